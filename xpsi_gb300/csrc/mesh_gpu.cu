@@ -14,17 +14,17 @@
 //   3. one thread per cell: the corner / centre membership tests; cells
 //      wholly inside or outside get their area at once, cells cut by a
 //      region boundary (~1 %) are queued;
-//   4. one group of 16 lanes per queued cell, taken from a shared counter:
-//      its area quadrature, group-cooperative (the 21 or 42 Gauss-Kronrod
-//      nodes of a step over the lanes, the rule's sums reduced lane-parallel,
-//      the interval list in shared memory) -- the same adaptive scheme the
-//      host builder runs serially.
+//   4. one CTA of two warps per queued cell, taken from a shared counter: its
+//      area quadrature, a panel to each warp (21 Gauss-Kronrod nodes over the
+//      lanes, the interval list in shared memory) -- the same adaptive scheme
+//      the host builder runs serially.
 // The per-thread quadratures of steps 1-2 keep their interval list (128
 // intervals) in local memory; the host builder's limit of 4000 gives bitwise
 // the same meshes (these integrals converge in far fewer intervals).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "../../include/xpsi_gb300.h"
@@ -107,166 +107,213 @@ __global__ void __launch_bounds__(128) mesh_rows_kernel(const MeshJob *jobs, con
 }
 
 // ---------------------------------------------------------------------------
-// Group-cooperative form of the quadrature of mesh_math.h (qag21, dyadic,
-// integrate): a group of kGrp = 16 lanes (half a warp) integrates one cell.
-// Lane l of the group evaluates nodes l, l + 16 and l + 32 of the step's one
-// or two 21-point panels, so the 42 nodes of a bisection step take three
-// passes (88 % of the lane slots; one cell per warp took two passes of 32,
-// 66 %).  Sums are xor-butterfly reductions within the group, identical in
-// each of its lanes, so the control flow is group-uniform; the two groups of
-// a warp run independently (group masks on every shuffle and sync).
+// The quadrature of mesh_math.h (qag21, dyadic, integrate) by a CTA of two
+// warps: a bisection step's two 21-point panels go one to each warp, a node
+// to a lane, and the first warp finishes both (the rule's error formula of
+// the two panels side by side on its even and odd lanes), keeps the list and
+// picks the next interval while the second waits.  The bound is the FP64
+// pipe: a warp's FP64 instruction takes it 64 cycles (76 with all four
+// partitions busy) however many lanes it has, so what counts is FP64
+// instructions per warp; and a cell's bisections are a serial chain (10-50
+// steps, up to the list's 128 where an arc ends inside the cell), which is
+// what a small batch waits for.  The sums pack two of the rule's four sums
+// into a warp's two halves.  Every thread takes the same branches.  Measured
+// against 16 lanes of a warp per cell: one blackbody spot (148 cut cells)
+// 2.07 -> 0.38 ms, 100 of them 6.4 -> 6.2 ms (345 FP64 instructions per cell
+// and step, the pipe 84 % busy).
 // ---------------------------------------------------------------------------
-constexpr int kGrp = 16;
-constexpr int kWarpList = 128;
-struct WarpList {
-  double al[kWarpList], bl[kWarpList], rl[kWarpList], el[kWarpList];
-};
-struct Grp {
-  int l;          // lane within the group
-  unsigned mask;  // the group's lanes
+constexpr int kCutThreads = 64;
+constexpr int kCutList = 128;
+struct CutList {
+  double al[kCutList], bl[kCutList], rl[kCutList], el[kCutList];
+  double panel[2][4];  // Kronrod, Gauss, |f| and |f - mean| sums of the step's panels
+  double next[2], out;  // the next interval; the integral
+  int go;               // another step follows
 };
 
-__device__ __forceinline__ double gsum(const Grp &g, double v) {
+__device__ __forceinline__ int k21_slot(int n) { return n < 10 ? n : (n == 10 ? 10 : n - 11); }
+
+// one panel by the calling warp, the four sums into `out`.  Lanes 0-15 carry
+// a node each and lanes 16-20 the other five, which fold onto five of the
+// first 16.  The pairing and the order of the sums are those of 16 lanes
+// taking the 42 nodes of a step in turn (first panel: nodes l and l + 16;
+// second: nodes l - 5 and l + 11), the order in which the meshes were always
+// summed.
+template <typename F>
+__device__ __forceinline__ void warp_panel(const F &f, bool second, double a, double b,
+                                           double *out) {
+  const int lane = threadIdx.x & 31;
+  const double c = 0.5 * (a + b), h = 0.5 * (b - a);
+  double v = 0.0;
+  if (lane < 21) {
+    const int m = lane >= 16 ? lane : (second ? (lane < 5 ? lane + 11 : lane - 5) : lane);
+    const double x = m == 10 ? 0.0 : XG_K21_X[k21_slot(m)];
+    // c - h x, c, c + h x
+    v = f(fma(h, m < 10 ? -x : x, c));
+  }
+  // the first half of the warp sums with the Kronrod weights, the second
+  // with the Gauss weights; then the first |f - mean|, the second |f|
+  const int fold = second ? 5 : 0, lo = lane & 15;
+  const int m1 = second ? (lo < 5 ? lo + 11 : lo - 5) : lo;
+  const bool two = lo >= fold && lo < fold + 5;
+  const int m2 = lo - fold + 16;
+  const double v1 = __shfl_sync(0xffffffffu, v, lo);
+  const double v2 = __shfl_sync(0xffffffffu, v, two ? m2 : lo);
+  const double wk1 = XG_K21_WK[k21_slot(m1)], wk2 = two ? XG_K21_WK[k21_slot(m2)] : 0.0;
+  double w1 = wk1, w2 = wk2;
+  if (lane >= 16) {
+    w1 = XG_K21_WG[k21_slot(m1)];
+    w2 = two ? XG_K21_WG[k21_slot(m2)] : 0.0;
+  }
+  double s = fma(w2, v2, w1 * v1);
 #pragma unroll
-  for (int o = kGrp / 2; o > 0; o >>= 1) v += __shfl_xor_sync(g.mask, v, o);
-  return v;
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  const double mean = lane < 16 ? 0.5 * s : 0.0;
+  double t = fma(wk2, fabs(v2 - mean), wk1 * fabs(v1 - mean));
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lo == 0) {
+    out[lane >> 4] = s;
+    out[2 + (lane >> 4)] = t;
+  }
 }
 
 struct WPanel {
   double res, err, rabs, rasc;
 };
-
-__device__ __forceinline__ int k21_slot(int n) { return n < 10 ? n : (n == 10 ? 10 : n - 11); }
-__device__ __forceinline__ double k21_node(double a, double b, int n) {
-  const double c = 0.5 * (a + b), h = 0.5 * (b - a);
-  if (n < 10) return c - h * XG_K21_X[n];
-  if (n == 10) return c;
-  return c + h * XG_K21_X[n - 11];
+__device__ __forceinline__ bool below(double a, double b) {
+  return ordered_bits(a) < ordered_bits(b);
 }
-__device__ __forceinline__ WPanel k21_finish(double rk, double rg, double ra, double rc,
-                                             double a, double b) {
+// result and error estimate of a panel from its sums (QUADPACK's formulas;
+// the tests on non-negative finite values by their bit patterns)
+__device__ __forceinline__ WPanel k21_finish(const double *p, double a, double b) {
   const double h = 0.5 * (b - a), ah = fabs(h);
+  const double rk = p[0], rg = p[1];
   WPanel P;
   P.res = rk * h;
-  ra *= ah;
-  rc *= ah;
+  const double rc = p[2] * ah, ra = p[3] * ah;
   double e = fabs((rk - rg) * h);
-  if (rc != 0.0 && e != 0.0) {
+  if (ordered_bits(rc) != 0 && ordered_bits(e) != 0) {
     const double x = 200.0 * e / rc, sc = x * sqrt(x);  // x^1.5 without pow
-    e = sc < 1.0 ? rc * sc : rc;
+    e = below(sc, 1.0) ? rc * sc : rc;
   }
   const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
-  if (ra > dmin / (50.0 * eps)) e = (e < 50.0 * eps * ra) ? 50.0 * eps * ra : e;
+  if (below(dmin / (50.0 * eps), ra)) {
+    const double fl = 50.0 * eps * ra;
+    if (below(e, fl)) e = fl;
+  }
   P.err = e;
   P.rabs = ra;
   P.rasc = rc;
   return P;
 }
 
-template <typename F>
-__device__ void grp_k21(const F &f, const Grp &g, double a1, double b1, double a2, double b2,
-                        bool two, WPanel &P1, WPanel &P2) {
-  const int total = two ? 42 : 21;
-  double fv[3];
-  double rk1 = 0.0, rg1 = 0.0, ra1 = 0.0, rk2 = 0.0, rg2 = 0.0, ra2 = 0.0;
-#pragma unroll
-  for (int p = 0; p < 3; p++) {
-    const int n = g.l + p * kGrp;
-    fv[p] = 0.0;
-    if (n < total) {
-      const bool first = n < 21;
-      const int m = first ? n : n - 21;
-      const double v = f(first ? k21_node(a1, b1, m) : k21_node(a2, b2, m));
-      fv[p] = v;
-      const int s = k21_slot(m);
-      const double wk = XG_K21_WK[s], wg = XG_K21_WG[s];
-      if (first) { rk1 += wk * v; rg1 += wg * v; ra1 += wk * fabs(v); }
-      else { rk2 += wk * v; rg2 += wg * v; ra2 += wk * fabs(v); }
-    }
+// the first interval of largest error, compared as signed 64-bit patterns
+// (the errors are non-negative): identical in every lane
+__device__ __forceinline__ int worst_interval(const double *el, int size, int lane) {
+  long long e = LLONG_MIN;
+  int k = 0;
+  for (int i = lane; i < size; i += 32) {
+    const long long v = __double_as_longlong(el[i]);
+    if (v > e) { e = v; k = i; }
   }
-  rk1 = gsum(g, rk1); rg1 = gsum(g, rg1); ra1 = gsum(g, ra1);
-  if (two) { rk2 = gsum(g, rk2); rg2 = gsum(g, rg2); ra2 = gsum(g, ra2); }
-  const double mean1 = 0.5 * rk1, mean2 = 0.5 * rk2;
-  double rc1 = 0.0, rc2 = 0.0;
-#pragma unroll
-  for (int p = 0; p < 3; p++) {
-    const int n = g.l + p * kGrp;
-    if (n < total) {
-      if (n < 21) rc1 += XG_K21_WK[k21_slot(n)] * fabs(fv[p] - mean1);
-      else rc2 += XG_K21_WK[k21_slot(n - 21)] * fabs(fv[p] - mean2);
-    }
-  }
-  P1 = k21_finish(rk1, rg1, ra1, gsum(g, rc1), a1, b1);
-  if (two) P2 = k21_finish(rk2, rg2, ra2, gsum(g, rc2), a2, b2);
+  const int hi = (int)(e >> 32);
+  const int mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)e : 0u;
+  const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
+  return (int)__reduce_min_sync(0xffffffffu,
+                                (hi == mh && (unsigned)e == ml) ? (unsigned)k : 0x7fffffffu);
 }
 
 template <typename F>
-__device__ double grp_qag21(const F &f, double a, double b, double epsabs, double er,
-                            WarpList &L, const Grp &g) {
+__device__ double cta_qag21(const F &f, double a, double b, double epsabs, double er,
+                            CutList &L) {
   const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
-  WPanel P0, Pu;
-  grp_k21(f, g, a, b, 0.0, 0.0, false, P0, Pu);
-  const double r0 = P0.res, e0 = P0.err;
-  double tol = (epsabs < er * fabs(r0)) ? er * fabs(r0) : epsabs;
-  if ((e0 <= 50.0 * eps * P0.rabs && e0 > tol) || (e0 <= tol && e0 != P0.rasc) || e0 == 0.0)
-    return r0;
-  __syncwarp(g.mask);
-  if (g.l == 0) { L.al[0] = a; L.bl[0] = b; L.rl[0] = r0; L.el[0] = e0; }
-  __syncwarp(g.mask);
-  int size = 1, iter = 1, k = 0, rnd1 = 0, rnd2 = 0, fail = 0;
-  double area = r0, errsum = e0;
-  do {
-    const double ai = L.al[k], bi = L.bl[k], ri = L.rl[k], ei = L.el[k];
-    const double a1 = ai, b1 = 0.5 * (ai + bi), a2 = b1, b2 = bi;
-    WPanel P1, P2;
-    grp_k21(f, g, a1, b1, a2, b2, true, P1, P2);
-    const double r1 = P1.res, e1 = P1.err, r2 = P2.res, e2 = P2.err;
-    const double r12 = r1 + r2, e12 = e1 + e2;
-    errsum += e12 - ei;
-    area += r12 - ri;
-    if (P1.rasc != e1 && P2.rasc != e2) {
-      if (fabs(ri - r12) <= 1.0e-5 * fabs(r12) && e12 >= 0.99 * ei) rnd1++;
-      if (iter >= 10 && e12 > ei) rnd2++;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // the first panel
+  if (w == 0) {
+    warp_panel(f, false, a, b, L.panel[0]);
+    __syncwarp();
+    const WPanel P = k21_finish(L.panel[0], a, b);
+    const double r0 = P.res, e0 = P.err;
+    const double tol = (epsabs < er * fabs(r0)) ? er * fabs(r0) : epsabs;
+    const bool done = (e0 <= 50.0 * eps * P.rabs && e0 > tol) || (e0 <= tol && e0 != P.rasc) ||
+                      e0 == 0.0;
+    if (lane == 0) {
+      L.al[0] = a; L.bl[0] = b; L.rl[0] = r0; L.el[0] = e0;
+      L.next[0] = a; L.next[1] = b;
+      L.out = r0;
+      L.go = !done;
     }
-    tol = (epsabs < er * fabs(area)) ? er * fabs(area) : epsabs;
-    if (errsum > tol) {
-      if (rnd1 >= 6 || rnd2 >= 20) fail = 2;
-      const double edge = (1.0 + 100.0 * eps) * (fabs(a2) + 1000.0 * dmin);
-      if (fabs(a1) <= edge && fabs(b2) <= edge) fail = 3;
-    }
-    const int nw = size++;
-    __syncwarp(g.mask);
-    if (g.l == 0) {
-      if (e2 > e1) {
-        L.al[k] = a2; L.bl[k] = b2; L.rl[k] = r2; L.el[k] = e2;
-        L.al[nw] = a1; L.bl[nw] = b1; L.rl[nw] = r1; L.el[nw] = e1;
+  }
+  __syncthreads();
+  double area = L.rl[0], errsum = L.el[0];
+  int size = 1, iter = 1, k = 0, rnd1 = 0, rnd2 = 0;
+  while (L.go) {
+    const double ai = L.next[0], bi = L.next[1];
+    const double mid = 0.5 * (ai + bi);
+    warp_panel(f, w == 1, w ? mid : ai, w ? bi : mid, L.panel[w]);
+    __syncthreads();
+    if (w == 0) {
+      const double ri = L.rl[k], ei = L.el[k];
+      // even lanes finish the first panel, odd lanes the second
+      const bool odd = lane & 1;
+      const WPanel P = k21_finish(L.panel[odd], odd ? mid : ai, odd ? bi : mid);
+      const double r1 = __shfl_sync(0xffffffffu, P.res, 0), r2 = __shfl_sync(0xffffffffu, P.res, 1);
+      const double e1 = __shfl_sync(0xffffffffu, P.err, 0), e2 = __shfl_sync(0xffffffffu, P.err, 1);
+      const bool flat = __any_sync(0xffffffffu, ordered_bits(P.rasc) == ordered_bits(P.err));
+      const double r12 = r1 + r2, e12 = e1 + e2;
+      errsum += e12 - ei;
+      area += r12 - ri;
+      if (!flat) {
+        if (!below(1.0e-5 * fabs(r12), fabs(ri - r12)) && !below(e12, 0.99 * ei)) rnd1++;
+        if (iter >= 10 && below(ei, e12)) rnd2++;
+      }
+      const double rt = er * fabs(area);
+      const double tol = below(epsabs, rt) ? rt : epsabs;
+      const bool above = below(tol, errsum);
+      int fail = 0;
+      if (above) {
+        if (rnd1 >= 6 || rnd2 >= 20) fail = 2;
+        const double edge = (1.0 + 100.0 * eps) * (fabs(mid) + 1000.0 * dmin);
+        if (!below(edge, fabs(ai)) && !below(edge, fabs(bi))) fail = 3;
+      }
+      const int nw = size++;
+      const bool swap = below(e1, e2);  // the half of larger error stays in place
+      if (lane == 0) {
+        L.al[k] = swap ? mid : ai; L.bl[k] = swap ? bi : mid;
+        L.rl[k] = swap ? r2 : r1; L.el[k] = swap ? e2 : e1;
+        L.al[nw] = swap ? ai : mid; L.bl[nw] = swap ? mid : bi;
+        L.rl[nw] = swap ? r1 : r2; L.el[nw] = swap ? e1 : e2;
+      }
+      __syncwarp();
+      iter++;
+      const bool go = iter < kCutList && !fail && above;
+      if (go) {
+        k = worst_interval(L.el, size, lane);
+        if (lane == 0) {
+          L.next[0] = L.al[k];
+          L.next[1] = L.bl[k];
+        }
       } else {
-        L.al[k] = a1; L.bl[k] = b1; L.rl[k] = r1; L.el[k] = e1;
-        L.al[nw] = a2; L.bl[nw] = b2; L.rl[nw] = r2; L.el[nw] = e2;
+        double sum = 0.0;
+        for (int i = 0; i < size; i++) sum += L.rl[i];
+        if (lane == 0) {
+          L.out = sum;
+          L.go = 0;
+        }
       }
     }
-    __syncwarp(g.mask);
-    // the interval of largest error, compared by bit pattern: the errors are
-    // non-negative, so their patterns order as 64-bit integers like the
-    // values (the integer pipe instead of FP64 compares; the first of equal
-    // errors wins, as before)
-    k = 0;
-    long long ek = __double_as_longlong(L.el[0]);
-    for (int i = 1; i < size; i++) {
-      const long long e = __double_as_longlong(L.el[i]);
-      if (e > ek) { ek = e; k = i; }
-    }
-    iter++;
-  } while (iter < kWarpList && !fail && errsum > tol);
-  double sum = 0.0;
-  for (int i = 0; i < size; i++) sum += L.rl[i];
-  __syncwarp(g.mask);
-  return sum;
+    __syncthreads();
+  }
+  const double r = L.out;
+  __syncthreads();  // the next integral's first panel rewrites the list
+  return r;
 }
 
 template <typename F>
-__device__ double grp_dyadic(const F &f, double lo, double hi, bool toward_lo, double er,
-                             WarpList &L, const Grp &g) {
+__device__ double cta_dyadic(const F &f, double lo, double hi, bool toward_lo, double er,
+                             CutList &L) {
   const double Lw = hi - lo;
   double sum = 0.0;
   int seen = 0, quiet = 0;
@@ -275,7 +322,7 @@ __device__ double grp_dyadic(const F &f, double lo, double hi, bool toward_lo, d
     const double p0 = toward_lo ? lo + s1 : hi - s0;
     const double p1 = toward_lo ? lo + s0 : hi - s1;
     if (!(p0 < p1) || (toward_lo ? p0 <= lo : p1 >= hi)) break;
-    const double r = grp_qag21(f, p0, p1, 0.0, er, L, g);
+    const double r = cta_qag21(f, p0, p1, 0.0, er, L);
     sum += r;
     if (r != 0.0) seen = 1;
     if (seen && fabs(r) <= 1.0e-17 * fabs(sum)) {
@@ -288,22 +335,22 @@ __device__ double grp_dyadic(const F &f, double lo, double hi, bool toward_lo, d
 }
 
 template <typename F>
-__device__ double grp_integrate(const F &f, double a, double b, double epsabs, double epsrel,
-                                WarpList &L, const Grp &g) {
+__device__ double cta_integrate(const F &f, double a, double b, double epsabs, double epsrel,
+                                CutList &L) {
   double sign = 1.0;
   if (b < a) { const double t = a; a = b; b = t; sign = -1.0; }
   if (a == b) return 0.0;
   double er = (1.0e-13 < epsrel) ? 1.0e-13 : epsrel;
   if (epsabs <= 0.0 && er < 50.0 * 2.220446049250313e-16) er = 50.0 * 2.220446049250313e-16;
-  double r = grp_qag21(f, a, b, epsabs, er, L, g);
+  double r = cta_qag21(f, a, b, epsabs, er, L);
   if (r == 0.0) {
     const double fa = f(a), fb = f(b);
     if (fa != 0.0 || fb != 0.0) {
       const double m = 0.5 * (a + b);
-      const double rl = fa != 0.0 ? grp_dyadic(f, a, m, true, er, L, g)
-                                  : grp_qag21(f, a, m, 0.0, er, L, g);
-      const double rr = fb != 0.0 ? grp_dyadic(f, m, b, false, er, L, g)
-                                  : grp_qag21(f, m, b, 0.0, er, L, g);
+      const double rl = fa != 0.0 ? cta_dyadic(f, a, m, true, er, L)
+                                  : cta_qag21(f, a, m, 0.0, er, L);
+      const double rr = fb != 0.0 ? cta_dyadic(f, m, b, false, er, L)
+                                  : cta_qag21(f, m, b, 0.0, er, L);
       r = rl + rr;
     }
   }
@@ -366,26 +413,19 @@ __global__ void __launch_bounds__(128) mesh_cells_kernel(const MeshJob *jobs, in
   }
 }
 
-// one group of 16 lanes per queued cell: the area quadrature of a cell cut
-// by a boundary.  The groups take the next queued cell from a shared counter
-// (n_queue[1]) when they finish one, as the cells' costs differ by 5x or
-// more (10-50 bisection steps); each cell's result is independent of which
-// group integrates it.
-constexpr int kBoundaryWarps = 4;
-__global__ void __launch_bounds__(32 * kBoundaryWarps, 4) mesh_boundary_kernel(
+// one CTA per queued cell: the area quadrature of a cell cut by a boundary.
+// A CTA starts with the cell of its own index (a small batch's cells spread
+// over the SMs) and takes the next from a shared counter (n_queue[1]) when it
+// finishes one, as the cells' costs differ by 5x or more (10-50 bisection
+// steps); each cell's result is independent of which CTA integrates it.
+constexpr int kCutCtasPerSm = 8;
+__global__ void __launch_bounds__(kCutThreads, kCutCtasPerSm) mesh_boundary_kernel(
     const MeshJob *jobs, int n_mesh, xgpu_mesh_batch_out o, const double *row_tmp,
     const int64_t *queue, unsigned *n_queue) {
-  __shared__ WarpList lists[2 * kBoundaryWarps];
-  const int lane = threadIdx.x & 31, half = lane / kGrp;
-  const int grp = (threadIdx.x >> 5) * 2 + half;
-  const Grp gp{lane - half * kGrp, 0xFFFFu << (kGrp * half)};
-  WarpList &L = lists[grp];
+  __shared__ CutList L;
+  __shared__ unsigned s_q;
   const unsigned n = n_queue[0];
-  for (;;) {
-    unsigned q = 0;
-    if (gp.l == 0) q = atomicAdd(&n_queue[1], 1u);
-    q = __shfl_sync(gp.mask, q, half * kGrp);
-    if (q >= n) break;
+  for (unsigned q = blockIdx.x; q < n; q = s_q) {
     const int64_t c = queue[q];
     const int m = mesh_of_cell(jobs, n_mesh, c);
     const MeshJob &J = jobs[m];
@@ -397,15 +437,20 @@ __global__ void __launch_bounds__(32 * kBoundaryWarps, 4) mesh_boundary_kernel(
     double pa, pb;
     mesh_cell_kind(J.pl, i, j, lower, upper, row_tmp[4 * row + 2], pa, pb);
     const Region g = mesh_region(J.pl);
-    const CellIntegrand f{J.s, g, pa, pb};
-    double integral = grp_integrate(f, lower, upper, 0.0, 1.0e-8, L, gp);
+    CutCell f;
+    f.init(CellIntegrand{J.s, g, pa, pb}, lower, upper);
+    double integral = cta_integrate(f, lower, upper, 0.0, 1.0e-8, L);
     if (are_equal(integral, 0.0)) {
       double tmin, tmax;
       if (cell_fallback_interval(lower, upper, pa, pb, g, tmin, tmax))
-        integral = grp_integrate(f, tmin, tmax, 0.0, 1.0e-8, L, gp);
+        integral = cta_integrate(f, tmin, tmax, 0.0, 1.0e-8, L);
     }
-    if (gp.l == 0) put_area(J, o, c, i, j, J.s.R_eq * J.s.R_eq * integral);
-    __syncwarp(gp.mask);
+    __syncthreads();  // every thread has read the last s_q
+    if (threadIdx.x == 0) {
+      put_area(J, o, c, i, j, J.s.R_eq * J.s.R_eq * integral);
+      s_q = gridDim.x + atomicAdd(&n_queue[1], 1u);
+    }
+    __syncthreads();
   }
 }
 
@@ -464,8 +509,8 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
   mesh_rows_kernel<<<(unsigned)n, 128, smem, st>>>(d_jobs, tab, *out, row_tmp, mesh_tmp);
   mesh_cells_kernel<<<(unsigned)((n_cells + 127) / 128), 128, 0, st>>>(
       d_jobs, n, n_cells, *out, row_tmp, mesh_tmp, queue, n_queue);
-  mesh_boundary_kernel<<<152 * 8, 32 * kBoundaryWarps, 0, st>>>(d_jobs, n, *out, row_tmp, queue,
-                                                                 n_queue);
+  mesh_boundary_kernel<<<152 * kCutCtasPerSm, kCutThreads, 0, st>>>(d_jobs, n, *out, row_tmp,
+                                                                     queue, n_queue);
   const cudaError_t e = cudaGetLastError();
   cudaFreeAsync(d_jobs, st);
   cudaFreeAsync(tab, st);

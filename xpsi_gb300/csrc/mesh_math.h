@@ -15,6 +15,7 @@
 #pragma once
 #include <math.h>
 #include <stddef.h>
+#include <string.h>
 
 #include "gk_nodes.h"
 
@@ -418,6 +419,157 @@ struct CellIntegrand {
     const double radius = radiusNormalised(mu, s.epsilon, s.zeta, s.shape);
     const double ft2 = f_theta_sq(mu, st, radius, s.epsilon, s.zeta, s.shape);
     return dphi * radius * radius * sqrt(1.0 + ft2) * st;
+  }
+};
+
+// ---------------------------------------------------------------------------
+// The integrand of a cut cell (CellIntegrand, the same bits)
+// without the inverse cosines and divisions whose values cannot matter.  A
+// region boundary's azimuth at colatitude theta enters the cell's share of
+// the ring only where it falls inside the cell's azimuths [pa, pb]; whether
+// it does is decided on its cosine, as a product comparison against the
+// cosines of the cell's nearest and farthest azimuths (1e-12 of slack, 1e4
+// times the rounding of either side; what lies within the slack, or near the
+// ends of the cosine's range, takes the full form).  Of a bisection's nodes
+// most see at most one of the two boundaries inside the cell.
+// On the GPU every FP64 instruction of a warp, comparisons included, takes the
+// FP64 pipe 64 cycles or more, so tests go through the sign of a fused
+// product or the bit patterns (integer pipe).
+// ---------------------------------------------------------------------------
+// a < b and a <= b of finite doubles by their bit patterns (-0 equals 0)
+XG_HD inline long long ordered_bits(double v) {
+#ifdef __CUDA_ARCH__
+  const long long b = __double_as_longlong(v);
+#else
+  long long b;
+  memcpy(&b, &v, sizeof(b));
+#endif
+  return b < 0 ? -(b & 0x7fffffffffffffffLL) : b;
+}
+XG_HD inline bool negative(double v) { return ordered_bits(v) < 0; }
+
+// get_interval for finite ends, on the bit patterns
+XG_HD inline double get_interval_bits(double a, double b, double LB, double UB) {
+  const long long ia = ordered_bits(a), ib = ordered_bits(b);
+  const long long il = ordered_bits(LB), iu = ordered_bits(UB);
+  int ac = (il <= ia && ia <= iu), bc = (il <= ib && ib <= iu);
+  if (ac == 0) ac = 2 * (int)(ia > iu);
+  if (bc == 0) bc = 2 * (int)(ib > iu);
+  // one subtraction, its operands chosen without branches
+  const bool up_b = (ac == bc && ac == 1) || (bc == 1 && ac == 0);
+  const bool up_U = bc == 2 && ac != 2;
+  if (!up_b && !up_U) return 0.0;
+  return (up_b ? b : UB) - (ac == 1 ? a : LB);
+}
+
+struct CutCell {
+  CellIntegrand f;
+  // cosines of the smallest and largest azimuthal distance between the cell
+  // and the ceding region's meridian (azimuth 0) and the superseding one's,
+  // moved outward by the slack
+  double c_near, c_far, s_near, s_far;
+  // the colatitudes integrated over never reach the pole (no theta counts as
+  // 0), never come near the superseding region
+  bool off_pole, no_super;
+  XG_HD void init(const CellIntegrand &fi, double lower, double upper) {
+    constexpr double kSlack = 1.0e-12;
+    f = fi;
+    const double pa = f.pa, pb = f.pb;
+    c_near = ((pa <= 0.0 && 0.0 <= pb) ? 1.0 : cos(fmin(fabs(pa), fabs(pb)))) + kSlack;
+    c_far = cos(fmin(PI, fmax(fabs(pa), fabs(pb)))) - kSlack;
+    double qa = pa - f.g.superAzi, qb = pb - f.g.superAzi;
+    if (0.5 * (qa + qb) > PI) { qa -= TWO_PI; qb -= TWO_PI; }
+    if (0.5 * (qa + qb) < -PI) { qa += TWO_PI; qb += TWO_PI; }
+    s_near = ((qa <= 0.0 && 0.0 <= qb) ? 1.0 : cos(fmin(fabs(qa), fabs(qb)))) + kSlack;
+    s_far = cos(fmin(PI, fmax(fabs(qa), fabs(qb)))) - kSlack;
+    // a cell that reaches past the far meridian, or a superseding azimuth
+    // outside [-pi, pi] (its arc's ends are wrapped once only): no fast
+    // classification (nothing passes these tests)
+    if (fmax(fabs(pa), fabs(pb)) > PI) { c_near = 4.0; c_far = -4.0; }
+    if (fabs(f.g.superAzi) > PI || fmax(fabs(qa), fabs(qb)) > PI) { s_near = 4.0; s_far = -4.0; }
+    off_pole = fmin(lower, upper) > 1.0e-6;
+    const double lo = fmin(lower, upper) - 1.0e-9, hi = fmax(lower, upper) + 1.0e-9;
+    no_super = lo > f.g.superColat + f.g.superRadius || hi < f.g.superColat - f.g.superRadius;
+  }
+  // 0: the boundary's azimuth may fall inside the cell; 1: it lies beyond
+  // the cell (the cell is inside the region's arc); 2: the cell is outside
+  XG_HD static int side(double num, double den, double c_near, double c_far) {
+    constexpr double kEnd = 1.0 - 1.0e-9;
+    // den > 1e-9, |num| < kEnd den
+    if (!negative(1.0e-9 - den)) return 0;
+    if (!negative(fma(-kEnd, den, num)) || !negative(fma(-kEnd, den, -num))) return 0;
+    if (negative(fma(-c_far, den, num))) return 1;
+    if (negative(fma(c_near, den, -num))) return 2;
+    return 0;
+  }
+  XG_HD double operator()(double theta) const {
+    if (!off_pole && are_equal(theta, 0.0)) return 0.0;
+    double mu, st;
+#ifdef __CUDA_ARCH__
+    sincos(theta, &st, &mu);
+#else
+    mu = cos(theta);
+    st = sin(theta);
+#endif
+    const Region &g = f.g;
+    const int cede = side(g.cos_cede - g.cos_colat * mu, g.sin_colat * st, c_near, c_far);
+    if (cede == 2) return 0.0;
+    double dphi;
+    const bool far = no_super || negative(g.superRadius - fabs(theta - g.superColat));
+    const int sup = far ? 2 : side(g.cos_sr - g.cos_sc * mu, g.sin_sc * st, s_near, s_far);
+    if (sup == 1) return 0.0;
+    if (cede == 1 && sup == 2) {
+      dphi = f.pb - f.pa;
+    } else {
+      bool zero;
+      dphi = extent(theta, mu, st, cede == 1, far, sup == 2, zero);
+      if (zero || ordered_bits(dphi) == 0) return 0.0;
+    }
+    const Star &s = f.s;
+    const double radius = radiusNormalised(mu, s.epsilon, s.zeta, s.shape);
+    const double ft2 = f_theta_sq(mu, st, radius, s.epsilon, s.zeta, s.shape);
+    return dphi * radius * radius * sqrt(1.0 + ft2) * st;
+  }
+  // ring_extent with the ceding arc known to hold the whole cell (cede_in:
+  // any arc beyond the cell gives the same bits, so the full circle stands
+  // in), the superseding arc absent at this colatitude (far) or known to
+  // miss the cell (sup_out)
+  XG_HD double extent(double theta, double mu, double st, bool cede_in, bool far, bool sup_out,
+                      bool &zero) const {
+    const Region &g = f.g;
+    zero = false;
+    if (sup_out) {
+      const double aUB = eval_phi_cs(mu, st, g.cos_colat, g.sin_colat, g.cos_cede);
+      if (negative(aUB)) {
+        zero = !(theta + g.colat < g.cedeRadius);
+        if (zero) return 0.0;
+        return far ? get_interval_bits(f.pa, f.pb, -PI, 0.0) +
+                         get_interval_bits(f.pa, f.pb, 0.0, PI)
+                   : get_interval_bits(f.pa, f.pb, -PI, PI);
+      }
+      if (far && ordered_bits(aUB) > 0)
+        // the absent arc is the empty one at azimuth 0
+        return get_interval_bits(f.pa, f.pb, -aUB, 0.0) +
+               get_interval_bits(f.pa, f.pb, 0.0, aUB);
+      return get_interval_bits(f.pa, f.pb, -aUB, aUB);
+    }
+    if (cede_in) {
+      // the superseding arc cuts the cell (or may)
+      double cUB = eval_phi_cs(mu, st, g.cos_sc, g.sin_sc, g.cos_sr);
+      if (negative(cUB)) {
+        zero = true;
+        return 0.0;
+      }
+      double cLB = -cUB;
+      cUB += g.superAzi;
+      cLB += g.superAzi;
+      if (negative(PI - cUB)) cUB -= TWO_PI;
+      if (negative(cLB + PI)) cLB += TWO_PI;
+      if (ordered_bits(cUB) >= ordered_bits(cLB))
+        return get_interval_bits(f.pa, f.pb, -PI, cLB) + get_interval_bits(f.pa, f.pb, cUB, PI);
+      return get_interval_bits(f.pa, f.pb, cUB, cLB);
+    }
+    return ring_extent(theta, mu, st, g, true, f.pa, f.pb, zero);
   }
 };
 
