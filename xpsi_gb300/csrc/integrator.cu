@@ -13,8 +13,8 @@
 //      profile column, which leaf's radiation it carries (or zero);
 //   3. per chunk of energies: the specific intensities of every column
 //      (:445-478) -> Akima-periodic piece coefficients in shared memory
-//      (:566-569) -> every (phase, cell) thread-task evaluates the piece once
-//      per energy and accumulates A_ij * max(S, 0) (:571-598) in registers;
+//      (:566-569) -> the sums of A_ij max(S, 0) over cells x phases
+//      (:571-598), from power sums over runs of cells in one knot interval;
 //   4. per-chunk partial sums are reduced in a fixed order and divided by
 //      E keV (:605-612), so results are bitwise reproducible run to run.
 //
@@ -608,9 +608,20 @@ struct Layout {
   size_t bytes;
 };
 
+// the coefficients' area: rows (PieceRows) has one energy slot more per knot
+// and also holds the staged deflection table while an image's leaf geometry
+// runs (the pieces are formed after it), so that two CTAs fit an SM
+__host__ __device__ inline size_t coef_bytes(int ec, int N_L, int piece_bytes, int N_R,
+                                             bool rows) {
+  const size_t c = (size_t)(ec + (rows ? 1 : 0)) * N_L * piece_bytes;
+  const size_t d = ((size_t)N_R * sizeof(double) + 15) & ~size_t(15);
+  return rows && d > c ? d : c;
+}
+
 // nmu, nE: Num4D grid sizes (0 when no mesh uses the numerical atmosphere)
 __host__ __device__ inline Layout make_layout(int N_L, int N_P, int N_E, int nmu = 0,
-                                              int nE = 0, int piece_bytes = 32, int N_R = 0) {
+                                              int nE = 0, int piece_bytes = 32, int N_R = 0,
+                                              bool rows = false) {
   Layout L;
   L.N_L = N_L;
   L.nmu = nmu;
@@ -620,13 +631,13 @@ __host__ __device__ inline Layout make_layout(int N_L, int N_P, int N_E, int nmu
   while (ec > 8 && (size_t)ec * N_L * piece_bytes > 96 * 1024) ec /= 2;
   L.EC = ec;
   L.bytes = (size_t)5 * N_L * sizeof(double)      // phase, leafphase, Z, ABB, GEOM
-            + (size_t)ec * N_L * piece_bytes       // coefficients
+            + coef_bytes(ec, N_L, piece_bytes, N_R, rows)
             + (size_t)(nmu + nE) * 5 * sizeof(double)  // Num4D grids + inverse denominators
             + (size_t)(nmu + nE) * 5 * sizeof(float)   // their FP32 copies (mixed form)
             + (size_t)3 * nE * sizeof(float)           // energy-grid node offsets (mixed)
             + (size_t)nE * sizeof(int)                 // slab column exponents (FP64 form)
             + (size_t)(5 * N_L + 4 * kMaxCellsF + kMaxEnergiesF) * sizeof(float)
-            + (size_t)N_R * sizeof(double)  // staged deflection table
+            + (size_t)(rows ? 0 : N_R) * sizeof(double)  // staged deflection table
             + (size_t)(ec + N_L) * sizeof(double)  // lgE, lzs
             + (size_t)2 * N_L * sizeof(DF)         // ih, ih2
             + (size_t)(4 * N_L + 8 + ec) * sizeof(int) + 64;
@@ -641,10 +652,11 @@ inline size_t geometry_bytes(int N_L, int N_R) {
 }
 
 __device__ GeoSmem carve(char *base, int N_L, int EC, double **coef, int nmu = 0, int nE = 0,
-                         AtmSmem *atm = nullptr, int piece_bytes = 32, int N_R = 0) {
+                         AtmSmem *atm = nullptr, int piece_bytes = 32, int N_R = 0,
+                         bool rows = false) {
   GeoSmem g;
   double *d = reinterpret_cast<double *>(base);
-  g.rD = d; d += N_R;
+  g.rD = d; d += rows ? 0 : N_R;
   g.phase = d; d += N_L;
   g.leafphase = d; d += N_L;
   g.Z = d; d += N_L;
@@ -655,7 +667,9 @@ __device__ GeoSmem carve(char *base, int N_L, int EC, double **coef, int nmu = 0
   g.ih = reinterpret_cast<DF *>(d); d += N_L;
   g.ih2 = reinterpret_cast<DF *>(d); d += N_L;
   d = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(d) + 15) & ~uintptr_t(15));
-  *coef = d; d += (size_t)EC * N_L * piece_bytes / 8;
+  *coef = d;
+  if (rows) g.rD = d;
+  d += coef_bytes(EC, N_L, piece_bytes, N_R, rows) / 8;
   if (atm) {
     atm->gmu = d; d += nmu;
     atm->gE = d; d += nE;
@@ -766,16 +780,17 @@ constexpr int kWrapLimit = 1024;  // 2 pi shifts of a cell phase (a few suffice)
 // (:575-586), with phases as unevaluated float pairs (hi + lo) and error-free
 // sums, so the offset t keeps ~1e-14 rad absolute accuracy instead of one
 // FP32 ulp of the phase (~5e-7 rad)
+template <bool kCached>
 struct CellPhaseF {
   const float *knot, *knot_lo;
   int N_L;
   float x_lo, x_hi, ph, ph_lo, tp, tp_lo;
-  const float *cphi, *cphi_lo;  // cached pairs, or null
+  const float *cphi, *cphi_lo;  // the parallel's cell azimuths as pairs (kCached)
   const double *cphi_d;
   // interval and offset th + tl of cell j's phase
   __device__ __forceinline__ int offset(int j, int hint, float &th, float &tl) const {
     float cp, cp_lo;
-    if (cphi) {
+    if (kCached) {
       cp = cphi[j];
       cp_lo = cphi_lo[j];
     } else {
@@ -823,16 +838,20 @@ struct CellPhaseF {
   }
 };
 
+template <bool kCached>
 struct AreaF {
-  const float *Af;  // cached, or null
+  const float *Af;  // the parallel's cell areas (kCached)
   const double *A;
-  __device__ __forceinline__ float operator()(int j) const { return Af ? Af[j] : (float)A[j]; }
+  __device__ __forceinline__ float operator()(int j) const {
+    return kCached ? Af[j] : (float)A[j];
+  }
 };
+template <bool kCached>
 struct AreaDF {
-  const float *Ah, *Al;  // cached pairs, or null
+  const float *Ah, *Al;  // the parallel's cell areas as pairs (kCached)
   const double *A;
   __device__ __forceinline__ DF operator()(int j) const {
-    return Ah ? DF{Ah[j], Al[j]} : df_split(A[j]);
+    return kCached ? DF{Ah[j], Al[j]} : df_split(A[j]);
   }
 };
 
@@ -866,14 +885,45 @@ __device__ __forceinline__ bool cell_phase_sums(const CP &cp, const AR &area, in
   return true;
 }
 
+// ---------------------------------------------------------------------------
+// The FP64 form's Akima pieces of a chunk of energies in shared memory:
+// piece (iv, e) is two float4, (y, k1) and (k2, k3) as float pairs, at
+// iv * es + e of two arrays.  Energies are adjacent, so the lanes of a group
+// that take the energies of one knot interval read consecutive float4; the
+// row stride es = EC + 1 (odd) keeps accesses along iv (column intensities,
+// the per-cell form) off a single bank group.
+// ---------------------------------------------------------------------------
+struct PieceRows {
+  float4 *a, *b;
+  int es;
+  __device__ __forceinline__ PieceDF at(int iv, int e) const {
+    const float4 p = a[iv * es + e], q = b[iv * es + e];
+    return PieceDF{{p.x, p.y}, {p.z, p.w}, {q.x, q.y}, {q.z, q.w}};
+  }
+  __device__ __forceinline__ DF &y(int iv, int e) const {
+    return *reinterpret_cast<DF *>(&a[iv * es + e]);
+  }
+  __device__ __forceinline__ double &yd(int iv, int e) const {
+    return *reinterpret_cast<double *>(&a[iv * es + e]);
+  }
+  __device__ __forceinline__ int &ex(int iv, int e) const {
+    return reinterpret_cast<int *>(&a[iv * es + e])[2];
+  }
+  __device__ __forceinline__ void put_k(int iv, int e, DF k1, DF k2, DF k3) const {
+    float4 &p = a[iv * es + e];
+    p.z = k1.h;
+    p.w = k1.l;
+    b[iv * es + e] = make_float4(k2.h, k2.l, k3.h, k3.l);
+  }
+};
+
 // the FP64 path's form of cell_phase_sums, in double-float arithmetic on
 // scaled pieces (the sign test is on the high part: h + l has the sign of h;
 // with the elsewhere correction every value is added, :593-594)
 template <typename CP, typename AR>
 __device__ __forceinline__ bool cell_phase_sums_df(const CP &cp, const AR &area, int S1,
-                                                   const int32_t *rad, const PieceDF *pc, int N_L,
-                                                   int pb, int ne, bool add_all,
-                                                   DF (&acc)[kEPT]) {
+                                                   const int32_t *rad, const PieceRows &pc,
+                                                   int pb, bool add_all, DF (&acc)[kEPT]) {
   int hint = -1;
   for (int j = 0; j < S1; j++) {
     if (rad[j] != 1) continue;
@@ -888,7 +938,7 @@ __device__ __forceinline__ bool cell_phase_sums_df(const CP &cp, const AR &area,
     // kEPT independent double-float chains interleave
 #pragma unroll
     for (int e = 0; e < kEPT; e++) {
-      const PieceDF q = pc[(pb + e) * N_L + iv];
+      const PieceDF q = pc.at(iv, pb + e);
       const DF sv = df_fma(t, df_fma(t, df_fma(t, q.k3, q.k2), q.k1), q.y);
       const DF nx = df_fma(A, sv, acc[e]);
       const bool take = add_all || sv.h > 0.0f;
@@ -900,11 +950,11 @@ __device__ __forceinline__ bool cell_phase_sums_df(const CP &cp, const AR &area,
 }
 
 // ---------------------------------------------------------------------------
-// Power-sum form of the FP64 path's cell x phase sums.  At a signal phase k
-// the cells of a parallel fall, in azimuth order, into runs of consecutive
-// radiating cells whose wrapped phase lies in the same knot interval iv (a
-// run ends where the interval changes).  Over a run every energy row
-// evaluates the same cubic piece, so
+// Power-sum form of the FP64 path's cell x phase sums (the form that runs).
+// At a signal phase k the cells of a parallel fall, in azimuth order, into
+// runs of consecutive radiating cells whose wrapped phase lies in the same
+// knot interval iv (a run ends where the interval changes).  Over a run every
+// energy row evaluates the same cubic piece, so
 //     sum_j A_j S_E(t_j) = y W0 + k1 W1 + k2 W2 + k3 W3,  Wp = sum_j A_j t_j^p,
 // and the power sums Wp depend on the geometry only: they are formed once
 // per (parallel, image) and reused by all N_E energies.  This holds where
@@ -916,52 +966,84 @@ __device__ __forceinline__ bool cell_phase_sums_df(const CP &cp, const AR &area,
 // (the curve lies in their convex hull), with a margin of 1e-5 of the
 // piece's scale so that rounding cannot flip the classification.
 //
-// Run records live in global scratch, per chunk: for cell half c (the two
-// halves of the parallel's cells are walked by different threads) and run r
-// of phase k, record (c w_cap + r) N_P + k (consecutive phases adjacent, so a
-// warp's tasks load them coalesced): two float4 with the float pairs of
-// W0, W1 and W2, W3, and an int with the interval (bits 0-9), the first
-// cell (bits 10-19) and the cell span (bits 20-29).
+// What bounds the sums is FP32 issue: 41 instructions per run and energy
+// (four products of pairs into a running pair, below) where the
+// per-cell form spends 62 per cell and energy, and a parallel has about
+// three cells per run.  The lanes of a group of EC take the chunk's energies
+// of one signal phase: they share the run list, the knot interval and the
+// records, so nothing diverges and the pieces are read as consecutive
+// float4; with lanes over the phases (each its own runs and intervals) the
+// same sums ran no faster than the per-cell form.
+//
+// Run records live in global scratch (L2), per CTA: run r of cell half c (the
+// two halves of the parallel's cells are walked by different threads) of
+// phase k is record (2 k + c) w_cap + r: two float4 with the float pairs of
+// W0, W1 and W2, W3, and an int with the interval (bits 0-9), the first cell
+// (bits 10-19) and the cell span (bits 20-29).  A group stages kStage records
+// at a time in shared memory (one load per lane, a block ahead): read one by
+// one from L2 they cost 600 cycles a run against the 100 of its arithmetic.
 // ---------------------------------------------------------------------------
 __host__ __device__ inline size_t integrate_wsum_bytes_dev(int N_P, int cap) {
   const size_t n = (size_t)2 * cap * N_P;
   return (n * (2 * sizeof(float4) + sizeof(int)) + 255) & ~size_t(255);
 }
+constexpr int kStage = 8;
+struct RunStage {  // the last record is empty
+  float4 w[2 * kStage + 2];
+  uint4 meta[kStage + 1];  // interval and cells, class masks of the interval
+};
 
 struct WRuns {
-  float4 *wa, *wb;
+  float4 *w;
   int *meta;
-  int cap, N_P;
-  __device__ __forceinline__ size_t rec(int half, int r, int k) const {
-    return ((size_t)half * cap + r) * N_P + k;
+  int cap;
+  __device__ __forceinline__ size_t first(int k, int half) const {
+    return (size_t)(2 * k + half) * cap;
   }
 };
 
 __device__ __forceinline__ WRuns wruns_of(unsigned char *base, int cap, int N_P) {
   const size_t n = (size_t)2 * cap * N_P;
   WRuns w;
-  w.wa = reinterpret_cast<float4 *>(base);
-  w.wb = w.wa + n;
-  w.meta = reinterpret_cast<int *>(w.wb + n);
+  w.w = reinterpret_cast<float4 *>(base);
+  w.meta = reinterpret_cast<int *>(w.w + 2 * n);
   w.cap = cap;
-  w.N_P = N_P;
   return w;
 }
 
-// piece classes: 0 adds nothing, 1 power sums, 2 cell by cell
-__device__ __forceinline__ uint8_t piece_class(const PieceDF &q, float h) {
+// |y| + |k1| h + |k2| h^2 + |k3| h^3 up to which a piece takes the power sums
+// (a row's largest value is in [0.5, 1)): beyond it, at a knot interval much
+// wider than its neighbours, the four terms cancel
+constexpr float kPieceScale = 4.0f;
+// knot intervals shorter than this are walked cell by cell: a cell's offset
+// may leave [0, h] by the rounding of its phase there
+constexpr float kShortKnot = 1.0e-4f;
+
+// piece classes: 0 adds nothing, 1 power sums, 2 cell by cell; yn and tr are
+// the value and the tangent at the right knot.  The Bernstein coefficients
+// are the end values and the ends' tangent points y + k1 h / 3 and yn - tr h
+// / 3.  One that is zero because the knot is dark and its tangent flat (what
+// Akima's weights give next to a dark stretch, to rounding) bounds the curve
+// at zero to rounding, so it does not make the piece a sign-changing one: most
+// pieces at the edges of dark stretches are of that kind.
+__device__ __forceinline__ int piece_class(const PieceDF &q, float yn, float tr, float h,
+                                           bool add_all) {
   const float y = q.y.h, a1 = q.k1.h * h, a2 = q.k2.h * h * h, a3 = q.k3.h * h * h * h;
   const float scale = fabsf(y) + fabsf(a1) + fabsf(a2) + fabsf(a3);
   if (scale == 0.0f) return 0;
-  const float b1 = y + a1 * (1.0f / 3.0f);
-  const float b2 = y + a1 * (2.0f / 3.0f) + a2 * (1.0f / 3.0f);
-  const float b3 = y + a1 + a2 + a3;
-  const float lo = fminf(fminf(y, b1), fminf(b2, b3));
-  const float hi = fmaxf(fmaxf(y, b1), fmaxf(b2, b3));
-  const float margin = 1.0e-5f * scale;
-  if (lo > margin) return 1;
-  if (hi < -margin) return 0;
-  return 2;
+  if (!(scale <= kPieceScale) || h < kShortKnot) return 2;
+  if (add_all) return 1;
+  const float margin = 1.0e-5f * scale, flat = 1.0e-11f * scale, ar = tr * h;
+  // -1, 0 or 1: a coefficient's sign; 2: too close to zero to tell
+  auto sign = [&](float b, bool zero) {
+    return zero ? 0 : (b > margin ? 1 : (b < -margin ? -1 : 2));
+  };
+  const int s0 = sign(y, y == 0.0f), s3 = sign(yn, yn == 0.0f);
+  const int s1 = sign(y + a1 * (1.0f / 3.0f), y == 0.0f && fabsf(a1) <= flat);
+  const int s2 = sign(yn - ar * (1.0f / 3.0f), yn == 0.0f && fabsf(ar) <= flat);
+  const int lo = min(min(s0, s1), min(s2, s3)), hi = max(max(s0, s1), max(s2, s3));
+  if (hi == 2) return 2;
+  return lo >= 0 ? 1 : (hi <= 0 ? 0 : 2);
 }
 
 // the runs of signal phase k over cells [jb, je) of the parallel; returns
@@ -974,9 +1056,9 @@ __device__ __forceinline__ int build_runs(const CP &cp, const AR &area, int jb, 
   const DF zero{0.0f, 0.0f};
   DF w0 = zero, w1 = zero, w2 = zero, w3 = zero;
   auto flush = [&]() {
-    const size_t r = w.rec(half, n, k);
-    w.wa[r] = make_float4(w0.h, w0.l, w1.h, w1.l);
-    w.wb[r] = make_float4(w2.h, w2.l, w3.h, w3.l);
+    const size_t r = w.first(k, half) + n;
+    w.w[2 * r] = make_float4(w0.h, w0.l, w1.h, w1.l);
+    w.w[2 * r + 1] = make_float4(w2.h, w2.l, w3.h, w3.l);
     w.meta[r] = cur | (j0 << 10) | (span << 20);
     n++;
   };
@@ -1007,86 +1089,143 @@ __device__ __forceinline__ int build_runs(const CP &cp, const AR &area, int jb, 
 // the run's cells one by one (a piece whose sign changes on its interval)
 template <typename CP, typename AR>
 __device__ __forceinline__ DF run_cells(const CP &cp, const AR &area, const int32_t *rad, int iv,
-                                     int j0, int span, const PieceDF &q, DF acc) {
+                                        int j0, int span, const PieceDF &q, bool add_all, DF acc) {
   for (int j = j0; j < j0 + span; j++) {
     if (rad[j] != 1) continue;
     DF t;
     if (cp(j, iv, t) != iv) continue;
     const DF sv = df_fma(t, df_fma(t, df_fma(t, q.k3, q.k2), q.k1), q.y);
-    if (sv.h > 0.0f) acc = df_fma(area(j), sv, acc);
+    if (add_all || sv.h > 0.0f) acc = df_fma(area(j), sv, acc);
   }
   return acc;
 }
 
-// sums at signal phase k for the energies pb .. pb+kEPT-1 of the chunk from
-// the power sums of the runs of one half of the parallel's cells.  The lanes of a warp take consecutive phases,
-// so the r-th runs of neighbouring lanes lie in different intervals and
-// carry different piece classes: every energy's power-sum term is formed on
-// every lane and kept where the class is 1 (a select, no branch), and the
-// runs whose piece changes sign are only noted here and walked cell by cell
-// after the last run, so that one lane's cell walk does not hold up the
-// others run after run.  The next run's record is loaded before the current
-// one is used.
-constexpr int kDeferRuns = 24;  // sign-changing (run, energy) items noted per task
+// the power of two above v >= 0 (the smallest normal number for v = 0), or
+// twice it
+__device__ __forceinline__ float lead_of(float v, bool twice) {
+  return __int_as_float((__float_as_int(v) & 0x7f800000) + ((twice ? 2 : 1) << 23));
+}
 
+// s += a b, the rounding going to x: |s| exceeds the product, so d = t - s is
+// exact and fma(a, b, -d) is what t lost
+__device__ __forceinline__ void lead_acc(float a, float b, float &s, float &x) {
+  const float t = __fmaf_rn(a, b, s);
+  const float d = __fsub_rn(t, s);
+  x = __fadd_rn(x, __fmaf_rn(a, b, -d));
+  s = t;
+}
+
+// sum at signal phase k for energy slot e of the chunk, from the power sums
+// of the parallel's runs; a group of EC lanes (a divisor of the warp) calls it
+// with its own k, all groups of the warp together.  A run's four products are
+// added to a lead, the power of two above the sum of their magnitudes (what
+// some of them take away leaves it above the rest), so that each is added by
+// one FMA whose error two more instructions recover exactly -- against the six
+// of an error-free sum of unordered terms; their cross products and errors
+// gather in x at the run's own magnitude, and the run's value joins the pair
+// (s, c) by one error-free sum; taking the lead off is exact where the run's
+// value is positive or, with values of either sign (add_all), the lead twice
+// as large.  (A lead common to all runs saves nine
+// instructions and loses two bits.)  flags[2 iv]: energies of interval iv that are
+// not of class 1; flags[2 iv + 1]: those of them that add nothing; a run none
+// of whose energies adds anything is dropped when it is staged.
 template <typename CP, typename AR>
-__device__ __forceinline__ void run_sums(const CP &cp, const AR &area, const int32_t *rad,
-                                         const WRuns &w, const int *nruns, int k, int half,
-                                         const PieceDF *pc, const uint8_t *cls, int N_L, int EC,
-                                         int pb, DF (&acc)[kEPT]) {
-  uint32_t defer[kDeferRuns];
-  int nd = 0;
-  const int n = nruns[half * w.N_P + k];
-  float4 a4, b4;
-  int meta = 0;
-  if (n > 0) {
-    const size_t ri = w.rec(half, 0, k);
-    a4 = w.wa[ri];
-    b4 = w.wb[ri];
-    meta = w.meta[ri];
-  }
-  for (int r = 0; r < n; r++) {
-    const DF W0{a4.x, a4.y}, W1{a4.z, a4.w}, W2{b4.x, b4.y}, W3{b4.z, b4.w};
-    const int iv = meta & 1023;
-    if (r + 1 < n) {
-      const size_t ri = w.rec(half, r + 1, k);
-      a4 = w.wa[ri];
-      b4 = w.wb[ri];
-      meta = w.meta[ri];
-    }
-    // slots past the chunk's energies have class 0
+__device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_t *rad,
+                                      const WRuns &w, int n0, int n1, int k, int EC, int ne,
+                                      const PieceRows &pc, const uint32_t *flags,
+                                      RunStage *stages, bool add_all) {
+  const int lane = threadIdx.x & 31, e = threadIdx.x % EC, sub = lane / EC;
+  RunStage &st = stages[threadIdx.x / EC];
+  const uint32_t lit = ne == 32 ? 0xffffffffu : ((1u << ne) - 1u);
+  float s = 0.0f, c = 0.0f;
+  DF walked{0.0f, 0.0f};
+  const int n = n0 + n1;
+  const int n_max = __reduce_max_sync(0xffffffffu, n);
+  const size_t f0 = w.first(k, 0), f1 = w.first(k, 1) - n0;
+  float4 v[2];
+  int mt = 0;
+  // lane e of the group loads half a record (EC = 8: two halves)
+  auto fetch = [&](int b) {
 #pragma unroll
-    for (int e = 0; e < kEPT; e++) {
-      const uint8_t c = cls[iv * EC + pb + e];
-      const PieceDF q = pc[(pb + e) * N_L + iv];
-      float sh = acc[e].h, sl = acc[e].l;
-      df_acc_mul(q.y, W0, sh, sl);
-      df_acc_mul(q.k1, W1, sh, sl);
-      df_acc_mul(q.k2, W2, sh, sl);
-      df_acc_mul(q.k3, W3, sh, sl);
-      if (c == 1) acc[e] = fast_two_sum(sh, sl);
-      if (c == 2) {
-        if (nd < kDeferRuns) {
-          defer[nd++] = ((uint32_t)r << 4) | (uint32_t)e;
-        } else {
-          const int m = w.meta[w.rec(half, r, k)];
-          acc[e] = df_add(acc[e], run_cells(cp, area, rad, iv, (m >> 10) & 1023,
-                                            (m >> 20) & 1023, q, DF{0.0f, 0.0f}));
+    for (int z = 0; z < 2; z++) {
+      const int h = e + z * EC, i = b + (h >> 1);
+      if (h < 2 * kStage && i < n && (z == 0 || EC < 2 * kStage))
+        v[z] = w.w[2 * ((i < n0 ? f0 : f1) + i) + (h & 1)];
+    }
+    const int i = b + e;
+    if (e < kStage && i < n) mt = w.meta[(i < n0 ? f0 : f1) + i];
+  };
+  fetch(0);
+  for (int b = 0; b < n_max; b += kStage) {
+    __syncwarp();  // the last block's readers are done
+    bool alive = false;
+    if (e < 2 * kStage) st.w[e] = v[0];
+    if (EC < 2 * kStage) st.w[e + EC] = v[1];
+    if (e < kStage && b + e < n) {
+      const int iv = mt & 1023;
+      const uint2 fl = *reinterpret_cast<const uint2 *>(flags + 2 * iv);
+      st.meta[e] = make_uint4((uint32_t)mt, fl.x, fl.y, 0u);
+      alive = (fl.x & fl.y & lit) != lit;
+    }
+    uint32_t todo = __ballot_sync(0xffffffffu, alive) >> (sub * EC);
+    todo &= (1u << kStage) - 1u;
+    __syncwarp();
+    if (b + kStage < n) fetch(b + kStage);
+    // two runs at a time (the last may be the empty record): their chains are
+    // independent, and the groups of the warp stay together
+    while (__any_sync(0xffffffffu, todo != 0u)) {
+      float h[2], x[2];
+#pragma unroll
+      for (int z = 0; z < 2; z++) {
+        const int r = todo ? __ffs(todo) - 1 : kStage;
+        todo &= todo - 1;
+        const uint4 m = st.meta[r];
+        const int iv = (int)(m.x & 1023u);
+        const float4 p = pc.a[iv * pc.es + e], q = pc.b[iv * pc.es + e];
+        const float4 A = st.w[2 * r], B = st.w[2 * r + 1];
+        x[z] = __fmul_rn(p.x, A.y);
+        x[z] = __fmaf_rn(p.y, A.x, x[z]);
+        x[z] = __fmaf_rn(p.z, A.w, x[z]);
+        x[z] = __fmaf_rn(p.w, A.z, x[z]);
+        x[z] = __fmaf_rn(q.x, B.y, x[z]);
+        x[z] = __fmaf_rn(q.y, B.x, x[z]);
+        x[z] = __fmaf_rn(q.z, B.w, x[z]);
+        x[z] = __fmaf_rn(q.w, B.z, x[z]);
+        // (a power sum is negative where rounding put a cell's offset below
+        // its knot)
+        const float mag = __fmaf_rn(
+            fabsf(q.z), fabsf(B.z),
+            __fmaf_rn(fabsf(q.x), fabsf(B.x), __fmaf_rn(fabsf(p.z), fabsf(A.z),
+                                                        __fmul_rn(fabsf(p.x), fabsf(A.x)))));
+        const float lead = lead_of(mag, add_all);
+        float v = lead;
+        lead_acc(p.x, A.x, v, x[z]);
+        lead_acc(p.z, A.z, v, x[z]);
+        lead_acc(q.x, B.x, v, x[z]);
+        lead_acc(q.z, B.z, v, x[z]);
+        h[z] = __fsub_rn(v, lead);
+        const bool odd = r < kStage && ((m.y >> e) & 1u);
+        if (odd) h[z] = x[z] = 0.0f;
+        if (__any_sync(0xffffffffu, odd)) {
+          if (odd && !((m.z >> e) & 1u))
+            walked = run_cells(cp, area, rad, iv, (int)((m.x >> 10) & 1023u),
+                               (int)((m.x >> 20) & 1023u),
+                               PieceDF{{p.x, p.y}, {p.z, p.w}, {q.x, q.y}, {q.z, q.w}}, add_all,
+                               walked);
+          __syncwarp();
         }
+      }
+#pragma unroll
+      for (int z = 0; z < 2; z++) {
+        float t, err;
+        two_sum(s, h[z], t, err);
+        const DF sc = fast_two_sum(t, __fadd_rn(c, __fadd_rn(err, x[z])));
+        s = sc.h;
+        c = sc.l;
       }
     }
   }
-  for (int d = 0; d < nd; d++) {
-    const uint32_t it = defer[d];
-    const int r = (int)(it >> 4), ed = (int)(it & 15u);
-    const int m = w.meta[w.rec(half, r, k)];
-    const int iv = m & 1023;
-    const DF add = run_cells(cp, area, rad, iv, (m >> 10) & 1023, (m >> 20) & 1023,
-                             pc[(pb + ed) * N_L + iv], DF{0.0f, 0.0f});
-#pragma unroll
-    for (int e = 0; e < kEPT; e++)
-      if (e == ed) acc[e] = df_add(acc[e], add);
-  }
+  return df_add(df_norm(s, c), walked);
 }
 
 // ---------------------------------------------------------------------------
@@ -1154,21 +1293,24 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
   const bool erest = (M.atm == 6);
   const bool num4d = (M.atm == 2) || tab2;
   const int nmu = a.atmos.I ? a.atmos.nmu : 0, nEt = a.atmos.I ? a.atmos.nE : 0;
-  const Layout L = make_layout(N_L, N_P, N_E, nmu, nEt, (int)sizeof(PieceT<WT>), a.N_R);
+  const Layout L =
+      make_layout(N_L, N_P, N_E, nmu, nEt, (int)sizeof(PieceT<WT>), a.N_R, !kMixed);
   const int EC = L.EC;
   double *coef;
   AtmSmem as{};
-  GeoSmem g = carve(smem, N_L, EC, &coef, nmu, nEt, &as, (int)sizeof(PieceT<WT>), a.N_R);
-  PieceT<WT> *co4 = reinterpret_cast<PieceT<WT> *>(coef);
+  GeoSmem g = carve(smem, N_L, EC, &coef, nmu, nEt, &as, (int)sizeof(PieceT<WT>), a.N_R, !kMixed);
+  PieceT<WT> *co4 = reinterpret_cast<PieceT<WT> *>(coef);  // mixed form
+  const PieceRows pr{reinterpret_cast<float4 *>(coef),
+                     reinterpret_cast<float4 *>(coef) + (size_t)N_L * (EC + 1), EC + 1};
   __shared__ int s_J, s_top, s_any, s_jalt;
   // a beaming modification's (abb, bbb, cbb, dbb, nimu) for the parallel
   __shared__ double s_beam[5];
-  // power-sum form (FP64 path with scratch): run counts per (cell half,
-  // signal phase) and the class of every piece of the chunk; the run
+  // power-sum form (FP64 path with scratch): run counts and areas per (cell
+  // half, signal phase) and the piece classes of the chunk; the run
   // records live in one of a.w_slots scratch slots, taken for the CTA's
   // lifetime (at most 2 CTAs per SM are resident, the pool has more slots;
   // a CTA that finds none after a bounded search runs the per-cell form)
-  __shared__ int s_wslot, s_next;
+  __shared__ int s_wslot;
   bool use_w = !kMixed && a.wsum != nullptr;
   if (use_w) {
     if (threadIdx.x == 0) {
@@ -1182,8 +1324,25 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
     __syncthreads();
     use_w = s_wslot >= 0;
   }
-  int *s_nruns = reinterpret_cast<int *>(g.sc_exp + EC);
-  uint8_t *s_cls = reinterpret_cast<uint8_t *>(s_nruns + 2 * N_P);
+  // class masks [N_L][2], run counts [2][N_P], the signal phases, staged runs
+  // per group
+  uint32_t *s_flags = reinterpret_cast<uint32_t *>(
+      (reinterpret_cast<uintptr_t>(g.sc_exp + EC) + 7) & ~uintptr_t(7));
+  int *s_nruns = reinterpret_cast<int *>(s_flags + 2 * N_L);
+  // the signal phases as float pairs
+  float2 *s_phase = reinterpret_cast<float2 *>(
+      (reinterpret_cast<uintptr_t>(s_nruns + 2 * N_P) + 15) & ~uintptr_t(15));
+  RunStage *s_stages = reinterpret_cast<RunStage *>(
+      (reinterpret_cast<uintptr_t>(s_phase + N_P) + 15) & ~uintptr_t(15));
+  for (int t = threadIdx.x; t < N_P; t += blockDim.x) {
+    const DF v = df_split(a.phases[t]);
+    s_phase[t] = make_float2(v.h, v.l);
+  }
+  if (use_w)
+    for (int t = threadIdx.x; t < kThreads / EC; t += blockDim.x) {
+      s_stages[t].w[2 * kStage] = s_stages[t].w[2 * kStage + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      s_stages[t].meta[kStage] = make_uint4(0u, 0u, 0u, 0u);
+    }
   const WRuns wr = use_w ? wruns_of(a.wsum + (size_t)s_wslot *
                                                  integrate_wsum_bytes_dev(N_P, a.w_cap),
                                     a.w_cap, N_P)
@@ -1226,12 +1385,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
   }
   const double norm = num4d ? kErg / kHKeV : kErg * kPlanck;
   double *part = a.partial + (size_t)chunk * N_E * N_P;
-  // the power sums' second cell half adds into its own partial
-  double *part2 = a.partial2 ? a.partial2 + (size_t)chunk * N_E * N_P : nullptr;
-  for (int t = threadIdx.x; t < N_E * N_P; t += blockDim.x) {
-    part[t] = 0.0;
-    if (part2) part2[t] = 0.0;
-  }
+  for (int t = threadIdx.x; t < N_E * N_P; t += blockDim.x) part[t] = 0.0;
   __syncthreads();
   const double mu_max = num4d ? a.atmos.mu[a.atmos.nmu - 1] : 0.0;
   const double mu_top3 = num4d ? a.atmos.mu[a.atmos.nmu - 3] : 0.0;
@@ -1360,6 +1514,11 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
     const double *cellPhi = a.phi + M.cell_off + (int64_t)i * M.S1;
     const int32_t *rad = a.radiates + M.cell_off + (int64_t)i * M.S1;
     for (int I = 0; I < c.IO; I++) {
+      if (!kMixed && I > 0) {  // the last image's pieces overwrote the staged table
+        for (int t = threadIdx.x; t < a.N_R; t += blockDim.x)
+          g.rD[t] = a.deflection[row * a.N_R + t];
+        __syncthreads();
+      }
       for (int k = threadIdx.x; k < leaf_lim; k += blockDim.x)
         leaf_geometry(c, I, k, N_L, leaf_lim, a.leaves, g);
       __syncthreads();
@@ -1416,25 +1575,26 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
         }
       }
       __syncthreads();
+      constexpr float tp = (float)kTwoPi;
+      auto cell_phase = [&](auto cached, int k) {
+        const float2 ph = s_phase[k];
+        return CellPhaseF<decltype(cached)::value>{as.fphase, as.fphase_lo, N_L, as.fphase[0],
+                                   as.fphase[N_L - 1], ph.x, ph.y, tp,
+                                   (float)(kTwoPi - (double)tp), as.fcphi, as.fcphi_lo, cellPhi};
+      };
       if (use_w) {
         // the runs of every signal phase, each half of the cells by its own
         // thread (energy independent: formed once per parallel and image)
         const int hc = (M.S1 + 1) / 2;
-        const bool cached = M.S1 <= kMaxCellsF;
-        const AreaDF ar{cached ? as.fcarea : nullptr, cached ? as.fcarea_lo : nullptr, cellA};
+        const AreaDF<true> ar{as.fcarea, as.fcarea_lo, cellA};
         for (int t = threadIdx.x; t < 2 * N_P; t += blockDim.x) {
           const int k = t % N_P, half = t / N_P;
-          const double phd = a.phases[k];
-          const float ph = (float)phd;
-          const float tp = (float)kTwoPi;
-          const CellPhaseF cp{as.fphase, as.fphase_lo, N_L, as.fphase[0], as.fphase[N_L - 1], ph,
-                              (float)(phd - (double)ph), tp, (float)(kTwoPi - (double)tp),
-                              cached ? as.fcphi : nullptr, cached ? as.fcphi_lo : nullptr,
-                              cellPhi};
-          int n = build_runs(cp, ar, half * hc, min(M.S1, (half + 1) * hc), rad, wr, half, k);
+          const CellPhaseF<true> cp = cell_phase(std::true_type{}, k);
+          const int n = build_runs(cp, ar, half * hc, min(M.S1, (half + 1) * hc), rad, wr, half, k);
           if (n < 0) {
+            // no cell of the parallel is added at this phase (either half's
+            // failure voids both, as in the per-cell form)
             atomicExch(&a.member_status[m], (int)kPulseFail);
-            n = 0;
           }
           s_nruns[half * N_P + k] = n;
         }
@@ -1520,9 +1680,8 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
                   if (dfy) {
                     // y = I 2^xr col_factor kept as a double-float mantissa
                     // and an exponent (no round trip through FP64)
-                    Piece &o = co4[pl * N_L + col];
-                    *reinterpret_cast<DF *>(&o.y) = df_mul(I, cf_m);
-                    *reinterpret_cast<int *>(&o.k1) = xr + cf_x;
+                    pr.y(col, pl) = df_mul(I, cf_m);
+                    pr.ex(col, pl) = xr + cf_x;
                     continue;
                   }
                   I_E = df_value(I) * pow2_double(xr) * p3;
@@ -1556,7 +1715,8 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
                 }
               }
             }
-            co4[pl * N_L + col].y = y;
+            if constexpr (kMixed) co4[pl * N_L + col].y = y;
+            else pr.yd(col, pl) = y;
           }
         }
         if (!kMixed && M.beam_opt > 0) {
@@ -1567,7 +1727,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
             const int p = e0 + pl;
             const int s = g.src[col];
             if (s < 0) continue;
-            const double I_raw = (double)co4[pl * N_L + col].y;
+            const double I_raw = pr.yd(col, pl);
             double I_E;
             if (num4d) {
               const double v3 = erest ? (g.lgE[pl] / g.lzs[s]) * 0.001956951 : g.lgE[pl] - g.lzs[s];
@@ -1589,7 +1749,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
             }
             const double I_c =
                 corr ? eval_bb(a.energies[p] / g.Z[s], kT_c) * (kErg * kPlanck) : 0.0;
-            co4[pl * N_L + col].y = (WT)((I_E * norm - I_c) * g.GEOM[s]);
+            pr.yd(col, pl) = (I_E * norm - I_c) * g.GEOM[s];
           }
         }
         __syncthreads();
@@ -1631,144 +1791,136 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
           // largest profile value lies in [0.5, 1): double-float values then
           // keep the row's full relative precision whatever its magnitude
           const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-          PieceDF *pc = reinterpret_cast<PieceDF *>(co4);
-          if (dfy) {
-            // values m 2^x (mantissa in the y slot, exponent in k1's): the
-            // row's largest exponent from the bits, then each value times
-            // 2^(x - that) in float arithmetic (exact)
-            for (int pl = warp; pl < ne; pl += kThreads / 32) {
-              MaxExponent mx;
-              for (int col = lane; col < N_L; col += 32) {
-                const Piece &o = co4[pl * N_L + col];
-                const float h = reinterpret_cast<const DF *>(&o.y)->h;
+          for (int pl = warp; pl < ne; pl += kThreads / 32) {
+            MaxExponent mx;
+            for (int col = lane; col < N_L; col += 32) {
+              if (dfy) {
+                // values m 2^x: the exponent from the bits
+                const float h = pr.y(col, pl).h;
                 if (h != 0.0f && h == h) {
                   if (isinf(h)) mx.inf = true;
-                  else mx.e = max(mx.e, *reinterpret_cast<const int *>(&o.k1) + float_exponent(h));
+                  else mx.e = max(mx.e, pr.ex(col, pl) + float_exponent(h));
                 }
+              } else {
+                mx.fold(pr.yd(col, pl));
               }
-              mx.merge_warp();
-              if (lane == 0) g.sc_exp[pl] = mx.exponent();
             }
-            __syncthreads();
-            for (int t = threadIdx.x; t < ne * N_L; t += blockDim.x) {
-              const DF m = *reinterpret_cast<const DF *>(&co4[t].y);
-              const int x = *reinterpret_cast<const int *>(&co4[t].k1);
-              pc[t].y = m.h == 0.0f ? DF{0.0f, 0.0f} : df_times_pow2(m, x - g.sc_exp[t / N_L]);
-            }
-          } else {
-            for (int pl = warp; pl < ne; pl += kThreads / 32) {
-              MaxExponent mx;
-              for (int col = lane; col < N_L; col += 32) mx.fold((double)co4[pl * N_L + col].y);
-              mx.merge_warp();
-              if (lane == 0) g.sc_exp[pl] = mx.exponent();
-            }
-            __syncthreads();
-            for (int t = threadIdx.x; t < ne * N_L; t += blockDim.x) {
-              const double v = (double)co4[t].y;
-              pc[t].y = df_split(scale_pow2(v, -g.sc_exp[t / N_L]));
+            mx.merge_warp();
+            if (lane == 0) g.sc_exp[pl] = mx.exponent();
+          }
+          __syncthreads();
+          for (int t = threadIdx.x; t < EC * N_L; t += blockDim.x) {
+            const int col = t / EC, pl = t - col * EC;
+            if (pl >= ne) continue;
+            if (dfy) {  // the value times 2^(x - the row's) in float arithmetic (exact)
+              const DF m = pr.y(col, pl);
+              pr.y(col, pl) = m.h == 0.0f ? DF{0.0f, 0.0f}
+                                          : df_times_pow2(m, pr.ex(col, pl) - g.sc_exp[pl]);
+            } else {
+              pr.y(col, pl) = df_split(scale_pow2(pr.yd(col, pl), -g.sc_exp[pl]));
             }
           }
           __syncthreads();
-          for (int t = threadIdx.x; t < ne * strips; t += blockDim.x) {
-            const int pl = t / strips, i0 = (t - pl * strips) * kStrip;
+          // a group of EC lanes takes a strip, a lane an energy; the classes
+          // of a piece's energies are gathered by ballot
+          const int sub = lane / EC;
+          for (int t = threadIdx.x; t < ((EC * strips + 31) & ~31); t += blockDim.x) {
+            const int pl = t % EC, i0 = (t / EC) * kStrip;
             const int i1 = min(i0 + kStrip, n_iv);
-            PieceDF *yr = pc + pl * N_L;
+            const bool on = pl < ne;
             auto chord = [&](int j) -> DF {
               const int q = periodic_chord(j, N_L);
-              return df_mul(df_sub(yr[q + 1].y, yr[q].y), g.ih[q]);
+              return df_mul(df_sub(pr.y(q + 1, pl), pr.y(q, pl)), g.ih[q]);
             };
-            DF m0 = chord(i0 - 2), m1 = chord(i0 - 1), m2 = chord(i0), m3 = chord(i0 + 1),
-               m4 = chord(i0 + 2);
-            for (int iv = i0; iv < i1; iv++) {
-              if (iv > i0) {
-                m0 = m1; m1 = m2; m2 = m3; m3 = m4;
-                m4 = chord(iv + 2);
+            DF m0{}, m1{}, m2{}, m3{}, m4{};
+            if (on && i0 < i1) {
+              m0 = chord(i0 - 2); m1 = chord(i0 - 1); m2 = chord(i0); m3 = chord(i0 + 1);
+              m4 = chord(i0 + 2);
+            }
+            for (int z = 0; z < kStrip; z++) {
+              const int iv = i0 + z;
+              const bool here = on && iv < i1;
+              int cls = 1;
+              if (here) {
+                if (z > 0) {
+                  m0 = m1; m1 = m2; m2 = m3; m3 = m4;
+                  m4 = chord(iv + 2);
+                }
+                DF k1, k2, k3, tr;
+                akima_piece_df(m0, m1, m2, m3, m4, g.ih[iv], g.ih2[iv], k1, k2, k3, tr);
+                pr.put_k(iv, pl, k1, k2, k3);
+                const float h = (as.fphase[iv + 1] - as.fphase[iv]) +
+                                (as.fphase_lo[iv + 1] - as.fphase_lo[iv]);
+                cls = piece_class(PieceDF{pr.y(iv, pl), k1, k2, k3}, pr.y(iv + 1, pl).h, tr.h, h,
+                                  corr);
               }
-              DF k1, k2, k3;
-              akima_piece_df(m0, m1, m2, m3, m4, g.ih[iv], g.ih2[iv], k1, k2, k3);
-              yr[iv].k1 = k1;
-              yr[iv].k2 = k2;
-              yr[iv].k3 = k3;
+              const uint32_t odd = __ballot_sync(0xffffffffu, cls != 1);
+              const uint32_t none = __ballot_sync(0xffffffffu, cls == 0);
+              if (pl == 0 && iv < i1) {
+                const uint32_t mask = EC == 32 ? 0xffffffffu : ((1u << EC) - 1u);
+                s_flags[2 * iv] = (odd >> (sub * EC)) & mask;
+                s_flags[2 * iv + 1] = (none >> (sub * EC)) & mask;
+              }
             }
           }
           __syncthreads();
-          // the class of every piece for the power sums, [N_L][EC] (0
-          // beyond the chunk's energies); every nonzero value is added with
-          // the elsewhere correction (:593-594)
-          if (use_w) for (int t = threadIdx.x; t < EC * N_L; t += blockDim.x) {
-            const int iv = t / EC, pl = t - iv * EC;
-            uint8_t cl = 0;
-            if (pl < ne && iv < N_L - 1) {
-              const PieceDF &q = pc[pl * N_L + iv];
-              cl = piece_class(q, as.fphase[iv + 1] - as.fphase[iv]);
-              if (corr && cl == 0 &&
-                  (q.y.h != 0.0f || q.k1.h != 0.0f || q.k2.h != 0.0f || q.k3.h != 0.0f))
-                cl = 1;
-              if (corr) cl = cl ? 1 : 0;
-            }
-            s_cls[t] = cl;
-          }
-          if (threadIdx.x == 0) s_next = blockDim.x;
-          if (use_w) __syncthreads();
         }
-        // cell x phase accumulation (:571-598).  The power-sum form splits
-        // each task into its two cell halves (units u < ntasks: half 0,
-        // u >= ntasks: half 1, adding into part2); a warp takes its first 32
-        // consecutive units by index and further blocks of 32 from a shared
-        // counter, so the uneven run counts of the phases even out over the
-        // CTA while a warp's lanes keep consecutive phases
-        const int nunits = use_w ? 2 * ntasks : ntasks;
-        const int lane = threadIdx.x & 31;
-        for (int u = threadIdx.x; u - lane < nunits;
-             u = use_w ? __shfl_sync(0xffffffffu, lane == 0 ? atomicAdd(&s_next, 32) : 0, 0) + lane
-                       : u + (int)blockDim.x) {
-          if (u >= nunits) continue;
-          const int half = u >= ntasks ? 1 : 0;
-          const int task = u - half * ntasks;
-          const int k = task % N_P, grp = task / N_P;
-          const int pb = grp * kEPT;
-          if (pb >= ne) continue;
-          const double phd = a.phases[k];
-          const float ph = (float)phd;
-          const float tp = (float)kTwoPi;
-          const bool cached = M.S1 <= kMaxCellsF;
-          const CellPhaseF cp{as.fphase, as.fphase_lo, N_L, as.fphase[0], as.fphase[N_L - 1], ph,
-                              (float)(phd - (double)ph), tp, (float)(kTwoPi - (double)tp),
-                              cached ? as.fcphi : nullptr, cached ? as.fcphi_lo : nullptr,
-                              cellPhi};
-          if constexpr (kMixed) {
-            WT acc[kEPT];
-#pragma unroll
-            for (int e = 0; e < kEPT; e++) acc[e] = WT(0);
-            const AreaF ar{cached ? as.fcarea : nullptr, cellA};
-            if (!cell_phase_sums<WT>(cp, ar, M.S1, rad, co4, N_L, pb, ne, acc)) {
-              atomicExch(&a.member_status[m], (int)kPulseFail);
-              continue;
-            }
-#pragma unroll
-            for (int e = 0; e < kEPT; e++)
-              if (pb + e < ne) part[(size_t)(e0 + pb + e) * N_P + k] += (double)acc[e] * fix;
-          } else {
-            DF acc[kEPT];
-#pragma unroll
-            for (int e = 0; e < kEPT; e++) acc[e] = DF{0.0f, 0.0f};
-            const AreaDF ar{cached ? as.fcarea : nullptr, cached ? as.fcarea_lo : nullptr, cellA};
-            if (use_w) {
-              run_sums(cp, ar, rad, wr, s_nruns, k, half,
-                       reinterpret_cast<const PieceDF *>(co4), s_cls, N_L, EC, pb, acc);
-            } else if (!cell_phase_sums_df(cp, ar, M.S1, rad,
-                                           reinterpret_cast<const PieceDF *>(co4), N_L, pb, ne,
-                                           corr, acc)) {
-              atomicExch(&a.member_status[m], (int)kPulseFail);
-              continue;
-            }
-            double *dst = half ? part2 : part;
-#pragma unroll
-            for (int e = 0; e < kEPT; e++)
-              if (pb + e < ne)
-                dst[(size_t)(e0 + pb + e) * N_P + k] +=
-                    scale_pow2(df_value(acc[e]), g.sc_exp[pb + e]);
+        // cell x phase accumulation (:571-598).  Power sums: a group of EC
+        // lanes takes a signal phase, a lane an energy.  Per-cell form: a
+        // thread takes a signal phase and kEPT energies.
+        if (use_w) {
+          const int e = threadIdx.x % EC;
+          for (int k0 = 0; k0 < N_P; k0 += kThreads / EC) {
+            const int k = k0 + threadIdx.x / EC, kc = min(k, N_P - 1);
+            const AreaDF<true> ar{as.fcarea, as.fcarea_lo, cellA};
+            int n0 = s_nruns[kc], n1 = s_nruns[N_P + kc];
+            if (n0 < 0 || n1 < 0 || k >= N_P) n0 = n1 = 0;
+            const DF v = run_sum(cell_phase(std::true_type{}, kc), ar, rad, wr, n0, n1, kc,
+                                 EC, ne, pr, s_flags, s_stages,
+                                 corr);
+            // partials [N_P][N_E]: the lanes' energies are adjacent
+            if (e < ne && k < N_P)
+              part[(size_t)k * N_E + e0 + e] += scale_pow2(df_value(v), g.sc_exp[e]);
           }
+        } else {
+          auto sums = [&](auto cached) {
+            constexpr bool kCached = decltype(cached)::value;
+            for (int task = threadIdx.x; task < ntasks; task += blockDim.x) {
+              const int k = task % N_P, grp = task / N_P;
+              const int pb = grp * kEPT;
+              if (pb >= ne) continue;
+              const CellPhaseF<kCached> cp = cell_phase(cached, k);
+              if constexpr (kMixed) {
+                WT acc[kEPT];
+#pragma unroll
+                for (int e = 0; e < kEPT; e++) acc[e] = WT(0);
+                const AreaF<kCached> ar{as.fcarea, cellA};
+                if (!cell_phase_sums<WT>(cp, ar, M.S1, rad, co4, N_L, pb, ne, acc)) {
+                  atomicExch(&a.member_status[m], (int)kPulseFail);
+                  continue;
+                }
+#pragma unroll
+                for (int e = 0; e < kEPT; e++)
+                  if (pb + e < ne) part[(size_t)(e0 + pb + e) * N_P + k] += (double)acc[e] * fix;
+              } else {
+                DF acc[kEPT];
+#pragma unroll
+                for (int e = 0; e < kEPT; e++) acc[e] = DF{0.0f, 0.0f};
+                const AreaDF<kCached> ar{as.fcarea, as.fcarea_lo, cellA};
+                if (!cell_phase_sums_df(cp, ar, M.S1, rad, pr, pb, corr, acc)) {
+                  atomicExch(&a.member_status[m], (int)kPulseFail);
+                  continue;
+                }
+#pragma unroll
+                for (int e = 0; e < kEPT; e++)
+                  if (pb + e < ne)
+                    part[(size_t)k * N_E + e0 + pb + e] +=
+                        scale_pow2(df_value(acc[e]), g.sc_exp[pb + e]);
+              }
+            }
+          };
+          if (M.S1 <= kMaxCellsF) sums(std::true_type{});
+          else sums(std::false_type{});
         }
         __syncthreads();
       }
@@ -2031,19 +2183,22 @@ __global__ void __launch_bounds__(kThreads, 1) stokes_kernel(IntegrateArgs a) {
         const double phd = a.phases[k];
         const float ph = (float)phd;
         const float tp = (float)kTwoPi;
-        const bool cached = M.S1 <= kMaxCellsF;
-        const CellPhaseF cp{as.fphase, as.fphase_lo, N_L, as.fphase[0], as.fphase[N_L - 1], ph,
-                            (float)(phd - (double)ph), tp, (float)(kTwoPi - (double)tp),
-                            cached ? as.fcphi : nullptr, cached ? as.fcphi_lo : nullptr,
-                            cellPhi};
-        const AreaDF ar{cached ? as.fcarea : nullptr, cached ? as.fcarea_lo : nullptr, cellA};
         DF aI[kEPT], aQ[kEPT], aU[kEPT];
 #pragma unroll
         for (int e = 0; e < kEPT; e++) aI[e] = aQ[e] = aU[e] = DF{0.0f, 0.0f};
-        if (!cell_phase_sums_stokes(cp, ar, M.S1, rad, reinterpret_cast<const PieceDF *>(coI),
-                                    reinterpret_cast<const PieceDF *>(coQ),
-                                    reinterpret_cast<const PieceDF *>(coU), N_L, pb, ne, corr, aI,
-                                    aQ, aU)) {
+        auto sums = [&](auto cached) {
+          constexpr bool kCached = decltype(cached)::value;
+          const CellPhaseF<kCached> cp{as.fphase, as.fphase_lo, N_L, as.fphase[0],
+                                       as.fphase[N_L - 1], ph, (float)(phd - (double)ph), tp,
+                                       (float)(kTwoPi - (double)tp), as.fcphi, as.fcphi_lo,
+                                       cellPhi};
+          const AreaDF<kCached> ar{as.fcarea, as.fcarea_lo, cellA};
+          return cell_phase_sums_stokes(cp, ar, M.S1, rad, reinterpret_cast<const PieceDF *>(coI),
+                                        reinterpret_cast<const PieceDF *>(coQ),
+                                        reinterpret_cast<const PieceDF *>(coU), N_L, pb, ne, corr,
+                                        aI, aQ, aU);
+        };
+        if (!(M.S1 <= kMaxCellsF ? sums(std::true_type{}) : sums(std::false_type{}))) {
           atomicExch(&a.member_status[m], (int)kPulseFail);
           continue;
         }
@@ -2326,11 +2481,11 @@ __global__ void reduce_flux_kernel(IntegrateArgs a) {
   const int c0 = a.chunk_first[m], c1 = a.chunk_first[m + 1];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int c = c0; c < c1; c++)
-      s += a.partial2 ? a.partial[(size_t)c * n + t] + a.partial2[(size_t)c * n + t]
-                      : a.partial[(size_t)c * n + t];
-    const int p = t / a.N_P;
-    a.flux[M.flux_off + t] = s / (a.energies[p] * kKeV);
+    for (int c = c0; c < c1; c++) s += a.partial[(size_t)c * n + t];
+    // the FP64 form's partials are [N_P][N_E], the mixed form's [N_E][N_P]
+    const int p = a.mixed ? t / a.N_P : t % a.N_E;
+    const int k = a.mixed ? t - p * a.N_P : t / a.N_E;
+    a.flux[M.flux_off + (int64_t)p * a.N_P + k] = s / (a.energies[p] * kKeV);
   }
 }
 
@@ -2359,10 +2514,14 @@ size_t integrate_wsum_bytes(int N_P, int max_cells, int *w_cap) {
 void launch_integrate(const IntegrateArgs &a, cudaStream_t st) {
   if (a.n_members <= 0) return;
   const int pb = a.mixed ? (int)sizeof(PieceT<float>) : (int)sizeof(PieceT<double>);
-  Layout L = a.atmos.I ? make_layout(a.N_L, a.N_P, a.N_E, a.atmos.nmu, a.atmos.nE, pb, a.N_R)
-                       : make_layout(a.N_L, a.N_P, a.N_E, 0, 0, pb, a.N_R);
-  // run counts [2][N_P] and piece classes [EC][N_L] after the layout
-  const size_t bytes = L.bytes + (size_t)2 * a.N_P * sizeof(int) + (size_t)L.EC * a.N_L + 16;
+  Layout L = make_layout(a.N_L, a.N_P, a.N_E, a.atmos.I ? a.atmos.nmu : 0,
+                         a.atmos.I ? a.atmos.nE : 0, pb, a.N_R, !a.mixed);
+  // class masks [N_L][2], run counts [2][N_P], the signal phases [N_P] and the
+  // groups' staged runs after the layout
+  const size_t bytes = L.bytes + (size_t)2 * a.N_L * sizeof(uint32_t) +
+                       (size_t)2 * a.N_P * sizeof(int) +
+                       (size_t)a.N_P * sizeof(float2) + 64 +
+                       (a.mixed ? 0 : (size_t)(kThreads / L.EC) * sizeof(RunStage));
   // the work plan from the parallels' costs (needs the ray tables)
   if (a.n_rows > 0) row_cost_kernel<<<(unsigned)((a.n_rows * 32 + 255) / 256), 256, 0, st>>>(a);
   plan_chunks_kernel<<<1, kPlanThreads, 0, st>>>(a);
