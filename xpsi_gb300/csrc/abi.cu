@@ -276,48 +276,52 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
   const int64_t max_chunks = std::min<int64_t>(2 * target_chunks + n_meshes, n_rows) + 16;
   if (max_chunks > (int64_t)INT32_MAX / 2) return fail_msg("too many meshes in one call");
   const int n_chunks = (int)max_chunks;
-  Dev dm, dr0, dr1, dfirst, dorder, dcount, drowcost, dchunkcost, dpart, dstate;
+  int dev = 0, sms = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int ctas = 2 * std::max(1, sms);  // two integrator CTAs are resident per SM
+  const int EC = xg::integrate_energy_chunk(N_L, N_P, N_E, mixed);
+  const int n_eg = 1;
+  Dev dm;
   int rc;
   if ((rc = upload(dm, reinterpret_cast<const xg::MemberDesc *>(meshes), n_meshes, st))) return rc;
-  if ((rc = dalloc(dr0, (size_t)n_chunks * sizeof(int64_t), st)) ||
-      (rc = dalloc(dr1, (size_t)n_chunks * sizeof(int64_t), st)) ||
-      (rc = dalloc(dfirst, (size_t)(n_meshes + 1) * sizeof(int32_t), st)) ||
-      (rc = dalloc(dorder, (size_t)n_chunks * sizeof(int32_t), st)) ||
-      (rc = dalloc(dcount, sizeof(int32_t), st)) ||
-      (rc = dalloc(drowcost, (size_t)std::max<int64_t>(1, n_rows) * sizeof(float), st)) ||
-      (rc = dalloc(dchunkcost, (size_t)n_chunks * sizeof(float), st)))
-    return rc;
-  // each chunk's CTA zeroes its own partial before accumulating
-  size_t part_n = (size_t)n_chunks * N_E * N_P;
-  if ((rc = dalloc(dpart, part_n * sizeof(double), st))) return rc;
-  if ((rc = dalloc(dstate, (size_t)3 * n_rows + 16, st))) return rc;
-  Dev dslab;
-  if (d->atmos.intensity != nullptr && !table2d &&
-      (rc = dalloc(dslab, (size_t)n_chunks * d->atmos.nmu * d->atmos.nE * sizeof(double), st)))
-    return rc;
-  CK(cudaMemsetAsync(d->mesh_status, 0, n_meshes * sizeof(int32_t), st));
   // run records of the FP64 form's power sums (parallels of up to 256 cells,
   // which the integrator holds in shared memory, and 1024 leaves; beyond that
   // the per-cell form runs)
-  Dev dwsum;
   int w_cap = 0;
   int max_cells = 0;
   for (int m = 0; m < n_meshes; m++) max_cells = std::max(max_cells, (int)meshes[m].S1);
   const bool use_w = !mixed && max_cells <= 256 && N_L <= 1024 && wsum_enabled();
-  // a slot per CTA that can be resident (at most 2 per SM), twice over
-  int w_slots = 0;
-  Dev dwbusy;
-  if (use_w) {
-    int dev = 0, sms = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    w_slots = 4 * std::max(1, sms);
-    const size_t w_chunk = xg::integrate_wsum_bytes(N_P, max_cells, &w_cap);
-    if ((rc = dalloc(dwsum, (size_t)w_slots * w_chunk, st)) ||
-        (rc = dalloc(dwbusy, (size_t)w_slots * sizeof(int32_t), st)))
-      return rc;
-    CK(cudaMemsetAsync(dwbusy.p, 0, (size_t)w_slots * sizeof(int32_t), st));
-  }
+  const bool tab4 = d->atmos.intensity != nullptr && !table2d;
+  // geometry records: two images per parallel and some room (a parallel near
+  // the photon sphere has up to about eight; the integrator forms those that
+  // find no room again), then one per CTA
+  const int64_t img = xg::integrate_image_doubles(N_L);
+  const int64_t geo_cap = 2 * n_rows + 1024;
+  // one allocation for the call's scratch, parts at 256-byte boundaries
+  size_t total = 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  const size_t o_r0 = part((size_t)n_chunks * 8), o_r1 = part((size_t)n_chunks * 8);
+  const size_t o_first = part((size_t)(n_meshes + 1) * 4), o_order = part((size_t)n_chunks * 4);
+  const size_t o_count = part(64), o_rowcost = part((size_t)std::max<int64_t>(1, n_rows) * 4);
+  const size_t o_chunkcost = part((size_t)n_chunks * 4);
+  // each item's CTA zeroes its own part of a partial before accumulating
+  const size_t o_part = part((size_t)n_chunks * N_E * N_P * 8);
+  const size_t o_state = part((size_t)3 * n_rows + 16);
+  const size_t o_slab = part(tab4 ? (size_t)ctas * d->atmos.nmu * d->atmos.nE * 8 : 0);
+  const size_t o_wsum =
+      part(use_w ? (size_t)ctas * xg::integrate_wsum_bytes(N_P, max_cells, &w_cap) : 0);
+  const size_t o_lgE = part((size_t)N_E * 8);
+  const size_t o_geo = part((size_t)(geo_cap + ctas) * img * 8);
+  const size_t o_info = part((size_t)std::max<int64_t>(1, n_rows) * sizeof(xg::RowInfo));
+  Dev dscratch;
+  if ((rc = dalloc(dscratch, total, st))) return rc;
+  unsigned char *sp = dscratch.as<unsigned char>();
+  CK(cudaMemsetAsync(d->mesh_status, 0, n_meshes * sizeof(int32_t), st));
 
   xg::IntegrateArgs a{};
   a.n_members = n_meshes;
@@ -339,24 +343,32 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
                         (int)d->atmos.nmu, (int)d->atmos.nE, d->atmos.intensity_f32};
   a.max_chunks = n_chunks;
   a.target_chunks = (int)target_chunks;
-  a.chunk_r0 = dr0.as<int64_t>();
-  a.chunk_r1 = dr1.as<int64_t>();
-  a.partial = dpart.as<double>();
-  a.chunk_first = dfirst.as<int32_t>();
-  a.chunk_order = dorder.as<int32_t>();
-  a.chunk_count = dcount.as<int32_t>();
-  a.row_cost = drowcost.as<float>();
-  a.chunk_cost = dchunkcost.as<float>();
-  uint8_t *sb = dstate.as<uint8_t>();
+  a.chunk_r0 = reinterpret_cast<int64_t *>(sp + o_r0);
+  a.chunk_r1 = reinterpret_cast<int64_t *>(sp + o_r1);
+  a.partial = reinterpret_cast<double *>(sp + o_part);
+  a.chunk_first = reinterpret_cast<int32_t *>(sp + o_first);
+  a.chunk_order = reinterpret_cast<int32_t *>(sp + o_order);
+  a.chunk_count = reinterpret_cast<int32_t *>(sp + o_count);
+  a.item_next = a.chunk_count + 1;
+  a.geo_count = reinterpret_cast<unsigned long long *>(sp + o_count + 16);
+  a.row_cost = reinterpret_cast<float *>(sp + o_rowcost);
+  a.chunk_cost = reinterpret_cast<float *>(sp + o_chunkcost);
+  uint8_t *sb = sp + o_state;
   a.row_has_eval = sb; a.row_last_top = sb + n_rows; a.row_entry_top = sb + 2 * n_rows;
+  a.n_eg = n_eg;
+  a.EC = EC;
+  a.ctas = ctas;
+  a.lgE = reinterpret_cast<double *>(sp + o_lgE);
+  a.geo = reinterpret_cast<double *>(sp + o_geo);
+  a.geo_cap = geo_cap;
+  a.row_info = reinterpret_cast<xg::RowInfo *>(sp + o_info);
+  a.table2d = table2d;
   a.member_status = d->mesh_status;
   a.flux = d->flux;
   a.flop_counter = d->flop_counter;
-  a.slab = d->atmos.intensity != nullptr && !table2d ? dslab.as<double>() : nullptr;
-  a.wsum = use_w ? dwsum.as<unsigned char>() : nullptr;
+  a.slab = tab4 ? reinterpret_cast<double *>(sp + o_slab) : nullptr;
+  a.wsum = use_w ? sp + o_wsum : nullptr;
   a.w_cap = w_cap;
-  a.w_slots = w_slots;
-  a.w_slot_busy = use_w ? dwbusy.as<int32_t>() : nullptr;
   a.mixed = mixed;
   xg::launch_integrate(a, st);
   CK(cudaGetLastError());

@@ -5,7 +5,8 @@
 // atmospheres.
 //
 // Work decomposition (one CTA per chunk of consecutive parallels of one mesh):
-//   1. leaf geometry, one thread per leaf pair (k, N_L-1-k): image deflection,
+//   1. leaf geometry, in a pre-pass with a CTA per parallel, one thread per leaf
+//      pair (k, N_L-1-k): image deflection,
 //      cos alpha / lag / d cos alpha from the Steffen ray tables, Doppler and
 //      aberration factors (:342-441);
 //   2. one thread runs the sequential visibility state machine that fills the
@@ -56,6 +57,7 @@ struct RowCtx {
   int S1, N_R, J, IO;
   const double *D, *CA, *LG;  // ray tables of the row
   int jalt;                   // first ray with deflection > pi/2
+  double alt_xmin;            // cos(D[jalt])
   double radius, Grav_z, cos_gamma, sin_gamma, cos_th, sin_th, th_over_pi, beta, Lorentz;
   double maxDefl, cos_i, sin_i, inclination;
   double vec0, vec1;
@@ -75,7 +77,56 @@ struct GeoSmem {
 };
 
 
-// per-leaf geometry, integrator_for_azimuthal_invariance.pyx:342-441
+// v below w, both finite, by the bit patterns (-0 counts as 0): a comparison
+// on the integer pipe (the FP64 pipe takes 64 cycles or more for it)
+__device__ __forceinline__ long long ordered(double v) {
+  const long long b = __double_as_longlong(v);
+  return b < 0 ? -(b & 0x7fffffffffffffffLL) : b;
+}
+// locate() on a table of non-negative values
+__device__ __forceinline__ int locate_bits(const double *x, int n, double v) {
+  const long long vb = __double_as_longlong(v);
+  int lo = 0, hi = n - 1;
+  while (hi > lo + 1) {
+    const int mid = (lo + hi) >> 1;
+    if (__double_as_longlong(x[mid]) > vb) hi = mid; else lo = mid;
+  }
+  return lo;
+}
+
+// knot spacings around interval i of an n-knot table, for steffen_piece's
+// slopes: one table's spacings serve several value tables
+struct SteffenH {
+  double h, hl, hr;
+  bool first, last;
+};
+// steffen_piece() with the spacings given and the values at i - 1 .. i + 2
+// (the same operations)
+__device__ __forceinline__ Cubic steffen_from(const SteffenH &g, double x0, double ym, double y0,
+                                              double y1, double y2) {
+  const double s = (y1 - y0) / g.h;
+  auto slope = [](double sl, double sr, double hl, double hr) {
+    const double p = (sl * hr + sr * hl) / (hl + hr);
+    const double mag = fmin(fabs(sl), fmin(fabs(sr), 0.5 * fabs(p)));
+    return (copysign(1.0, sl) + copysign(1.0, sr)) * mag;
+  };
+  const double d0 = g.first ? s : slope((y0 - ym) / g.hl, s, g.hl, g.h);
+  const double d1 = g.last ? s : slope(s, (y2 - y1) / g.hr, g.h, g.hr);
+  Cubic c;
+  c.x0 = x0;
+  c.y0 = y0;
+  c.k1 = d0;
+  c.k2 = (3.0 * s - 2.0 * d0 - d1) / g.h;
+  c.k3 = (d0 + d1 - 2.0 * s) / (g.h * g.h);
+  return c;
+}
+
+// per-leaf geometry, integrator_for_azimuthal_invariance.pyx:342-441.  The
+// interval of the main table is found once for cos alpha and lag, each
+// table's piece formed once for value and derivative, and the interval of the
+// reversed table on cos(deflection) found from the main one's (its knots are
+// the cosines of the same deflections), so four cosines replace a bisection's
+// ten.
 __device__ void leaf_geometry(const RowCtx &c, int I, int k, int N_L, int leaf_lim,
                               const double *leaves, GeoSmem &g) {
   double cos_psi = c.cos_i * c.cos_th + c.sin_i * c.sin_th * cos(leaves[k]);
@@ -89,20 +140,58 @@ __device__ void leaf_geometry(const RowCtx &c, int I, int k, int N_L, int leaf_l
     sin_psi = sin(psi);
   }
   const int N_R = c.N_R;
-  MainX mx{c.D};
-  AltX ax{c.D, c.jalt};
-  AltY ay{c.CA, c.jalt};
-  const double alt_xmin = cos(c.D[c.jalt]);
   int calc = 0, term = 0;
-  double sin_alpha = 0.0, mu = 0.0, cos_a;
+  double sin_alpha = 0.0, mu = 0.0, cos_a = 0.0, dca = 0.0;
+  int iv = 0;
+  SteffenH hm{};
+  bool alt = false;
   if (psi <= c.maxDefl) {
     if (psi < c.D[0] || psi > c.D[N_R - 1]) {
       term = 1;
     } else {
-      if (psi <= kHalfPi && cos_psi >= alt_xmin)
-        steffen_eval(ax, ay, c.jalt + 1, cos_psi, &cos_a, nullptr);
-      else
-        steffen_eval(mx, ArrY{c.CA}, N_R, psi, &cos_a, nullptr);
+      alt = psi <= kHalfPi && cos_psi >= c.alt_xmin;
+      iv = locate_bits(c.D, N_R, psi);
+      hm.h = c.D[iv + 1] - c.D[iv];
+      hm.first = iv == 0;
+      hm.last = iv + 1 == N_R - 1;
+      if (!hm.first) hm.hl = c.D[iv] - c.D[iv - 1];
+      if (!hm.last) hm.hr = c.D[iv + 2] - c.D[iv + 1];
+      Cubic q;
+      double at;
+      if (alt) {
+        // knots x(t) = cos(D[jalt - t]), t = 0 .. jalt, ascending; x(t) <= cos psi
+        AltX ax{c.D, c.jalt};
+        const int n = c.jalt + 1;
+        const long long v = ordered(cos_psi);
+        int t = min(max(c.jalt - iv - 1, 0), n - 2);
+        double x0 = ax(t), x1 = ax(t + 1);
+        while (t < n - 2 && ordered(x1) <= v) {
+          t++;
+          x0 = x1;
+          x1 = ax(t + 1);
+        }
+        while (t > 0 && ordered(x0) > v) {
+          t--;
+          x1 = x0;
+          x0 = ax(t);
+        }
+        SteffenH ha;
+        ha.h = x1 - x0;
+        ha.first = t == 0;
+        ha.last = t + 1 == n - 1;
+        ha.hl = ha.first ? 1.0 : x0 - ax(t - 1);
+        ha.hr = ha.last ? 1.0 : ax(t + 2) - x1;
+        const int d = c.jalt - t;  // the value table's index of knot t
+        q = steffen_from(ha, x0, ha.first ? 0.0 : c.CA[d + 1], c.CA[d], c.CA[d - 1],
+                         ha.last ? 0.0 : c.CA[d - 2]);
+        at = cos_psi;
+      } else {
+        q = steffen_from(hm, c.D[iv], hm.first ? 0.0 : c.CA[iv - 1], c.CA[iv], c.CA[iv + 1],
+                         hm.last ? 0.0 : c.CA[iv + 2]);
+        at = psi;
+      }
+      cos_a = cubic_eval(q, at);
+      dca = cubic_deriv(q, at);
       sin_alpha = sqrt(1.0 - cos_a * cos_a);
       mu = cos_a * c.cos_gamma;
       if (!are_equal(psi, 0.0)) {
@@ -114,17 +203,13 @@ __device__ void leaf_geometry(const RowCtx &c, int I, int k, int N_L, int leaf_l
     }
   }
   if (calc && !term) {
-    double deriv;
-    if (psi <= kHalfPi && cos_psi >= alt_xmin) {
-      steffen_eval(ax, ay, c.jalt + 1, cos_psi, nullptr, &deriv);
-    } else {
-      steffen_eval(mx, ArrY{c.CA}, N_R, psi, nullptr, &deriv);
-      // the reference's exp(log|deriv| - log|sin psi|), as the quotient
-      // (the same zero, infinite and NaN cases; an ulp apart)
-      deriv = fabs(deriv) / fabs(sin_psi);
-    }
-    double plag;
-    steffen_eval(mx, ArrY{c.LG}, N_R, psi, &plag, nullptr);
+    double deriv = dca;
+    // the reference's exp(log|deriv| - log|sin psi|), as the quotient
+    // (the same zero, infinite and NaN cases; an ulp apart)
+    if (!alt) deriv = fabs(deriv) / fabs(sin_psi);
+    const Cubic ql = steffen_from(hm, c.D[iv], hm.first ? 0.0 : c.LG[iv - 1], c.LG[iv],
+                                  c.LG[iv + 1], hm.last ? 0.0 : c.LG[iv + 2]);
+    const double plag = cubic_eval(ql, psi);
     for (int ks = 0; ks < 2; ks++) {
       if ((0 < k && k < leaf_lim - 1) || (k == 0 && ks == 0) ||
           (k == leaf_lim - 1 && N_L % 2 == 1 && ks == 0) ||
@@ -161,10 +246,10 @@ __device__ void leaf_geometry(const RowCtx &c, int I, int k, int N_L, int leaf_l
 // Returns through g.flags: [0] terminate, [1] no visibility in this image.
 // Tracks the Num4D call-history flag `top` (last evaluated mu*eta above the
 // table's third-to-last mu node) and marks columns whose first energy sees a
-// clamped mu.
+// clamped mu; *first receives the first evaluated leaf.
 __device__ void state_machine(int N_L, int leaf_lim, const double *leaves, GeoSmem &g,
                               bool num4d, double mu_top3, double mu_max, int &top,
-                              int &any_eval) {
+                              int &any_eval, int *first = nullptr) {
   int InvisFlag = 2, InvisPhase = 0;
   double step;
   int term = 0;
@@ -186,6 +271,7 @@ __device__ void state_machine(int N_L, int leaf_lim, const double *leaves, GeoSm
             g.clamp0[kdx] = (a > mu_max && !top) ? 1 : 0;
             top = (a > mu_top3) ? 1 : 0;
           }
+          if (!any_eval && first) *first = kdx;
           any_eval = 1;
         }
       }
@@ -226,54 +312,59 @@ __device__ void state_machine(int N_L, int leaf_lim, const double *leaves, GeoSm
       invis = 1;
     } else {
       for (int m = 1; m < N_L; m++)
-        if (g.phase[m] <= g.phase[m - 1]) { term = 1; break; }
+        if (!(ordered(g.phase[m]) > ordered(g.phase[m - 1]))) { term = 1; break; }
     }
   }
   g.flags[0] = term;
   g.flags[1] = invis;
 }
 
+// the parallel's context, formed by the first warp (the FP64 pipe takes an
+// instruction of every warp in turn, so one warp's worth serves the CTA) into
+// `sc`; false when no cell of it radiates.  Ends with a block barrier.
 __device__ bool load_row(const IntegrateArgs &a, const MemberDesc &M, int64_t row, int i,
-                         RowCtx &c, int *s_J) {
-  // first radiating cell of the parallel (:286-296), found by the first warp
-  const int32_t *rad = a.radiates + M.cell_off + (int64_t)i * M.S1;
+                         RowCtx &c, RowCtx *sc) {
+  // first radiating cell of the parallel (:286-296)
   if (threadIdx.x < 32) {
+    const int32_t *rad = a.radiates + M.cell_off + (int64_t)i * M.S1;
     int best = M.S1;
     for (int j = threadIdx.x; j < M.S1; j += 32)
       if (rad[j] == 1) { best = min(best, j); break; }
     for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (threadIdx.x == 0) *s_J = best;
+    RowCtx r{};
+    r.J = best;
+    r.S1 = M.S1;
+    if (best < M.S1) {
+      r.N_R = a.N_R;
+      r.D = a.deflection + row * a.N_R;
+      r.CA = a.cos_alpha + row * a.N_R;
+      r.LG = a.lag + row * a.N_R;
+      r.jalt = a.N_R - 1;  // set by stage_deflection()
+      r.radius = a.radius[row];
+      r.Grav_z = sqrt(1.0 - a.u[row]);
+      r.cos_gamma = a.cos_gamma[row];
+      r.sin_gamma = sqrt(1.0 - r.cos_gamma * r.cos_gamma);
+      double th = a.theta0[row];
+      r.cos_th = cos(th);
+      r.sin_th = sin(th);
+      r.th_over_pi = th / kPi;
+      r.beta = r.radius * M.omega * r.sin_th / (kC * r.Grav_z);
+      r.Lorentz = sqrt(1.0 - r.beta * r.beta);
+      r.maxDefl = a.maxDeflection[row];
+      r.inclination = M.inclination;
+      r.cos_i = cos(M.inclination);
+      r.sin_i = sin(M.inclination);
+      r.IO = M.image_order_limit > 0 ? M.image_order_limit : (int)ceil(r.maxDefl / kPi);
+      const double *vec = a.params + (M.cell_off + (int64_t)i * M.S1 + best) * a.n_params;
+      r.vec0 = vec[0];
+      r.vec1 = vec[1];
+    }
+    if (threadIdx.x == 0) *sc = r;
   }
   __syncthreads();
-  int J = *s_J;
+  c = *sc;
   __syncthreads();
-  if (J >= M.S1) return false;
-  c.S1 = M.S1;
-  c.N_R = a.N_R;
-  c.J = J;
-  c.D = a.deflection + row * a.N_R;
-  c.CA = a.cos_alpha + row * a.N_R;
-  c.LG = a.lag + row * a.N_R;
-  c.jalt = a.N_R - 1;  // set by stage_deflection()
-  c.radius = a.radius[row];
-  c.Grav_z = sqrt(1.0 - a.u[row]);
-  c.cos_gamma = a.cos_gamma[row];
-  c.sin_gamma = sqrt(1.0 - c.cos_gamma * c.cos_gamma);
-  double th = a.theta0[row];
-  c.cos_th = cos(th);
-  c.sin_th = sin(th);
-  c.th_over_pi = th / kPi;
-  c.beta = c.radius * M.omega * c.sin_th / (kC * c.Grav_z);
-  c.Lorentz = sqrt(1.0 - c.beta * c.beta);
-  c.maxDefl = a.maxDeflection[row];
-  c.inclination = M.inclination;
-  c.cos_i = cos(M.inclination);
-  c.sin_i = sin(M.inclination);
-  c.IO = M.image_order_limit > 0 ? M.image_order_limit : (int)ceil(c.maxDefl / kPi);
-  const double *vec = a.params + (M.cell_off + (int64_t)i * M.S1 + J) * a.n_params;
-  c.vec0 = vec[0];
-  c.vec1 = vec[1];
-  return true;
+  return c.J < M.S1;
 }
 
 // Copy the parallel's deflection table to shared memory (the leaf searches
@@ -286,10 +377,11 @@ __device__ void stage_deflection(RowCtx &c, GeoSmem &g, int *s_jalt) {
   if (threadIdx.x == 0) *s_jalt = N_R - 1;
   __syncthreads();
   for (int t = threadIdx.x; t < N_R - 1; t += blockDim.x)
-    if (g.rD[t] > kHalfPi) atomicMin(s_jalt, t);
+    if (ordered(g.rD[t]) > ordered(kHalfPi)) atomicMin(s_jalt, t);
   __syncthreads();
   c.jalt = *s_jalt;
   c.D = g.rD;
+  c.alt_xmin = cos(c.D[c.jalt]);
   __syncthreads();
 }
 
@@ -434,85 +526,6 @@ __device__ __forceinline__ DF df_scale(DF a, int d) {
   return DF{a.h * f, a.l * f};
 }
 
-// Num4D intensity of the FP64 form from a slab held as double-float pairs
-// whose energy-node columns are scaled by 2^-xe: the same stencils as
-// eval_num4d_e, with the energy coordinate's offset from the stencil base
-// formed in FP64 (as the reference's differences) and the Lagrange products
-// and the 4 x 4 contraction in double-float arithmetic (~2^-48 relative, on
-// the FP32 pipes).  The float pre-tests leave the FP64 comparisons to the
-// grid's ends and to ties of the rounded coordinate.  Returns the stencil
-// sum before the positive part (the caller clamps it at 0), in units of
-// `scale` (the largest of the four nodes' column scales).
-struct MuStencilDF {
-  int b2;
-  DF w2[4];
-};
-__device__ __forceinline__ MuStencilDF mu_stencil_df(const Atmos4D &A, const AtmSmem &as,
-                                                     double mu, bool clamp_mu) {
-  const MuStencil m = mu_stencil(A, as, mu, clamp_mu);
-  MuStencilDF d;
-  d.b2 = m.b2;
-#pragma unroll
-  for (int k = 0; k < 4; k++) d.w2[k] = df_split(m.w2[k]);
-  return d;
-}
-// the contracted table's value at (mu stencil m, v3) as a double-float times
-// 2^xr (xr the largest column exponent of the energy stencil)
-__device__ __forceinline__ DF eval_num4d_dfx(const Atmos4D &A, const AtmSmem &as, const DF *slab,
-                                             const MuStencilDF &m, double v3, int &xr) {
-  const int nE = A.nE;
-  float vf = (float)v3;
-  if (vf <= as.fgE[0] && v3 < as.gE[0]) {
-    v3 = as.gE[0];
-    vf = as.fgE[0];
-  }
-  if (vf >= as.fgE[nE - 1] && v3 > as.gE[nE - 1]) {
-    v3 = as.gE[nE - 1];
-    vf = as.fgE[nE - 1];
-  }
-  // stencil_base_guided with the FP64 step-down tested only where the
-  // rounded node does not lie below the rounded coordinate (g > v implies
-  // fg >= vf, rounding being monotone)
-  int lo = 0, hi = nE - 1;
-  while (hi > lo + 1) {
-    const int mid = (lo + hi) >> 1;
-    if (as.fgE[mid] > vf) hi = mid; else lo = mid;
-  }
-  while (lo > 0 && as.fgE[lo] >= vf && as.gE[lo] > v3) lo--;
-  int b3 = lo - 1;
-  if (b3 < 0) b3 = 0;
-  if (b3 > nE - 4) b3 = nE - 4;
-  const DF u0 = df_split(v3 - as.gE[b3]);
-  const DF *o = as.dgEo + 3 * b3;
-  const DF u1 = df_sub(u0, o[0]), u2 = df_sub(u0, o[1]), u3 = df_sub(u0, o[2]);
-  const DF u01 = df_mul(u0, u1), u23 = df_mul(u2, u3);
-  const DF *S = as.dsE + 4 * b3;
-  // the nodes' column scales relative to the largest of the four (<= 1)
-  const int x0 = as.xe[b3], x1 = as.xe[b3 + 1], x2 = as.xe[b3 + 2], x3 = as.xe[b3 + 3];
-  xr = max(max(x0, x1), max(x2, x3));
-  const DF w3[4] = {df_scale(df_mul(df_mul(u1, u23), S[0]), x0 - xr),
-                    df_scale(df_mul(df_mul(u0, u23), S[1]), x1 - xr),
-                    df_scale(df_mul(df_mul(u01, u3), S[2]), x2 - xr),
-                    df_scale(df_mul(df_mul(u01, u2), S[3]), x3 - xr)};
-  float sh = 0.0f, sl = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const DF *r = slab + (size_t)(m.b2 + k) * nE + b3;
-    float th = 0.0f, tl = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; i++) df_acc_mul(w3[i], r[i], th, tl);
-    df_acc_mul(m.w2[k], df_norm(th, tl), sh, sl);
-  }
-  return df_norm(sh, sl);
-}
-// the same with the factor 2^xr returned as a double
-__device__ __forceinline__ DF eval_num4d_df(const Atmos4D &A, const AtmSmem &as, const DF *slab,
-                                            const MuStencilDF &m, double v3, double &scale) {
-  int xr;
-  const DF v = eval_num4d_dfx(A, as, slab, m, v3, xr);
-  scale = pow2_double(xr);
-  return v;
-}
 // binary exponent x of |f| = m 2^x, m in [0.5, 1), of a nonzero finite float
 // from its bit pattern
 __device__ __forceinline__ int float_exponent(float f) {
@@ -556,44 +569,26 @@ __device__ __forceinline__ void lagrange_wf(const float *P, const float *S, int 
 }
 
 // Num4D intensity in the mixed form: the slab and the Lagrange weights in
-// FP32, the mu stencil formed once per profile column; the energy
-// coordinate v3 = log10 E - log10 Z - log10 E_eff and its offset from the
-// stencil base in FP64, so the weights see the FP32 rounding of an offset of
-// a few grid spacings (~1e-9 absolute) rather than that of the coordinate
-// (~3e-8, the same on every evaluation of a parallel: a systematic shift).
-struct MuStencilF {
-  int b2;
-  float w2[4];
-};
-__device__ __forceinline__ MuStencilF mu_stencil_f(const Atmos4D &A, const AtmSmem &as, float mu,
-                                                   bool clamp_mu) {
-  float v2 = mu;
-  const float mu_hi = as.fgmu[A.nmu - 1];
-  if (v2 > mu_hi && clamp_mu) v2 = mu_hi;
-  if (v2 < as.fgmu[0]) v2 = as.fgmu[0];
-  MuStencilF m;
-  m.b2 = stencil_base_f(as.fgmu, A.nmu, v2);
-  lagrange_wf(as.fgmu, as.fsmu, m.b2, v2, m.w2);
-  return m;
-}
-__device__ __forceinline__ float eval_num4d_f(const Atmos4D &A, const AtmSmem &as,
-                                              const float *slab, const MuStencilF &m, double v3,
-                                              float p3) {
-  if (v3 < as.gE[0]) v3 = as.gE[0];
-  if (v3 > as.gE[A.nE - 1]) v3 = as.gE[A.nE - 1];
-  const int b3 = stencil_base_guided(as.gE, as.fgE, A.nE, v3);
-  const float u = (float)(v3 - as.gE[b3]);
-  const float *o = as.fgEo + 3 * b3;  // node offsets gE[b3 + i] - gE[b3], i = 1..3
+// FP32, the mu stencil (b2, w2) formed once per profile column; the energy
+// coordinate's offset u from the stencil base b3 is the rounding of an exact
+// one, so the weights see the FP32 rounding of an offset of a few grid
+// spacings (~1e-9 absolute) rather than that of the coordinate (~3e-8, the
+// same on every evaluation of a parallel: a systematic shift).
+__device__ __forceinline__ float eval_num4d_f(const float *offs, const float *space, int nE,
+                                              const float *slab, int b2, float4 w2, int b3,
+                                              float u, float p3) {
+  const float *o = offs + 3 * b3;  // node offsets gE[b3 + i] - gE[b3], i = 1..3
   const float d0 = u, d1 = u - o[0], d2 = u - o[1], d3 = u - o[2];
-  const float *S = as.fsE + 4 * b3;
+  const float *S = space + 4 * b3;
   const float w3[4] = {d1 * d2 * d3 * S[0], d0 * d2 * d3 * S[1], d0 * d1 * d3 * S[2],
                        d0 * d1 * d2 * S[3]};
+  const float w[4] = {w2.x, w2.y, w2.z, w2.w};
   float I = 0.0f;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const float *r = slab + (size_t)(m.b2 + k) * A.nE + b3;
+    const float *r = slab + (size_t)(b2 + k) * nE + b3;
     const float t = w3[0] * r[0] + w3[1] * r[1] + w3[2] * r[2] + w3[3] * r[3];
-    I += m.w2[k] * t;
+    I += w[k] * t;
   }
   if (I < 0.0f) return 0.0f;
   return I * p3;
@@ -603,41 +598,37 @@ __device__ __forceinline__ float eval_bb_f(float E, float kT) {
   return E * E * E / expm1f(E / kT);
 }
 
+// energies per chunk: as many as keep every thread in the per-cell sums and the
+// coefficients within 96 KB
+__host__ __device__ inline int energy_chunk(int N_L, int N_P, int N_E, int piece_bytes) {
+  int ec = 8;
+  while (ec < 32 && (long)N_P * (ec * 2 / kEPT) <= kThreads && ec * 2 <= N_E + kEPT) ec *= 2;
+  while (ec > 8 && (size_t)ec * N_L * piece_bytes > 96 * 1024) ec /= 2;
+  return ec;
+}
+
 struct Layout {
   int N_L, EC, nmu, nE;
   size_t bytes;
 };
 
-// the coefficients' area: rows (PieceRows) has one energy slot more per knot
-// and also holds the staged deflection table while an image's leaf geometry
-// runs (the pieces are formed after it), so that two CTAs fit an SM
-__host__ __device__ inline size_t coef_bytes(int ec, int N_L, int piece_bytes, int N_R,
-                                             bool rows) {
-  const size_t c = (size_t)(ec + (rows ? 1 : 0)) * N_L * piece_bytes;
-  const size_t d = ((size_t)N_R * sizeof(double) + 15) & ~size_t(15);
-  return rows && d > c ? d : c;
-}
-
 // nmu, nE: Num4D grid sizes (0 when no mesh uses the numerical atmosphere)
 __host__ __device__ inline Layout make_layout(int N_L, int N_P, int N_E, int nmu = 0,
-                                              int nE = 0, int piece_bytes = 32, int N_R = 0,
-                                              bool rows = false) {
+                                              int nE = 0, int piece_bytes = 32, int N_R = 0) {
   Layout L;
   L.N_L = N_L;
   L.nmu = nmu;
   L.nE = nE;
-  int ec = 8;
-  while (ec < 32 && (long)N_P * (ec * 2 / kEPT) <= kThreads && ec * 2 <= N_E + kEPT) ec *= 2;
-  while (ec > 8 && (size_t)ec * N_L * piece_bytes > 96 * 1024) ec /= 2;
+  const int ec = energy_chunk(N_L, N_P, N_E, piece_bytes);
   L.EC = ec;
   L.bytes = (size_t)5 * N_L * sizeof(double)      // phase, leafphase, Z, ABB, GEOM
-            + coef_bytes(ec, N_L, piece_bytes, N_R, rows)
+            + (size_t)ec * N_L * piece_bytes       // coefficients
             + (size_t)(nmu + nE) * 5 * sizeof(double)  // Num4D grids + inverse denominators
             + (size_t)(nmu + nE) * 5 * sizeof(float)   // their FP32 copies (mixed form)
             + (size_t)3 * nE * sizeof(float)           // energy-grid node offsets (mixed)
             + (size_t)nE * sizeof(int)                 // slab column exponents (FP64 form)
             + (size_t)(5 * N_L + 4 * kMaxCellsF + kMaxEnergiesF) * sizeof(float)
-            + (size_t)(rows ? 0 : N_R) * sizeof(double)  // staged deflection table
+            + (size_t)N_R * sizeof(double)  // staged deflection table
             + (size_t)(ec + N_L) * sizeof(double)  // lgE, lzs
             + (size_t)2 * N_L * sizeof(DF)         // ih, ih2
             + (size_t)(4 * N_L + 8 + ec) * sizeof(int) + 64;
@@ -645,18 +636,17 @@ __host__ __device__ inline Layout make_layout(int N_L, int N_P, int N_E, int nmu
 }
 
 // bytes carve() takes with no coefficients and no atmosphere arrays (the
-// Num4D pre-pass)
+// geometry pre-pass)
 inline size_t geometry_bytes(int N_L, int N_R) {
   return (size_t)N_R * sizeof(double) + (size_t)8 * N_L * sizeof(double) + 16 /* alignment */ +
          (size_t)(4 * N_L + 8) * sizeof(int) + 16;
 }
 
 __device__ GeoSmem carve(char *base, int N_L, int EC, double **coef, int nmu = 0, int nE = 0,
-                         AtmSmem *atm = nullptr, int piece_bytes = 32, int N_R = 0,
-                         bool rows = false) {
+                         AtmSmem *atm = nullptr, int piece_bytes = 32, int N_R = 0) {
   GeoSmem g;
   double *d = reinterpret_cast<double *>(base);
-  g.rD = d; d += rows ? 0 : N_R;
+  g.rD = d; d += N_R;
   g.phase = d; d += N_L;
   g.leafphase = d; d += N_L;
   g.Z = d; d += N_L;
@@ -667,9 +657,7 @@ __device__ GeoSmem carve(char *base, int N_L, int EC, double **coef, int nmu = 0
   g.ih = reinterpret_cast<DF *>(d); d += N_L;
   g.ih2 = reinterpret_cast<DF *>(d); d += N_L;
   d = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(d) + 15) & ~uintptr_t(15));
-  *coef = d;
-  if (rows) g.rD = d;
-  d += coef_bytes(EC, N_L, piece_bytes, N_R, rows) / 8;
+  *coef = d; d += (size_t)EC * N_L * piece_bytes / 8;
   if (atm) {
     atm->gmu = d; d += nmu;
     atm->gE = d; d += nE;
@@ -710,46 +698,131 @@ __device__ GeoSmem carve(char *base, int N_L, int EC, double **coef, int nmu = 0
 }
 
 // ---------------------------------------------------------------------------
-// Pre-pass for Num4D: per parallel, does it evaluate the atmosphere, and does
-// its last evaluation leave the mu stencil at the top of the table?
+// Geometry pre-pass, one CTA per parallel: its images' leaf geometry and
+// visibility, once, into a record per image that the integrator's CTAs read
+// (however many share the parallel's energies), and for the table
+// atmospheres whether the parallel evaluates the atmosphere and whether its
+// last evaluation leaves the mu stencil at the top of the table.  The work is
+// FP64 (trigonometry, the Steffen pieces, a serial walk over the leaves):
+// here many parallels' CTAs share an SM and keep the pipe busy, in the
+// integrator two of a CTA's warps ran it and the rest waited.
+//
+// Record of an image, per profile column: the knot's phase, 1 / redshift
+// factor Z, cosine mu eta, geometric factor (doubles, [N_L] each), then a
+// byte: kColLit the column carries a leaf's radiation (else it is dark and
+// the three values are undefined), kColClamp its first energy sees the mu
+// clamp, kColFirst it is the parallel's first evaluation.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) num4d_prepass_kernel(IntegrateArgs a) {
+constexpr unsigned kColLit = 1, kColClamp = 2, kColFirst = 4;
+constexpr int kImgTerm = 1 << 30;  // the image after the parallel's records is the terminate
+
+__host__ __device__ inline int64_t image_doubles(int N_L) { return 4 * (int64_t)N_L + (N_L + 7) / 8; }
+
+// one image of the parallel by the whole CTA: leaf geometry, state machine
+// and, when it is visible, the record (rec, or none when null).  s[0], s[1], s[2]: the mu stencil's top
+// state, any evaluation so far, the parallel's first evaluated leaf.  Returns
+// 0 visible, 1 not visible, 2 terminate.  Ends with a block barrier.
+__device__ int image_record(const RowCtx &c, int I, int N_L, const double *leaves, GeoSmem &g,
+                            bool table, double mu_top3, double mu_max, int *s, int *s_z,
+                            double *rec) {
+  const int leaf_lim = (N_L % 2 == 0) ? N_L / 2 : (N_L + 1) / 2;
+  for (int k = threadIdx.x; k < leaf_lim; k += blockDim.x)
+    leaf_geometry(c, I, k, N_L, leaf_lim, leaves, g);
+  __syncthreads();
+  const bool before = s[1] != 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int top = s[0], any = s[1], first = s[2];
+    state_machine(N_L, leaf_lim, leaves, g, table, mu_top3, mu_max, top, any, &first);
+    s[0] = top;
+    s[1] = any;
+    s[2] = first;
+  }
+  __syncthreads();
+  const int out = g.flags[0] ? 2 : (g.flags[1] ? 1 : 0);
+  if (out == 0) {
+    uint8_t *fl = reinterpret_cast<uint8_t *>(rec + 4 * (size_t)N_L);
+    float zlo = INFINITY, zhi = 0.0f;
+    for (int t = threadIdx.x; t < N_L; t += blockDim.x) {
+      const int q = g.src[t];
+      if (rec) rec[t] = g.phase[t];
+      unsigned f = 0;
+      if (q >= 0) {
+        if (rec) {
+          rec[N_L + t] = g.Z[q];
+          rec[2 * N_L + t] = g.ABB[q];
+          rec[3 * N_L + t] = g.GEOM[q];
+        }
+        zlo = fminf(zlo, (float)g.Z[q]);
+        zhi = fmaxf(zhi, (float)g.Z[q]);
+        f = kColLit | ((table && g.clamp0[q]) ? kColClamp : 0u) |
+            ((!before && q == s[2]) ? kColFirst : 0u);
+      }
+      if (rec) fl[t] = (uint8_t)f;
+    }
+    if (s_z) {  // the lit columns' smallest and largest Z (positive floats order as ints)
+      atomicMin(&s_z[0], __float_as_int(zlo));
+      atomicMax(&s_z[1], __float_as_int(zhi));
+    }
+  }
+  __syncthreads();
+  return out;
+}
+
+__global__ void __launch_bounds__(128) geometry_kernel(IntegrateArgs a) {
   extern __shared__ __align__(16) char smem[];
   const int64_t row = blockIdx.x;
   const int m = a.row_member[row];
   const MemberDesc M = a.members[m];
   const int i = (int)(row - M.row_off);
   const int N_L = a.N_L;
-  const int leaf_lim = (N_L % 2 == 0) ? N_L / 2 : (N_L + 1) / 2;
   double *coef;
   GeoSmem g = carve(smem, N_L, 0, &coef, 0, 0, nullptr, 32, a.N_R);
-  __shared__ int s_J, s_any, s_top, s_jalt;
+  __shared__ RowCtx s_row;
+  __shared__ int s_jalt, s_state[3], s_z[2];
+  __shared__ long long s_base;
   RowCtx c;
-  if (threadIdx.x == 0) { s_any = 0; s_top = 0; }
-  if (!load_row(a, M, row, i, c, &s_J)) {
-    if (threadIdx.x == 0) { a.row_has_eval[row] = 0; a.row_last_top[row] = 0; }
-    return;
+  if (threadIdx.x == 0) {
+    s_state[0] = s_state[1] = s_state[2] = 0;
+    s_z[0] = __float_as_int(INFINITY);
+    s_z[1] = 0;
+    s_base = -1;
   }
-  stage_deflection(c, g, &s_jalt);
-  const double mu_max = a.atmos.mu[a.atmos.nmu - 1], mu_top3 = a.atmos.mu[a.atmos.nmu - 3];
-  for (int I = 0; I < c.IO; I++) {
-    for (int k = threadIdx.x; k < leaf_lim; k += blockDim.x)
-      leaf_geometry(c, I, k, N_L, leaf_lim, a.leaves, g);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int top = s_top, any = s_any;
-      state_machine(N_L, leaf_lim, a.leaves, g, true, mu_top3, mu_max, top, any);
-      s_top = top;
-      s_any = any;
+  const bool lit = load_row(a, M, row, i, c, &s_row);
+  int n = 0;
+  if (lit) {
+    if (threadIdx.x == 0 && a.geo) {
+      const long long b = (long long)atomicAdd(a.geo_count, (unsigned long long)c.IO);
+      s_base = b + c.IO <= a.geo_cap ? b : -1;
     }
-    __syncthreads();
-    int stop = g.flags[0] | g.flags[1];
-    __syncthreads();
-    if (stop) break;
+    stage_deflection(c, g, &s_jalt);
+    const bool table = a.atmos.I != nullptr;
+    const double mu_max = table ? a.atmos.mu[a.atmos.nmu - 1] : 0.0;
+    const double mu_top3 = table ? a.atmos.mu[a.atmos.nmu - 3] : 0.0;
+    for (int I = 0; I < c.IO; I++) {
+      // (without room for the parallel's images the integrator forms them again)
+      double *rec = s_base >= 0 ? a.geo + (s_base + I) * image_doubles(N_L) : nullptr;
+      const int got = image_record(c, I, N_L, a.leaves, g, table, mu_top3, mu_max, s_state, s_z,
+                                   rec);
+      if (got == 0) { n++; continue; }
+      if (got == 2) n |= kImgTerm;
+      break;
+    }
   }
   if (threadIdx.x == 0) {
-    a.row_has_eval[row] = (uint8_t)s_any;
-    a.row_last_top[row] = (uint8_t)s_top;
+    if (a.row_has_eval) {
+      a.row_has_eval[row] = (uint8_t)s_state[1];
+      a.row_last_top[row] = (uint8_t)s_state[0];
+    }
+    if (a.row_info) {
+      RowInfo r;
+      r.geo = s_base;
+      r.images = n;
+      r.cell = c.J;
+      r.z_lo = __int_as_float(s_z[0]);
+      r.z_hi = __int_as_float(s_z[1]);
+      a.row_info[row] = r;
+    }
   }
 }
 
@@ -1129,23 +1202,18 @@ __device__ __forceinline__ void lead_acc(float a, float b, float &s, float &x) {
 // instructions and loses two bits.)  flags[2 iv]: energies of interval iv that are
 // not of class 1; flags[2 iv + 1]: those of them that add nothing; a run none
 // of whose energies adds anything is dropped when it is staged.
-template <typename CP, typename AR>
-__device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_t *rad,
-                                      const WRuns &w, int n0, int n1, int k, int EC, int ne,
-                                      const PieceRows &pc, const uint32_t *flags,
-                                      RunStage *stages, bool add_all) {
-  const int lane = threadIdx.x & 31, e = threadIdx.x % EC, sub = lane / EC;
-  RunStage &st = stages[threadIdx.x / EC];
-  const uint32_t lit = ne == 32 ? 0xffffffffu : ((1u << ne) - 1u);
-  float s = 0.0f, c = 0.0f;
-  DF walked{0.0f, 0.0f};
-  const int n = n0 + n1;
-  const int n_max = __reduce_max_sync(0xffffffffu, n);
-  const size_t f0 = w.first(k, 0), f1 = w.first(k, 1) - n0;
+// (n0, n1: the run counts of phase k's two halves; k2, m0, m1: the same of
+// the group's next phase, whose first block is fetched while the last one of
+// this phase is used)
+struct RunFetch {
   float4 v[2];
   int mt = 0;
-  // lane e of the group loads half a record (EC = 8: two halves)
-  auto fetch = [&](int b) {
+  // records b .. b + kStage - 1 of phase k: lane e of the group loads half a
+  // record (EC = 8: two halves) and, the first kStage lanes, its int
+  __device__ __forceinline__ void fetch(const WRuns &w, int k, int n0, int n1, int b, int e,
+                                        int EC) {
+    const int n = n0 + n1;
+    const size_t f0 = w.first(k, 0), f1 = w.first(k, 1) - n0;
 #pragma unroll
     for (int z = 0; z < 2; z++) {
       const int h = e + z * EC, i = b + (h >> 1);
@@ -1154,23 +1222,38 @@ __device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_
     }
     const int i = b + e;
     if (e < kStage && i < n) mt = w.meta[(i < n0 ? f0 : f1) + i];
-  };
-  fetch(0);
+  }
+};
+template <typename CP, typename AR>
+__device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_t *rad,
+                                      const WRuns &w, int k, int n0, int n1, int k2, int m0,
+                                      int m1, int EC, int ne, const PieceRows &pc,
+                                      const uint32_t *flags, RunStage *stages, bool add_all,
+                                      RunFetch &rf) {
+  const int lane = threadIdx.x & 31, e = threadIdx.x % EC, sub = lane / EC;
+  RunStage &st = stages[threadIdx.x / EC];
+  const uint32_t lit = ne == 32 ? 0xffffffffu : ((1u << ne) - 1u);
+  float s = 0.0f, c = 0.0f;
+  DF walked{0.0f, 0.0f};
+  const int n = n0 + n1;
+  const int n_max = __reduce_max_sync(0xffffffffu, n);
+  if (n_max == 0) rf.fetch(w, k2, m0, m1, 0, e, EC);
   for (int b = 0; b < n_max; b += kStage) {
     __syncwarp();  // the last block's readers are done
     bool alive = false;
-    if (e < 2 * kStage) st.w[e] = v[0];
-    if (EC < 2 * kStage) st.w[e + EC] = v[1];
+    if (e < 2 * kStage) st.w[e] = rf.v[0];
+    if (EC < 2 * kStage) st.w[e + EC] = rf.v[1];
     if (e < kStage && b + e < n) {
-      const int iv = mt & 1023;
+      const int iv = rf.mt & 1023;
       const uint2 fl = *reinterpret_cast<const uint2 *>(flags + 2 * iv);
-      st.meta[e] = make_uint4((uint32_t)mt, fl.x, fl.y, 0u);
+      st.meta[e] = make_uint4((uint32_t)rf.mt, fl.x, fl.y, 0u);
       alive = (fl.x & fl.y & lit) != lit;
     }
     uint32_t todo = __ballot_sync(0xffffffffu, alive) >> (sub * EC);
     todo &= (1u << kStage) - 1u;
     __syncwarp();
-    if (b + kStage < n) fetch(b + kStage);
+    if (b + kStage < n_max) rf.fetch(w, k, n0, n1, b + kStage, e, EC);
+    else rf.fetch(w, k2, m0, m1, 0, e, EC);
     // two runs at a time (the last may be the empty record): their chains are
     // independent, and the groups of the warp stay together
     while (__any_sync(0xffffffffu, todo != 0u)) {
@@ -1269,8 +1352,216 @@ __device__ double beamed_intensity(int opt, const double *b, double E, double mu
 }
 
 // ---------------------------------------------------------------------------
-// main integrator kernel: one CTA per chunk of parallels of one mesh
+// double <-> float-pair conversions on the integer pipe.  A conversion
+// instruction between the two widths takes the FP64 pipe as long as a DFMA
+// (64 cycles or more per warp), and a split is four FP64 instructions, a
+// joined and scaled pair four; these are about fifteen integer ones.
 // ---------------------------------------------------------------------------
+// df_split(v 2^e) (ties of the high part aside, which split the same value)
+__device__ __forceinline__ DF df_split_bits(double v, int e) {
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  const int ev = (hi >> 20) & 0x7ff, E = ev - 1023 + e;
+  if (ev == 0 || ev == 0x7ff || E < -70 || E > 120) {
+    if ((hi & 0x7fffffff) == 0 && lo == 0) return DF{0.0f, 0.0f};
+    return df_split(scale_pow2(v, e));
+  }
+  int top = ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29);
+  int r = lo & 0x1fffffff;
+  if (r & 0x10000000) {
+    top += 1;
+    r -= 0x20000000;
+  }
+  const int sign = hi & 0x80000000;
+  DF d;
+  d.h = __int_as_float((((E + 127) << 23) + top) | sign);
+  d.l = (float)r * __int_as_float(((E - 52 + 127) << 23) | sign);
+  return d;
+}
+// df_value(a) 2^e, rounded once to a double (|a.l| at most half an ulp of a.h)
+__device__ __forceinline__ double df_join_bits(DF a, int e) {
+  const int hb = __float_as_int(a.h), eh = ((hb >> 23) & 0xff) - 127;
+  const int ex = eh + e;
+  if (eh < -60 || eh > 100 || ex < -1020 || ex > 1020) {
+    if (a.h == 0.0f) return 0.0;
+    return scale_pow2(df_value(a), e);
+  }
+  // in units of 2^(eh - 52): the high part's 24 bits and the low part rounded
+  const int li = __float2int_rn(a.l * __int_as_float((52 - eh + 127) << 23));
+  const bool neg = hb < 0;
+  long long m = ((long long)((hb & 0x7fffff) | 0x800000) << 29) + (neg ? -li : li);
+  int x = ex;
+  if (m < (1ll << 52)) {
+    m <<= 1;
+    x -= 1;
+  }
+  const long long bits = ((long long)(x + 1023) << 52) + (m - (1ll << 52));
+  return __longlong_as_double(neg ? bits | (long long)0x8000000000000000ull : bits);
+}
+
+// Energy coordinates log10 E as 64-bit integers in units of 2^-54: the
+// differences log10 E - log10 Z - log10 E_eff - node are exact, on the integer
+// pipe (in FP64 each rounds at 2^-52 and takes the FP64 pipe seven
+// instructions per column value, comparisons and conversions included).
+constexpr double kFix = 18014398509481984.0;  // 2^54
+__device__ __forceinline__ long long fix_of(double v) { return __double2ll_rn(v * kFix); }
+// u / 2^54 as a float pair
+__device__ __forceinline__ DF fix_df(long long u) {
+  const int uh = (int)(u >> 32);
+  if (uh >= (1 << 24) || uh < -(1 << 24)) return df_split((double)u * (1.0 / kFix));
+  const unsigned ul = (unsigned)u;
+  constexpr float s32 = 0x1p-22f, s16 = 0x1p-38f, s0 = 0x1p-54f;
+  // three exact pieces; fast_two_sum's condition holds for the first two (the
+  // high one is 0 or at least 2^-22)
+  const DF a = fast_two_sum((float)uh * s32, (float)(ul >> 16) * s16);
+  return fast_two_sum(a.h, __fadd_rn(a.l, (float)(ul & 0xffffu) * s0));
+}
+// the base node of the 4-point stencil around v on an ascending grid of n
+// nodes, and lo the largest node index <= n - 2 at or below v (0 below the
+// grid); lo < 0 on entry: unknown, else a walk from it
+__device__ __forceinline__ int stencil_base_fix(const long long *g, int n, long long v, int &lo) {
+  if (lo < 0) {
+    lo = 0;
+    int hi = n - 1;
+    while (hi > lo + 1) {
+      const int mid = (lo + hi) >> 1;
+      if (g[mid] > v) hi = mid; else lo = mid;
+    }
+  } else {
+    while (lo < n - 2 && g[lo + 1] <= v) lo++;
+    while (lo > 0 && g[lo] > v) lo--;
+  }
+  return min(max(lo - 1, 0), n - 4);
+}
+
+// Num4D intensity of the FP64 form from a slab held as double-float pairs
+// whose energy-node columns are scaled by 2^-xe: the reference's stencils,
+// with the energy coordinate's offset u from the stencil's base node b3 exact
+// and the Lagrange products and the 4 x 4 contraction in double-float
+// arithmetic (~2^-48 relative, on the FP32 pipes).  Returns the stencil sum
+// before the positive part (the caller clamps it at 0) as a double-float
+// times 2^xr (xr the largest column exponent of the energy stencil).
+struct EGrid {
+  const DF *o, *s;  // offsets g[b + i] - g[b] (i = 1..3) and inverse Lagrange denominators
+  const int *xe;
+  int nE;
+};
+__device__ __forceinline__ DF eval_num4d_dfx(const EGrid &E, const DF *slab, int b2, const DF *w2,
+                                             int b3, DF u0, int &xr) {
+  const DF *o = E.o + 3 * b3;
+  const DF u1 = df_sub(u0, o[0]), u2 = df_sub(u0, o[1]), u3 = df_sub(u0, o[2]);
+  const DF u01 = df_mul(u0, u1), u23 = df_mul(u2, u3);
+  const DF *S = E.s + 4 * b3;
+  // the nodes' column scales relative to the largest of the four (<= 1)
+  const int x0 = E.xe[b3], x1 = E.xe[b3 + 1], x2 = E.xe[b3 + 2], x3 = E.xe[b3 + 3];
+  xr = max(max(x0, x1), max(x2, x3));
+  const DF w3[4] = {df_scale(df_mul(df_mul(u1, u23), S[0]), x0 - xr),
+                    df_scale(df_mul(df_mul(u0, u23), S[1]), x1 - xr),
+                    df_scale(df_mul(df_mul(u01, u3), S[2]), x2 - xr),
+                    df_scale(df_mul(df_mul(u01, u2), S[3]), x3 - xr)};
+  float sh = 0.0f, sl = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const DF *r = slab + (size_t)(b2 + k) * E.nE + b3;
+    float th = 0.0f, tl = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) df_acc_mul(w3[i], r[i], th, tl);
+    df_acc_mul(w2[k], df_norm(th, tl), sh, sl);
+  }
+  return df_norm(sh, sl);
+}
+
+// ---------------------------------------------------------------------------
+// main integrator kernel
+// ---------------------------------------------------------------------------
+// shared memory of the integrator, in order (offsets for the launch, pointers
+// in the kernel)
+struct IntSmem {
+  char *piece;  // the chunk's pieces; the leaf geometry's arrays where a CTA forms it itself
+  double *Z, *abb, *geom;          // per profile column
+  long long *lz;                   // log10 Z + log10 E_eff in units of 2^-54
+  double *lzd;                     // 2-D tables: log10 Z, or Z (E in electron rest energies)
+  DF *ih, *ih2;                    // 1 / h and 1 / h^2 of the phase intervals (FP64 form)
+  DF *mw;                          // [4] mu stencil weights per column (FP64 form, 4-D table)
+  float4 *mwf;                     // the same (mixed form)
+  DF *cfm;                         // norm 10^(3 log T) GEOM as mantissa and exponent
+  int *cfx, *mb, *flag;            // exponent; mu stencil base; kCol* bits
+  float *fphase, *fphase_lo, *fh, *finvZ, *fgeom;
+  double *gmu, *smu, *gE, *sE;     // grids and inverse Lagrange denominators
+  long long *gEi;                  // energy grid in units of 2^-54
+  DF *dgEo, *dsE;
+  float *fgmu, *fgE, *fsmu, *fsE, *fgEo;
+  int *xe;
+  float *fcphi, *fcphi_lo, *fcarea, *fcarea_lo;
+  long long *lgE;                  // the chunk's log10 E in units of 2^-54
+  double *lgEd;                    // 2-D tables: log10 E, or E
+  int *sc_exp;
+  uint32_t *flags;
+  int *nruns;
+  float2 *phase;
+  RunStage *stages;
+  size_t bytes;
+};
+template <bool kMixed>
+__host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC, int nmu, int nE,
+                                            bool tab2) {
+  IntSmem o{};
+  size_t at = 0;
+  auto take = [&](auto *&p, size_t n) {
+    using T = std::remove_reference_t<decltype(*p)>;
+    at = (at + 15) & ~size_t(15);
+    p = reinterpret_cast<T *>(base + at);
+    at += n * sizeof(T);
+  };
+  const size_t pieces = kMixed ? (size_t)EC * N_L * sizeof(PieceT<float>)
+                               : (size_t)2 * (EC + 1) * N_L * sizeof(float4);
+  const size_t geo = (size_t)N_L * 8 * sizeof(double) + (size_t)(4 * N_L + 8) * sizeof(int) + 64;
+  take(o.piece, pieces > geo ? pieces : geo);
+  take(o.Z, N_L); take(o.abb, N_L); take(o.geom, N_L);
+  const bool tab4 = nE > 0 && !tab2;
+  if (tab4) take(o.lz, N_L);
+  if (tab2) take(o.lzd, N_L);
+  if (!kMixed) { take(o.ih, N_L); take(o.ih2, N_L); }
+  if (tab4 && !kMixed) { take(o.mw, 4 * N_L); take(o.cfm, N_L); take(o.cfx, N_L); }
+  if (tab4 && kMixed) take(o.mwf, N_L);
+  if (tab4) take(o.mb, N_L);
+  take(o.flag, N_L);
+  take(o.fphase, N_L); take(o.fphase_lo, N_L);
+  if (kMixed) { take(o.fh, N_L); take(o.finvZ, N_L); take(o.fgeom, N_L); }
+  if (nE > 0) { take(o.gmu, nmu); take(o.smu, 4 * nmu); take(o.fgmu, nmu); }
+  if (tab2) { take(o.gE, nE); take(o.sE, 4 * nE); take(o.fgE, nE); }
+  if (tab4) take(o.gEi, nE);
+  if (tab4 && !kMixed) { take(o.dgEo, 3 * nE); take(o.dsE, 4 * nE); take(o.xe, nE); }
+  if (tab4 && kMixed) { take(o.fsmu, 4 * nmu); take(o.fsE, 4 * nE); take(o.fgEo, 3 * nE); }
+  take(o.fcphi, kMaxCellsF); take(o.fcphi_lo, kMaxCellsF);
+  take(o.fcarea, kMaxCellsF); take(o.fcarea_lo, kMaxCellsF);
+  if (tab4) take(o.lgE, EC);
+  if (tab2) take(o.lgEd, EC);
+  take(o.sc_exp, EC);
+  take(o.phase, N_P);
+  if (!kMixed) {
+    take(o.flags, 2 * N_L); take(o.nruns, 2 * N_P);
+    take(o.stages, kThreads / EC);
+  }
+  o.bytes = (at + 15) & ~size_t(15);
+  return o;
+}
+
+// a parallel's atmosphere constants, formed by one warp
+struct RowAtm {
+  double vec0, vec1, kT, kT_c, p3, lgE_eff, wT[4], wg[4];
+  int bT, bg;
+};
+
+// One CTA takes items (a chunk of consecutive parallels of one mesh, and one
+// of n_eg groups of its energy chunks) from a shared counter.  Bound: FP32
+// issue and the FP64 pipe about equally, two CTAs of 8 warps per SM (pieces and
+// grids fill half an SM's shared memory).  What FP64 is left per parallel is
+// the table contraction over the reachable energy nodes and, per image, the mu
+// stencils and 1 / h of the knots; energy coordinates are integers, and values
+// change between double and float pair on the integer pipe.  24 vectors at
+// sqrt_num_cells 96 (two Num4D regions, 128 leaves, 128 energies): 30 ms with
+// those in FP64 and the geometry formed here, 16.7 ms now; 100 blackbody spots
+// (64 leaves, 64 energies): 4.7 ms, 1.9 ms now.
 // WT = double: the plain FP64 drop-in.  WT = float: the mixed-precision form
 // (geometry, visibility and knots in FP64; atmosphere, Akima pieces and the
 // cell x phase sums in FP32; per-chunk partials in FP64).
@@ -1278,659 +1569,736 @@ template <typename WT>
 __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a) {
   constexpr bool kMixed = std::is_same<WT, float>::value;
   extern __shared__ __align__(16) char smem[];
-  if ((int)blockIdx.x >= *a.chunk_count) return;
-  const int chunk = a.chunk_order[blockIdx.x];
-  const int64_t r0 = a.chunk_r0[chunk], r1 = a.chunk_r1[chunk];
-  const int m = a.row_member[r0];
-  const MemberDesc M = a.members[m];
-  const int N_L = a.N_L, N_E = a.N_E, N_P = a.N_P;
-  const int leaf_lim = (N_L % 2 == 0) ? N_L / 2 : (N_L + 1) / 2;
+  const int N_L = a.N_L, N_E = a.N_E, N_P = a.N_P, EC = a.EC;
+  const int nmu = a.atmos.I ? a.atmos.nmu : 0, nEt = a.atmos.I ? a.atmos.nE : 0;
   // 2-D tables (atmos.I is [nmu][nE], no 10^(3 log T)): atm 4, Pol_Num2D's
   // I on (mu, log10 E') (hot_Num2D.pyx:187-400); atm 6, a split atmosphere
   // reduced once per call to (mu, E) with E' in electron rest energies
   // (integrator_for_azimuthal_invariance_split.pyx:270-275,457-476)
-  const bool tab2 = (M.atm == 4 || M.atm == 6) && !kMixed;
-  const bool erest = (M.atm == 6);
-  const bool num4d = (M.atm == 2) || tab2;
-  const int nmu = a.atmos.I ? a.atmos.nmu : 0, nEt = a.atmos.I ? a.atmos.nE : 0;
-  const Layout L =
-      make_layout(N_L, N_P, N_E, nmu, nEt, (int)sizeof(PieceT<WT>), a.N_R, !kMixed);
-  const int EC = L.EC;
-  double *coef;
-  AtmSmem as{};
-  GeoSmem g = carve(smem, N_L, EC, &coef, nmu, nEt, &as, (int)sizeof(PieceT<WT>), a.N_R, !kMixed);
-  PieceT<WT> *co4 = reinterpret_cast<PieceT<WT> *>(coef);  // mixed form
-  const PieceRows pr{reinterpret_cast<float4 *>(coef),
-                     reinterpret_cast<float4 *>(coef) + (size_t)N_L * (EC + 1), EC + 1};
-  __shared__ int s_J, s_top, s_any, s_jalt;
+  const bool tab2 = a.table2d && !kMixed;
+  const IntSmem sm = int_smem<kMixed>(smem, N_L, N_P, EC, nmu, nEt, a.table2d != 0);
+  PieceT<WT> *co4 = reinterpret_cast<PieceT<WT> *>(sm.piece);  // mixed form
+  const PieceRows pr{reinterpret_cast<float4 *>(sm.piece),
+                     reinterpret_cast<float4 *>(sm.piece) + (size_t)N_L * (EC + 1), EC + 1};
+  __shared__ RowAtm s_ra;
+  __shared__ RowCtx s_row;
+  __shared__ int s_item, s_jalt, s_state[3], s_win[2];
+  __shared__ float s_erange[2];
   // a beaming modification's (abb, bbb, cbb, dbb, nimu) for the parallel
   __shared__ double s_beam[5];
-  // power-sum form (FP64 path with scratch): run counts and areas per (cell
-  // half, signal phase) and the piece classes of the chunk; the run
-  // records live in one of a.w_slots scratch slots, taken for the CTA's
-  // lifetime (at most 2 CTAs per SM are resident, the pool has more slots;
-  // a CTA that finds none after a bounded search runs the per-cell form)
-  __shared__ int s_wslot;
-  bool use_w = !kMixed && a.wsum != nullptr;
-  if (use_w) {
-    if (threadIdx.x == 0) {
-      int got = -1;
-      for (int i = 0; i < 4 * a.w_slots && got < 0; i++) {
-        const int sl = (int)((blockIdx.x + i) % a.w_slots);
-        if (atomicCAS(&a.w_slot_busy[sl], 0, 1) == 0) got = sl;
-      }
-      s_wslot = got;
-    }
-    __syncthreads();
-    use_w = s_wslot >= 0;
-  }
-  // class masks [N_L][2], run counts [2][N_P], the signal phases, staged runs
-  // per group
-  uint32_t *s_flags = reinterpret_cast<uint32_t *>(
-      (reinterpret_cast<uintptr_t>(g.sc_exp + EC) + 7) & ~uintptr_t(7));
-  int *s_nruns = reinterpret_cast<int *>(s_flags + 2 * N_L);
-  // the signal phases as float pairs
-  float2 *s_phase = reinterpret_cast<float2 *>(
-      (reinterpret_cast<uintptr_t>(s_nruns + 2 * N_P) + 15) & ~uintptr_t(15));
-  RunStage *s_stages = reinterpret_cast<RunStage *>(
-      (reinterpret_cast<uintptr_t>(s_phase + N_P) + 15) & ~uintptr_t(15));
-  for (int t = threadIdx.x; t < N_P; t += blockDim.x) {
-    const DF v = df_split(a.phases[t]);
-    s_phase[t] = make_float2(v.h, v.l);
-  }
-  if (use_w)
-    for (int t = threadIdx.x; t < kThreads / EC; t += blockDim.x) {
-      s_stages[t].w[2 * kStage] = s_stages[t].w[2 * kStage + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      s_stages[t].meta[kStage] = make_uint4(0u, 0u, 0u, 0u);
-    }
-  const WRuns wr = use_w ? wruns_of(a.wsum + (size_t)s_wslot *
+  // power-sum form (FP64 path with scratch)
+  const bool use_w = !kMixed && a.wsum != nullptr;
+  const WRuns wr = use_w ? wruns_of(a.wsum + (size_t)blockIdx.x *
                                                  integrate_wsum_bytes_dev(N_P, a.w_cap),
                                     a.w_cap, N_P)
                          : WRuns{};
-  double *slab = nullptr;
-  float *slabf = nullptr;
-  if (num4d) {
-    stage_table_grids(a.atmos, as, nmu, nEt);
-    // the mixed form's FP32 interpolation data
-    if (kMixed) {
-      for (int t = threadIdx.x; t < min(N_E, kMaxEnergiesF); t += blockDim.x)
-        as.fE[t] = (float)a.energies[t];
-      for (int t = threadIdx.x; t < 4 * nmu; t += blockDim.x) as.fsmu[t] = (float)as.smu[t];
-      for (int t = threadIdx.x; t < 4 * nEt; t += blockDim.x) as.fsE[t] = (float)as.sE[t];
-      for (int t = threadIdx.x; t < 3 * nEt; t += blockDim.x) {
-        const int b = t / 3, i = t - 3 * b + 1;
-        as.fgEo[t] = b + i < nEt ? (float)(as.gE[b + i] - as.gE[b]) : 0.0f;
-      }
-    }
-    slab = tab2 ? const_cast<double *>(a.atmos.I) : a.slab + (size_t)chunk * nmu * nEt;
-    slabf = reinterpret_cast<float *>(slab);
-    if (!kMixed && !tab2) {
-      // the energy grid's node offsets and inverse denominators as
-      // double-float pairs for eval_num4d_df (sE converted in place)
-      for (int t = threadIdx.x; t < 3 * nEt; t += blockDim.x) {
-        const int b = t / 3, i = t - 3 * b + 1;
-        as.dgEo[t] = b + i < nEt ? df_split(as.gE[b + i] - as.gE[b]) : DF{0.0f, 0.0f};
-      }
-      for (int t = threadIdx.x; t < 4 * nEt; t += blockDim.x) {
-        const double v = as.sE[t];
-        as.dsE[t] = df_split(v);
-      }
-    }
-    __syncthreads();
-  }
-  if (kMixed && !num4d) {
-    for (int t = threadIdx.x; t < min(N_E, kMaxEnergiesF); t += blockDim.x)
-      as.fE[t] = (float)a.energies[t];
-    __syncthreads();
-  }
-  const double norm = num4d ? kErg / kHKeV : kErg * kPlanck;
-  double *part = a.partial + (size_t)chunk * N_E * N_P;
-  for (int t = threadIdx.x; t < N_E * N_P; t += blockDim.x) part[t] = 0.0;
-  __syncthreads();
-  const double mu_max = num4d ? a.atmos.mu[a.atmos.nmu - 1] : 0.0;
-  const double mu_top3 = num4d ? a.atmos.mu[a.atmos.nmu - 3] : 0.0;
-  const int groups = EC / kEPT;
-  const int ntasks = N_P * groups;
-  // algorithmic FLOPs per (parallel, image), the cost model of the
-  // likelihood path: leaf work N_L (60 + N_E f_atm) and spline work
-  // N_E (30 N_L + C N_P 14), f_atm 12 (blackbody) or 1350 (4-D table)
-  double flops = 0.0;
-  const double f_atm = num4d ? 1350.0 : 12.0;
-
-  for (int64_t row = r0; row < r1; row++) {
-    const int i = (int)(row - M.row_off);
-    RowCtx c;
-    if (!load_row(a, M, row, i, c, &s_J)) continue;
-    stage_deflection(c, g, &s_jalt);
-    if (threadIdx.x == 0) {
-      s_top = num4d ? (int)a.row_entry_top[row] : 0;
-      s_any = 0;
-      // parameters 2-6 of the parallel's first radiating cell
-      if (M.beam_opt > 0) {
-        const double *vec = a.params + (M.cell_off + (int64_t)i * M.S1 + c.J) * a.n_params;
-        for (int b = 0; b < 5; b++) s_beam[b] = vec[2 + b];
-      }
-    }
-    __syncthreads();
-    double E_eff = 0.0, p3 = 0.0;
-    if (tab2) {
-      p3 = 1.0;
-    } else if (num4d) {
-      // contract the (log T, log g) stencil of this parallel once:
-      // slab[mu][logE] = sum_ij w_T[i] w_g[j] table[bT+i][bg+j][mu][logE]
-      double vT = c.vec0, vg = c.vec1;
-      if (vT < a.atmos.logT[0]) vT = a.atmos.logT[0];
-      if (vT > a.atmos.logT[a.atmos.nT - 1]) vT = a.atmos.logT[a.atmos.nT - 1];
-      if (vg < a.atmos.logg[0]) vg = a.atmos.logg[0];
-      if (vg > a.atmos.logg[a.atmos.ng - 1]) vg = a.atmos.logg[a.atmos.ng - 1];
-      const int bT = stencil_base(a.atmos.logT, a.atmos.nT, vT);
-      const int bg = stencil_base(a.atmos.logg, a.atmos.ng, vg);
-      double wT[4], wg[4];
-      lagrange4(a.atmos.logT, bT, vT, wT);
-      lagrange4(a.atmos.logg, bg, vg, wg);
-      const size_t S1t = (size_t)nmu * nEt, S0t = (size_t)a.atmos.ng * S1t;
-      if (kMixed && a.atmos.I32 != nullptr) {
-        // FP32 contraction from the FP32 copy of the table
-        const float *basef = a.atmos.I32 + bT * S0t + bg * S1t;
-        float wTf[4], wgf[4];
-#pragma unroll
-        for (int ii = 0; ii < 4; ii++) {
-          wTf[ii] = (float)wT[ii];
-          wgf[ii] = (float)wg[ii];
+  double *slab = a.slab ? a.slab + (size_t)blockIdx.x * nmu * nEt : nullptr;
+  float *slabf = reinterpret_cast<float *>(slab);
+  const DF *slabd = reinterpret_cast<const DF *>(slab);
+  AtmSmem as{};  // the FP64 stencil functions' view of the grids
+  if (nEt > 0) {
+    as.gmu = sm.gmu; as.smu = sm.smu; as.fgmu = sm.fgmu;
+    as.gE = sm.gE; as.sE = sm.sE; as.fgE = sm.fgE;
+    const double *mu = a.atmos.mu, *lE = a.atmos.logE;
+    for (int t = threadIdx.x; t < nmu; t += blockDim.x) {
+      sm.gmu[t] = mu[t];
+      sm.fgmu[t] = (float)mu[t];
+      if (t <= nmu - 4) {
+        double s4[4];
+        lagrange_space(mu, t, s4);
+        for (int q = 0; q < 4; q++) {
+          sm.smu[4 * t + q] = s4[q];
+          if (kMixed) sm.fsmu[4 * t + q] = (float)s4[q];
         }
-        for (int t = threadIdx.x; t < (int)S1t; t += blockDim.x) {
-          float r = 0.0f;
-#pragma unroll
-          for (int ii = 0; ii < 4; ii++) {
-            const float *q = basef + ii * S0t + t;
-            float u = wgf[0] * __ldg(q) + wgf[1] * __ldg(q + S1t) + wgf[2] * __ldg(q + 2 * S1t) +
-                      wgf[3] * __ldg(q + 3 * S1t);
-            r += wTf[ii] * u;
-          }
-          slabf[t] = r;
-        }
+      }
+    }
+    for (int t = threadIdx.x; t < nEt; t += blockDim.x) {
+      double s4[4] = {0.0, 0.0, 0.0, 0.0};
+      if (t <= nEt - 4) lagrange_space(lE, t, s4);
+      if (a.table2d) {
+        sm.gE[t] = lE[t];
+        sm.fgE[t] = (float)lE[t];
+        for (int q = 0; q < 4; q++) sm.sE[4 * t + q] = s4[q];
       } else {
-        const double *base = a.atmos.I + bT * S0t + bg * S1t;
-        double mx = 0.0;
-        for (int t = threadIdx.x; t < (int)S1t; t += blockDim.x) {
-          double r = 0.0;
-#pragma unroll
-          for (int ii = 0; ii < 4; ii++) {
-            const double *q = base + ii * S0t + t;
-            double u = wg[0] * __ldg(q) + wg[1] * __ldg(q + S1t) + wg[2] * __ldg(q + 2 * S1t) +
-                       wg[3] * __ldg(q + 3 * S1t);
-            r += wT[ii] * u;
-          }
-          if (kMixed) {
-            slabf[t] = (float)r;
-          } else {
-            slab[t] = r;
-            mx = fmax(mx, fabs(r));
-          }
+        sm.gEi[t] = fix_of(lE[t]);
+        for (int q = 0; q < 4; q++) {
+          if (kMixed) sm.fsE[4 * t + q] = (float)s4[q];
+          else sm.dsE[4 * t + q] = df_split(s4[q]);
         }
-        if (!kMixed) {
-          // the FP64 form keeps the slab as double-float pairs, each energy
-          // node's column (all mu) scaled by 2^-xe[e] (exact), xe the binary
-          // exponent of its largest value, so that the pairs keep full
-          // relative precision across the table's exponential tail
-          for (int e = threadIdx.x; e < nEt; e += blockDim.x) as.xe[e] = kZeroExp;
-          __syncthreads();
-          for (int t = threadIdx.x; t < (int)S1t; t += blockDim.x)
-            atomicMax(&as.xe[t % nEt], binary_exponent(slab[t]));
-          __syncthreads();
-          DF *slabd = reinterpret_cast<DF *>(slab);
-          for (int t = threadIdx.x; t < (int)S1t; t += blockDim.x) {
-            const double r = slab[t];
-            slabd[t] = df_split(r * pow2_double(-as.xe[t % nEt]));
-          }
+        for (int q = 0; q < 3; q++) {
+          const double o = t + q + 1 < nEt ? lE[t + q + 1] - lE[t] : 0.0;
+          if (kMixed) sm.fgEo[3 * t + q] = (float)o;
+          else sm.dgEo[3 * t + q] = df_split(o);
         }
       }
-      E_eff = (kKB / kKeV) * pow(10.0, c.vec0);
-      p3 = pow(10.0, 3.0 * vT);
-      __syncthreads();
     }
-    // the FP64 form's double-float slab (energy columns scaled by 2^-xe)
-    const DF *slabd = reinterpret_cast<const DF *>(slab);
-    const double kT = (kKB / kKeV) * pow(10.0, c.vec0);
-    const float kT_f = (float)kT;
-    // mixed form: the FP32 roundings of the constant factors norm and
-    // 10^(3 log T) are undone exactly on the parallel's FP64 partials
-    const float p3f = (float)p3;
-    const double fix = num4d ? (norm * p3) / ((double)(float)norm * (double)p3f)
-                             : norm / (double)(float)norm;
-    const double lg_Eeff = (num4d && !tab2) ? log10(E_eff) : 0.0;
-    // the elsewhere correction's blackbody temperature at the parallel's
-    // first radiating cell (:469-476)
-    const bool corr = !kMixed && a.correction != nullptr;
+  }
+  const EGrid eg4{sm.dgEo, sm.dsE, sm.xe, nEt};
+  for (int t = threadIdx.x; t < N_P; t += blockDim.x) {
+    const DF v = df_split(a.phases[t]);
+    sm.phase[t] = make_float2(v.h, v.l);
+  }
+  if (use_w)
+    for (int t = threadIdx.x; t < kThreads / EC; t += blockDim.x) {
+      sm.stages[t].w[2 * kStage] = sm.stages[t].w[2 * kStage + 1] =
+          make_float4(0.f, 0.f, 0.f, 0.f);
+      sm.stages[t].meta[kStage] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_iv = N_L - 1, strips = (n_iv + kStrip - 1) / kStrip;
+  // energy chunks of equal size, at most EC energies each
+  const int nec = (N_E + EC - 1) / EC, ec = (N_E + nec - 1) / nec;
+  // a thread's profile columns and its share of their energies: with N_L
+  // columns or fewer than threads a column belongs to `parts` threads
+  const int parts = max(1, kThreads / N_L);
+  const int part0 = N_L <= kThreads ? threadIdx.x / N_L : 0;
+  const int col0 = N_L <= kThreads ? (part0 < parts ? (int)threadIdx.x - part0 * N_L : N_L)
+                                   : threadIdx.x;
+  const double mu_max = nEt ? a.atmos.mu[nmu - 1] : 0.0;
+  const double mu_top3 = nEt ? a.atmos.mu[nmu - 3] : 0.0;
+  const bool corr = !kMixed && a.correction != nullptr;
+  constexpr float tp = (float)kTwoPi;
+  const int n_items = *a.chunk_count * a.n_eg;
+
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = atomicAdd(a.item_next, 1);
+    __syncthreads();
+    const int item = s_item;
+    if (item >= n_items) break;
+    const int chunk = a.chunk_order[item / a.n_eg], eg = item % a.n_eg;
+    const int ec_lo = (int)((long long)nec * eg / a.n_eg);
+    const int ec_hi = (int)((long long)nec * (eg + 1) / a.n_eg);
+    const int e_lo = ec_lo * ec, e_hi = min(N_E, ec_hi * ec);
+    const int64_t r0 = a.chunk_r0[chunk], r1 = a.chunk_r1[chunk];
+    const int m = a.row_member[r0];
+    const MemberDesc M = a.members[m];
+    const bool erest = (M.atm == 6);
+    const bool num4d = (M.atm == 2) || tab2;
+    const bool t4 = num4d && !tab2;
+    const double norm = num4d ? kErg / kHKeV : kErg * kPlanck;
     // the plain Num4D columns without beaming or correction keep their
     // intensities as double-float mantissas with exponents up to the row
     // scaling (uniform over the CTA: a chunk is one mesh's rows)
-    const bool dfy = !kMixed && num4d && !tab2 && M.beam_opt == 0 && !corr;
-    const double kT_c =
-        corr ? (kKB / kKeV) *
-                   pow(10.0, a.correction[(M.cell_off + (int64_t)i * M.S1 + c.J) * a.n_correction])
-             : 0.0;
-    const double *cellA = a.cellArea + M.cell_off + (int64_t)i * M.S1;
-    const double *cellPhi = a.phi + M.cell_off + (int64_t)i * M.S1;
-    const int32_t *rad = a.radiates + M.cell_off + (int64_t)i * M.S1;
-    for (int I = 0; I < c.IO; I++) {
-      if (!kMixed && I > 0) {  // the last image's pieces overwrote the staged table
-        for (int t = threadIdx.x; t < a.N_R; t += blockDim.x)
-          g.rD[t] = a.deflection[row * a.N_R + t];
-        __syncthreads();
+    const bool dfy = !kMixed && t4 && M.beam_opt == 0 && !corr;
+    double *part = a.partial + (size_t)chunk * N_E * N_P;
+    // partials: FP64 form [N_P][N_E] (the sums' lanes are energies), mixed [N_E][N_P]
+    for (int t = threadIdx.x; t < N_P * (e_hi - e_lo); t += blockDim.x) {
+      const int k = t / (e_hi - e_lo), e = e_lo + t - k * (e_hi - e_lo);
+      part[kMixed ? (size_t)e * N_P + k : (size_t)k * N_E + e] = 0.0;
+    }
+    if (t4 && warp == 0) {  // the item's range of log10 E
+      float lo = INFINITY, hi = -INFINITY;
+      for (int p = e_lo + lane; p < e_hi; p += 32) {
+        lo = fminf(lo, (float)a.lgE[p]);
+        hi = fmaxf(hi, (float)a.lgE[p]);
       }
-      for (int k = threadIdx.x; k < leaf_lim; k += blockDim.x)
-        leaf_geometry(c, I, k, N_L, leaf_lim, a.leaves, g);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int top = s_top, any = s_any;
-        state_machine(N_L, leaf_lim, a.leaves, g, num4d, mu_top3, mu_max, top, any);
-        s_top = top;
-        s_any = any;
+      for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
       }
-      __syncthreads();
-      const int term = g.flags[0], invis = g.flags[1];
-      if (term) {
-        if (threadIdx.x == 0) {
-          atomicExch(&a.member_status[m], (int)kPulseFail);
-          if (use_w) atomicExch(&a.w_slot_busy[s_wslot], 0);
-        }
-        return;
-      }
-      if (invis) break;
-      // phase knots, cell azimuths and areas as float pairs for the cell x
-      // phase sums (both forms)
-      for (int t = threadIdx.x; t < N_L; t += blockDim.x) {
-        const float hi = (float)g.phase[t];
-        as.fphase[t] = hi;
-        as.fphase_lo[t] = (float)(g.phase[t] - (double)hi);
-      }
-      if (M.S1 <= kMaxCellsF) {
-        for (int t = threadIdx.x; t < M.S1; t += blockDim.x) {
-          const float hi = (float)cellPhi[t];
-          as.fcphi[t] = hi;
-          as.fcphi_lo[t] = (float)(cellPhi[t] - (double)hi);
-          const float ah = (float)cellA[t];
-          as.fcarea[t] = ah;
-          as.fcarea_lo[t] = (float)(cellA[t] - (double)ah);
-        }
-      }
-      if (!kMixed) {
-        for (int t = threadIdx.x; t < N_L - 1; t += blockDim.x) {
-          const double h = g.phase[t + 1] - g.phase[t];
-          g.ih[t] = df_split(1.0 / h);
-          g.ih2[t] = df_split(1.0 / (h * h));
-        }
-      }
-      for (int t = threadIdx.x; t < N_L; t += blockDim.x) {
-        const int sidx = g.src[t];
-        if (sidx >= 0) {
-          if (kMixed) {
-            as.finvZ[sidx] = (float)(1.0 / g.Z[sidx]);
-            as.fabb[sidx] = (float)g.ABB[sidx];
-            as.fgeom[sidx] = (float)g.GEOM[sidx];
-          }
-          if (erest) g.lzs[sidx] = g.Z[sidx];
-          else if (num4d) g.lzs[sidx] = log10(g.Z[sidx]) + lg_Eeff;
-        }
-      }
-      __syncthreads();
-      constexpr float tp = (float)kTwoPi;
-      auto cell_phase = [&](auto cached, int k) {
-        const float2 ph = s_phase[k];
-        return CellPhaseF<decltype(cached)::value>{as.fphase, as.fphase_lo, N_L, as.fphase[0],
-                                   as.fphase[N_L - 1], ph.x, ph.y, tp,
-                                   (float)(kTwoPi - (double)tp), as.fcphi, as.fcphi_lo, cellPhi};
-      };
-      if (use_w) {
-        // the runs of every signal phase, each half of the cells by its own
-        // thread (energy independent: formed once per parallel and image)
-        const int hc = (M.S1 + 1) / 2;
-        const AreaDF<true> ar{as.fcarea, as.fcarea_lo, cellA};
-        for (int t = threadIdx.x; t < 2 * N_P; t += blockDim.x) {
-          const int k = t % N_P, half = t / N_P;
-          const CellPhaseF<true> cp = cell_phase(std::true_type{}, k);
-          const int n = build_runs(cp, ar, half * hc, min(M.S1, (half + 1) * hc), rad, wr, half, k);
-          if (n < 0) {
-            // no cell of the parallel is added at this phase (either half's
-            // failure voids both, as in the per-cell form)
-            atomicExch(&a.member_status[m], (int)kPulseFail);
-          }
-          s_nruns[half * N_P + k] = n;
-        }
-        __syncthreads();
-      }
-      if (threadIdx.x == 0 && a.flop_counter) {
-        int Cr = 0;
-        for (int j = 0; j < M.S1; j++) Cr += (rad[j] == 1);
-        flops += (double)N_L * (60.0 + N_E * f_atm) +
-                 (double)N_E * (30.0 * N_L + (double)Cr * N_P * 14.0);
-      }
+      if (lane == 0) { s_erange[0] = lo; s_erange[1] = hi; }
+    }
+    // algorithmic FLOPs per (parallel, image), the cost model of the
+    // likelihood path: leaf work N_L (60 + N_E f_atm) and spline work
+    // N_E (30 N_L + C N_P 14), f_atm 12 (blackbody) or 1350 (4-D table)
+    double flops = 0.0;
+    const double f_atm = num4d ? 1350.0 : 12.0;
 
-      for (int e0 = 0; e0 < N_E; e0 += EC) {
-        const int ne = min(EC, N_E - e0);
-        if (num4d) {
-          for (int t = threadIdx.x; t < ne; t += blockDim.x)
-            g.lgE[t] = erest ? a.energies[e0 + t] : log10(a.energies[e0 + t]);
-          __syncthreads();
+    for (int64_t row = r0; row < r1; row++) {
+      const RowInfo ri = a.row_info[row];
+      const int images = ri.images & ~kImgTerm;
+      const int i = (int)(row - M.row_off);
+      const double *cellA = a.cellArea + M.cell_off + (int64_t)i * M.S1;
+      const double *cellPhi = a.phi + M.cell_off + (int64_t)i * M.S1;
+      const int32_t *rad = a.radiates + M.cell_off + (int64_t)i * M.S1;
+      if (images > 0) {
+        __syncthreads();  // the last parallel's readers are done
+        if (warp == 0) {
+          const int64_t cell = M.cell_off + (int64_t)i * M.S1 + ri.cell;
+          const double *vec = a.params + cell * a.n_params;
+          const double v0 = vec[0], v1 = vec[1];
+          double vT = v0, vg = v1;
+          if (t4) {
+            if (vT < a.atmos.logT[0]) vT = a.atmos.logT[0];
+            if (vT > a.atmos.logT[a.atmos.nT - 1]) vT = a.atmos.logT[a.atmos.nT - 1];
+            if (vg < a.atmos.logg[0]) vg = a.atmos.logg[0];
+            if (vg > a.atmos.logg[a.atmos.ng - 1]) vg = a.atmos.logg[a.atmos.ng - 1];
+          }
+          // lane by lane the same instructions: the powers 10^(log T), 10^(3
+          // log T), the elsewhere's; the T and g stencils
+          const double pw = pow(10.0, lane == 0 ? v0
+                                      : lane == 1 ? 3.0 * vT
+                                      : (corr ? a.correction[cell * a.n_correction] : 0.0));
+          const double kT = (kKB / kKeV) * __shfl_sync(0xffffffffu, pw, 0);
+          const double p3 = __shfl_sync(0xffffffffu, pw, 1);
+          const double kT_c = (kKB / kKeV) * __shfl_sync(0xffffffffu, pw, 2);
+          if (t4 && lane < 2) {
+            const double *P = lane ? a.atmos.logg : a.atmos.logT;
+            const int n = lane ? a.atmos.ng : a.atmos.nT;
+            const double x = lane ? vg : vT;
+            const int b = stencil_base(P, n, x);
+            double w[4];
+            lagrange4(P, b, x, w);
+            for (int q = 0; q < 4; q++) (lane ? s_ra.wg : s_ra.wT)[q] = w[q];
+            if (lane) s_ra.bg = b; else s_ra.bT = b;
+          }
+          if (lane == 0) {
+            s_ra.vec0 = v0;
+            s_ra.vec1 = v1;
+            s_ra.kT = kT;
+            s_ra.kT_c = corr ? kT_c : 0.0;
+            s_ra.p3 = t4 ? p3 : 1.0;
+            s_ra.lgE_eff = t4 ? log10(kT) : 0.0;
+            s_state[0] = num4d ? (int)a.row_entry_top[row] : 0;
+            s_state[1] = s_state[2] = 0;
+            // parameters 2-6 of the parallel's first radiating cell
+            if (M.beam_opt > 0)
+              for (int b = 0; b < 5; b++) s_beam[b] = vec[2 + b];
+            if (t4) {
+              // the energy nodes any of the item's columns can reach: from the
+              // range of log10 E and of the lit columns' Z, with slack well
+              // above the floats' rounding
+              const float l = (float)s_ra.lgE_eff;
+              const float vlo = s_erange[0] - log10f(ri.z_hi) - l - 1.0e-3f;
+              const float vhi = s_erange[1] - log10f(ri.z_lo) - l + 1.0e-3f;
+              int lo0 = -1, lo1 = -1;
+              const int b0 = stencil_base_fix(sm.gEi, nEt, fix_of((double)vlo), lo0);
+              const int b1 = stencil_base_fix(sm.gEi, nEt, fix_of((double)vhi), lo1);
+              s_win[0] = b0;
+              s_win[1] = b1 + 4;
+            }
+          }
+        } else if (M.S1 <= kMaxCellsF) {
+          // cell azimuths and areas as float pairs
+          for (int t = threadIdx.x - 32; t < M.S1; t += blockDim.x - 32) {
+            const DF p = df_split_bits(cellPhi[t], 0), ar = df_split_bits(cellA[t], 0);
+            sm.fcphi[t] = p.h;
+            sm.fcphi_lo[t] = p.l;
+            sm.fcarea[t] = ar.h;
+            sm.fcarea_lo[t] = ar.l;
+          }
         }
-        // specific intensities of every profile column (:445-478).  With
-        // N_L dividing the block size a thread keeps one column for all its
-        // energies, so its mu stencil (FP64 form) is formed once.
-        {
-          int mu_col = -1;
-          MuStencil ms{};
-          MuStencilF msf{};
-          MuStencilDF msd{};
-          double col_factor = 0.0;  // norm 10^(3 log T) GEOM of the column
-          DF cf_m{0.0f, 0.0f};      // col_factor = cf_m 2^cf_x (dfy form)
-          int cf_x = 0;
-          for (int t = threadIdx.x; t < ne * N_L; t += blockDim.x) {
-            const int pl = t / N_L, col = t - pl * N_L;
-            const int p = e0 + pl;
-            const int s = g.src[col];
-            WT y = WT(0);
-            if (s >= 0) {
+        __syncthreads();
+      }
+      const double p3 = s_ra.p3, kT = s_ra.kT, kT_c = s_ra.kT_c;
+      const float kT_f = (float)kT, p3f = (float)p3;
+      // mixed form: the FP32 roundings of the constant factors norm and
+      // 10^(3 log T) are undone exactly on the parallel's FP64 partials
+      const double fix = !kMixed ? 1.0
+                         : num4d ? (norm * p3) / ((double)(float)norm * (double)p3f)
+                                 : norm / (double)(float)norm;
+      if (images > 0 && t4) {
+        // contract the (log T, log g) stencil of this parallel once over the
+        // reachable energy nodes:
+        // slab[mu][logE] = sum_ij w_T[i] w_g[j] table[bT+i][bg+j][mu][logE]
+        const int n0 = s_win[0], wn = s_win[1] - n0, nw = nmu * wn;
+        double wT[4], wg[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) { wT[q] = s_ra.wT[q]; wg[q] = s_ra.wg[q]; }
+        const size_t S1t = (size_t)nmu * nEt, S0t = (size_t)a.atmos.ng * S1t;
+        const size_t base = s_ra.bT * S0t + s_ra.bg * S1t;
+        if (kMixed && a.atmos.I32 != nullptr) {
+          // FP32 contraction from the FP32 copy of the table
+          float wTf[4], wgf[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) { wTf[q] = (float)wT[q]; wgf[q] = (float)wg[q]; }
+          for (int w = threadIdx.x; w < nw; w += blockDim.x) {
+            const int mu_i = w / wn, t = mu_i * nEt + n0 + (w - mu_i * wn);
+            float r = 0.0f;
+#pragma unroll
+            for (int ii = 0; ii < 4; ii++) {
+              const float *q = a.atmos.I32 + base + ii * S0t + t;
+              float u = wgf[0] * __ldg(q) + wgf[1] * __ldg(q + S1t) + wgf[2] * __ldg(q + 2 * S1t) +
+                        wgf[3] * __ldg(q + 3 * S1t);
+              r += wTf[ii] * u;
+            }
+            slabf[t] = r;
+          }
+        } else {
+          if (!kMixed) {
+            for (int e = threadIdx.x; e < wn; e += blockDim.x) sm.xe[n0 + e] = kZeroExp;
+            __syncthreads();
+          }
+          for (int w = threadIdx.x; w < nw; w += blockDim.x) {
+            const int mu_i = w / wn, e = n0 + (w - mu_i * wn), t = mu_i * nEt + e;
+            double r = 0.0;
+#pragma unroll
+            for (int ii = 0; ii < 4; ii++) {
+              const double *q = a.atmos.I + base + ii * S0t + t;
+              double u = wg[0] * __ldg(q) + wg[1] * __ldg(q + S1t) + wg[2] * __ldg(q + 2 * S1t) +
+                         wg[3] * __ldg(q + 3 * S1t);
+              r += wT[ii] * u;
+            }
+            if (kMixed) {
+              slabf[t] = (float)r;
+            } else {
+              slab[t] = r;
+              atomicMax(&sm.xe[e], binary_exponent(r));
+            }
+          }
+          if (!kMixed) {
+            // the FP64 form keeps the slab as double-float pairs, each energy
+            // node's column (all mu) scaled by 2^-xe[e] (exact), xe the binary
+            // exponent of its largest value, so that the pairs keep full
+            // relative precision across the table's exponential tail
+            __syncthreads();
+            DF *o = reinterpret_cast<DF *>(slab);
+            for (int w = threadIdx.x; w < nw; w += blockDim.x) {
+              const int mu_i = w / wn, e = n0 + (w - mu_i * wn), t = mu_i * nEt + e;
+              o[t] = df_split_bits(slab[t], -sm.xe[e]);
+            }
+          }
+        }
+        __syncthreads();
+      }
+      for (int I = 0; I < images; I++) {
+        const double *rec;
+        if (ri.geo >= 0) {
+          rec = a.geo + (ri.geo + I) * image_doubles(N_L);
+        } else {
+          // no room was left for the parallel's records: form the image here
+          double *own = a.geo + (a.geo_cap + blockIdx.x) * image_doubles(N_L);
+          double *coef;
+          GeoSmem g = carve(sm.piece, N_L, 0, &coef, 0, 0, nullptr, 32, 0);
+          RowCtx c;
+          load_row(a, M, row, i, c, &s_row);
+          if (threadIdx.x == 0) s_jalt = c.N_R - 1;
+          __syncthreads();
+          for (int t = threadIdx.x; t < c.N_R - 1; t += blockDim.x)
+            if (ordered(c.D[t]) > ordered(kHalfPi)) atomicMin(&s_jalt, t);
+          __syncthreads();
+          c.jalt = s_jalt;
+          c.alt_xmin = cos(c.D[c.jalt]);
+          image_record(c, I, N_L, a.leaves, g, num4d, mu_top3, mu_max, s_state, nullptr, own);
+          rec = own;
+        }
+        const uint8_t *rfl = reinterpret_cast<const uint8_t *>(rec + 4 * (size_t)N_L);
+        // (the parallel's entry state was not known to the pre-pass; a record
+        // formed here has it)
+        const bool entry_top = num4d && ri.geo >= 0 && a.row_entry_top[row] != 0;
+        for (int t = threadIdx.x; t < N_L; t += blockDim.x) {
+          unsigned f = rfl[t];
+          if (entry_top && (f & kColFirst)) f &= ~kColClamp;
+          sm.flag[t] = (int)f;
+          const double ph = rec[t];
+          const DF pd = df_split_bits(ph, 0);
+          sm.fphase[t] = pd.h;
+          sm.fphase_lo[t] = pd.l;
+          if (t < N_L - 1) {
+            const double h = rec[t + 1] - ph;
+            if (kMixed) {
+              sm.fh[t] = (float)h;
+            } else {
+              const double r = 1.0 / h;
+              sm.ih[t] = df_split_bits(r, 0);
+              sm.ih2[t] = df_split_bits(1.0 / (h * h), 0);
+            }
+          }
+          if (f & kColLit) {
+            const double Z = rec[N_L + t], abb = rec[2 * N_L + t], geom = rec[3 * N_L + t];
+            sm.Z[t] = Z;
+            sm.abb[t] = abb;
+            sm.geom[t] = geom;
+            if (kMixed) {
+              sm.finvZ[t] = (float)(1.0 / Z);
+              sm.fgeom[t] = (float)geom;
+            }
+            if (tab2) sm.lzd[t] = erest ? Z : log10(Z);
+            if (t4) {
+              sm.lz[t] = fix_of(log10(Z) + s_ra.lgE_eff);
+              if constexpr (kMixed) {
+                const float v = fmaxf((float)abb, sm.fgmu[0]);
+                const int b = stencil_base_f(sm.fgmu, nmu, v);
+                float w[4];
+                lagrange_wf(sm.fgmu, sm.fsmu, b, v, w);
+                sm.mb[t] = b;
+                sm.mwf[t] = make_float4(w[0], w[1], w[2], w[3]);
+              } else {
+                const MuStencil ms = mu_stencil(a.atmos, as, abb, false);
+                sm.mb[t] = ms.b2;
+#pragma unroll
+                for (int q = 0; q < 4; q++) sm.mw[4 * t + q] = df_split_bits(ms.w2[q], 0);
+                const double cf = norm * p3 * geom;
+                MaxExponent mx;
+                mx.fold(cf);
+                const int x = mx.exponent();
+                sm.cfx[t] = x;
+                sm.cfm[t] = df_split_bits(cf, -x);
+              }
+            }
+          }
+        }
+        __syncthreads();
+        auto cell_phase = [&](auto cached, int k) {
+          const float2 ph = sm.phase[k];
+          return CellPhaseF<decltype(cached)::value>{
+              sm.fphase, sm.fphase_lo, N_L, sm.fphase[0], sm.fphase[N_L - 1], ph.x, ph.y, tp,
+              (float)(kTwoPi - (double)tp), sm.fcphi, sm.fcphi_lo, cellPhi};
+        };
+        if (use_w) {
+          // the runs of every signal phase, each half of the cells by its own
+          // thread (energy independent: formed once per parallel and image)
+          const int hc = (M.S1 + 1) / 2;
+          const AreaDF<true> ar{sm.fcarea, sm.fcarea_lo, cellA};
+          for (int t = threadIdx.x; t < 2 * N_P; t += blockDim.x) {
+            const int k = t % N_P, half = t / N_P;
+            const CellPhaseF<true> cp = cell_phase(std::true_type{}, k);
+            const int n =
+                build_runs(cp, ar, half * hc, min(M.S1, (half + 1) * hc), rad, wr, half, k);
+            // no cell of the parallel is added at this phase where one cannot
+            // be wrapped (either half's failure voids both, as in the per-cell
+            // form)
+            if (n < 0) atomicExch(&a.member_status[m], (int)kPulseFail);
+            sm.nruns[half * N_P + k] = n;
+          }
+        }
+        if (threadIdx.x == 0 && a.flop_counter && eg == 0) {
+          int Cr = 0;
+          for (int j = 0; j < M.S1; j++) Cr += (rad[j] == 1);
+          flops += (double)N_L * (60.0 + N_E * f_atm) +
+                   (double)N_E * (30.0 * N_L + (double)Cr * N_P * 14.0);
+        }
+
+        for (int e0 = e_lo; e0 < e_hi; e0 += ec) {
+          const int ne = min(ec, e_hi - e0);
+          if (num4d) {
+            for (int t = threadIdx.x; t < ne; t += blockDim.x) {
+              if (tab2) sm.lgEd[t] = erest ? a.energies[e0 + t] : a.lgE[e0 + t];
+              else sm.lgE[t] = fix_of(a.lgE[e0 + t]);
+            }
+          }
+          __syncthreads();
+          // specific intensities of every profile column (:445-478): a thread
+          // takes one column and every parts-th energy of the chunk, so the
+          // energy stencil moves by a node or two from one to the next
+          for (int col = col0; col < N_L; col += kThreads) {
+            const int f = sm.flag[col];
+            int lo = -1;
+            MuStencil ms{};
+            if (tab2 && (f & kColLit)) ms = mu_stencil(a.atmos, as, sm.abb[col], false);
+            for (int pl = part0; pl < ne; pl += parts) {
+              const int p = e0 + pl;
+              if (!(f & kColLit)) {
+                if constexpr (kMixed) co4[pl * N_L + col].y = 0.0f;
+                else if (dfy) pr.y(col, pl) = DF{0.0f, 0.0f};
+                else pr.yd(col, pl) = 0.0;
+                continue;
+              }
+              // a leaf's first energy may see the clamped mu; with beaming
+              // option 3 every call is followed by calls up to mu = 1, so no
+              // out-of-table mu is ever clamped
+              const bool clamp = p == 0 && (f & kColClamp) && M.beam_opt != 3;
+              int b3 = 0;
+              DF u{0.0f, 0.0f};
+              if (t4) {
+                long long v = sm.lgE[pl] - sm.lz[col];
+                v = max(v, sm.gEi[0]);
+                v = min(v, sm.gEi[nEt - 1]);
+                b3 = stencil_base_fix(sm.gEi, nEt, v, lo);
+                u = fix_df(v - sm.gEi[b3]);
+              }
               if constexpr (kMixed) {
                 float I_E;
-                if (num4d) {
-                  // atm 6: E' = E / Z in electron rest energies (:457-458)
-                  const double v3 = erest ? (g.lgE[pl] / g.lzs[s]) * 0.001956951
-                                          : g.lgE[pl] - g.lzs[s];
-                  if (p == 0 && g.clamp0[s]) {
-                    I_E = eval_num4d_f(a.atmos, as, slabf,
-                                       mu_stencil_f(a.atmos, as, as.fabb[s], true), v3, p3f);
-                  } else {
-                    if (s != mu_col) {
-                      msf = mu_stencil_f(a.atmos, as, as.fabb[s], false);
-                      mu_col = s;
-                    }
-                    I_E = eval_num4d_f(a.atmos, as, slabf, msf, v3, p3f);
+                if (t4) {
+                  int b2 = sm.mb[col];
+                  float4 w2 = sm.mwf[col];
+                  if (clamp) {
+                    const float v = fminf((float)sm.abb[col], sm.fgmu[nmu - 1]);
+                    b2 = stencil_base_f(sm.fgmu, nmu, v);
+                    float w[4];
+                    lagrange_wf(sm.fgmu, sm.fsmu, b2, v, w);
+                    w2 = make_float4(w[0], w[1], w[2], w[3]);
                   }
+                  I_E = eval_num4d_f(sm.fgEo, sm.fsE, nEt, slabf, b2, w2, b3, u.h, p3f);
                 } else {
-                  const float Ef = p < kMaxEnergiesF ? as.fE[p] : (float)a.energies[p];
-                  I_E = eval_bb_f(Ef * as.finvZ[s], kT_f);
+                  I_E = eval_bb_f((float)a.energies[p] * sm.finvZ[col], kT_f);
                 }
-                y = (WT)((float)norm * I_E * as.fgeom[s]);
+                co4[pl * N_L + col].y = (float)norm * I_E * sm.fgeom[col];
               } else {
                 double I_E;
-                if (num4d && !tab2) {
-                  // the contracted 4-D table in double-float (eval_num4d_df);
-                  // with beaming option 3 every call is followed by calls up
-                  // to mu = 1, so no out-of-table mu is ever clamped
-                  const double v3 = g.lgE[pl] - g.lzs[s];
-                  if (s != mu_col) {
-                    msd = mu_stencil_df(a.atmos, as, g.ABB[s], false);
-                    col_factor = norm * p3 * g.GEOM[s];
-                    if (dfy) {
-                      MaxExponent mx;
-                      mx.fold(col_factor);
-                      cf_x = mx.exponent();
-                      cf_m = df_split(scale_pow2(col_factor, -cf_x));
-                    }
-                    mu_col = s;
-                  }
+                if (t4) {
                   int xr;
-                  DF I = (p == 0 && g.clamp0[s] && M.beam_opt != 3)
-                             ? eval_num4d_dfx(a.atmos, as, slabd,
-                                              mu_stencil_df(a.atmos, as, g.ABB[s], true), v3,
-                                              xr)
-                             : eval_num4d_dfx(a.atmos, as, slabd, msd, v3, xr);
+                  DF I;
+                  if (clamp) {
+                    const MuStencil mc = mu_stencil(a.atmos, as, sm.abb[col], true);
+                    DF w2[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) w2[q] = df_split(mc.w2[q]);
+                    I = eval_num4d_dfx(eg4, slabd, mc.b2, w2, b3, u, xr);
+                  } else {
+                    I = eval_num4d_dfx(eg4, slabd, sm.mb[col], sm.mw + 4 * col, b3, u, xr);
+                  }
                   if (I.h < 0.0f) I = DF{0.0f, 0.0f};
                   if (dfy) {
                     // y = I 2^xr col_factor kept as a double-float mantissa
                     // and an exponent (no round trip through FP64)
-                    pr.y(col, pl) = df_mul(I, cf_m);
-                    pr.ex(col, pl) = xr + cf_x;
+                    pr.y(col, pl) = df_mul(I, sm.cfm[col]);
+                    pr.ex(col, pl) = xr + sm.cfx[col];
                     continue;
                   }
                   I_E = df_value(I) * pow2_double(xr) * p3;
                 } else if (num4d) {
                   // atm 6: E' = E / Z in electron rest energies (:457-458)
-                  const double v3 = erest ? (g.lgE[pl] / g.lzs[s]) * 0.001956951
-                                          : g.lgE[pl] - g.lzs[s];
-                  // with beaming option 3 every call is followed by calls up
-                  // to mu = 1, so no out-of-table mu is ever clamped
-                  if (p == 0 && g.clamp0[s] && M.beam_opt != 3) {
-                    I_E = eval_num4d_e(a.atmos, as, slab, mu_stencil(a.atmos, as, g.ABB[s], true),
-                                       v3, p3);
-                  } else {
-                    if (s != mu_col) {
-                      ms = mu_stencil(a.atmos, as, g.ABB[s], false);
-                      mu_col = s;
-                    }
-                    I_E = eval_num4d_e(a.atmos, as, slab, ms, v3, p3);
-                  }
+                  const double v3 = erest ? (sm.lgEd[pl] / sm.lzd[col]) * 0.001956951
+                                          : sm.lgEd[pl] - sm.lzd[col];
+                  I_E = eval_num4d_e(a.atmos, as, a.atmos.I,
+                                     clamp ? mu_stencil(a.atmos, as, sm.abb[col], true) : ms, v3,
+                                     p3);
                 } else {
-                  I_E = eval_bb(a.energies[p] / g.Z[s], kT);
+                  I_E = eval_bb(a.energies[p] / sm.Z[col], kT);
                   // the burst blackbody's limb darkening (hot_BB_burst.pyx)
-                  if (M.atm == 3) I_E = I_E * (0.421 + 0.868 * g.ABB[s]);
+                  if (M.atm == 3) I_E = I_E * (0.421 + 0.868 * sm.abb[col]);
                 }
-                {
-                  const double I_c =
-                      corr ? eval_bb(a.energies[p] / g.Z[s], kT_c) * (kErg * kPlanck) : 0.0;
-                  // with a beaming modification the raw intensity is kept
-                  // here and modified in the pass below
-                  y = (WT)(M.beam_opt > 0 ? I_E : (I_E * norm - I_c) * g.GEOM[s]);
-                }
+                const double I_c =
+                    corr ? eval_bb(a.energies[p] / sm.Z[col], kT_c) * (kErg * kPlanck) : 0.0;
+                // with a beaming modification the raw intensity is kept
+                // here and modified in the pass below
+                pr.yd(col, pl) = M.beam_opt > 0 ? I_E : (I_E * norm - I_c) * sm.geom[col];
               }
             }
-            if constexpr (kMixed) co4[pl * N_L + col].y = y;
-            else pr.yd(col, pl) = y;
-          }
-        }
-        if (!kMixed && M.beam_opt > 0) {
-          // the beaming modification (hot_wrapper.pyx:153-199) of every
-          // column intensity of the chunk, by the thread that formed it
-          for (int t = threadIdx.x; t < ne * N_L; t += blockDim.x) {
-            const int pl = t / N_L, col = t - pl * N_L;
-            const int p = e0 + pl;
-            const int s = g.src[col];
-            if (s < 0) continue;
-            const double I_raw = pr.yd(col, pl);
-            double I_E;
-            if (num4d) {
-              const double v3 = erest ? (g.lgE[pl] / g.lzs[s]) * 0.001956951 : g.lgE[pl] - g.lzs[s];
-              const double Ep = erest ? v3 : a.energies[p] / g.Z[s];
-              I_E = beamed_intensity(M.beam_opt, s_beam, Ep, g.ABB[s], I_raw, [&](double mu_k) {
-                if (tab2)
-                  return eval_num4d_e(a.atmos, as, slab, mu_stencil(a.atmos, as, mu_k, false),
-                                      v3, p3);
-                double scale;
-                const DF I = eval_num4d_df(a.atmos, as, slabd,
-                                           mu_stencil_df(a.atmos, as, mu_k, false), v3, scale);
-                return I.h < 0.0f ? 0.0 : df_value(I) * scale * p3;
-              });
-            } else {
-              const double Ep = a.energies[p] / g.Z[s];
-              const double I0 = eval_bb(Ep, kT);  // the blackbody has no mu dependence
-              I_E = beamed_intensity(M.beam_opt, s_beam, Ep, g.ABB[s], I_raw,
-                                     [&](double) { return I0; });
-            }
-            const double I_c =
-                corr ? eval_bb(a.energies[p] / g.Z[s], kT_c) * (kErg * kPlanck) : 0.0;
-            pr.yd(col, pl) = (I_E * norm - I_c) * g.GEOM[s];
-          }
-        }
-        __syncthreads();
-        // Akima-periodic piece coefficients (:566-569): a thread builds kStrip
-        // consecutive pieces of one energy row from a sliding window of the
-        // five chords each piece needs, so each chord is formed once per
-        // strip instead of five times
-        const int n_iv = N_L - 1, strips = (n_iv + kStrip - 1) / kStrip;
-        if constexpr (kMixed) {
-          for (int t = threadIdx.x; t < ne * strips; t += blockDim.x) {
-            const int pl = t / strips, i0 = (t - pl * strips) * kStrip;
-            const int i1 = min(i0 + kStrip, n_iv);
-            PieceT<WT> *yr = co4 + pl * N_L;
-            auto chord = [&](int j) -> WT {
-              const int q = periodic_chord(j, N_L);
-              // knot spacings from the FP64 knots: adjacent knots closer
-              // than an FP32 ulp stay distinct
-              return (yr[q + 1].y - yr[q].y) / (WT)(g.phase[q + 1] - g.phase[q]);
-            };
-            WT m0 = chord(i0 - 2), m1 = chord(i0 - 1), m2 = chord(i0), m3 = chord(i0 + 1),
-               m4 = chord(i0 + 2);
-            for (int iv = i0; iv < i1; iv++) {
-              if (iv > i0) {
-                m0 = m1; m1 = m2; m2 = m3; m3 = m4;
-                m4 = chord(iv + 2);
+            if (!kMixed && M.beam_opt > 0 && (f & kColLit)) {
+              // the beaming modification (hot_wrapper.pyx:153-199) of the
+              // column's intensities
+              int lb = -1;
+              for (int pl = part0; pl < ne; pl += parts) {
+                const int p = e0 + pl;
+                const double I_raw = pr.yd(col, pl);
+                double I_E;
+                if (num4d) {
+                  int b3 = 0;
+                  DF u{0.0f, 0.0f};
+                  double v3 = 0.0;
+                  if (t4) {
+                    long long v = sm.lgE[pl] - sm.lz[col];
+                    v = max(v, sm.gEi[0]);
+                    v = min(v, sm.gEi[nEt - 1]);
+                    b3 = stencil_base_fix(sm.gEi, nEt, v, lb);
+                    u = fix_df(v - sm.gEi[b3]);
+                  } else {
+                    v3 = erest ? (sm.lgEd[pl] / sm.lzd[col]) * 0.001956951
+                               : sm.lgEd[pl] - sm.lzd[col];
+                  }
+                  const double Ep = erest ? v3 : a.energies[p] / sm.Z[col];
+                  I_E = beamed_intensity(M.beam_opt, s_beam, Ep, sm.abb[col], I_raw,
+                                         [&](double mu_k) {
+                    const MuStencil mk = mu_stencil(a.atmos, as, mu_k, false);
+                    if (tab2) return eval_num4d_e(a.atmos, as, a.atmos.I, mk, v3, p3);
+                    DF w2[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) w2[q] = df_split(mk.w2[q]);
+                    int xr;
+                    const DF I = eval_num4d_dfx(eg4, slabd, mk.b2, w2, b3, u, xr);
+                    return I.h < 0.0f ? 0.0 : df_value(I) * pow2_double(xr) * p3;
+                  });
+                } else {
+                  const double Ep = a.energies[p] / sm.Z[col];
+                  const double I0 = eval_bb(Ep, kT);  // the blackbody has no mu dependence
+                  I_E = beamed_intensity(M.beam_opt, s_beam, Ep, sm.abb[col], I_raw,
+                                         [&](double) { return I0; });
+                }
+                const double I_c =
+                    corr ? eval_bb(a.energies[p] / sm.Z[col], kT_c) * (kErg * kPlanck) : 0.0;
+                pr.yd(col, pl) = (I_E * norm - I_c) * sm.geom[col];
               }
-              WT k1, k2, k3;
-              const WT h = (WT)(g.phase[iv + 1] - g.phase[iv]);
-              akima_piece(m0, m1, m2, m3, m4, h, k1, k2, k3);
-              PieceT<WT> *o = yr + iv;
-              o->k1 = k1;
-              o->k2 = k2;
-              o->k3 = k3;
             }
           }
           __syncthreads();
-        } else {
-          // scale each energy row by a power of two (exact) so that its
-          // largest profile value lies in [0.5, 1): double-float values then
-          // keep the row's full relative precision whatever its magnitude
-          const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-          for (int pl = warp; pl < ne; pl += kThreads / 32) {
-            MaxExponent mx;
-            for (int col = lane; col < N_L; col += 32) {
-              if (dfy) {
-                // values m 2^x: the exponent from the bits
-                const float h = pr.y(col, pl).h;
-                if (h != 0.0f && h == h) {
-                  if (isinf(h)) mx.inf = true;
-                  else mx.e = max(mx.e, pr.ex(col, pl) + float_exponent(h));
-                }
-              } else {
-                mx.fold(pr.yd(col, pl));
-              }
-            }
-            mx.merge_warp();
-            if (lane == 0) g.sc_exp[pl] = mx.exponent();
-          }
-          __syncthreads();
-          for (int t = threadIdx.x; t < EC * N_L; t += blockDim.x) {
-            const int col = t / EC, pl = t - col * EC;
-            if (pl >= ne) continue;
-            if (dfy) {  // the value times 2^(x - the row's) in float arithmetic (exact)
-              const DF m = pr.y(col, pl);
-              pr.y(col, pl) = m.h == 0.0f ? DF{0.0f, 0.0f}
-                                          : df_times_pow2(m, pr.ex(col, pl) - g.sc_exp[pl]);
-            } else {
-              pr.y(col, pl) = df_split(scale_pow2(pr.yd(col, pl), -g.sc_exp[pl]));
-            }
-          }
-          __syncthreads();
-          // a group of EC lanes takes a strip, a lane an energy; the classes
-          // of a piece's energies are gathered by ballot
-          const int sub = lane / EC;
-          for (int t = threadIdx.x; t < ((EC * strips + 31) & ~31); t += blockDim.x) {
-            const int pl = t % EC, i0 = (t / EC) * kStrip;
-            const int i1 = min(i0 + kStrip, n_iv);
-            const bool on = pl < ne;
-            auto chord = [&](int j) -> DF {
-              const int q = periodic_chord(j, N_L);
-              return df_mul(df_sub(pr.y(q + 1, pl), pr.y(q, pl)), g.ih[q]);
-            };
-            DF m0{}, m1{}, m2{}, m3{}, m4{};
-            if (on && i0 < i1) {
-              m0 = chord(i0 - 2); m1 = chord(i0 - 1); m2 = chord(i0); m3 = chord(i0 + 1);
-              m4 = chord(i0 + 2);
-            }
-            for (int z = 0; z < kStrip; z++) {
-              const int iv = i0 + z;
-              const bool here = on && iv < i1;
-              int cls = 1;
-              if (here) {
-                if (z > 0) {
+          // Akima-periodic piece coefficients (:566-569): a thread builds kStrip
+          // consecutive pieces of one energy row from a sliding window of the
+          // five chords each piece needs, so each chord is formed once per
+          // strip instead of five times
+          if constexpr (kMixed) {
+            for (int t = threadIdx.x; t < ne * strips; t += blockDim.x) {
+              const int pl = t / strips, i0 = (t - pl * strips) * kStrip;
+              const int i1 = min(i0 + kStrip, n_iv);
+              PieceT<WT> *yr = co4 + pl * N_L;
+              auto chord = [&](int j) -> WT {
+                const int q = periodic_chord(j, N_L);
+                // knot spacings from the FP64 knots: adjacent knots closer
+                // than an FP32 ulp stay distinct
+                return (yr[q + 1].y - yr[q].y) / sm.fh[q];
+              };
+              WT m0 = chord(i0 - 2), m1 = chord(i0 - 1), m2 = chord(i0), m3 = chord(i0 + 1),
+                 m4 = chord(i0 + 2);
+              for (int iv = i0; iv < i1; iv++) {
+                if (iv > i0) {
                   m0 = m1; m1 = m2; m2 = m3; m3 = m4;
                   m4 = chord(iv + 2);
                 }
-                DF k1, k2, k3, tr;
-                akima_piece_df(m0, m1, m2, m3, m4, g.ih[iv], g.ih2[iv], k1, k2, k3, tr);
-                pr.put_k(iv, pl, k1, k2, k3);
-                const float h = (as.fphase[iv + 1] - as.fphase[iv]) +
-                                (as.fphase_lo[iv + 1] - as.fphase_lo[iv]);
-                cls = piece_class(PieceDF{pr.y(iv, pl), k1, k2, k3}, pr.y(iv + 1, pl).h, tr.h, h,
-                                  corr);
-              }
-              const uint32_t odd = __ballot_sync(0xffffffffu, cls != 1);
-              const uint32_t none = __ballot_sync(0xffffffffu, cls == 0);
-              if (pl == 0 && iv < i1) {
-                const uint32_t mask = EC == 32 ? 0xffffffffu : ((1u << EC) - 1u);
-                s_flags[2 * iv] = (odd >> (sub * EC)) & mask;
-                s_flags[2 * iv + 1] = (none >> (sub * EC)) & mask;
+                WT k1, k2, k3;
+                akima_piece(m0, m1, m2, m3, m4, (WT)sm.fh[iv], k1, k2, k3);
+                PieceT<WT> *o = yr + iv;
+                o->k1 = k1;
+                o->k2 = k2;
+                o->k3 = k3;
               }
             }
+            __syncthreads();
+          } else {
+            // scale each energy row by a power of two (exact) so that its
+            // largest profile value lies in [0.5, 1): double-float values then
+            // keep the row's full relative precision whatever its magnitude
+            for (int pl = warp; pl < ne; pl += kThreads / 32) {
+              MaxExponent mx;
+              for (int col = lane; col < N_L; col += 32) {
+                if (dfy) {
+                  // values m 2^x: the exponent from the bits
+                  const float h = pr.y(col, pl).h;
+                  if (h != 0.0f && h == h) {
+                    if (isinf(h)) mx.inf = true;
+                    else mx.e = max(mx.e, pr.ex(col, pl) + float_exponent(h));
+                  }
+                } else {
+                  mx.fold(pr.yd(col, pl));
+                }
+              }
+              mx.merge_warp();
+              if (lane == 0) sm.sc_exp[pl] = mx.exponent();
+            }
+            __syncthreads();
+            for (int t = threadIdx.x; t < EC * N_L; t += blockDim.x) {
+              const int col = t / EC, pl = t - col * EC;
+              if (pl >= ne) continue;
+              if (dfy) {  // the value times 2^(x - the row's) in float arithmetic (exact)
+                const DF mv = pr.y(col, pl);
+                pr.y(col, pl) = mv.h == 0.0f
+                                    ? DF{0.0f, 0.0f}
+                                    : df_times_pow2(mv, pr.ex(col, pl) - sm.sc_exp[pl]);
+              } else {
+                pr.y(col, pl) = df_split_bits(pr.yd(col, pl), -sm.sc_exp[pl]);
+              }
+            }
+            __syncthreads();
+            // a group of EC lanes takes a strip, a lane an energy; the classes
+            // of a piece's energies are gathered by ballot
+            const int sub = lane / EC;
+            for (int t = threadIdx.x; t < ((EC * strips + 31) & ~31); t += blockDim.x) {
+              const int pl = t % EC, i0 = (t / EC) * kStrip;
+              const int i1 = min(i0 + kStrip, n_iv);
+              const bool on = pl < ne;
+              auto chord = [&](int j) -> DF {
+                const int q = periodic_chord(j, N_L);
+                return df_mul(df_sub(pr.y(q + 1, pl), pr.y(q, pl)), sm.ih[q]);
+              };
+              DF m0{}, m1{}, m2{}, m3{}, m4{};
+              if (on && i0 < i1) {
+                m0 = chord(i0 - 2); m1 = chord(i0 - 1); m2 = chord(i0); m3 = chord(i0 + 1);
+                m4 = chord(i0 + 2);
+              }
+              for (int z = 0; z < kStrip; z++) {
+                const int iv = i0 + z;
+                const bool here = on && iv < i1;
+                int cls = 1;
+                if (here) {
+                  if (z > 0) {
+                    m0 = m1; m1 = m2; m2 = m3; m3 = m4;
+                    m4 = chord(iv + 2);
+                  }
+                  DF k1, k2, k3, tr;
+                  akima_piece_df(m0, m1, m2, m3, m4, sm.ih[iv], sm.ih2[iv], k1, k2, k3, tr);
+                  pr.put_k(iv, pl, k1, k2, k3);
+                  const float h = (sm.fphase[iv + 1] - sm.fphase[iv]) +
+                                  (sm.fphase_lo[iv + 1] - sm.fphase_lo[iv]);
+                  cls = piece_class(PieceDF{pr.y(iv, pl), k1, k2, k3}, pr.y(iv + 1, pl).h, tr.h,
+                                    h, corr);
+                }
+                const uint32_t odd = __ballot_sync(0xffffffffu, cls != 1);
+                const uint32_t none = __ballot_sync(0xffffffffu, cls == 0);
+                if (pl == 0 && iv < i1) {
+                  const uint32_t mask = EC == 32 ? 0xffffffffu : ((1u << EC) - 1u);
+                  sm.flags[2 * iv] = (odd >> (sub * EC)) & mask;
+                  sm.flags[2 * iv + 1] = (none >> (sub * EC)) & mask;
+                }
+              }
+            }
+            __syncthreads();
+          }
+          // cell x phase accumulation (:571-598).  Power sums: a group of EC
+          // lanes takes a signal phase, a lane an energy.  Per-cell form: a
+          // thread takes a signal phase and kEPT energies.
+          if (use_w) {
+            const int e = threadIdx.x % EC, grp = threadIdx.x / EC, step = kThreads / EC;
+            const AreaDF<true> ar{sm.fcarea, sm.fcarea_lo, cellA};
+            RunFetch rf;
+            auto counts = [&](int k, int &n0, int &n1) {
+              n0 = n1 = 0;
+              if (k < N_P) {
+                n0 = sm.nruns[k];
+                n1 = sm.nruns[N_P + k];
+                if (n0 < 0 || n1 < 0) n0 = n1 = 0;
+              }
+            };
+            int n0, n1;
+            counts(grp, n0, n1);
+            rf.fetch(wr, grp, n0, n1, 0, e, EC);
+            for (int k0 = 0; k0 < N_P; k0 += step) {
+              const int k = k0 + grp, kc = min(k, N_P - 1);
+              const bool mine = e < ne && k < N_P;
+              // partials [N_P][N_E]: the lanes' energies are adjacent
+              double *dst = part + (size_t)kc * N_E + e0 + e;
+              const double before = mine ? *dst : 0.0;
+              int m0, m1;
+              counts(k + step, m0, m1);
+              const DF v = run_sum(cell_phase(std::true_type{}, kc), ar, rad, wr, kc, n0, n1,
+                                   k + step, m0, m1, EC, ne, pr, sm.flags, sm.stages, corr, rf);
+              if (mine) *dst = before + df_join_bits(v, sm.sc_exp[e]);
+              n0 = m0;
+              n1 = m1;
+            }
+          } else {
+            const int ntasks = N_P * (EC / kEPT);
+            auto sums = [&](auto cached) {
+              constexpr bool kCached = decltype(cached)::value;
+              for (int task = threadIdx.x; task < ntasks; task += blockDim.x) {
+                const int k = task % N_P, grp = task / N_P;
+                const int pb = grp * kEPT;
+                if (pb >= ne) continue;
+                const CellPhaseF<kCached> cp = cell_phase(cached, k);
+                if constexpr (kMixed) {
+                  WT acc[kEPT];
+#pragma unroll
+                  for (int e = 0; e < kEPT; e++) acc[e] = WT(0);
+                  const AreaF<kCached> ar{sm.fcarea, cellA};
+                  if (!cell_phase_sums<WT>(cp, ar, M.S1, rad, co4, N_L, pb, ne, acc)) {
+                    atomicExch(&a.member_status[m], (int)kPulseFail);
+                    continue;
+                  }
+#pragma unroll
+                  for (int e = 0; e < kEPT; e++)
+                    if (pb + e < ne)
+                      part[(size_t)(e0 + pb + e) * N_P + k] += (double)acc[e] * fix;
+                } else {
+                  DF acc[kEPT];
+#pragma unroll
+                  for (int e = 0; e < kEPT; e++) acc[e] = DF{0.0f, 0.0f};
+                  const AreaDF<kCached> ar{sm.fcarea, sm.fcarea_lo, cellA};
+                  if (!cell_phase_sums_df(cp, ar, M.S1, rad, pr, pb, corr, acc)) {
+                    atomicExch(&a.member_status[m], (int)kPulseFail);
+                    continue;
+                  }
+#pragma unroll
+                  for (int e = 0; e < kEPT; e++)
+                    if (pb + e < ne)
+                      part[(size_t)k * N_E + e0 + pb + e] +=
+                          scale_pow2(df_value(acc[e]), sm.sc_exp[pb + e]);
+                }
+              }
+            };
+            if (M.S1 <= kMaxCellsF) sums(std::true_type{});
+            else sums(std::false_type{});
           }
           __syncthreads();
         }
-        // cell x phase accumulation (:571-598).  Power sums: a group of EC
-        // lanes takes a signal phase, a lane an energy.  Per-cell form: a
-        // thread takes a signal phase and kEPT energies.
-        if (use_w) {
-          const int e = threadIdx.x % EC;
-          for (int k0 = 0; k0 < N_P; k0 += kThreads / EC) {
-            const int k = k0 + threadIdx.x / EC, kc = min(k, N_P - 1);
-            const AreaDF<true> ar{as.fcarea, as.fcarea_lo, cellA};
-            int n0 = s_nruns[kc], n1 = s_nruns[N_P + kc];
-            if (n0 < 0 || n1 < 0 || k >= N_P) n0 = n1 = 0;
-            const DF v = run_sum(cell_phase(std::true_type{}, kc), ar, rad, wr, n0, n1, kc,
-                                 EC, ne, pr, s_flags, s_stages,
-                                 corr);
-            // partials [N_P][N_E]: the lanes' energies are adjacent
-            if (e < ne && k < N_P)
-              part[(size_t)k * N_E + e0 + e] += scale_pow2(df_value(v), g.sc_exp[e]);
-          }
-        } else {
-          auto sums = [&](auto cached) {
-            constexpr bool kCached = decltype(cached)::value;
-            for (int task = threadIdx.x; task < ntasks; task += blockDim.x) {
-              const int k = task % N_P, grp = task / N_P;
-              const int pb = grp * kEPT;
-              if (pb >= ne) continue;
-              const CellPhaseF<kCached> cp = cell_phase(cached, k);
-              if constexpr (kMixed) {
-                WT acc[kEPT];
-#pragma unroll
-                for (int e = 0; e < kEPT; e++) acc[e] = WT(0);
-                const AreaF<kCached> ar{as.fcarea, cellA};
-                if (!cell_phase_sums<WT>(cp, ar, M.S1, rad, co4, N_L, pb, ne, acc)) {
-                  atomicExch(&a.member_status[m], (int)kPulseFail);
-                  continue;
-                }
-#pragma unroll
-                for (int e = 0; e < kEPT; e++)
-                  if (pb + e < ne) part[(size_t)(e0 + pb + e) * N_P + k] += (double)acc[e] * fix;
-              } else {
-                DF acc[kEPT];
-#pragma unroll
-                for (int e = 0; e < kEPT; e++) acc[e] = DF{0.0f, 0.0f};
-                const AreaDF<kCached> ar{as.fcarea, as.fcarea_lo, cellA};
-                if (!cell_phase_sums_df(cp, ar, M.S1, rad, pr, pb, corr, acc)) {
-                  atomicExch(&a.member_status[m], (int)kPulseFail);
-                  continue;
-                }
-#pragma unroll
-                for (int e = 0; e < kEPT; e++)
-                  if (pb + e < ne)
-                    part[(size_t)k * N_E + e0 + pb + e] +=
-                        scale_pow2(df_value(acc[e]), g.sc_exp[pb + e]);
-              }
-            }
-          };
-          if (M.S1 <= kMaxCellsF) sums(std::true_type{});
-          else sums(std::false_type{});
-        }
-        __syncthreads();
+      }
+      if (ri.images & kImgTerm) {
+        // the reference terminates here: nothing after it in the chunk is added
+        if (threadIdx.x == 0) atomicExch(&a.member_status[m], (int)kPulseFail);
+        break;
       }
     }
+    if (threadIdx.x == 0 && a.flop_counter && flops > 0.0) atomicAdd(a.flop_counter, flops);
   }
-  if (use_w) {
-    __syncthreads();
-    if (threadIdx.x == 0) atomicExch(&a.w_slot_busy[s_wslot], 0);
-  }
-  if (threadIdx.x == 0 && a.flop_counter && flops > 0.0) atomicAdd(a.flop_counter, flops);
 }
 
 // ---------------------------------------------------------------------------
@@ -2008,10 +2376,11 @@ __global__ void __launch_bounds__(kThreads, 1) stokes_kernel(IntegrateArgs a) {
   int *scQ = reinterpret_cast<int *>(xd + 2 * N_L), *scU = scQ + EC;
   Piece *coI = reinterpret_cast<Piece *>(coef);
   Piece *coQ = coI + (size_t)EC * N_L, *coU = coQ + (size_t)EC * N_L;
-  __shared__ int s_J, s_jalt, s_top, s_any;
+  __shared__ int s_jalt, s_top, s_any;
+  __shared__ RowCtx s_row;
   double *part = a.partial + (size_t)row * 3 * N_E * N_P;
   RowCtx c;
-  if (!load_row(a, M, row, i, c, &s_J)) return;
+  if (!load_row(a, M, row, i, c, &s_row)) return;
   stage_deflection(c, g, &s_jalt);
   if (tab2) stage_table_grids(a.atmos, as, nmu, nEt);
   if (threadIdx.x == 0) {
@@ -2412,11 +2781,17 @@ __device__ int block_exclusive_scan(int v, int *s_buf, int &excl) {
 }
 
 // one CTA of kPlanThreads threads
+// (also the call's other constants: log10 of the energies, zeroed counters)
 __global__ void __launch_bounds__(kPlanThreads) plan_chunks_kernel(IntegrateArgs a) {
   __shared__ double s_sum[kPlanThreads];
   __shared__ int s_scan[kPlanThreads];
   __shared__ int s_hist[64], s_cur[64];
   const int t = threadIdx.x;
+  for (int p = t; p < a.N_E; p += kPlanThreads) a.lgE[p] = log10(a.energies[p]);
+  if (t == 0) {
+    *a.item_next = 0;
+    *a.geo_count = 0;
+  }
   // total cost (fixed summation order)
   double sum = 0.0;
   for (int64_t r = t; r < a.n_rows; r += kPlanThreads) sum += a.row_cost[r];
@@ -2491,18 +2866,14 @@ __global__ void reduce_flux_kernel(IntegrateArgs a) {
 
 }  // namespace
 
-// each parallel's entry state of a table atmosphere's mu walk: the
-// geometry pre-pass, then the per-mesh scan in call order
-static void launch_table_state(const IntegrateArgs &a, cudaStream_t st) {
-  const size_t pre_smem = geometry_bytes(a.N_L, a.N_R);
-  static bool pre_attr = false;
-  if (!pre_attr) {
-    cudaFuncSetAttribute(num4d_prepass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
-    pre_attr = true;
-  }
-  num4d_prepass_kernel<<<(unsigned)a.n_rows, 128, pre_smem, st>>>(a);
-  num4d_scan_kernel<<<(a.n_members + 127) / 128, 128, 0, st>>>(a);
+// the geometry pre-pass and, for a table atmosphere, each parallel's entry
+// state of the mu walk: a scan of the parallels in call order
+static void launch_geometry(const IntegrateArgs &a, cudaStream_t st) {
+  const size_t smem = geometry_bytes(a.N_L, a.N_R);
+  // (the attribute is per device: set on every launch, which is cheap)
+  cudaFuncSetAttribute(geometry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  geometry_kernel<<<(unsigned)a.n_rows, 128, smem, st>>>(a);
+  if (a.atmos.I != nullptr) num4d_scan_kernel<<<(a.n_members + 127) / 128, 128, 0, st>>>(a);
 }
 
 size_t integrate_wsum_bytes(int N_P, int max_cells, int *w_cap) {
@@ -2511,30 +2882,32 @@ size_t integrate_wsum_bytes(int N_P, int max_cells, int *w_cap) {
   return integrate_wsum_bytes_dev(N_P, cap);
 }
 
+int64_t integrate_image_doubles(int N_L) { return image_doubles(N_L); }
+
+int integrate_energy_chunk(int N_L, int N_P, int N_E, int mixed) {
+  return energy_chunk(N_L, N_P, N_E,
+                      mixed ? (int)sizeof(PieceT<float>) : (int)sizeof(PieceDF));
+}
+
 void launch_integrate(const IntegrateArgs &a, cudaStream_t st) {
   if (a.n_members <= 0) return;
-  const int pb = a.mixed ? (int)sizeof(PieceT<float>) : (int)sizeof(PieceT<double>);
-  Layout L = make_layout(a.N_L, a.N_P, a.N_E, a.atmos.I ? a.atmos.nmu : 0,
-                         a.atmos.I ? a.atmos.nE : 0, pb, a.N_R, !a.mixed);
-  // class masks [N_L][2], run counts [2][N_P], the signal phases [N_P] and the
-  // groups' staged runs after the layout
-  const size_t bytes = L.bytes + (size_t)2 * a.N_L * sizeof(uint32_t) +
-                       (size_t)2 * a.N_P * sizeof(int) +
-                       (size_t)a.N_P * sizeof(float2) + 64 +
-                       (a.mixed ? 0 : (size_t)(kThreads / L.EC) * sizeof(RunStage));
+  const int nmu = a.atmos.I ? a.atmos.nmu : 0, nE = a.atmos.I ? a.atmos.nE : 0;
   // the work plan from the parallels' costs (needs the ray tables)
   if (a.n_rows > 0) row_cost_kernel<<<(unsigned)((a.n_rows * 32 + 255) / 256), 256, 0, st>>>(a);
   plan_chunks_kernel<<<1, kPlanThreads, 0, st>>>(a);
-  // the attribute is per device: set it on every launch (cheap)
-  if (a.atmos.I != nullptr) launch_table_state(a, st);
+  if (a.n_rows > 0) launch_geometry(a, st);
+  const long items = (long)a.max_chunks * a.n_eg;
+  const unsigned ctas = (unsigned)(items < a.ctas ? items : a.ctas);
   if (a.mixed) {
+    const size_t bytes = int_smem<true>(nullptr, a.N_L, a.N_P, a.EC, nmu, nE, a.table2d).bytes;
     cudaFuncSetAttribute(integrate_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          200 * 1024);
-    integrate_kernel<float><<<a.max_chunks, kThreads, bytes, st>>>(a);
+    integrate_kernel<float><<<ctas, kThreads, bytes, st>>>(a);
   } else {
+    const size_t bytes = int_smem<false>(nullptr, a.N_L, a.N_P, a.EC, nmu, nE, a.table2d).bytes;
     cudaFuncSetAttribute(integrate_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          200 * 1024);
-    integrate_kernel<double><<<a.max_chunks, kThreads, bytes, st>>>(a);
+    integrate_kernel<double><<<ctas, kThreads, bytes, st>>>(a);
   }
   dim3 grid((a.N_E * a.N_P + 255) / 256, a.n_members);
   reduce_flux_kernel<<<grid, 256, 0, st>>>(a);
@@ -2559,7 +2932,7 @@ int launch_stokes(const IntegrateArgs &a, cudaStream_t st) {
   const int nmu = a.atmos.I ? a.atmos.nmu : 0, nE = a.atmos.I ? a.atmos.nE : 0;
   const size_t smem = stokes_smem(a.N_L, a.N_P, a.N_E, a.N_R, nmu, nE);
   if (smem > 227 * 1024) return -2;
-  if (a.atmos.I != nullptr) launch_table_state(a, st);
+  if (a.atmos.I != nullptr) launch_geometry(a, st);
   if (cudaFuncSetAttribute(stokes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return -5;

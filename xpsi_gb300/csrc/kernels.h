@@ -44,6 +44,14 @@ struct Atmos4D {
   const float *I32;  // FP32 copy of the table for the mixed form (or null)
 };
 
+// what the integrator needs to know of a parallel, from the geometry pre-pass
+struct RowInfo {
+  long long geo;     // first image record, or -1: form them again
+  int images;        // images with records (bit 30: the next one terminates)
+  int cell;          // first radiating cell
+  float z_lo, z_hi;  // range of 1 / redshift over the lit columns
+};
+
 struct IntegrateArgs {
   int n_members;
   int64_t n_rows;
@@ -68,8 +76,9 @@ struct IntegrateArgs {
   Atmos4D atmos;
   // work chunks, planned on the device from per-parallel costs before the
   // integrator runs (integrator.cu, plan_chunks_kernel): chunk c covers rows
-  // [chunk_r0[c], chunk_r1[c]) of one member; the grid is max_chunks CTAs and
-  // CTA b takes chunk chunk_order[b] (heaviest first) while b < *chunk_count
+  // [chunk_r0[c], chunk_r1[c]) of one member.  An item is a chunk and one of
+  // n_eg groups of its energy chunks (of at most EC energies); `ctas` CTAs take
+  // items from the counter item_next, chunk_order[0] (heaviest) first
   int max_chunks;           // bound on the planned chunks (2 target + members)
   int target_chunks;        // chunks the plan aims at
   int64_t *chunk_r0, *chunk_r1;  // [max_chunks]
@@ -77,6 +86,16 @@ struct IntegrateArgs {
   int32_t *chunk_first;     // [n_members + 1] first chunk of each member
   int32_t *chunk_order;     // [max_chunks]
   int32_t *chunk_count;     // [1]
+  int n_eg, EC, ctas;
+  int32_t *item_next;       // [1]
+  double *lgE;              // [N_E] log10 of the energies
+  // geometry records (integrator.cu): geo_cap slots, then one per CTA;
+  // geo_count: slots taken; all null for launch_stokes
+  double *geo;
+  long long geo_cap;
+  unsigned long long *geo_count;
+  RowInfo *row_info;        // [rows]
+  int table2d;              // the atmosphere is a 2-D table (atm 4, 6)
   float *row_cost;          // [n_rows] scratch: estimated cost of each parallel
   float *chunk_cost;        // [max_chunks] scratch
   // Num4D call-history state (see integrator.cu)
@@ -84,14 +103,11 @@ struct IntegrateArgs {
   int32_t *member_status;   // [n_members]
   double *flux;             // [..] at members[m].flux_off
   double *flop_counter;     // algorithmic FLOPs of the launch (atomic), or null
-  double *slab;             // [max_chunks][nmu][nE] contracted Num4D table (scratch)
+  double *slab;             // [ctas][nmu][nE] contracted Num4D table (scratch)
   // power sums of the cell x phase sums (FP64 form; scratch, or null for the
-  // per-cell form): w_slots slots of 2 * w_cap * N_P run records, a CTA
-  // holding one (w_slot_busy[slot] = 1) while it runs, see integrator.cu
+  // per-cell form): 2 * w_cap * N_P run records per CTA, see integrator.cu
   unsigned char *wsum = nullptr;
   int w_cap = 0;            // runs per (cell half, signal phase)
-  int w_slots = 0;
-  int32_t *w_slot_busy = nullptr;  // [w_slots], zero before the launch
   int mixed;                // 0: FP64 drop-in, 1: mixed-precision form
   double *flux_q = nullptr, *flux_u = nullptr;  // Stokes Q, U (launch_stokes only)
   // Stokes Q of a 2-D table atmosphere (atm 4, 6; launch_stokes only):
@@ -108,9 +124,12 @@ struct SplitArgs {
 };
 void launch_split_reduce(const SplitArgs &a, cudaStream_t st);
 void launch_integrate(const IntegrateArgs &a, cudaStream_t st);
-// scratch bytes per chunk of the FP64 integrator's power sums for parallels
-// of at most max_cells cells (w_cap runs per cell half and signal phase)
+// scratch bytes per CTA of the FP64 integrator's power sums for parallels of
+// at most max_cells cells (w_cap runs per cell half and signal phase); doubles
+// of an image's geometry record; energies per chunk
 size_t integrate_wsum_bytes(int N_P, int max_cells, int *w_cap);
+int64_t integrate_image_doubles(int N_L);
+int integrate_energy_chunk(int N_L, int N_P, int N_E, int mixed);
 // Stokes I (a.flux), Q, U for blackbody (1) and burst blackbody (3) members;
 // a.partial: stokes_partial_doubles(a) doubles, zeroed; a.chunk_* unused
 size_t stokes_partial_doubles(const IntegrateArgs &a);

@@ -81,6 +81,8 @@ def estimate_bytes(ev: BT.BatchEvaluator, P) -> int:
     b += n_m * (N_E * N_P + ev.q * N_P + ev.K * N_P) * 8
     b += P.V * ev.K * 12 + P.V * 12
     b += 8 * 152 * (N_E * N_P * 8)           # chunk partials (bounded)
+    # the integrator's geometry records: two images per parallel
+    b += (2 * P.n_rows + 1024) * (4 * 8 + 1) * ev.N_L
     if ev.atmos is not None:
         b += 8 * 152 * ev.atmos.nmu * ev.atmos.nE * 8
     if getattr(P, "else_V", 0):
