@@ -5,20 +5,22 @@
 // (the packing of xpsi/HotRegion.py:774-1017 / Likelihood.py:297-432 that
 // the host path does in numpy).
 //
-// Four launches over all meshes of the batch:
-//   1. the 1000-point table of area(colat..lims[1]) per mesh, one thread per
-//      entry (1000 independent adaptive quadratures);
-//   2. per mesh: the cell area and the S - 1 parallels (one thread, the
-//      reference's running sum), then one thread per parallel for its
-//      centre colatitude, radius, gravity, tilt and the packed row values;
-//   3. one thread per cell: the corner / centre membership tests; cells
+// Seven launches over all meshes of the batch:
+//   1. the 1000-point table of area(colat..lims[1]) per mesh, one thread (few
+//      meshes: one warp) per entry (1000 independent adaptive quadratures);
+//   2. per mesh: the cell area, the S - 1 parallels and the columns' edges (the
+//      reference's running sums), and the trigonometry the cells share;
+//   3. one warp per parallel: its centre colatitude, radius, gravity, tilt and
+//      the packed row values;
+//   4. one thread per cell: the corner / centre membership tests; cells
 //      wholly inside or outside get their area at once, cells cut by a
 //      region boundary (~1 %) are queued;
-//   4. one CTA of two warps per queued cell, taken from a shared counter: its
+//   5. one CTA of two warps per queued cell, taken from a shared counter: its
 //      area quadrature, a panel to each warp (21 Gauss-Kronrod nodes over the
 //      lanes, the interval list in shared memory) -- the same adaptive scheme
-//      the host builder runs serially.
-// The per-thread quadratures of steps 1-2 keep their interval list (128
+//      the host builder runs serially; two more launches for the pieces of
+//      cells touched at a corner.
+// The serial quadratures of steps 1 and 3 keep their interval list (128
 // intervals) in local memory; the host builder's limit of 4000 gives bitwise
 // the same meshes (these integrals converge in far fewer intervals).
 #include <cuda_runtime.h>
@@ -45,65 +47,239 @@ struct MeshJob {
   int antiphased;
 };
 
+// The area integral of mesh_math.h (integrateArea) by a warp: the first
+// panel's 21 nodes, one per lane, summed in the serial rule's order (the same
+// bits); the integrand is smooth, so a panel that does not converge, which
+// takes the serial bisection, is the exception.
+__device__ double warp_area(double lo, double hi, const Star &s, int av, DWork &w) {
+  const int lane = threadIdx.x & 31;
+  const int NH = XG_K21_HALF - 1;  // 10
+  if (!(hi > lo)) return integrateArea(lo, hi, s, av, w);
+  const double c = 0.5 * (lo + hi), h = 0.5 * (hi - lo), ah = fabs(h);
+  double v = 0.0;
+  if (lane < 21) {
+    const int jn = lane < 10 ? lane : lane - 10;  // 0-9: c - dx_j, 10-19: c + dx_j, 20: c
+    double theta = c;
+    if (lane < 20) {
+      const double dx = h * XG_K21_X[jn];
+      theta = lane < 10 ? c - dx : c + dx;
+    }
+    if (!are_equal(theta, 0.0)) {
+      const double mu = cos(theta);
+      const double radius = radiusNormalised(mu, s.epsilon, s.zeta, s.shape);
+      const double ft = f_theta(mu, radius, s.epsilon, s.zeta, s.shape);
+      v = radius * radius * sqrt(1.0 + ft * ft) * sin(theta);
+      if (av != 0) v = theta * v;
+    }
+  }
+  const double fc = __shfl_sync(0xffffffffu, v, 20);
+  double rk = XG_K21_WK[NH] * fc, rg = XG_K21_WG[NH] * fc, ra = fabs(rk);
+#pragma unroll 1
+  for (int q = 0; q < NH; q++) {
+    const double f1 = __shfl_sync(0xffffffffu, v, q), f2 = __shfl_sync(0xffffffffu, v, q + 10);
+    rk += XG_K21_WK[q] * (f1 + f2);
+    rg += XG_K21_WG[q] * (f1 + f2);
+    ra += XG_K21_WK[q] * (fabs(f1) + fabs(f2));
+  }
+  const double mean = 0.5 * rk;
+  double rc = XG_K21_WK[NH] * fabs(fc - mean);
+#pragma unroll 1
+  for (int q = 0; q < NH; q++) {
+    const double f1 = __shfl_sync(0xffffffffu, v, q), f2 = __shfl_sync(0xffffffffu, v, q + 10);
+    rc += XG_K21_WK[q] * (fabs(f1 - mean) + fabs(f2 - mean));
+  }
+  const double r0 = rk * h;
+  ra *= ah;
+  rc *= ah;
+  double e = fabs((rk - rg) * h);
+  if (rc != 0.0 && e != 0.0) {
+    const double x = 200.0 * e / rc, sc = x * sqrt(x);
+    e = sc < 1.0 ? rc * sc : rc;
+  }
+  const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
+  if (ra > dmin / (50.0 * eps)) e = (e < 50.0 * eps * ra) ? 50.0 * eps * ra : e;
+  const double er = 1.0e-13, tol = er * fabs(r0);
+  const bool done = (e <= 50.0 * eps * ra && e > tol) || (e <= tol && e != rc) || e == 0.0;
+  if (!done || r0 == 0.0) return integrateArea(lo, hi, s, av, w);
+  return s.R_eq * s.R_eq * r0;
+}
+
+// one entry per thread (many meshes), or per warp (kWarp: up to kWarpTables
+// meshes, where the batch leaves the chip idle and a thread's chain of 21
+// nodes is what it waits for: one mesh 87 us by threads)
+constexpr int kWarpTables = 8;
+template <bool kWarp>
 __global__ void __launch_bounds__(128) mesh_table_kernel(const MeshJob *jobs, double *tab) {
   const int m = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = kWarp ? blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)
+                      : blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= kAreaTab) return;
   const MeshJob &J = jobs[m];
   DWork w;
-  tab[(size_t)m * kAreaTab + i] =
-      integrateArea(mesh_table_colat(J.pl, i), J.pl.lims[1], J.s, 0, w);
+  const double lo = mesh_table_colat(J.pl, i), hi = J.pl.lims[1];
+  if (kWarp) {
+    const double A = warp_area(lo, hi, J.s, 0, w);
+    if ((threadIdx.x & 31) == 0) tab[(size_t)m * kAreaTab + i] = A;
+  } else {
+    tab[(size_t)m * kAreaTab + i] = integrateArea(lo, hi, J.s, 0, w);
+  }
 }
 
-// per mesh: parallels, then the rows.  row_tmp[row] = (lower, upper, colatC,
-// effective gravity); mesh_tmp[m] = (cellArea, eta)
-__global__ void __launch_bounds__(128) mesh_rows_kernel(const MeshJob *jobs, const double *tab,
-                                                        xgpu_mesh_batch_out o, double *row_tmp,
-                                                        double *mesh_tmp) {
+// what the cells of a mesh share, formed once: the region with its angles'
+// cosines and sines, and per column the azimuth of its left edge (the
+// reference's running sum of cell widths) and the cosines its membership tests
+// need
+struct MeshTrig {
+  Region g;
+  double cos_cr;  // cos of the ceding radius
+};
+struct ColTrig {
+  double left, c_left, s_left, c_mid, s_mid;  // cos of the azimuth from each region's meridian
+};
+struct RowTmp {
+  double lower, upper, colat, effGrav;
+  double cl, sl, cu, su, cc, sc;  // cos and sin of lower, upper, colat
+};
+
+// per mesh: the cell area, the parallels, the columns' edges.  The running
+// sums (parallels' areas, edges) are single threads' chains of additions; the
+// rest is a thread per parallel or column.
+__global__ void __launch_bounds__(128) mesh_parallels_kernel(const MeshJob *jobs,
+                                                             const double *tab, double *par_out,
+                                                             double *mesh_tmp, MeshTrig *trig,
+                                                             ColTrig *cols, int S_max) {
   extern __shared__ double sm[];
-  double *colat = sm, *par = sm + kAreaTab;
+  double *colat = sm, *eta_i = sm + kAreaTab, *edge = eta_i + S_max;
   const int m = blockIdx.x;
   const MeshJob &J = jobs[m];
-  const size_t S = J.pl.S;
+  const int S = (int)J.pl.S;
   const double *T = tab + (size_t)m * kAreaTab;
+  double cellArea, eta;
+  mesh_cell_area(J.pl, T[kAreaTab - 1], cellArea, eta);
   for (int i = threadIdx.x; i < kAreaTab; i += blockDim.x) colat[i] = mesh_table_colat(J.pl, i);
-  __syncthreads();
-  __shared__ double s_eta;
   if (threadIdx.x == 0) {
-    double cellArea, eta;
-    mesh_cell_area(J.pl, T[kAreaTab - 1], cellArea, eta);
-    mesh_parallels(J.pl, colat, T, eta, par);
-    s_eta = eta;
+    double i_eta = (double)J.pl.S * eta;
+    for (int i = 0; i + 1 < S; i++) {
+      i_eta -= eta;
+      eta_i[i] = i_eta;
+    }
     mesh_tmp[2 * m] = cellArea;
     mesh_tmp[2 * m + 1] = eta;
   }
+  if (threadIdx.x == 32) {
+    double e = J.pl.polar ? -PI : -J.pl.boundary_phi;
+    for (int j = 0; j <= S; j++) {
+      edge[j] = e;
+      e = e + J.pl.delta_phi;
+    }
+    MeshTrig t;
+    t.g = mesh_region(J.pl);
+    t.cos_cr = t.g.cos_cede;
+    trig[m] = t;
+  }
   __syncthreads();
-  const double eta = s_eta;
-  for (size_t i = threadIdx.x; i < S; i += blockDim.x) {
-    double lower, upper;
-    mesh_row_bounds(J.pl, par, i, lower, upper);
-    DWork w;
-    const RowOut r = mesh_row(J.s, lower, upper, eta, w);
-    const int64_t row = J.row_off + (int64_t)i;
-    row_tmp[4 * row] = lower;
-    row_tmp[4 * row + 1] = upper;
-    row_tmp[4 * row + 2] = r.colat;
-    row_tmp[4 * row + 3] = r.effGrav;
-    // packed row values, as the host packing forms them
-    const double u = J.r_s / r.r;
+  for (int i = threadIdx.x; i + 1 < S; i += blockDim.x)
+    par_out[(size_t)m * S_max + i] = steffen_at(T, colat, kAreaTab, eta_i[i]);
+  for (int j = threadIdx.x; j <= S; j += blockDim.x) {
+    ColTrig c;
+    const double l = edge[j], mid = l + 0.5 * J.pl.delta_phi;
+    c.left = l;
+    c.c_left = cos(l);
+    c.s_left = cos(l - J.pl.superAzi);
+    c.c_mid = cos(mid);
+    c.s_mid = cos(mid - J.pl.superAzi);
+    cols[(size_t)m * (S_max + 1) + j] = c;
+  }
+}
+
+// a warp per parallel: its centre colatitude, radius, gravity and tilt, the
+// packed row values (as the host packing forms them), and what its cells need
+__global__ void __launch_bounds__(128) mesh_rows_kernel(const MeshJob *jobs, int n_mesh,
+                                                        int64_t n_rows, const double *par,
+                                                        int S_max, const double *mesh_tmp,
+                                                        xgpu_mesh_batch_out o, RowTmp *row_tmp) {
+  const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= n_rows) return;
+  int lo = 0, hi = n_mesh - 1;
+  while (lo < hi) {  // last mesh whose row_off <= row
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].row_off <= row) lo = mid; else hi = mid - 1;
+  }
+  const int m = lo;
+  const MeshJob &J = jobs[m];
+  const size_t i = (size_t)(row - J.row_off);
+  double lower, upper;
+  mesh_row_bounds(J.pl, par + (size_t)m * S_max, i, lower, upper);
+  const double eta = mesh_tmp[2 * m + 1];
+  DWork w;
+  RowOut r;
+  r.colat = warp_area(lower, upper, J.s, 1, w) / eta;
+  mesh_row_at(J.s, r);
+  const double u = J.r_s / r.r;
+  double C = (1.0 / u - J.R_over_rs);
+  C += log((1.0 / u - 1.0) / (J.R_over_rs - 1.0));
+  C *= J.r_s / kC;
+  // one sine and cosine instruction stream for the three colatitudes
+  const int lane = threadIdx.x & 31;
+  const double th = lane == 0 ? lower : lane == 1 ? upper : r.colat;
+  const double ct = cos(th), st = sin(th);
+  RowTmp t;
+  t.lower = lower; t.upper = upper; t.colat = r.colat; t.effGrav = r.effGrav;
+  t.cl = __shfl_sync(0xffffffffu, ct, 0); t.sl = __shfl_sync(0xffffffffu, st, 0);
+  t.cu = __shfl_sync(0xffffffffu, ct, 1); t.su = __shfl_sync(0xffffffffu, st, 1);
+  t.cc = __shfl_sync(0xffffffffu, ct, 2); t.sc = __shfl_sync(0xffffffffu, st, 2);
+  if (lane == 0) {
+    row_tmp[row] = t;
     o.u[row] = u;
     o.r_s[row] = J.r_s;
     o.maxAlpha[row] = r.maxAlpha;
     o.radius[row] = r.r;
     o.cos_gamma[row] = r.cos_gamma;
     o.theta0[row] = J.pl.invert ? PI - r.colat : r.colat;
-    double C = (1.0 / u - J.R_over_rs);
-    C += log((1.0 / u - 1.0) / (J.R_over_rs - 1.0));
-    C *= J.r_s / kC;
     o.lag_C[row] = C;
     o.lag_scale[row] = J.lag_scale;
     o.row_mesh[row] = m;
   }
+}
+
+// mesh_cell_kind from the shared trigonometry: each test "angular distance
+// to a region's centre <= its radius" is decided on cosines, with the bit
+// patterns; one closer than 1e-12 to its edge (the rounding of either side is
+// 1e-15), or with a cosine at 1 to rounding, whose arccosine may be NaN, takes
+// eval_psi's arccosine (a mesh has a few: the edge cells' corners touch the
+// region's boundary).  p1-p5 as there.
+__device__ int cell_kind(const MeshPlan &pl, const MeshTrig &t, const RowTmp &r, const ColTrig &a,
+                         const ColTrig &b, size_t i) {
+  const Region &g = t.g;
+  auto near = [](double x, double cR) {
+    return negative(fabs(x - cR) - 1.0e-12) || !negative(fabs(x) - (1.0 - 1.0e-12));
+  };
+  auto corner = [&](double ct, double st, const double cphi, const double sphi) {
+    const double x = g.cos_colat * ct + g.sin_colat * st * cphi;
+    const bool in = near(x, t.cos_cr) ? acos(x) <= pl.cedeRadius : negative(t.cos_cr - x);
+    if (!in) return 2;
+    const double y = g.cos_sc * ct + g.sin_sc * st * sphi;
+    return (near(y, g.cos_sr) ? pl.superRadius <= acos(y) : negative(y - g.cos_sr)) ? 1 : 0;
+  };
+  int p1, p3;
+  const bool pole = pl.polar && i == 0;
+  if (pole) {
+    p1 = p3 = pl.cedeColat <= pl.cedeRadius ? (pl.superRadius <= pl.superColat ? 1 : 0) : 2;
+  } else {
+    p1 = corner(r.cl, r.sl, a.c_left, a.s_left);
+    p3 = corner(r.cl, r.sl, b.c_left, b.s_left);
+  }
+  const int p2 = corner(r.cu, r.su, a.c_left, a.s_left);
+  const int p4 = corner(r.cu, r.su, b.c_left, b.s_left);
+  const int p5 = corner(r.cc, r.sc, a.c_mid, a.s_mid);
+  if (!(p1 == p2 && p2 == p3 && p3 == p4 && p4 == p5)) return 2;
+  if (pl.superRadius > 0.0) {
+    auto in = [&](const double *q) {
+      return r.lower <= q[0] && q[0] <= r.upper && a.left <= q[1] && q[1] <= b.left;
+    };
+    if (in(pl.sp1) || in(pl.sp2) || in(pl.sp3) || in(pl.sp4)) return 2;
+  }
+  return p5 == 1 ? 1 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -311,18 +487,27 @@ __device__ double cta_qag21(const F &f, double a, double b, double epsabs, doubl
   return r;
 }
 
+// piece k of the dyadic cut of [lo, hi] toward an endpoint; false past the
+// last one (the cut has reached the endpoint's rounding)
+__device__ __forceinline__ bool dyadic_piece(double lo, double hi, bool toward_lo, int k,
+                                             double &p0, double &p1) {
+  const double Lw = hi - lo;
+  const double s1 = ldexp(Lw, -(k + 1)), s0 = ldexp(Lw, -k);
+  p0 = toward_lo ? lo + s1 : hi - s0;
+  p1 = toward_lo ? lo + s0 : hi - s1;
+  return p0 < p1 && !(toward_lo ? p0 <= lo : p1 >= hi);
+}
+// the sum over the pieces in turn, until four are negligible; the first
+// n_done pieces' integrals are given
 template <typename F>
 __device__ double cta_dyadic(const F &f, double lo, double hi, bool toward_lo, double er,
-                             CutList &L) {
-  const double Lw = hi - lo;
+                             CutList &L, const double *done, int n_done) {
   double sum = 0.0;
   int seen = 0, quiet = 0;
   for (int k = 0; k < 2100; k++) {
-    const double s1 = ldexp(Lw, -(k + 1)), s0 = ldexp(Lw, -k);
-    const double p0 = toward_lo ? lo + s1 : hi - s0;
-    const double p1 = toward_lo ? lo + s0 : hi - s1;
-    if (!(p0 < p1) || (toward_lo ? p0 <= lo : p1 >= hi)) break;
-    const double r = cta_qag21(f, p0, p1, 0.0, er, L);
+    double p0, p1;
+    if (!dyadic_piece(lo, hi, toward_lo, k, p0, p1)) break;
+    const double r = k < n_done ? done[k] : cta_qag21(f, p0, p1, 0.0, er, L);
     sum += r;
     if (r != 0.0) seen = 1;
     if (seen && fabs(r) <= 1.0e-17 * fabs(sum)) {
@@ -334,24 +519,45 @@ __device__ double cta_dyadic(const F &f, double lo, double hi, bool toward_lo, d
   return sum;
 }
 
+// the relative tolerance integrate() (mesh_math.h) runs at for CQUAD's 1e-8
+constexpr double kCutTol = 1.0e-13;
+
+// an integral whose interior nodes all see zero but an endpoint does not, cut
+// in two halves: dyadic pieces toward such an endpoint, else plainly
+struct DyadicSplit {
+  double a, b;
+  bool at_a, at_b;
+};
 template <typename F>
-__device__ double cta_integrate(const F &f, double a, double b, double epsabs, double epsrel,
-                                CutList &L) {
+__device__ double cta_halves(const F &f, const DyadicSplit &d, CutList &L, const double *done,
+                             int n_done) {
+  const double m = 0.5 * (d.a + d.b);
+  const double rl = d.at_a ? cta_dyadic(f, d.a, m, true, kCutTol, L, done, n_done)
+                    : n_done ? done[0] : cta_qag21(f, d.a, m, 0.0, kCutTol, L);
+  const double rr = d.at_b ? cta_dyadic(f, m, d.b, false, kCutTol, L, done + n_done, n_done)
+                    : n_done ? done[n_done] : cta_qag21(f, m, d.b, 0.0, kCutTol, L);
+  return rl + rr;
+}
+// integrate() of mesh_math.h over [a, b], a < b; true in `split` (when asked
+// for): the halves of d are left to the caller
+template <typename F>
+__device__ double cta_integrate(const F &f, double a, double b, CutList &L, DyadicSplit *d,
+                                bool &split) {
+  split = false;
   double sign = 1.0;
   if (b < a) { const double t = a; a = b; b = t; sign = -1.0; }
   if (a == b) return 0.0;
-  double er = (1.0e-13 < epsrel) ? 1.0e-13 : epsrel;
-  if (epsabs <= 0.0 && er < 50.0 * 2.220446049250313e-16) er = 50.0 * 2.220446049250313e-16;
-  double r = cta_qag21(f, a, b, epsabs, er, L);
+  double r = cta_qag21(f, a, b, 0.0, kCutTol, L);
   if (r == 0.0) {
     const double fa = f(a), fb = f(b);
     if (fa != 0.0 || fb != 0.0) {
-      const double m = 0.5 * (a + b);
-      const double rl = fa != 0.0 ? cta_dyadic(f, a, m, true, er, L)
-                                  : cta_qag21(f, a, m, 0.0, er, L);
-      const double rr = fb != 0.0 ? cta_dyadic(f, m, b, false, er, L)
-                                  : cta_qag21(f, m, b, 0.0, er, L);
-      r = rl + rr;
+      const DyadicSplit h{a, b, fa != 0.0, fb != 0.0};
+      if (d != nullptr && sign > 0.0) {
+        *d = h;
+        split = true;
+        return 0.0;
+      }
+      r = cta_halves(f, h, L, nullptr, 0);
     }
   }
   return sign * r;
@@ -381,8 +587,10 @@ __device__ __forceinline__ void put_area(const MeshJob &J, xgpu_mesh_batch_out &
 // one thread per cell of the batch (cells of mesh m at [cell_off, cell_off + S^2))
 __global__ void __launch_bounds__(128) mesh_cells_kernel(const MeshJob *jobs, int n_mesh,
                                                          int64_t n_cells, xgpu_mesh_batch_out o,
-                                                         const double *row_tmp,
+                                                         const RowTmp *row_tmp,
                                                          const double *mesh_tmp,
+                                                         const MeshTrig *trig,
+                                                         const ColTrig *cols, int S_max,
                                                          int64_t *queue, unsigned *n_queue) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n_cells) return;
@@ -391,19 +599,18 @@ __global__ void __launch_bounds__(128) mesh_cells_kernel(const MeshJob *jobs, in
   const size_t S = J.pl.S;
   const int64_t k = c - J.cell_off;
   const size_t i = (size_t)(k / (int64_t)S), j = (size_t)(k - (int64_t)i * (int64_t)S);
-  const int64_t row = J.row_off + (int64_t)i;
+  const RowTmp &r = row_tmp[J.row_off + (int64_t)i];
   // azimuth (shifted by the omitted region's azimuth, half a turn when
   // antiphased) and the atmosphere parameters of the cell
   double ph = mesh_phi(J.pl, j) - J.omit_azimuth;
   if (J.antiphased) ph = ph + PI;
   o.phi[c] = ph;
   o.params[2 * c] = J.logT;
-  o.params[2 * c + 1] = row_tmp[4 * row + 3];
+  o.params[2 * c + 1] = r.effGrav;
   const size_t j_max = J.pl.j_max;
   if (j < j_max) {
-    double leftmost, rightmost;
-    const int kind = mesh_cell_kind(J.pl, i, j, row_tmp[4 * row], row_tmp[4 * row + 1],
-                                    row_tmp[4 * row + 2], leftmost, rightmost);
+    const ColTrig *ct = cols + (size_t)m * (S_max + 1) + j;
+    const int kind = cell_kind(J.pl, trig[m], r, ct[0], ct[1], i);
     if (kind == 2) queue[atomicAdd(n_queue, 1u)] = c;
     else put_area(J, o, c, i, j, kind == 1 ? mesh_tmp[2 * m] : 0.0);
   } else if (!J.pl.sym || j < S - j_max) {
@@ -413,6 +620,54 @@ __global__ void __launch_bounds__(128) mesh_cells_kernel(const MeshJob *jobs, in
   }
 }
 
+// A cell that a region's arc touches at a corner only has an integral that the
+// first panel's nodes miss and its dyadic pieces resolve, some 60 quadratures
+// of about 7 bisections each: in turn 400 steps, ten times any other cell, so
+// its pieces are set aside (room for `cap` cells; one that finds none runs
+// them in turn), integrated a CTA each, and summed in order at the end.
+constexpr int kPieces = 64;  // of a half; what lies beyond is integrated in turn
+struct SplitCell {
+  int64_t cell;
+  DyadicSplit d;
+};
+struct SplitList {
+  SplitCell *cells;
+  double *piece;    // [cap][2][kPieces]
+  unsigned *count;  // cells set aside; the piece items' counter
+  unsigned cap;
+};
+
+// a queued cell's integrand
+__device__ __forceinline__ void cut_cell(const MeshJob *jobs, int n_mesh, const RowTmp *row_tmp,
+                                         const MeshTrig *trig, const ColTrig *cols, int S_max,
+                                         int64_t c, int &m, size_t &i, size_t &j, double &lower,
+                                         double &upper, CutCell &f) {
+  m = mesh_of_cell(jobs, n_mesh, c);
+  const MeshJob &J = jobs[m];
+  const size_t S = J.pl.S;
+  const int64_t k = c - J.cell_off;
+  i = (size_t)(k / (int64_t)S);
+  j = (size_t)(k - (int64_t)i * (int64_t)S);
+  const RowTmp &r = row_tmp[J.row_off + (int64_t)i];
+  lower = r.lower;
+  upper = r.upper;
+  const ColTrig *ct = cols + (size_t)m * (S_max + 1) + j;
+  f.init(CellIntegrand{J.s, trig[m].g, ct[0].left, ct[1].left}, lower, upper);
+}
+// the area from the first integral: the reference integrates again between
+// the boundary's crossings where it vanishes
+__device__ __forceinline__ void finish_cell(const MeshJob &J, xgpu_mesh_batch_out &o, int64_t c,
+                                            size_t i, size_t j, double lower, double upper,
+                                            const CutCell &f, double integral, CutList &L) {
+  if (are_equal(integral, 0.0)) {
+    double tmin, tmax;
+    bool split;
+    if (cell_fallback_interval(lower, upper, f.f.pa, f.f.pb, f.f.g, tmin, tmax))
+      integral = cta_integrate(f, tmin, tmax, L, nullptr, split);
+  }
+  if (threadIdx.x == 0) put_area(J, o, c, i, j, J.s.R_eq * J.s.R_eq * integral);
+}
+
 // one CTA per queued cell: the area quadrature of a cell cut by a boundary.
 // A CTA starts with the cell of its own index (a small batch's cells spread
 // over the SMs) and takes the next from a shared counter (n_queue[1]) when it
@@ -420,36 +675,86 @@ __global__ void __launch_bounds__(128) mesh_cells_kernel(const MeshJob *jobs, in
 // steps); each cell's result is independent of which CTA integrates it.
 constexpr int kCutCtasPerSm = 8;
 __global__ void __launch_bounds__(kCutThreads, kCutCtasPerSm) mesh_boundary_kernel(
-    const MeshJob *jobs, int n_mesh, xgpu_mesh_batch_out o, const double *row_tmp,
-    const int64_t *queue, unsigned *n_queue) {
+    const MeshJob *jobs, int n_mesh, xgpu_mesh_batch_out o, const RowTmp *row_tmp,
+    const MeshTrig *trig, const ColTrig *cols, int S_max, const int64_t *queue,
+    unsigned *n_queue, SplitList sl) {
   __shared__ CutList L;
   __shared__ unsigned s_q;
   const unsigned n = n_queue[0];
   for (unsigned q = blockIdx.x; q < n; q = s_q) {
     const int64_t c = queue[q];
-    const int m = mesh_of_cell(jobs, n_mesh, c);
-    const MeshJob &J = jobs[m];
-    const size_t S = J.pl.S;
-    const int64_t k = c - J.cell_off;
-    const size_t i = (size_t)(k / (int64_t)S), j = (size_t)(k - (int64_t)i * (int64_t)S);
-    const int64_t row = J.row_off + (int64_t)i;
-    const double lower = row_tmp[4 * row], upper = row_tmp[4 * row + 1];
-    double pa, pb;
-    mesh_cell_kind(J.pl, i, j, lower, upper, row_tmp[4 * row + 2], pa, pb);
-    const Region g = mesh_region(J.pl);
+    int m;
+    size_t i, j;
+    double lower, upper;
     CutCell f;
-    f.init(CellIntegrand{J.s, g, pa, pb}, lower, upper);
-    double integral = cta_integrate(f, lower, upper, 0.0, 1.0e-8, L);
-    if (are_equal(integral, 0.0)) {
-      double tmin, tmax;
-      if (cell_fallback_interval(lower, upper, pa, pb, g, tmin, tmax))
-        integral = cta_integrate(f, tmin, tmax, 0.0, 1.0e-8, L);
-    }
+    cut_cell(jobs, n_mesh, row_tmp, trig, cols, S_max, c, m, i, j, lower, upper, f);
+    DyadicSplit d;
+    bool split;
+    double integral = cta_integrate(f, lower, upper, L, &d, split);
     __syncthreads();  // every thread has read the last s_q
-    if (threadIdx.x == 0) {
-      put_area(J, o, c, i, j, J.s.R_eq * J.s.R_eq * integral);
-      s_q = gridDim.x + atomicAdd(&n_queue[1], 1u);
+    if (split) {
+      if (threadIdx.x == 0) {
+        const unsigned at = atomicAdd(&sl.count[0], 1u);
+        if (at < sl.cap) sl.cells[at] = SplitCell{c, d};
+        s_q = at;
+      }
+      __syncthreads();
+      const bool room = s_q < sl.cap;
+      __syncthreads();
+      if (!room) integral = cta_halves(f, d, L, nullptr, 0);
+      split = room;
     }
+    if (!split) finish_cell(jobs[m], o, c, i, j, lower, upper, f, integral, L);
+    if (threadIdx.x == 0) s_q = gridDim.x + atomicAdd(&n_queue[1], 1u);
+    __syncthreads();
+  }
+}
+
+// the dyadic pieces of the cells set aside, one CTA per piece
+__global__ void __launch_bounds__(kCutThreads, kCutCtasPerSm) mesh_pieces_kernel(
+    const MeshJob *jobs, int n_mesh, const RowTmp *row_tmp, const MeshTrig *trig,
+    const ColTrig *cols, int S_max, SplitList sl) {
+  __shared__ CutList L;
+  __shared__ unsigned s_q;
+  const unsigned n = min(sl.count[0], sl.cap) * (2u * kPieces);
+  for (unsigned q = blockIdx.x; q < n; q = s_q) {
+    const SplitCell sc = sl.cells[q / (2u * kPieces)];
+    const unsigned h = (q / kPieces) & 1u, k = q % kPieces;
+    const DyadicSplit &d = sc.d;
+    const double mid = 0.5 * (d.a + d.b), lo = h ? mid : d.a, hi = h ? d.b : mid;
+    double p0 = lo, p1 = hi;
+    const bool any = (h ? d.at_b : d.at_a) ? dyadic_piece(lo, hi, h == 0, (int)k, p0, p1) : k == 0;
+    if (any) {
+      int m;
+      size_t i, j;
+      double lower, upper;
+      CutCell f;
+      cut_cell(jobs, n_mesh, row_tmp, trig, cols, S_max, sc.cell, m, i, j, lower, upper, f);
+      const double r = cta_qag21(f, p0, p1, 0.0, kCutTol, L);
+      if (threadIdx.x == 0) sl.piece[q] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_q = gridDim.x + atomicAdd(&sl.count[1], 1u);
+    __syncthreads();
+  }
+}
+
+// ... and their areas, one CTA per cell
+__global__ void __launch_bounds__(kCutThreads) mesh_split_kernel(
+    const MeshJob *jobs, int n_mesh, xgpu_mesh_batch_out o, const RowTmp *row_tmp,
+    const MeshTrig *trig, const ColTrig *cols, int S_max, SplitList sl) {
+  __shared__ CutList L;
+  const unsigned n = min(sl.count[0], sl.cap);
+  for (unsigned q = blockIdx.x; q < n; q += gridDim.x) {
+    const SplitCell sc = sl.cells[q];
+    int m;
+    size_t i, j;
+    double lower, upper;
+    CutCell f;
+    cut_cell(jobs, n_mesh, row_tmp, trig, cols, S_max, sc.cell, m, i, j, lower, upper, f);
+    const double integral =
+        cta_halves(f, sc.d, L, sl.piece + (size_t)q * 2 * kPieces, kPieces);
+    finish_cell(jobs[m], o, sc.cell, i, j, lower, upper, f, integral, L);
     __syncthreads();
   }
 }
@@ -487,36 +792,65 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
     S_max = std::max(S_max, q.S);
   }
   if (rows != n_rows || cells != n_cells) return -2;
-  MeshJob *d_jobs = nullptr;
-  double *tab = nullptr, *row_tmp = nullptr, *mesh_tmp = nullptr;
-  int64_t *queue = nullptr;
-  unsigned *n_queue = nullptr;
-  if (cudaMallocAsync(&d_jobs, sizeof(MeshJob) * (size_t)n, st) != cudaSuccess) return -5;
-  if (cudaMallocAsync(&tab, sizeof(double) * (size_t)n * kAreaTab, st) != cudaSuccess ||
-      cudaMallocAsync(&row_tmp, sizeof(double) * 4 * (size_t)n_rows, st) != cudaSuccess ||
-      cudaMallocAsync(&mesh_tmp, sizeof(double) * 2 * (size_t)n, st) != cudaSuccess ||
-      cudaMallocAsync(&queue, sizeof(int64_t) * (size_t)n_cells, st) != cudaSuccess ||
-      cudaMallocAsync(&n_queue, 2 * sizeof(unsigned), st) != cudaSuccess) {
-    cudaFreeAsync(d_jobs, st);
-    return -5;
-  }
+  // one allocation for the call's scratch, parts at 256-byte boundaries
+  const int S_m = (int)S_max;
+  size_t total = 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  const size_t o_jobs = part(sizeof(MeshJob) * (size_t)n);
+  const size_t o_tab = part(sizeof(double) * (size_t)n * kAreaTab);
+  const size_t o_row = part(sizeof(RowTmp) * (size_t)n_rows);
+  const size_t o_mesh = part(sizeof(double) * 2 * (size_t)n);
+  const size_t o_par = part(sizeof(double) * (size_t)n * S_max);
+  const size_t o_trig = part(sizeof(MeshTrig) * (size_t)n);
+  const size_t o_cols = part(sizeof(ColTrig) * (size_t)n * (S_max + 1));
+  const size_t o_queue = part(sizeof(int64_t) * (size_t)n_cells);
+  const size_t o_count = part(4 * sizeof(unsigned));
+  SplitList sl{};
+  sl.cap = (unsigned)(4 * (size_t)n + 64);
+  const size_t o_split = part(sizeof(SplitCell) * sl.cap);
+  const size_t o_piece = part(sizeof(double) * 2 * kPieces * sl.cap);
+  unsigned char *base = nullptr;
+  if (cudaMallocAsync(reinterpret_cast<void **>(&base), total, st) != cudaSuccess) return -5;
+  MeshJob *d_jobs = reinterpret_cast<MeshJob *>(base + o_jobs);
+  double *tab = reinterpret_cast<double *>(base + o_tab);
+  RowTmp *row_tmp = reinterpret_cast<RowTmp *>(base + o_row);
+  double *mesh_tmp = reinterpret_cast<double *>(base + o_mesh);
+  double *par = reinterpret_cast<double *>(base + o_par);
+  MeshTrig *trig = reinterpret_cast<MeshTrig *>(base + o_trig);
+  ColTrig *cols = reinterpret_cast<ColTrig *>(base + o_cols);
+  int64_t *queue = reinterpret_cast<int64_t *>(base + o_queue);
+  unsigned *n_queue = reinterpret_cast<unsigned *>(base + o_count);
+  sl.cells = reinterpret_cast<SplitCell *>(base + o_split);
+  sl.piece = reinterpret_cast<double *>(base + o_piece);
+  sl.count = n_queue + 2;
   // (a copy from pageable memory has been staged when cudaMemcpyAsync
   // returns, so the host jobs may go out of scope)
   cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(MeshJob) * (size_t)n, cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(n_queue, 0, 2 * sizeof(unsigned), st);  // queue length, next cell
-  mesh_table_kernel<<<dim3((kAreaTab + 127) / 128, (unsigned)n), 128, 0, st>>>(d_jobs, tab);
-  const size_t smem = sizeof(double) * (kAreaTab + S_max);
-  mesh_rows_kernel<<<(unsigned)n, 128, smem, st>>>(d_jobs, tab, *out, row_tmp, mesh_tmp);
+  // queue length, next cell; cells set aside, next piece
+  cudaMemsetAsync(n_queue, 0, 4 * sizeof(unsigned), st);
+  if (n <= kWarpTables)
+    mesh_table_kernel<true><<<dim3((kAreaTab + 3) / 4, (unsigned)n), 128, 0, st>>>(d_jobs, tab);
+  else
+    mesh_table_kernel<false><<<dim3((kAreaTab + 127) / 128, (unsigned)n), 128, 0, st>>>(d_jobs,
+                                                                                       tab);
+  const size_t smem = sizeof(double) * (kAreaTab + 2 * S_max + 1);
+  mesh_parallels_kernel<<<(unsigned)n, 128, smem, st>>>(d_jobs, tab, par, mesh_tmp, trig, cols,
+                                                        S_m);
+  mesh_rows_kernel<<<(unsigned)((n_rows + 3) / 4), 128, 0, st>>>(d_jobs, n, n_rows, par, S_m,
+                                                                 mesh_tmp, *out, row_tmp);
   mesh_cells_kernel<<<(unsigned)((n_cells + 127) / 128), 128, 0, st>>>(
-      d_jobs, n, n_cells, *out, row_tmp, mesh_tmp, queue, n_queue);
-  mesh_boundary_kernel<<<152 * kCutCtasPerSm, kCutThreads, 0, st>>>(d_jobs, n, *out, row_tmp,
-                                                                     queue, n_queue);
+      d_jobs, n, n_cells, *out, row_tmp, mesh_tmp, trig, cols, S_m, queue, n_queue);
+  mesh_boundary_kernel<<<152 * kCutCtasPerSm, kCutThreads, 0, st>>>(
+      d_jobs, n, *out, row_tmp, trig, cols, S_m, queue, n_queue, sl);
+  mesh_pieces_kernel<<<152 * kCutCtasPerSm, kCutThreads, 0, st>>>(d_jobs, n, row_tmp, trig, cols,
+                                                                 S_m, sl);
+  mesh_split_kernel<<<(unsigned)std::min<size_t>(sl.cap, 152), kCutThreads, 0, st>>>(
+      d_jobs, n, *out, row_tmp, trig, cols, S_m, sl);
   const cudaError_t e = cudaGetLastError();
-  cudaFreeAsync(d_jobs, st);
-  cudaFreeAsync(tab, st);
-  cudaFreeAsync(row_tmp, st);
-  cudaFreeAsync(mesh_tmp, st);
-  cudaFreeAsync(queue, st);
-  cudaFreeAsync(n_queue, st);
+  cudaFreeAsync(base, st);
   return e == cudaSuccess ? 0 : -5;
 }

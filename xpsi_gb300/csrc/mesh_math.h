@@ -512,64 +512,77 @@ struct CutCell {
     st = sin(theta);
 #endif
     const Region &g = f.g;
-    const int cede = side(g.cos_cede - g.cos_colat * mu, g.sin_colat * st, c_near, c_far);
+    const double na = g.cos_cede - g.cos_colat * mu, da = g.sin_colat * st;
+    const double nc = g.cos_sr - g.cos_sc * mu, dc = g.sin_sc * st;
+    const int cede = side(na, da, c_near, c_far);
     if (cede == 2) return 0.0;
-    double dphi;
     const bool far = no_super || negative(g.superRadius - fabs(theta - g.superColat));
-    const int sup = far ? 2 : side(g.cos_sr - g.cos_sc * mu, g.sin_sc * st, s_near, s_far);
+    const int sup = far ? 2 : side(nc, dc, s_near, s_far);
     if (sup == 1) return 0.0;
-    if (cede == 1 && sup == 2) {
-      dphi = f.pb - f.pa;
-    } else {
-      bool zero;
-      dphi = extent(theta, mu, st, cede == 1, far, sup == 2, zero);
-      if (zero || ordered_bits(dphi) == 0) return 0.0;
+    double dphi = f.pb - f.pa;
+    if (cede == 0 || sup == 0) {
+      // the boundary azimuths that matter: one inverse cosine for the lanes
+      // that need one of the two, a second only for those that need both
+      const double phi1 = edge_azimuth(cede == 0 ? na : nc, cede == 0 ? da : dc);
+      double phi2 = phi1;
+      if (cede == 0 && sup == 0) phi2 = edge_azimuth(nc, dc);
+      dphi = extent(theta, cede, sup, far, phi1, phi2);
+      if (ordered_bits(dphi) == 0) return 0.0;
     }
     const Star &s = f.s;
     const double radius = radiusNormalised(mu, s.epsilon, s.zeta, s.shape);
     const double ft2 = f_theta_sq(mu, st, radius, s.epsilon, s.zeta, s.shape);
     return dphi * radius * radius * sqrt(1.0 + ft2) * st;
   }
-  // ring_extent with the ceding arc known to hold the whole cell (cede_in:
-  // any arc beyond the cell gives the same bits, so the full circle stands
-  // in), the superseding arc absent at this colatitude (far) or known to
-  // miss the cell (sup_out)
-  XG_HD double extent(double theta, double mu, double st, bool cede_in, bool far, bool sup_out,
-                      bool &zero) const {
+  // eval_phi_cs from its numerator and denominator (the range check by bits)
+  XG_HD static double edge_azimuth(double num, double den) {
+    const double c = num / den;
+    if (negative(c + 1.0) || negative(1.0 - c) || c != c) return -1.0;
+    return acos(c);
+  }
+  // ring_extent from the boundary azimuths (aUB the ceding arc's, cUB the
+  // superseding one's; -1 where the ring does not meet the boundary), 0 where
+  // it reports none.  cede 1: the ceding arc holds the whole cell, any arc
+  // beyond the cell gives the same bits and the full circle stands in; sup 2:
+  // the superseding arc misses the cell or (far) is absent, when it counts as
+  // the empty arc at azimuth 0
+  XG_HD double extent(double theta, int cede, int sup, bool far, double aUB, double cUB) const {
     const Region &g = f.g;
-    zero = false;
-    if (sup_out) {
-      const double aUB = eval_phi_cs(mu, st, g.cos_colat, g.sin_colat, g.cos_cede);
-      if (negative(aUB)) {
-        zero = !(theta + g.colat < g.cedeRadius);
-        if (zero) return 0.0;
-        return far ? get_interval_bits(f.pa, f.pb, -PI, 0.0) +
-                         get_interval_bits(f.pa, f.pb, 0.0, PI)
-                   : get_interval_bits(f.pa, f.pb, -PI, PI);
-      }
-      if (far && ordered_bits(aUB) > 0)
-        // the absent arc is the empty one at azimuth 0
-        return get_interval_bits(f.pa, f.pb, -aUB, 0.0) +
-               get_interval_bits(f.pa, f.pb, 0.0, aUB);
-      return get_interval_bits(f.pa, f.pb, -aUB, aUB);
+    const double pa = f.pa, pb = f.pb;
+    auto I = [&](double lo, double hi) { return get_interval_bits(pa, pb, lo, hi); };
+    if (cede == 1) aUB = PI;
+    else if (negative(aUB)) {
+      if (!(theta + g.colat < g.cedeRadius)) return 0.0;
+      aUB = PI;
     }
-    if (cede_in) {
-      // the superseding arc cuts the cell (or may)
-      double cUB = eval_phi_cs(mu, st, g.cos_sc, g.sin_sc, g.cos_sr);
-      if (negative(cUB)) {
-        zero = true;
-        return 0.0;
-      }
-      double cLB = -cUB;
+    const double aLB = -aUB;
+    if (sup == 2 && !far) return I(aLB, aUB);
+    double cLB = 0.0;
+    if (far) {
+      cUB = 0.0;
+    } else {
+      if (negative(cUB)) return 0.0;
+      cLB = -cUB;
       cUB += g.superAzi;
       cLB += g.superAzi;
       if (negative(PI - cUB)) cUB -= TWO_PI;
       if (negative(cLB + PI)) cLB += TWO_PI;
-      if (ordered_bits(cUB) >= ordered_bits(cLB))
-        return get_interval_bits(f.pa, f.pb, -PI, cLB) + get_interval_bits(f.pa, f.pb, cUB, PI);
-      return get_interval_bits(f.pa, f.pb, cUB, cLB);
     }
-    return ring_extent(theta, mu, st, g, true, f.pa, f.pb, zero);
+    const long long bu = ordered_bits(cUB), bl = ordered_bits(cLB);
+    const long long au = ordered_bits(aUB), al = ordered_bits(aLB);
+    if (bu >= bl) {
+      if (bl >= au || bu <= al) return I(aLB, aUB);
+      if (bl >= al && bu <= au) return I(aLB, cLB) + I(cUB, aUB);
+      if (bl < al && al < bu && bu <= au) return I(cUB, aUB);
+      if (al <= bl && bl < au && au < bu) return I(aLB, cLB);
+      return 0.0;
+    }
+    if (bu >= au || bl <= al) return 0.0;
+    if (bu >= al && bl <= au) return I(cUB, cLB);
+    if (bu < al && al < bl && bl <= au) return I(aLB, cLB);
+    if (al <= bu && bu < au && au < bl) return I(cUB, aUB);
+    if (bu < al && bl > au) return I(aLB, aUB);
+    return 0.0;
   }
 };
 
@@ -792,11 +805,9 @@ struct RowOut {
 };
 
 // per-parallel quantities: the area-weighted centre colatitude, radius,
-// effective gravity and surface tilt (mesh.pyx:140-170)
-template <typename W>
-XG_QD inline RowOut mesh_row(const Star &s, double lower, double upper, double eta, W &w) {
-  RowOut o;
-  o.colat = integrateArea(lower, upper, s, 1, w) / eta;
+// effective gravity and surface tilt (mesh.pyx:140-170); mesh_row_at: from the
+// colatitude
+XG_HD inline void mesh_row_at(const Star &s, RowOut &o) {
   const double mu = cos(o.colat);
   const double radius = radiusNormalised(mu, s.epsilon, s.zeta, s.shape);
   o.r = radius * s.R_eq;
@@ -804,6 +815,12 @@ XG_QD inline RowOut mesh_row(const Star &s, double lower, double upper, double e
   const double ft = f_theta(mu, radius, s.epsilon, s.zeta, s.shape);
   o.cos_gamma = 1.0 / sqrt(1.0 + ft * ft);
   o.maxAlpha = PI_2 + acos(o.cos_gamma);
+}
+template <typename W>
+XG_QD inline RowOut mesh_row(const Star &s, double lower, double upper, double eta, W &w) {
+  RowOut o;
+  o.colat = integrateArea(lower, upper, s, 1, w) / eta;
+  mesh_row_at(s, o);
   return o;
 }
 
