@@ -332,6 +332,15 @@ int xgpu_rays_batch(int64_t n_rows, int N_R, const double *u,
                     double *cos_alpha, double *lag, double *maxDeflection,
                     int32_t *row_status, const double *lag_C,
                     const double *lag_scale, void *stream);
+/* The same with a choice of each integral's first panel: 31 points, which most
+ * rays need no more than (xgpu_rays_batch), or 61, the reference's rule from
+ * the start.  The two agree to 1e-14; what rounds to FP32 downstream (the
+ * mixed form) keeps its values to the last bit with 61. */
+int xgpu_rays_batch_rule(int64_t n_rows, int N_R, const double *u,
+                         const double *r_s, double *maxAlpha, double *deflection,
+                         double *cos_alpha, double *lag, double *maxDeflection,
+                         int32_t *row_status, const double *lag_C,
+                         const double *lag_scale, int first_points, void *stream);
 
 /* Integrator over n_meshes packed meshes.  `meshes` is a HOST array; every
  * other pointer is device memory.  flux receives [N_E][N_P] per mesh at

@@ -189,6 +189,8 @@ def _bind(L):
                                                     P, D, D, D, D, D, P, D, P, P, P, P,
                                                     P]),
         "xgpu_rays_batch": (C.c_int, [I64, C.c_int, P, P, P, P, P, P, P, P, P, P, P]),
+        "xgpu_rays_batch_rule": (C.c_int, [I64, C.c_int, P, P, P, P, P, P, P, P, P, P, C.c_int,
+                                           P]),
         "xgpu_integrate_batch": (C.c_int, [C.c_int, C.POINTER(Mesh), I64, C.c_int,
                                            C.c_int, C.c_int, C.c_int,
                                            C.POINTER(IntegrateBatchData), C.c_int, P]),
@@ -265,7 +267,7 @@ def _bind(L):
 
 EXPORTED = ["xgpu_abi_version", "xgpu_last_error", "xgpu_compute_rays", "xgpu_integrate",
             "xgpu_energy_integrator", "xgpu_response_fold", "xgpu_precomputation",
-            "xgpu_eval_marginal_likelihood", "xgpu_rays_batch", "xgpu_integrate_batch",
+            "xgpu_eval_marginal_likelihood", "xgpu_rays_batch", "xgpu_rays_batch_rule", "xgpu_integrate_batch",
             "xgpu_energy_batch", "xgpu_fold_batch", "xgpu_likelihood_batch",
             "xgpu_allocate_cells", "xgpu_cell_mesh", "xgpu_cell_mesh_many", "xgpu_peak_probe",
             "xgpu_likelihood_batch_static", "xgpu_integrate_batch_mixed",

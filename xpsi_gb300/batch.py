@@ -636,10 +636,13 @@ class BatchEvaluator:
         p = lambda x: x.data_ptr()
         L = lib()
         row = B["row"]
-        check(L.xgpu_rays_batch(P.n_rows, self.N_R, p(row["u"]), p(row["r_s"]),
-                                p(B["maxAlpha"]), p(B["defl"]), p(B["ca"]), p(B["lag"]),
-                                p(B["maxDefl"]), p(B["row_status"]), p(row["lag_C"]),
-                                p(row["lag_scale"]), st))
+        # the mixed form's FP32 roundings see the last bits of the tables: it
+        # keeps the 61-point rule's
+        rule = 61 if self.precision == "mixed" else 31
+        check(L.xgpu_rays_batch_rule(P.n_rows, self.N_R, p(row["u"]), p(row["r_s"]),
+                                     p(B["maxAlpha"]), p(B["defl"]), p(B["ca"]), p(B["lag"]),
+                                     p(B["maxDefl"]), p(B["row_status"]), p(row["lag_C"]),
+                                     p(row["lag_scale"]), rule, st))
         d = IntegrateBatchData()
         d.row_mesh = p(B["row_mesh"])
         d.radius, d.u, d.cos_gamma = p(row["radius"]), p(row["u"]), p(row["cos_gamma"])

@@ -190,10 +190,20 @@ int xgpu_rays_batch(int64_t n_rows, int N_R, const double *u, const double *r_s,
                     double *maxAlpha, double *deflection, double *cos_alpha, double *lag,
                     double *maxDeflection, int32_t *row_status, const double *lag_C,
                     const double *lag_scale, void *stream) {
+  return xgpu_rays_batch_rule(n_rows, N_R, u, r_s, maxAlpha, deflection, cos_alpha, lag,
+                              maxDeflection, row_status, lag_C, lag_scale, 31, stream);
+}
+
+int xgpu_rays_batch_rule(int64_t n_rows, int N_R, const double *u, const double *r_s,
+                         double *maxAlpha, double *deflection, double *cos_alpha, double *lag,
+                         double *maxDeflection, int32_t *row_status, const double *lag_C,
+                         const double *lag_scale, int first_points, void *stream) {
+  if (first_points != 31 && first_points != 61)
+    return fail_msg("the first panel has 31 or 61 points");
   if (N_R < 3) return fail_msg("num_rays must be at least 3");
   if (n_rows > INT32_MAX) return fail_msg("too many rows in one launch");
   xg::RaysArgs a{(int)n_rows, N_R, u, r_s, maxAlpha, deflection, cos_alpha, lag,
-                 maxDeflection, row_status, lag_C, lag_scale};
+                 maxDeflection, row_status, lag_C, lag_scale, first_points == 31};
   xg::launch_rays(a, static_cast<cudaStream_t>(stream));
   CK(cudaGetLastError());
   return 0;

@@ -401,6 +401,53 @@ __device__ __forceinline__ double pow2_double(int x) {
 __device__ __forceinline__ double scale_pow2(double v, int e) {
   return (e >= -1022 && e <= 1023) ? v * pow2_double(e) : ldexp(v, e);
 }
+// ---------------------------------------------------------------------------
+// double <-> float-pair conversions on the integer pipe.  A conversion
+// instruction between the two widths takes the FP64 pipe as long as a DFMA
+// (64 cycles or more per warp), and a split is four FP64 instructions, a
+// joined and scaled pair four; these are about fifteen integer ones.
+// ---------------------------------------------------------------------------
+// df_split(v 2^e) (ties of the high part aside, which split the same value)
+__device__ __forceinline__ DF df_split_bits(double v, int e) {
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  const int ev = (hi >> 20) & 0x7ff, E = ev - 1023 + e;
+  if (ev == 0 || ev == 0x7ff || E < -70 || E > 120) {
+    if ((hi & 0x7fffffff) == 0 && lo == 0) return DF{0.0f, 0.0f};
+    return df_split(scale_pow2(v, e));
+  }
+  int top = ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29);
+  int r = lo & 0x1fffffff;
+  if (r & 0x10000000) {
+    top += 1;
+    r -= 0x20000000;
+  }
+  const int sign = hi & 0x80000000;
+  DF d;
+  d.h = __int_as_float((((E + 127) << 23) + top) | sign);
+  d.l = (float)r * __int_as_float(((E - 52 + 127) << 23) | sign);
+  return d;
+}
+// df_value(a) 2^e, rounded once to a double (|a.l| at most half an ulp of a.h)
+__device__ __forceinline__ double df_join_bits(DF a, int e) {
+  const int hb = __float_as_int(a.h), eh = ((hb >> 23) & 0xff) - 127;
+  const int ex = eh + e;
+  if (eh < -60 || eh > 100 || ex < -1020 || ex > 1020) {
+    if (a.h == 0.0f) return 0.0;
+    return scale_pow2(df_value(a), e);
+  }
+  // in units of 2^(eh - 52): the high part's 24 bits and the low part rounded
+  const int li = __float2int_rn(a.l * __int_as_float((52 - eh + 127) << 23));
+  const bool neg = hb < 0;
+  long long m = ((long long)((hb & 0x7fffff) | 0x800000) << 29) + (neg ? -li : li);
+  int x = ex;
+  if (m < (1ll << 52)) {
+    m <<= 1;
+    x -= 1;
+  }
+  const long long bits = ((long long)(x + 1023) << 52) + (m - (1ll << 52));
+  return __longlong_as_double(neg ? bits | (long long)0x8000000000000000ull : bits);
+}
+
 // the largest frexp exponent of |v| over a lane's values, from the bit
 // patterns (integer work): fold() each value, exponent() at the end gives
 // what frexp(max |v|) gives, 0 when the largest is 0, infinite or NaN

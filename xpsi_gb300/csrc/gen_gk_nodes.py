@@ -1,9 +1,9 @@
 """Compute Gauss-Kronrod (G_n, K_{2n+1}) nodes and weights in high precision.
 
-Nodes for the ray (61-point) and window (21-point) quadratures; it writes the 61-point
-Kronrod extension of the 30-point Gauss-Legendre rule (the rule the ray
-integrals use, QUADPACK key 6) and the 21-point extension of the 10-point
-rule.  They are derived here from their definition, not taken from any
+Nodes for the ray (61-point, first tried with 31) and window (21-point)
+quadratures; it writes the 61-point Kronrod extension of the 30-point
+Gauss-Legendre rule (the rule the ray integrals use, QUADPACK key 6) and the
+31- and 21-point extensions of the 15- and 10-point rules.  They are derived here from their definition, not taken from any
 library table:
 
 * Gauss nodes are the roots of P_n, weights 2 / ((1 - x^2) P_n'(x)^2).
@@ -95,7 +95,7 @@ def main():
              "#define GK_TABLE static const double",
              "#define GK_TABLE_F static const float",
              "#endif", ""]
-    for n in (10, 30):
+    for n in (10, 15, 30):
         nodes, kw, gx, gw = kronrod(n)
         # keep x >= 0 half: index 0 = largest node; the centre node is last
         half = n + 1

@@ -20,6 +20,7 @@ struct RaysArgs {
   int32_t *row_status;    // [rows] or null
   const double *lag_C;     // [rows] lag calibration offset (s) or null
   const double *lag_scale; // [rows] 2 pi f_mode
+  int first31;             // try one 31-point panel before the 61-point bisection
 };
 void launch_rays(const RaysArgs &a, cudaStream_t st);
 

@@ -2,9 +2,11 @@
 // mesh parallel.  Replaces xpsi/cellmesh/rays.pyx:249-390 (compute_rays) and
 // its per-ray quadrature rayIntegrator (:90-247).
 //
-// Work decomposition: one CTA per mesh row ("parallel"), one thread per ray;
-// each thread runs its 2 or 4 QUADPACK-QAG / Gauss-Kronrod-61 integrals to
-// epsrel 1e-12, the reference's quadrature problem, with the deflection and
+// Work decomposition: one CTA per mesh row ("parallel"; several where rows are
+// few), one thread per ray;
+// each thread runs its 2 or 4 QUADPACK-QAG integrals to epsrel 1e-12 (one
+// 31-point panel where that meets it, else the reference's Gauss-Kronrod-61
+// bisection), with the deflection and
 // lag integrals over the same interval taken as a pair (their integrands
 // share the square root, so each node is evaluated once for both):
 // interval bookkeeping and error control in FP64, every panel's integrand
@@ -68,7 +70,7 @@ __device__ __forceinline__ void gk61_pair_panel(const P &pf, double a, double b,
                                                 double err[2], double rabs[2], double rasc[2]) {
   constexpr int NH = XG_K61_HALF - 1;
   const double cd = 0.5 * (a + b), hd = 0.5 * (b - a);
-  const DF c = df_split(cd), h = df_split(hd);
+  const DF c = df_split_bits(cd, 0), h = df_split_bits(hd, 0);
   float fv1[2][NH], fv2[2][NH];
   DF fc[2];
   pf(c, fc[0], fc[1]);
@@ -132,6 +134,64 @@ __device__ __forceinline__ void gk61_pair_panel(const P &pf, double a, double b,
   }
 }
 
+// The 31-point rule over [a, b] for the two integrals of a pair; true when
+// both meet the tolerance by QUADPACK's own error estimate (taken in float:
+// the half-width cancels from the ratio to the tolerance), with the results
+// in r.  Nearly every ray of a star away from the photon sphere does (all of
+// them for r_s / r below 0.6, half at 0.655), agreeing with the 61-point rule
+// to 1e-15, at half its evaluations.
+template <typename P>
+__device__ __forceinline__ bool gk31_pair(const P &pf, double a, double b, double r[2]) {
+  constexpr int NH = XG_K31_HALF - 1;
+  const double cd = 0.5 * (a + b), hd = 0.5 * (b - a);
+  const DF c = df_split_bits(cd, 0), h = df_split_bits(hd, 0);
+  float fv1[2][NH], fv2[2][NH];
+  DF fc[2];
+  pf(c, fc[0], fc[1]);
+  DF rk[2], rg[2];
+  const DF wkc{XG_K31_WK2[2 * NH], XG_K31_WK2[2 * NH + 1]};
+  const DF wgc{XG_K31_WG2[2 * NH], XG_K31_WG2[2 * NH + 1]};
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    rk[q] = df_mul(wkc, fc[q]);
+    rg[q] = df_mul(wgc, fc[q]);
+  }
+#pragma unroll 1
+  for (int j = 0; j < NH; j++) {
+    const DF dx = df_mul(h, DF{XG_K31_X2[2 * j], XG_K31_X2[2 * j + 1]});
+    DF f1[2], f2[2];
+    pf(df_sub(c, dx), f1[0], f1[1]);
+    pf(df_add(c, dx), f2[0], f2[1]);
+    const DF wk{XG_K31_WK2[2 * j], XG_K31_WK2[2 * j + 1]};
+    const DF wg{XG_K31_WG2[2 * j], XG_K31_WG2[2 * j + 1]};
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      fv1[q][j] = f1[q].h;
+      fv2[q][j] = f2[q].h;
+      const DF s2 = df_add(f1[q], f2[q]);
+      rk[q] = df_fma(wk, s2, rk[q]);
+      if (wg.h != 0.0f) rg[q] = df_fma(wg, s2, rg[q]);
+    }
+  }
+  bool ok = true;
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const float mean = 0.5f * rk[q].h;
+    float rc = wkc.h * fabsf(fc[q].h - mean);
+#pragma unroll 1
+    for (int j = 0; j < NH; j++)
+      rc += XG_K31_WK2[2 * j] * (fabsf(fv1[q][j] - mean) + fabsf(fv2[q][j] - mean));
+    const float dk = fabsf(df_sub(rk[q], rg[q]).h);
+    // err = rasc min(1, (200 |K - G| / rasc)^1.5); a NaN fails
+    const float x = 200.0f * dk / rc, e = rc * fminf(1.0f, x * sqrtf(x));
+    ok = ok && (dk == 0.0f || e <= 0.9e-12f * fabsf(rk[q].h)) && isfinite(rk[q].h);
+  }
+  if (!ok) return false;
+  r[0] = df_join_bits(rk[0], 0) * hd;
+  r[1] = df_join_bits(rk[1], 0) * hd;
+  return true;
+}
+
 // QUADPACK QAG at relative 1e-12, limit 100 (rays.pyx:140-236) for the two
 // integrals of a pair over the same interval: the first panel's tests are
 // QUADPACK's for each integral, and while either error is above its
@@ -139,13 +199,18 @@ __device__ __forceinline__ void gk61_pair_panel(const P &pf, double a, double b,
 // is largest is bisected (both integrals refined there).  Each integral is
 // thus at least as accurate as its own QAG run would leave it.  Statuses:
 // 0, 11 (limit), 18 (round-off), 21 (bad integrand), as qag_panels.
-template <typename P>
+template <bool k31, typename P>
 __device__ int q61_pair(const P &pf, double a, double b, double &r1, double &r2) {
   constexpr int LIMIT = 100;
   const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
   const double epsrel = 1.0e-12;
   double al[LIMIT], bl[LIMIT], rl[2][LIMIT], el[2][LIMIT];
   double r0[2], e0[2], ra0[2], rc0[2];
+  if (k31 && gk31_pair(pf, a, b, r0)) {
+    r1 = r0[0];
+    r2 = r0[1];
+    return 0;
+  }
   gk61_pair_panel(pf, a, b, r0, e0, ra0, rc0);
   bool done[2];
   int st0[2];
@@ -239,9 +304,14 @@ __device__ __forceinline__ double turning_radius(double b) {
   return 2.0 * b * cos((atan(sqrt(4.0 * b * b * i27 - 1.0)) - kPi) * i3) * isq3;
 }
 
-// u_sq1u = u sqrt(1 - u), formed once per row (rays.pyx forms it per ray)
-__device__ void ray_integrate(double cos_alpha, double r_s, double u, double u_sq1u, double &d,
-                              double &l) {
+// what a row's rays share: u sqrt(1 - u), 1 / u, 1 / (1/u - 1) as a pair, 1 / c
+struct RowRay {
+  double r_s, u, u_sq1u, iu;
+  DF q;
+};
+template <bool k31>
+__device__ void ray_integrate(double cos_alpha, const RowRay &R, double &d, double &l) {
+  const double r_s = R.r_s, u = R.u;
   const int EFAILED = 5;
   int status = 0;
   double sas = 1.0 - cos_alpha * cos_alpha;
@@ -251,12 +321,12 @@ __device__ void ray_integrate(double cos_alpha, double r_s, double u, double u_s
   // rounds to pi/2 from a cosine a few ulps below zero: there it is formed
   double alpha = cos_alpha >= 0.0 ? 0.0 : kPi;
   if (fabs(cos_alpha) < 1.0e-15) alpha = acos(cos_alpha);
-  double b = sa / u_sq1u;
+  double b = sa / R.u_sq1u;
   d = 0.0;
   l = 0.0;
   if (b <= kBPhotonSphere) {
-    const OutDef fd{df_split(1.0 - sas), df_split(sas), df_split(1.0 / (1.0 / u - 1.0))};
-    status = q61_pair(OutPair{fd}, 0.0, 1.0, d, l);
+    const OutDef fd{df_split_bits(1.0 - sas, 0), df_split_bits(sas, 0), R.q};
+    status = q61_pair<k31>(OutPair{fd}, 0.0, 1.0, d, l);
     if (status == EFAILED) d = nan("");
     if (status != EFAILED) {
       d *= 2.0 * b * u;
@@ -265,15 +335,15 @@ __device__ void ray_integrate(double cos_alpha, double r_s, double u, double u_s
   } else if (alpha <= kPi / 2.0) {
     double rc, wR;
     if (are_equal(sa, 1.0)) {
-      rc = 1.0 / u;
+      rc = R.iu;
       wR = 0.0;
     } else {
       rc = turning_radius(b);
       wR = sqrt(1.0 - rc * u);
     }
     if (isnan(wR)) wR = 0.0;
-    const InDef fd{df_split(1.0 / (rc - 1.0))};
-    status = q61_pair(InPair{fd}, wR, 1.0, d, l);
+    const InDef fd{df_split_bits(1.0 / (rc - 1.0), 0)};
+    status = q61_pair<k31>(InPair{fd}, wR, 1.0, d, l);
     if (status == EFAILED) d = nan("");
     if (status != EFAILED) {
       const double irc = 1.0 / rc;
@@ -284,106 +354,82 @@ __device__ void ray_integrate(double cos_alpha, double r_s, double u, double u_s
     double rc = turning_radius(b);
     double wR = sqrt(1.0 - rc * u);
     if (isnan(wR)) wR = 0.0;
-    const InDef fd{df_split(1.0 / (rc - 1.0))};
+    const InDef fd{df_split_bits(1.0 / (rc - 1.0), 0)};
     double d1, d0, l1, l0;
-    status = q61_pair(InPair{fd}, 0.0, 1.0, d1, l1);
+    status = q61_pair<k31>(InPair{fd}, 0.0, 1.0, d1, l1);
     if (status == EFAILED) d = nan("");
     if (status != EFAILED) {
-      status = q61_pair(InPair{fd}, wR, 1.0, d0, l0);
+      status = q61_pair<k31>(InPair{fd}, wR, 1.0, d0, l0);
       if (status == EFAILED) d = nan("");
     }
     if (status != EFAILED) {
       const double irc = 1.0 / rc;
       d = 2.0 * b * (2.0 * d1 - d0) * irc;
       l = 2.0 * b * b * r_s * (2.0 * l1 - l0) * irc;
-      double cor = 1.0 / u - rc + log((1.0 / u - 1.0) / (rc - 1.0));
+      double cor = R.iu - rc + log((R.iu - 1.0) / (rc - 1.0));
       l += 2.0 * r_s * cor;
     }
   }
   if (status != EFAILED) l /= kC;
 }
 
-__global__ void __launch_bounds__(128) rays_kernel(RaysArgs a) {
-  const int row = blockIdx.x;
-  if (row >= a.n_rows) return;
+// rays.pyx:310-320: the largest ray angle of the row
+__device__ double clamped_max_alpha(double u, double ma) {
+  double extreme = 0.0;
+  if (u < 2.0 / 3.0)
+    extreme = kPi - asin(sqrt(1.0 - u) * kBPhotonSphere * u);
+  else if (are_equal(u, 2.0 / 3.0))
+    extreme = kPi / 2.0;
+  else if (2.0 / 3.0 < u && u < 1.0)
+    extreme = asin(sqrt(1.0 - u) * kBPhotonSphere * u);
+  const double eps = 1.0e-8;
+  return ma >= (1.0 - eps) * extreme ? (1.0 - eps) * extreme : ma;
+}
+
+// a row's checks, repair and lag calibration, by a CTA after its rays
+__device__ void finish_row(const RaysArgs &a, int row, double ma) {
   const int N_R = a.N_R;
-  const double u = a.u[row];
-  const double r_s = a.r_s_row[row];
   double *D = a.deflection + (size_t)row * N_R;
-  double *CA = a.cos_alpha + (size_t)row * N_R;
   double *L = a.lag + (size_t)row * N_R;
-  __shared__ double s_inc;
-  if (threadIdx.x == 0) {
-    // rays.pyx:310-320
-    double extreme = 0.0;
-    if (u < 2.0 / 3.0)
-      extreme = kPi - asin(sqrt(1.0 - u) * kBPhotonSphere * u);
-    else if (are_equal(u, 2.0 / 3.0))
-      extreme = kPi / 2.0;
-    else if (2.0 / 3.0 < u && u < 1.0)
-      extreme = asin(sqrt(1.0 - u) * kBPhotonSphere * u);
-    double ma = a.maxAlpha[row];
-    const double eps = 1.0e-8;
-    if (ma >= (1.0 - eps) * extreme) ma = (1.0 - eps) * extreme;
-    a.maxAlpha[row] = ma;
-    s_inc = (1.0 - cos(ma)) / ((double)N_R - 1.0);
-  }
-  __syncthreads();
-  const double inc = s_inc;
-  const double u_sq1u = u * sqrt(1.0 - u);
-  for (int j = threadIdx.x; j < N_R; j += blockDim.x) {
-    double ca = 1.0 - (double)j * inc;
-    if (j == 0) {
-      CA[0] = 1.0;
-      D[0] = 0.0;
-      L[0] = 0.0;
-      continue;
-    }
-    CA[j] = ca;
-    double d, l;
-    ray_integrate(ca, r_s, u, u_sq1u, d, l);
-    D[j] = d;  // raw values; repaired below
-    L[j] = l;
-  }
-  __syncthreads();
   // rays.pyx:322-371: a row whose values are all finite, in [0, 100 pi] and
   // rising at the last ray needs no repair (the walk below changes nothing
   // there); the CTA checks that in parallel and only other rows take the
-  // sequential walk
+  // sequential walk.  (In range: the bits as an integer from 0 to those of
+  // 100 pi; -0 does not occur.)
   int bad = 0;
   for (int j = 1 + threadIdx.x; j < N_R; j += blockDim.x) {
-    const double rp = D[j];
-    bad |= (isnan(rp) || rp < 0.0 || rp > 100.0 * kPi) ? 1 : 0;
+    const long long rp = __double_as_longlong(D[j]);
+    bad |= (rp < 0 || rp > __double_as_longlong(100.0 * kPi)) ? 1 : 0;
   }
   const int any_bad = __syncthreads_or(bad);
-  if (!any_bad && threadIdx.x == 0) {
-    const int term = N_R >= 2 && !(D[N_R - 1] > D[N_R - 2]);
-    a.maxDeflection[row] = D[N_R - 1];
-    if (a.row_status) a.row_status[row] = term ? kRayFail : kOk;
-  }
-  if (any_bad && threadIdx.x == 0) {
-    // rays.pyx:322-371, sequential NaN repair by linear interpolation
+  if (threadIdx.x == 0) {
+    a.maxAlpha[row] = ma;
     int term = 0;
-    int icount = 0, iidx = 0;
-    for (int j = 1; j < N_R; j++) {
-      double rp = D[j], lp = L[j];
-      if (j == N_R - 1 && (isnan(rp) || rp <= D[j - 1])) {
-        term = 1;
-        break;
-      } else if (icount > 0 && !isnan(rp) && 0.0 <= rp && rp < 100.0 * kPi && rp > D[iidx]) {
-        double delta = (double)icount + 1.0;
-        for (int k = 1; k <= icount; k++) {
-          double v = rp * (double)k;
-          v += D[iidx] * (delta - (double)k);
-          D[iidx + k] = v / delta;
-          double w = lp * (double)k;
-          w += L[iidx] * (delta - (double)k);
-          L[iidx + k] = w / delta;
+    if (!any_bad) {
+      term = N_R >= 2 && !(D[N_R - 1] > D[N_R - 2]);
+    } else {
+      // rays.pyx:322-371, sequential NaN repair by linear interpolation
+      int icount = 0, iidx = 0;
+      for (int j = 1; j < N_R; j++) {
+        double rp = D[j], lp = L[j];
+        if (j == N_R - 1 && (isnan(rp) || rp <= D[j - 1])) {
+          term = 1;
+          break;
+        } else if (icount > 0 && !isnan(rp) && 0.0 <= rp && rp < 100.0 * kPi && rp > D[iidx]) {
+          double delta = (double)icount + 1.0;
+          for (int k = 1; k <= icount; k++) {
+            double v = rp * (double)k;
+            v += D[iidx] * (delta - (double)k);
+            D[iidx + k] = v / delta;
+            double w = lp * (double)k;
+            w += L[iidx] * (delta - (double)k);
+            L[iidx + k] = w / delta;
+          }
+          icount = 0;
+        } else if (isnan(rp) || rp < 0.0 || rp > 100.0 * kPi) {
+          if (icount == 0) iidx = j - 1;
+          icount++;
         }
-        icount = 0;
-      } else if (isnan(rp) || rp < 0.0 || rp > 100.0 * kPi) {
-        if (icount == 0) iidx = j - 1;
-        icount++;
       }
     }
     a.maxDeflection[row] = D[N_R - 1];
@@ -397,9 +443,80 @@ __global__ void __launch_bounds__(128) rays_kernel(RaysArgs a) {
   }
 }
 
+// kSplit: a row's rays are shared by a.parts CTAs, a ray to a thread, and
+// rays_finish_kernel follows; else a CTA has a whole row.
+template <bool kSplit, bool k31>
+__global__ void __launch_bounds__(128) rays_kernel(RaysArgs a, int parts) {
+  const int row = kSplit ? blockIdx.x / parts : blockIdx.x;
+  const int N_R = a.N_R;
+  const double u = a.u[row];
+  double *D = a.deflection + (size_t)row * N_R;
+  double *CA = a.cos_alpha + (size_t)row * N_R;
+  double *L = a.lag + (size_t)row * N_R;
+  __shared__ double s_inc, s_ma;
+  __shared__ RowRay s_row;
+  if (threadIdx.x == 0) {
+    const double ma = clamped_max_alpha(u, a.maxAlpha[row]);
+    s_ma = ma;
+    s_inc = (1.0 - cos(ma)) / ((double)N_R - 1.0);
+  }
+  if (threadIdx.x == 32) {
+    RowRay r;
+    r.r_s = a.r_s_row[row];
+    r.u = u;
+    r.u_sq1u = u * sqrt(1.0 - u);
+    r.iu = 1.0 / u;
+    r.q = df_split(1.0 / (r.iu - 1.0));
+    s_row = r;
+  }
+  __syncthreads();
+  const double inc = s_inc;
+  const RowRay R = s_row;
+  const int j0 = kSplit ? (blockIdx.x - row * parts) * blockDim.x : 0;
+  const int j1 = kSplit ? min(N_R, j0 + (int)blockDim.x) : N_R;
+  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
+    double ca = 1.0 - (double)j * inc;
+    if (j == 0) {
+      CA[0] = 1.0;
+      D[0] = 0.0;
+      L[0] = 0.0;
+      continue;
+    }
+    CA[j] = ca;
+    double d, l;
+    ray_integrate<k31>(ca, R, d, l);
+    D[j] = d;  // raw values; repaired below
+    L[j] = l;
+  }
+  if (!kSplit) {
+    __syncthreads();
+    finish_row(a, row, s_ma);
+  }
+}
+
+__global__ void __launch_bounds__(128) rays_finish_kernel(RaysArgs a) {
+  const int row = blockIdx.x;
+  // (one thread's arithmetic; the others need no value)
+  const double ma = threadIdx.x == 0 ? clamped_max_alpha(a.u[row], a.maxAlpha[row]) : 0.0;
+  finish_row(a, row, ma);
+}
+
 void launch_rays(const RaysArgs &a, cudaStream_t st) {
   if (a.n_rows <= 0) return;
-  rays_kernel<<<a.n_rows, 128, 0, st>>>(a);
+  // Rows of a CTA each, its threads taking every 128th ray, until they fill
+  // the chip about twice over (152 SMs x 4 CTAs); below that a ray per thread:
+  // 64 rows of 1024 rays ran 252 us with 8 rays in turn on 64 SMs.
+  const int parts = (a.N_R + 127) / 128;
+  if (a.n_rows < 1216 && parts > 1) {
+    const unsigned grid = (unsigned)(a.n_rows * parts);
+    if (a.first31) rays_kernel<true, true><<<grid, 128, 0, st>>>(a, parts);
+    else rays_kernel<true, false><<<grid, 128, 0, st>>>(a, parts);
+    rays_finish_kernel<<<a.n_rows, 128, 0, st>>>(a);
+  } else if (a.first31) {
+    rays_kernel<false, true><<<a.n_rows, 128, 0, st>>>(a, 1);
+  } else {
+    rays_kernel<false, false><<<a.n_rows, 128, 0, st>>>(a, 1);
+  }
 }
 
 }  // namespace xg
