@@ -2,8 +2,7 @@
 // mesh parallel.  Replaces xpsi/cellmesh/rays.pyx:249-390 (compute_rays) and
 // its per-ray quadrature rayIntegrator (:90-247).
 //
-// Work decomposition: one CTA per mesh row ("parallel"; several where rows are
-// few), one thread per ray;
+// Work decomposition: several CTAs per mesh row ("parallel"), one thread per ray;
 // each thread runs its 2 or 4 QUADPACK-QAG integrals to epsrel 1e-12 (one
 // 31-point panel where that meets it, else the reference's Gauss-Kronrod-61
 // bisection), with the deflection and
@@ -65,8 +64,10 @@ struct InPair {
 
 // gk_panel_df for the two integrands of a pair at once (the same nodes,
 // weights and error estimate per integrand)
+// (not inlined: one copy per integrand pair, so that the kernel's code stays in
+// the instruction cache)
 template <typename P>
-__device__ __forceinline__ void gk61_pair_panel(const P &pf, double a, double b, double res[2],
+__device__ __noinline__ void gk61_pair_panel(const P &pf, double a, double b, double res[2],
                                                 double err[2], double rabs[2], double rasc[2]) {
   constexpr int NH = XG_K61_HALF - 1;
   const double cd = 0.5 * (a + b), hd = 0.5 * (b - a);
@@ -141,7 +142,7 @@ __device__ __forceinline__ void gk61_pair_panel(const P &pf, double a, double b,
 // them for r_s / r below 0.6, half at 0.655), agreeing with the 61-point rule
 // to 1e-15, at half its evaluations.
 template <typename P>
-__device__ __forceinline__ bool gk31_pair(const P &pf, double a, double b, double r[2]) {
+__device__ __noinline__ bool gk31_pair(const P &pf, double a, double b, double r[2]) {
   constexpr int NH = XG_K31_HALF - 1;
   const double cd = 0.5 * (a + b), hd = 0.5 * (b - a);
   const DF c = df_split_bits(cd, 0), h = df_split_bits(hd, 0);
@@ -200,17 +201,12 @@ __device__ __forceinline__ bool gk31_pair(const P &pf, double a, double b, doubl
 // thus at least as accurate as its own QAG run would leave it.  Statuses:
 // 0, 11 (limit), 18 (round-off), 21 (bad integrand), as qag_panels.
 template <bool k31, typename P>
-__device__ int q61_pair(const P &pf, double a, double b, double &r1, double &r2) {
+__device__ __noinline__ int q61_pair(const P &pf, double a, double b, double &r1, double &r2) {
   constexpr int LIMIT = 100;
   const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
   const double epsrel = 1.0e-12;
   double al[LIMIT], bl[LIMIT], rl[2][LIMIT], el[2][LIMIT];
   double r0[2], e0[2], ra0[2], rc0[2];
-  if (k31 && gk31_pair(pf, a, b, r0)) {
-    r1 = r0[0];
-    r2 = r0[1];
-    return 0;
-  }
   gk61_pair_panel(pf, a, b, r0, e0, ra0, rc0);
   bool done[2];
   int st0[2];
@@ -293,6 +289,19 @@ __device__ int q61_pair(const P &pf, double a, double b, double &r1, double &r2)
 }
 
 
+// the two integrals of a pair, by the 31-point rule where it suffices
+template <bool k31, typename P>
+__device__ __forceinline__ int pair_integral(const P &pf, double a, double b, double &r1,
+                                             double &r2) {
+  double r[2];
+  if (k31 && gk31_pair(pf, a, b, r)) {
+    r1 = r[0];
+    r2 = r[1];
+    return 0;
+  }
+  return q61_pair<k31>(pf, a, b, r1, r2);
+}
+
 // rays.pyx:90-247; returns deflection in d, lag in seconds in l
 // the turning radius r_c / r_s of a ray of impact parameter b / r_s
 // (rays.pyx:156, :194): 2 b cos((atan(sqrt(4 b^2 / 27 - 1)) - pi) / 3) / sqrt 3,
@@ -326,15 +335,19 @@ __device__ void ray_integrate(double cos_alpha, const RowRay &R, double &d, doub
   l = 0.0;
   if (b <= kBPhotonSphere) {
     const OutDef fd{df_split_bits(1.0 - sas, 0), df_split_bits(sas, 0), R.q};
-    status = q61_pair<k31>(OutPair{fd}, 0.0, 1.0, d, l);
+    status = pair_integral<k31>(OutPair{fd}, 0.0, 1.0, d, l);
     if (status == EFAILED) d = nan("");
     if (status != EFAILED) {
       d *= 2.0 * b * u;
       l *= 2.0 * b * b * u * r_s;
     }
-  } else if (alpha <= kPi / 2.0) {
+  } else {
+    // inward rays (alpha > pi/2) reach the turning point and come back: their
+    // integrals take the whole range [0, 1] twice less the part beyond the
+    // surface [wR, 1], the outward ones that part alone
+    const bool back = alpha > kPi / 2.0;
     double rc, wR;
-    if (are_equal(sa, 1.0)) {
+    if (!back && are_equal(sa, 1.0)) {
       rc = R.iu;
       wR = 0.0;
     } else {
@@ -342,32 +355,34 @@ __device__ void ray_integrate(double cos_alpha, const RowRay &R, double &d, doub
       wR = sqrt(1.0 - rc * u);
     }
     if (isnan(wR)) wR = 0.0;
-    const InDef fd{df_split_bits(1.0 / (rc - 1.0), 0)};
-    status = q61_pair<k31>(InPair{fd}, wR, 1.0, d, l);
-    if (status == EFAILED) d = nan("");
-    if (status != EFAILED) {
-      const double irc = 1.0 / rc;
-      d *= 2.0 * b * irc;
-      l *= 2.0 * b * b * r_s * irc;
+    const InPair fd{InDef{df_split_bits(1.0 / (rc - 1.0), 0)}};
+    double d1 = 0.0, l1 = 0.0, d0 = 0.0, l0 = 0.0;
+#pragma unroll 1
+    for (int z = back ? 0 : 1; z < 2 && status != EFAILED; z++) {
+      double di, li;
+      status = pair_integral<k31>(fd, z == 0 ? 0.0 : wR, 1.0, di, li);
+      if (z == 0) {
+        d1 = di;
+        l1 = li;
+      } else {
+        d0 = di;
+        l0 = li;
+      }
     }
-  } else if (alpha > kPi / 2.0) {
-    double rc = turning_radius(b);
-    double wR = sqrt(1.0 - rc * u);
-    if (isnan(wR)) wR = 0.0;
-    const InDef fd{df_split_bits(1.0 / (rc - 1.0), 0)};
-    double d1, d0, l1, l0;
-    status = q61_pair<k31>(InPair{fd}, 0.0, 1.0, d1, l1);
-    if (status == EFAILED) d = nan("");
-    if (status != EFAILED) {
-      status = q61_pair<k31>(InPair{fd}, wR, 1.0, d0, l0);
-      if (status == EFAILED) d = nan("");
-    }
-    if (status != EFAILED) {
+    if (status == EFAILED) {
+      d = nan("");
+      l = l1 + l0;
+    } else {
       const double irc = 1.0 / rc;
-      d = 2.0 * b * (2.0 * d1 - d0) * irc;
-      l = 2.0 * b * b * r_s * (2.0 * l1 - l0) * irc;
-      double cor = R.iu - rc + log((R.iu - 1.0) / (rc - 1.0));
-      l += 2.0 * r_s * cor;
+      if (back) {
+        d = 2.0 * b * (2.0 * d1 - d0) * irc;
+        l = 2.0 * b * b * r_s * (2.0 * l1 - l0) * irc;
+        double cor = R.iu - rc + log((R.iu - 1.0) / (rc - 1.0));
+        l += 2.0 * r_s * cor;
+      } else {
+        d = d0 * (2.0 * b * irc);
+        l = l0 * (2.0 * b * b * r_s * irc);
+      }
     }
   }
   if (status != EFAILED) l /= kC;
@@ -387,7 +402,10 @@ __device__ double clamped_max_alpha(double u, double ma) {
 }
 
 // a row's checks, repair and lag calibration, by a CTA after its rays
-__device__ void finish_row(const RaysArgs &a, int row, double ma) {
+__global__ void __launch_bounds__(128) rays_finish_kernel(RaysArgs a) {
+  const int row = blockIdx.x;
+  // (one thread's arithmetic; the others need no value)
+  const double ma = threadIdx.x == 0 ? clamped_max_alpha(a.u[row], a.maxAlpha[row]) : 0.0;
   const int N_R = a.N_R;
   double *D = a.deflection + (size_t)row * N_R;
   double *L = a.lag + (size_t)row * N_R;
@@ -443,21 +461,25 @@ __device__ void finish_row(const RaysArgs &a, int row, double ma) {
   }
 }
 
-// kSplit: a row's rays are shared by a.parts CTAs, a ray to a thread, and
-// rays_finish_kernel follows; else a CTA has a whole row.
-template <bool kSplit, bool k31>
+// A row's rays are shared by `parts` CTAs, a ray to a thread, and
+// rays_finish_kernel follows.  (A CTA with a whole row in turn ran 8 % slower:
+// its warps waited for the rays near the limb.)  Bound: FP32 issue through
+// long dependent double-float chains, 45-60 % of the issue slots, and the
+// instruction cache.  24 vectors (5628 rows of 1024 rays): 7.9 ms with 61
+// points everywhere and every panel inlined, 4.3 ms now (61 points alone: 64
+// vectors' 10810 rows 13.7 -> 7.7 ms); 64 rows: 252 us in turn on 64 SMs, 67 us.
+template <bool k31>
 __global__ void __launch_bounds__(128) rays_kernel(RaysArgs a, int parts) {
-  const int row = kSplit ? blockIdx.x / parts : blockIdx.x;
+  const int row = blockIdx.x / parts;
   const int N_R = a.N_R;
   const double u = a.u[row];
   double *D = a.deflection + (size_t)row * N_R;
   double *CA = a.cos_alpha + (size_t)row * N_R;
   double *L = a.lag + (size_t)row * N_R;
-  __shared__ double s_inc, s_ma;
+  __shared__ double s_inc;
   __shared__ RowRay s_row;
   if (threadIdx.x == 0) {
     const double ma = clamped_max_alpha(u, a.maxAlpha[row]);
-    s_ma = ma;
     s_inc = (1.0 - cos(ma)) / ((double)N_R - 1.0);
   }
   if (threadIdx.x == 32) {
@@ -472,50 +494,33 @@ __global__ void __launch_bounds__(128) rays_kernel(RaysArgs a, int parts) {
   __syncthreads();
   const double inc = s_inc;
   const RowRay R = s_row;
-  const int j0 = kSplit ? (blockIdx.x - row * parts) * blockDim.x : 0;
-  const int j1 = kSplit ? min(N_R, j0 + (int)blockDim.x) : N_R;
-  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-    double ca = 1.0 - (double)j * inc;
-    if (j == 0) {
-      CA[0] = 1.0;
-      D[0] = 0.0;
-      L[0] = 0.0;
-      continue;
-    }
-    CA[j] = ca;
-    double d, l;
-    ray_integrate<k31>(ca, R, d, l);
-    D[j] = d;  // raw values; repaired below
-    L[j] = l;
-  }
-  if (!kSplit) {
-    __syncthreads();
-    finish_row(a, row, s_ma);
-  }
-}
-
-__global__ void __launch_bounds__(128) rays_finish_kernel(RaysArgs a) {
-  const int row = blockIdx.x;
-  // (one thread's arithmetic; the others need no value)
-  const double ma = threadIdx.x == 0 ? clamped_max_alpha(a.u[row], a.maxAlpha[row]) : 0.0;
-  finish_row(a, row, ma);
+  const int j = (blockIdx.x - row * parts) * blockDim.x + threadIdx.x;
+  if (j >= N_R) return;
+  double ca = 1.0 - (double)j * inc, d = 0.0, l = 0.0;
+  if (j == 0) ca = 1.0;
+  else ray_integrate<k31>(ca, R, d, l);
+  CA[j] = ca;
+  D[j] = d;  // raw values; checked and repaired by rays_finish_kernel
+  L[j] = l;
 }
 
 void launch_rays(const RaysArgs &a, cudaStream_t st) {
   if (a.n_rows <= 0) return;
-  // Rows of a CTA each, its threads taking every 128th ray, until they fill
-  // the chip about twice over (152 SMs x 4 CTAs); below that a ray per thread:
-  // 64 rows of 1024 rays ran 252 us with 8 rays in turn on 64 SMs.
   const int parts = (a.N_R + 127) / 128;
-  if (a.n_rows < 1216 && parts > 1) {
-    const unsigned grid = (unsigned)(a.n_rows * parts);
-    if (a.first31) rays_kernel<true, true><<<grid, 128, 0, st>>>(a, parts);
-    else rays_kernel<true, false><<<grid, 128, 0, st>>>(a, parts);
-    rays_finish_kernel<<<a.n_rows, 128, 0, st>>>(a);
-  } else if (a.first31) {
-    rays_kernel<false, true><<<a.n_rows, 128, 0, st>>>(a, 1);
-  } else {
-    rays_kernel<false, false><<<a.n_rows, 128, 0, st>>>(a, 1);
+  // (rows per launch so that the grid stays within its limit)
+  const int64_t most = (int64_t)INT32_MAX / parts;
+  for (int64_t r0 = 0; r0 < a.n_rows; r0 += most) {
+    RaysArgs b = a;
+    const int64_t n = a.n_rows - r0 < most ? a.n_rows - r0 : most;
+    b.n_rows = (int)n;
+    b.u += r0; b.r_s_row += r0; b.maxAlpha += r0; b.maxDeflection += r0;
+    b.deflection += r0 * a.N_R; b.cos_alpha += r0 * a.N_R; b.lag += r0 * a.N_R;
+    if (b.row_status) b.row_status += r0;
+    if (b.lag_C) { b.lag_C += r0; b.lag_scale += r0; }
+    const unsigned grid = (unsigned)(n * parts);
+    if (b.first31) rays_kernel<true><<<grid, 128, 0, st>>>(b, parts);
+    else rays_kernel<false><<<grid, 128, 0, st>>>(b, parts);
+    rays_finish_kernel<<<(unsigned)n, 128, 0, st>>>(b);
   }
 }
 
