@@ -570,7 +570,7 @@ __device__ __forceinline__ void lagrange_wf(const float *P, const float *S, int 
 
 // Num4D intensity in the mixed form: the slab and the Lagrange weights in
 // FP32, the mu stencil (b2, w2) formed once per profile column; the energy
-// coordinate's offset u from the stencil base b3 is the rounding of an exact
+// coordinate's offset u from the stencil base b3 is the rounding of an FP64
 // one, so the weights see the FP32 rounding of an offset of a few grid
 // spacings (~1e-9 absolute) rather than that of the coordinate (~3e-8, the
 // same on every evaluation of a parallel: a systematic shift).
@@ -1432,7 +1432,9 @@ struct IntSmem {
   char *piece;  // the chunk's pieces; the leaf geometry's arrays where a CTA forms it itself
   double *Z, *abb, *geom;          // per profile column
   long long *lz;                   // log10 Z + log10 E_eff in units of 2^-54
-  double *lzd;                     // 2-D tables: log10 Z, or Z (E in electron rest energies)
+  // the same in FP64: 2-D tables (log10 Z, or Z with E in electron rest
+  // energies) and the mixed form
+  double *lzd;
   DF *ih, *ih2;                    // 1 / h and 1 / h^2 of the phase intervals (FP64 form)
   DF *mw;                          // [4] mu stencil weights per column (FP64 form, 4-D table)
   float4 *mwf;                     // the same (mixed form)
@@ -1446,7 +1448,7 @@ struct IntSmem {
   int *xe;
   float *fcphi, *fcphi_lo, *fcarea, *fcarea_lo;
   long long *lgE;                  // the chunk's log10 E in units of 2^-54
-  double *lgEd;                    // 2-D tables: log10 E, or E
+  double *lgEd;                    // the same in FP64 (2-D tables: log10 E, or E)
   int *sc_exp;
   uint32_t *flags;
   int *nruns;
@@ -1472,7 +1474,7 @@ __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC
   take(o.Z, N_L); take(o.abb, N_L); take(o.geom, N_L);
   const bool tab4 = nE > 0 && !tab2;
   if (tab4) take(o.lz, N_L);
-  if (tab2) take(o.lzd, N_L);
+  if (tab2 || (tab4 && kMixed)) take(o.lzd, N_L);
   if (!kMixed) { take(o.ih, N_L); take(o.ih2, N_L); }
   if (tab4 && !kMixed) { take(o.mw, 4 * N_L); take(o.cfm, N_L); take(o.cfx, N_L); }
   if (tab4 && kMixed) take(o.mwf, N_L);
@@ -1484,11 +1486,13 @@ __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC
   if (tab2) { take(o.gE, nE); take(o.sE, 4 * nE); take(o.fgE, nE); }
   if (tab4) take(o.gEi, nE);
   if (tab4 && !kMixed) { take(o.dgEo, 3 * nE); take(o.dsE, 4 * nE); take(o.xe, nE); }
-  if (tab4 && kMixed) { take(o.fsmu, 4 * nmu); take(o.fsE, 4 * nE); take(o.fgEo, 3 * nE); }
+  if (tab4 && kMixed) {
+    take(o.fsmu, 4 * nmu); take(o.fsE, 4 * nE); take(o.fgEo, 3 * nE); take(o.gE, nE);
+  }
   take(o.fcphi, kMaxCellsF); take(o.fcphi_lo, kMaxCellsF);
   take(o.fcarea, kMaxCellsF); take(o.fcarea_lo, kMaxCellsF);
   if (tab4) take(o.lgE, EC);
-  if (tab2) take(o.lgEd, EC);
+  if (tab2 || (tab4 && kMixed)) take(o.lgEd, EC);
   take(o.sc_exp, EC);
   take(o.phase, N_P);
   if (!kMixed) {
@@ -1574,6 +1578,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
         for (int q = 0; q < 4; q++) sm.sE[4 * t + q] = s4[q];
       } else {
         sm.gEi[t] = fix_of(lE[t]);
+        if (kMixed) sm.gE[t] = lE[t];
         for (int q = 0; q < 4; q++) {
           if (kMixed) sm.fsE[4 * t + q] = (float)s4[q];
           else sm.dsE[4 * t + q] = df_split(s4[q]);
@@ -1859,8 +1864,10 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
             }
             if (tab2) sm.lzd[t] = erest ? Z : log10(Z);
             if (t4) {
-              sm.lz[t] = fix_of(log10(Z) + s_ra.lgE_eff);
+              const double lz = log10(Z) + s_ra.lgE_eff;
+              sm.lz[t] = fix_of(lz);
               if constexpr (kMixed) {
+                sm.lzd[t] = lz;
                 const float v = fmaxf((float)abb, sm.fgmu[0]);
                 const int b = stencil_base_f(sm.fgmu, nmu, v);
                 float w[4];
@@ -1919,6 +1926,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
             for (int t = threadIdx.x; t < ne; t += blockDim.x) {
               if (tab2) sm.lgEd[t] = erest ? a.energies[e0 + t] : a.lgE[e0 + t];
               else sm.lgE[t] = fix_of(a.lgE[e0 + t]);
+              if (kMixed) sm.lgEd[t] = a.lgE[e0 + t];
             }
           }
           __syncthreads();
@@ -1945,11 +1953,18 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
               int b3 = 0;
               DF u{0.0f, 0.0f};
               if (t4) {
-                long long v = sm.lgE[pl] - sm.lz[col];
-                v = max(v, sm.gEi[0]);
+                const long long v0 = sm.lgE[pl] - sm.lz[col];
+                long long v = max(v0, sm.gEi[0]);
                 v = min(v, sm.gEi[nEt - 1]);
                 b3 = stencil_base_fix(sm.gEi, nEt, v, lo);
-                u = fix_df(v - sm.gEi[b3]);
+                if (kMixed) {
+                  // (the FP32 rounding of the offset sees its FP64 value)
+                  const double vd = v == v0 ? sm.lgEd[pl] - sm.lzd[col]
+                                            : sm.gE[v0 < v ? 0 : nEt - 1];
+                  u.h = (float)(vd - sm.gE[b3]);
+                } else {
+                  u = fix_df(v - sm.gEi[b3]);
+                }
               }
               if constexpr (kMixed) {
                 float I_E;
