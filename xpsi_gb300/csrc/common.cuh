@@ -62,6 +62,23 @@ __device__ __forceinline__ int locate(const T *x, int n, T v) {
   return lo;
 }
 
+// v below w, both finite, by the bit patterns (-0 counts as 0): a comparison
+// on the integer pipe (the FP64 pipe takes 64 cycles or more for it)
+__device__ __forceinline__ long long ordered(double v) {
+  const long long b = __double_as_longlong(v);
+  return b < 0 ? -(b & 0x7fffffffffffffffLL) : b;
+}
+// locate() on a table of non-negative values
+__device__ __forceinline__ int locate_bits(const double *x, int n, double v) {
+  const long long vb = __double_as_longlong(v);
+  int lo = 0, hi = n - 1;
+  while (hi > lo + 1) {
+    const int mid = (lo + hi) >> 1;
+    if (__double_as_longlong(x[mid]) > vb) hi = mid; else lo = mid;
+  }
+  return lo;
+}
+
 // ---------------------------------------------------------------------
 // Steffen (1990) monotone cubic, evaluated without a coefficient table: the
 // node slopes of interval i need only y[i-1..i+2].  End slopes are the end

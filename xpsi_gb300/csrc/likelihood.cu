@@ -170,7 +170,7 @@ __device__ __forceinline__ int akima_pieces_warp_df(const double *x, const doubl
   }
   if (inf || e == INT_MIN) e = 0;
   // yd (in k3[] for now) and the chords
-  for (int q = lane; q < n; q += 32) k3[q] = df_split(ldexp(y[q], -e));
+  for (int q = lane; q < n; q += 32) k3[q] = df_split_bits(y[q], -e);
   __syncwarp();
   for (int q = lane; q < n - 1; q += 32)
     ch[q] = df_mul(df_sub(k3[q + 1], k3[q]), ih[q]);
@@ -200,7 +200,7 @@ __device__ __forceinline__ DF akima_integral_df(const double *x, const DF *yd, i
                                                 const DF *k1, const DF *k2, const DF *k3,
                                                 double lo, double hi) {
   const DF third{0.3333333432674408f, -9.934107758624577e-09f};
-  const int ia = locate(x, n, lo), ib = locate(x, n, hi);
+  const int ia = locate_bits(x, n, lo), ib = locate_bits(x, n, hi);
   DF acc{0.0f, 0.0f};
   for (int i = ia; i <= ib; i++) {
     const double u = (i == ia) ? lo - x[i] : 0.0;
@@ -212,7 +212,7 @@ __device__ __forceinline__ DF akima_integral_df(const double *x, const DF *yd, i
     const double ts[2] = {w, u};
 #pragma unroll
     for (int z = 0; z < 2; z++) {
-      const DF t = df_split(ts[z]);
+      const DF t = df_split_bits(ts[z], 0);
       F[z] = df_mul(t, df_fma(t, df_fma(t, df_fma(t, c3, c2), c1), yd[i]));
     }
     acc = df_add(acc, df_sub(F[0], F[1]));
@@ -428,6 +428,59 @@ __device__ double warp_dyadic(const Marg &m, WarpSmem &w, int lane, double lo, d
   return sum;
 }
 
+// A 61-point Gauss-Kronrod panel over [a, b] by the warp, two nodes to a lane
+// (61 of its 64 slots).  The integrand is an exponential, so its own sum is
+// the rule's |f| sum; the error estimate is QUADPACK's.
+__device__ __forceinline__ void warp_panel61(const Marg &m, int lane, double a, double b,
+                                             double &res, double &err) {
+  const int NH = XG_K61_HALF - 1;  // 30
+  const double c = 0.5 * (a + b), h = 0.5 * (b - a);
+  double f[2] = {0.0, 0.0}, wk[2] = {0.0, 0.0}, wg[2] = {0.0, 0.0};
+#pragma unroll 1
+  for (int z = 0; z < 2; z++) {
+    const int n = lane + 32 * z;
+    if (n > 2 * NH) break;
+    const int s = n <= NH ? n : n - NH - 1;
+    const double x = n < NH ? -XG_K61_X[s] : (n == NH ? 0.0 : XG_K61_X[s]);
+    f[z] = marginal_integrand(m, fma(h, x, c));
+    wk[z] = XG_K61_WK[s];
+    wg[z] = XG_K61_WG[s];
+  }
+  const double rk = warp_sum(fma(wk[1], f[1], wk[0] * f[0]));
+  const double rg = warp_sum(fma(wg[1], f[1], wg[0] * f[0]));
+  const double mean = 0.5 * rk;
+  const double rc = warp_sum(fma(wk[1], fabs(f[1] - mean), wk[0] * fabs(f[0] - mean))) * h;
+  res = rk * h;
+  double e = fabs((rk - rg) * h);
+  if (rc != 0.0 && e != 0.0) {
+    const double x = 200.0 * e / rc, sc = x * sqrt(x);
+    e = sc < 1.0 ? rc * sc : rc;
+  }
+  err = fmax(e, 50.0 * 2.220446049250313e-16 * res);
+}
+
+// The marginal integral over [a, b] from one such panel on each side of the
+// integrand's peak (one in all where the peak lies on an end): a window of
+// ten standard deviations either way is smooth enough that they meet the
+// adaptive rule's tolerance, at two node evaluations per lane and panel
+// against two for each of the eight or so bisections, whose sums and error
+// estimates (FP64, one per warp) were the kernel's larger half.  Returns false
+// where they do not.
+__device__ __forceinline__ bool warp_peak61(const Marg &m, int lane, double a, double b,
+                                            double er, double &out) {
+  const bool inside = a < m.Bi && m.Bi < b;
+  double r, e;
+  warp_panel61(m, lane, a, inside ? m.Bi : b, r, e);
+  if (inside) {
+    double r2, e2;
+    warp_panel61(m, lane, m.Bi, b, r2, e2);
+    r += r2;
+    e += e2;
+  }
+  out = r;
+  return r > 0.0 && e <= er * r;
+}
+
 // the marginal integral over [a, b]: adaptive GK21 at relative
 // min(epsrel, 1e-13); when every interior node sees zero but an endpoint
 // does not (a channel without counts has a window ~1e91 wide whose integrand
@@ -442,6 +495,8 @@ __device__ double warp_marginal(const Marg &m, WarpSmem &w, int lane, double a, 
   if (a == b) return 0.0;
   double er = epsrel < 1.0e-13 ? epsrel : 1.0e-13;
   if (epsabs <= 0.0 && er < 50.0 * eps) er = 50.0 * eps;
+  double peak;
+  if (m.rel && warp_peak61(m, lane, a, b, er, peak)) return sign * peak;
   double r = warp_qag21_core(m, w, lane, a, b, epsabs, er);
   if (r == 0.0) {
     double fa = marginal_integrand(m, a);
@@ -504,7 +559,7 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
         auto piece = [&](double lo, double hi) -> double {
           if (lo > hi || lo < xs[0] || hi > xs[N_P - 1]) return nan("");
           if (lo == hi) return 0.0;
-          return ldexp(df_value(akima_integral_df(xs, yd, N_P, k1, k2, k3, lo, hi)), ex);
+          return df_join_bits(akima_integral_df(xs, yd, N_P, k1, k2, k3, lo, hi), ex);
         };
         double val;
         if (pa < pb) {
@@ -704,18 +759,21 @@ __device__ __forceinline__ void comp_add(double &s, double &c, double x) {
   s = t;
 }
 
-// per-evaluation sum over channels and the reference's early exits: one
-// warp per evaluation; the first flagged channel (lowest index) decides the
+// per-evaluation sum over channels and the reference's early exits: one CTA
+// per evaluation; the first flagged channel (lowest index) decides the
 // early exit (:677-684, :423-429), otherwise the channel terms are summed
-// with compensation (each lane over its channels, then the lanes' sums and
-// corrections by a fixed butterfly: bitwise reproducible)
-__global__ void like_finalize_kernel(LikeArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (v >= a.n_vec) return;
+// with compensation (each thread over its channels, then the lanes' sums and
+// corrections by a fixed butterfly and the warps' in order: bitwise
+// reproducible)
+constexpr int kFinalWarps = 4;
+__global__ void __launch_bounds__(32 * kFinalWarps) like_finalize_kernel(LikeArgs a) {
+  __shared__ double s_s[kFinalWarps], s_c[kFinalWarps];
+  __shared__ int s_first[kFinalWarps];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int v = blockIdx.x;
   double LL = 0.0, LLc = 0.0;
   int first = 0x7fffffff;
-  for (int ch = lane; ch < a.K; ch += 32) {
+  for (int ch = threadIdx.x; ch < a.K; ch += blockDim.x) {
     const size_t o = (size_t)v * a.K + ch;
     if (a.chan_flag[o] != 0) {
       if (ch < first) first = ch;
@@ -736,6 +794,18 @@ __global__ void like_finalize_kernel(LikeArgs a) {
     LL = s;
     LLc = c;
   }
+  if (lane == 0) {
+    s_s[wid] = LL;
+    s_c[wid] = LLc;
+    s_first[wid] = first;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < kFinalWarps; w++) {
+    comp_add(LL, LLc, s_s[w]);
+    LLc += s_c[w];
+    first = min(first, s_first[w]);
+  }
   LL = LL + LLc;
   int st = kOk;
   if (first != 0x7fffffff) {
@@ -747,10 +817,8 @@ __global__ void like_finalize_kernel(LikeArgs a) {
     LL = a.llzero * (0.1 + 0.9 * U);
     st = (f == 1) ? kSlimCut : kQuadFail;
   }
-  if (lane == 0) {
-    a.loglike[v] = LL;
-    a.status[v] = st;
-  }
+  a.loglike[v] = LL;
+  a.status[v] = st;
 }
 
 }  // namespace
@@ -760,7 +828,7 @@ void launch_likelihood(const LikeArgs &a, cudaStream_t st) {
   if (warps <= 0) return;
   unsigned blocks = (unsigned)((warps + kWarps - 1) / kWarps);
   like_channel_kernel<<<blocks, 32 * kWarps, 0, st>>>(a);
-  like_finalize_kernel<<<(a.n_vec + 3) / 4, 128, 0, st>>>(a);
+  like_finalize_kernel<<<a.n_vec, 32 * kFinalWarps, 0, st>>>(a);
 }
 
 }  // namespace xg
