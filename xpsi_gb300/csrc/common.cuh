@@ -448,7 +448,7 @@ __device__ __forceinline__ DF df_split_bits(double v, int e) {
 __device__ __forceinline__ double df_join_bits(DF a, int e) {
   const int hb = __float_as_int(a.h), eh = ((hb >> 23) & 0xff) - 127;
   const int ex = eh + e;
-  if (eh < -60 || eh > 100 || ex < -1020 || ex > 1020) {
+  if (eh < -60 || eh > 126 || ex < -1020 || ex > 1020) {
     if (a.h == 0.0f) return 0.0;
     return scale_pow2(df_value(a), e);
   }

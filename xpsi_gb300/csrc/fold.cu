@@ -12,7 +12,8 @@
 //     stored transposed (q-major) for the tile loads;
 //  2. fold_cols_kernel: every column of every member's input likewise,
 //     2^sX[b][n];
-//  3. fold_df_kernel: 64 x 64 output tiles, 4 x 4 outputs per thread.  Per
+//  3. fold_df_kernel: 64 x 64 output tiles, 4 x 4 outputs per thread (32 x 32
+//     and 2 x 2 in small batches).  Per
 //     term the product's rounding error comes from an FMA (plus both cross
 //     terms), the rounded products are summed by error-free two-sums into s
 //     and every error into c; (s, c) is renormalised after each 16 terms; the
@@ -31,7 +32,7 @@
 namespace xg {
 namespace {
 
-constexpr int TM = 64, TN = 64, TK = 16;
+constexpr int TK = 16;
 constexpr int kFoldThreads = 256;
 constexpr int kRowsPerCta = kFoldThreads / 32;
 constexpr int kColGroups = kFoldThreads / 32;
@@ -65,7 +66,7 @@ FoldScratch carve(const FoldArgs &a, void *scratch) {
 }
 
 __device__ __forceinline__ float2 scaled_split(double v, int s) {
-  const DF d = df_split(scale_pow2(v, s));
+  const DF d = df_split_bits(v, s);
   return make_float2(d.h, d.l);
 }
 
@@ -117,18 +118,24 @@ __global__ void __launch_bounds__(kFoldThreads) fold_cols_kernel(FoldArgs a, Fol
   if (g == 0) f.sx[(size_t)b * a.N + n] = s;
 }
 
+// R x R outputs per thread, 16 R x 16 R output tiles: R = 4, or 2 where the
+// larger tiles would not fill the chip (one 1500 x 128 x 128 signal: 48 tiles
+// of 64, 67 us; 188 of 32, 30 us; 24 vectors, 2304 tiles of 64: 574 us); an
+// output's sum is the same either way.
+template <int R>
 __global__ void __launch_bounds__(kFoldThreads) fold_df_kernel(FoldArgs a, FoldScratch f) {
+  constexpr int TM = 16 * R, TN = 16 * R;
   __shared__ float2 sA[TK][TM];
   __shared__ float2 sB[TK][TN];
   const int b = blockIdx.z;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   const float2 *Xs = f.xs + (size_t)b * a.q * a.N;
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float s[4][4], c[4][4];
+  float s[R][R], c[R][R];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < R; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) s[i][j] = c[i][j] = 0.0f;
+    for (int j = 0; j < R; j++) s[i][j] = c[i][j] = 0.0f;
   const float2 zero = make_float2(0.0f, 0.0f);
   for (int k0 = 0; k0 < a.q; k0 += TK) {
     for (int t = threadIdx.x; t < TK * TM; t += kFoldThreads) {
@@ -144,26 +151,26 @@ __global__ void __launch_bounds__(kFoldThreads) fold_df_kernel(FoldArgs a, FoldS
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < TK; kk++) {
-      DF av[4], bv[4];
+      DF av[R], bv[R];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
+      for (int i = 0; i < R; i++) {
         const float2 v = sA[kk][ty + 16 * i];
         av[i] = DF{v.x, v.y};
       }
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
+      for (int j = 0; j < R; j++) {
         const float2 v = sB[kk][tx + 16 * j];
         bv[j] = DF{v.x, v.y};
       }
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int i = 0; i < R; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) df_acc_mul(av[i], bv[j], s[i][j], c[i][j]);
+        for (int j = 0; j < R; j++) df_acc_mul(av[i], bv[j], s[i][j], c[i][j]);
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < R; i++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
+      for (int j = 0; j < R; j++) {
         const DF r = df_norm(s[i][j], c[i][j]);
         s[i][j] = r.h;
         c[i][j] = r.l;
@@ -173,15 +180,15 @@ __global__ void __launch_bounds__(kFoldThreads) fold_df_kernel(FoldArgs a, FoldS
   double *Out = a.out + (size_t)b * a.K * a.N;
   const int *sx = f.sx + (size_t)b * a.N;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < R; i++) {
     const int gm = m0 + ty + 16 * i;
     if (gm >= a.K) continue;
     const int sm = f.sm[gm];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < R; j++) {
       const int gn = n0 + tx + 16 * j;
       if (gn < a.N)
-        Out[(size_t)gm * a.N + gn] = scale_pow2((double)s[i][j] + (double)c[i][j], -(sm + sx[gn]));
+        Out[(size_t)gm * a.N + gn] = df_join_bits(DF{s[i][j], c[i][j]}, -(sm + sx[gn]));
     }
   }
 }
@@ -200,8 +207,11 @@ void launch_fold(const FoldArgs &a, void *scratch, cudaStream_t st) {
   const int T = fold_target_exponent(a.q);
   fold_rows_kernel<<<(a.K + kRowsPerCta - 1) / kRowsPerCta, kFoldThreads, 0, st>>>(a, f, T);
   fold_cols_kernel<<<dim3((a.N + 31) / 32, a.batch), kFoldThreads, 0, st>>>(a, f, T);
-  dim3 grid((a.N + TN - 1) / TN, (a.K + TM - 1) / TM, a.batch);
-  fold_df_kernel<<<grid, kFoldThreads, 0, st>>>(a, f);
+  const int64_t tiles = (int64_t)((a.N + 63) / 64) * ((a.K + 63) / 64) * a.batch;
+  if (tiles < 304)  // below two tiles per SM (two signals, 96: 97 us, 37 us now)
+    fold_df_kernel<2><<<dim3((a.N + 31) / 32, (a.K + 31) / 32, a.batch), kFoldThreads, 0, st>>>(a, f);
+  else
+    fold_df_kernel<4><<<dim3((a.N + 63) / 64, (a.K + 63) / 64, a.batch), kFoldThreads, 0, st>>>(a, f);
 }
 
 }  // namespace xg
