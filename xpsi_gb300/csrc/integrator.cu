@@ -41,6 +41,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kEPT = 8;  // energies per accumulation task
 constexpr int kMaxCellsF = 256;  // cells per parallel held as FP32 pairs in shared memory
+constexpr int kMaxPhases = 1024;  // signal phases held as FP32 pairs in shared memory
 constexpr int kMaxEnergiesF = 256;  // energies held in FP32 (mixed form)
 constexpr int kStrip = 8;  // Akima pieces per thread, built from a sliding window of chords
 
@@ -1439,9 +1440,13 @@ struct IntSmem {
   RunStage *stages;
   size_t bytes;
 };
+// the integrator's dynamic shared memory at most (with the statically
+// allocated part, 227 KB): the form without runs takes every size that 200 KB
+// held with the pieces in rows of EC and the ray table staged per CTA
+constexpr size_t kIntSmemMax = 225 * 1024;
 template <bool kMixed>
 __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC, int nmu, int nE,
-                                            bool tab2) {
+                                            bool tab2, bool runs) {
   IntSmem o{};
   size_t at = 0;
   auto take = [&](auto *&p, size_t n) {
@@ -1477,11 +1482,9 @@ __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC
   if (tab4) take(o.lgE, EC);
   if (tab2 || (tab4 && kMixed)) take(o.lgEd, EC);
   take(o.sc_exp, EC);
-  take(o.phase, N_P);
-  if (!kMixed) {
-    take(o.flags, 2 * N_L); take(o.nruns, 2 * N_P);
-    take(o.stages, kThreads / EC);
-  }
+  if (N_P <= kMaxPhases) take(o.phase, N_P);
+  if (!kMixed) take(o.flags, 2 * N_L);
+  if (runs) { take(o.nruns, 2 * N_P); take(o.stages, kThreads / EC); }
   o.bytes = (at + 15) & ~size_t(15);
   return o;
 }
@@ -1516,7 +1519,9 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
   // reduced once per call to (mu, E) with E' in electron rest energies
   // (integrator_for_azimuthal_invariance_split.pyx:270-275,457-476)
   const bool tab2 = a.table2d && !kMixed;
-  const IntSmem sm = int_smem<kMixed>(smem, N_L, N_P, EC, nmu, nEt, a.table2d != 0);
+  // power-sum form (FP64 path with scratch)
+  const bool use_w = !kMixed && a.wsum != nullptr;
+  const IntSmem sm = int_smem<kMixed>(smem, N_L, N_P, EC, nmu, nEt, a.table2d != 0, use_w);
   PieceT<WT> *co4 = reinterpret_cast<PieceT<WT> *>(sm.piece);  // mixed form
   const PieceRows pr{reinterpret_cast<float4 *>(sm.piece),
                      reinterpret_cast<float4 *>(sm.piece) + (size_t)N_L * (EC + 1), EC + 1};
@@ -1526,8 +1531,6 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
   __shared__ float s_erange[2];
   // a beaming modification's (abb, bbb, cbb, dbb, nimu) for the parallel
   __shared__ double s_beam[5];
-  // power-sum form (FP64 path with scratch)
-  const bool use_w = !kMixed && a.wsum != nullptr;
   const WRuns wr = use_w ? wruns_of(a.wsum + (size_t)blockIdx.x *
                                                  integrate_wsum_bytes_dev(N_P, a.w_cap),
                                     a.w_cap, N_P)
@@ -1575,10 +1578,11 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
     }
   }
   const EGrid eg4{sm.dgEo, sm.dsE, sm.xe, nEt};
-  for (int t = threadIdx.x; t < N_P; t += blockDim.x) {
-    const DF v = df_split(a.phases[t]);
-    sm.phase[t] = make_float2(v.h, v.l);
-  }
+  if (sm.phase)
+    for (int t = threadIdx.x; t < N_P; t += blockDim.x) {
+      const DF v = df_split(a.phases[t]);
+      sm.phase[t] = make_float2(v.h, v.l);
+    }
   if (use_w)
     for (int t = threadIdx.x; t < kThreads / EC; t += blockDim.x) {
       sm.stages[t].w[2 * kStage] = sm.stages[t].w[2 * kStage + 1] =
@@ -1874,7 +1878,13 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
         }
         __syncthreads();
         auto cell_phase = [&](auto cached, int k) {
-          const float2 ph = sm.phase[k];
+          float2 ph;
+          if (sm.phase) {
+            ph = sm.phase[k];
+          } else {
+            const DF v = df_split(a.phases[k]);
+            ph = make_float2(v.h, v.l);
+          }
           return CellPhaseF<decltype(cached)::value>{
               sm.fphase, sm.fphase_lo, N_L, sm.fphase[0], sm.fphase[N_L - 1], ph.x, ph.y, tp,
               (float)(kTwoPi - (double)tp), sm.fcphi, sm.fcphi_lo, cellPhi};
@@ -2836,6 +2846,11 @@ size_t integrate_wsum_bytes(int N_P, int max_cells, int *w_cap) {
   return integrate_wsum_bytes_dev(N_P, cap);
 }
 
+bool integrate_runs_fit(int N_L, int N_P, int EC, int nmu, int nE, int table2d) {
+  return N_P <= kMaxPhases &&
+         int_smem<false>(nullptr, N_L, N_P, EC, nmu, nE, table2d, true).bytes <= kIntSmemMax;
+}
+
 int64_t integrate_image_doubles(int N_L) { return image_doubles(N_L); }
 
 int integrate_energy_chunk(int N_L, int N_P, int N_E, int mixed) {
@@ -2853,14 +2868,16 @@ void launch_integrate(const IntegrateArgs &a, cudaStream_t st) {
   const long items = (long)a.max_chunks * a.n_eg;
   const unsigned ctas = (unsigned)(items < a.ctas ? items : a.ctas);
   if (a.mixed) {
-    const size_t bytes = int_smem<true>(nullptr, a.N_L, a.N_P, a.EC, nmu, nE, a.table2d).bytes;
+    const size_t bytes = int_smem<true>(nullptr, a.N_L, a.N_P, a.EC, nmu, nE, a.table2d,
+                                              false).bytes;
     cudaFuncSetAttribute(integrate_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
+                         kIntSmemMax);
     integrate_kernel<float><<<ctas, kThreads, bytes, st>>>(a);
   } else {
-    const size_t bytes = int_smem<false>(nullptr, a.N_L, a.N_P, a.EC, nmu, nE, a.table2d).bytes;
+    const size_t bytes = int_smem<false>(nullptr, a.N_L, a.N_P, a.EC, nmu, nE, a.table2d,
+                                               a.wsum != nullptr).bytes;
     cudaFuncSetAttribute(integrate_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         200 * 1024);
+                         kIntSmemMax);
     integrate_kernel<double><<<ctas, kThreads, bytes, st>>>(a);
   }
   dim3 grid((a.N_E * a.N_P + 255) / 256, a.n_members);

@@ -129,6 +129,8 @@ void launch_integrate(const IntegrateArgs &a, cudaStream_t st);
 // at most max_cells cells (w_cap runs per cell half and signal phase); doubles
 // of an image's geometry record; energies per chunk
 size_t integrate_wsum_bytes(int N_P, int max_cells, int *w_cap);
+// whether the form with runs finds its shared memory
+bool integrate_runs_fit(int N_L, int N_P, int EC, int nmu, int nE, int table2d);
 int64_t integrate_image_doubles(int N_L);
 int integrate_energy_chunk(int N_L, int N_P, int N_E, int mixed);
 // Stokes I (a.flux), Q, U for blackbody (1) and burst blackbody (3) members;
