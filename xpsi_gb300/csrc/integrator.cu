@@ -915,31 +915,76 @@ struct AreaDF {
 // the reference adds an interpolant value when it is > 0 (:593-594)
 __device__ __forceinline__ bool positive(float v) { return v > 0.0f; }
 
-// sums over the radiating cells of one parallel at one signal phase for the
-// energies pb .. pb+kEPT-1 of the chunk; false when a cell phase cannot be
-// wrapped into the knot range (the reference's terminate)
-template <typename WT, typename CP, typename AR>
-__device__ __forceinline__ bool cell_phase_sums(const CP &cp, const AR &area, int S1,
-                                                const int32_t *rad, const PieceT<WT> *co4,
-                                                int N_L, int pb, int ne, WT (&acc)[kEPT]) {
-  int hint = -1;
-  for (int j = 0; j < S1; j++) {
-    if (rad[j] != 1) continue;
-    WT t;
-    const int iv = cp(j, hint, t);
-    if (iv < 0) return false;
-    hint = iv;
-    const WT A = area(j);
+// Mixed form: the sums over the radiating cells of one parallel at one signal
+// phase for the lane's Z energies; eight lanes share a phase, energies e + 8 z
+// of the chunk to lane e.  The lanes place a batch of eight cells (interval
+// and offset) in shared memory, then walk it in the cells' order; a piece is
+// read where the interval changes, about every third cell.  FP32 issue bounds
+// it: five instructions per cell and energy (three FMAs, the reference's test,
+// an FMA) and eight per cell that the Z energies share.  With lanes over the
+// phases each cell read eight pieces, every (phase, eight energies) placed
+// the cells again, and branches kept the eight chains from overlapping (issue
+// slots 42 % busy); with one energy per lane the shared part weighed most.
+// 64 vectors of two Num4D regions at sqrt_num_cells 96: 28.4 ms lanes over
+// phases, 19.6 one energy per lane, 14.7 now.
+// True in `bad`: a cell phase cannot be wrapped into the knot range (the
+// reference's terminate).
+constexpr int kCellLanes = 8;
+struct CellStage {
+  float2 ta[kThreads];  // offset and area
+  int iv[kThreads];
+};
+template <int Z, typename CP, typename AR>
+__device__ __forceinline__ void cell_phase_sums_f(const CP &cp, const AR &area, int S1,
+                                                  const int32_t *rad, const float4 *piece, int es,
+                                                  CellStage &cs, bool &bad, float (&acc)[Z]) {
+  const int lane = threadIdx.x & 31, e = lane % kCellLanes, shift = lane - e;
+  float2 *ta = cs.ta + (threadIdx.x - e);
+  int *ivs = cs.iv + (threadIdx.x - e);
+  int cur = -1;
+  bool lost = false;
+  float4 q[Z];
 #pragma unroll
-    for (int e = 0; e < kEPT; e++) {
-      if (pb + e < ne) {
-        const PieceT<WT> q = co4[(pb + e) * N_L + iv];
-        const WT sv = q.y + t * (q.k1 + t * (q.k2 + t * q.k3));
-        if (positive(sv)) acc[e] += A * sv;
+  for (int z = 0; z < Z; z++) {
+    acc[z] = 0.0f;
+    q[z] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (int b = 0; b < S1; b += kCellLanes) {
+    const int j = b + e;
+    const bool on = j < S1 && rad[j] == 1;
+    const uint32_t lit = __ballot_sync(0xffffffffu, on) & 0xffu;  // the same in every group
+    const int n = __popc(lit);
+    if (n == 0) continue;
+    __syncwarp();  // the last batch's readers are done
+    if (on) {
+      float t;
+      const int iv = cp(j, -1, t);
+      lost |= iv < 0;
+      const int at = __popc(lit & ((1u << e) - 1u));
+      ta[at] = make_float2(t, area(j));
+      ivs[at] = max(iv, 0);
+    }
+    __syncwarp();
+    const bool change = e < n && ivs[e] != (e > 0 ? ivs[e - 1] : cur);
+    uint32_t read = __ballot_sync(0xffffffffu, change) >> shift;
+    cur = ivs[n - 1];
+    for (int i = 0; i < n; i++) {
+      if (read & 1u) {
+        const float4 *p = piece + ivs[i] * es + e;
+#pragma unroll
+        for (int z = 0; z < Z; z++) q[z] = p[kCellLanes * z];
+      }
+      read >>= 1;
+      const float2 c = ta[i];
+#pragma unroll
+      for (int z = 0; z < Z; z++) {
+        const float sv =
+            __fmaf_rn(c.x, __fmaf_rn(c.x, __fmaf_rn(c.x, q[z].w, q[z].z), q[z].y), q[z].x);
+        if (positive(sv)) acc[z] = __fmaf_rn(c.y, sv, acc[z]);
       }
     }
   }
-  return true;
+  bad = ((__ballot_sync(0xffffffffu, lost) >> shift) & 0xffu) != 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -974,7 +1019,7 @@ struct PieceRows {
   }
 };
 
-// the FP64 path's form of cell_phase_sums, in double-float arithmetic on
+// the same sums cell by cell in double-float arithmetic, kEPT energies per thread, on
 // scaled pieces (the sign test is on the high part: h + l has the sign of h;
 // with the elsewhere correction every value is added, :593-594)
 template <typename CP, typename AR>
@@ -1438,6 +1483,7 @@ struct IntSmem {
   int *nruns;
   float2 *phase;
   RunStage *stages;
+  CellStage *cells;                // mixed form
   size_t bytes;
 };
 // the integrator's dynamic shared memory at most (with the statically
@@ -1455,7 +1501,7 @@ __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC
     p = reinterpret_cast<T *>(base + at);
     at += n * sizeof(T);
   };
-  const size_t pieces = kMixed ? (size_t)EC * N_L * sizeof(PieceT<float>)
+  const size_t pieces = kMixed ? (size_t)(EC + 1) * N_L * sizeof(PieceT<float>)
                                : (size_t)2 * (EC + 1) * N_L * sizeof(float4);
   const size_t geo = (size_t)N_L * 8 * sizeof(double) + (size_t)(4 * N_L + 8) * sizeof(int) + 64;
   take(o.piece, pieces > geo ? pieces : geo);
@@ -1484,6 +1530,7 @@ __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC
   take(o.sc_exp, EC);
   if (N_P <= kMaxPhases) take(o.phase, N_P);
   if (!kMixed) take(o.flags, 2 * N_L);
+  if (kMixed) take(o.cells, 1);
   if (runs) { take(o.nruns, 2 * N_P); take(o.stages, kThreads / EC); }
   o.bytes = (at + 15) & ~size_t(15);
   return o;
@@ -1630,7 +1677,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
     // partials: FP64 form [N_P][N_E] (the sums' lanes are energies), mixed [N_E][N_P]
     for (int t = threadIdx.x; t < N_P * (e_hi - e_lo); t += blockDim.x) {
       const int k = t / (e_hi - e_lo), e = e_lo + t - k * (e_hi - e_lo);
-      part[kMixed ? (size_t)e * N_P + k : (size_t)k * N_E + e] = 0.0;
+      part[(size_t)k * N_E + e] = 0.0;
     }
     if (t4 && warp == 0) {  // the item's range of log10 E
       float lo = INFINITY, hi = -INFINITY;
@@ -1882,7 +1929,8 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
           if (sm.phase) {
             ph = sm.phase[k];
           } else {
-            const DF v = df_split(a.phases[k]);
+            // (on the integer pipe: the compiler evaluates both sides)
+            const DF v = df_split_bits(a.phases[k], 0);
             ph = make_float2(v.h, v.l);
           }
           return CellPhaseF<decltype(cached)::value>{
@@ -1934,7 +1982,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
             for (int pl = part0; pl < ne; pl += parts) {
               const int p = e0 + pl;
               if (!(f & kColLit)) {
-                if constexpr (kMixed) co4[pl * N_L + col].y = 0.0f;
+                if constexpr (kMixed) co4[col * (EC + 1) + pl].y = 0.0f;
                 else if (dfy) pr.y(col, pl) = DF{0.0f, 0.0f};
                 else pr.yd(col, pl) = 0.0;
                 continue;
@@ -1975,7 +2023,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
                 } else {
                   I_E = eval_bb_f((float)a.energies[p] * sm.finvZ[col], kT_f);
                 }
-                co4[pl * N_L + col].y = (float)norm * I_E * sm.fgeom[col];
+                co4[col * (EC + 1) + pl].y = (float)norm * I_E * sm.fgeom[col];
               } else {
                 double I_E;
                 if (t4) {
@@ -2070,15 +2118,17 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
           // five chords each piece needs, so each chord is formed once per
           // strip instead of five times
           if constexpr (kMixed) {
-            for (int t = threadIdx.x; t < ne * strips; t += blockDim.x) {
-              const int pl = t / strips, i0 = (t - pl * strips) * kStrip;
+            for (int t = threadIdx.x; t < EC * strips; t += blockDim.x) {
+              const int pl = t % EC, i0 = (t / EC) * kStrip;
               const int i1 = min(i0 + kStrip, n_iv);
-              PieceT<WT> *yr = co4 + pl * N_L;
+              if (pl >= ne) continue;
+              PieceT<WT> *yr = co4 + pl;
+              const int es = EC + 1;
               auto chord = [&](int j) -> WT {
                 const int q = periodic_chord(j, N_L);
                 // knot spacings from the FP64 knots: adjacent knots closer
                 // than an FP32 ulp stay distinct
-                return (yr[q + 1].y - yr[q].y) / sm.fh[q];
+                return (yr[(q + 1) * es].y - yr[q * es].y) / sm.fh[q];
               };
               WT m0 = chord(i0 - 2), m1 = chord(i0 - 1), m2 = chord(i0), m3 = chord(i0 + 1),
                  m4 = chord(i0 + 2);
@@ -2089,7 +2139,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
                 }
                 WT k1, k2, k3;
                 akima_piece(m0, m1, m2, m3, m4, (WT)sm.fh[iv], k1, k2, k3);
-                PieceT<WT> *o = yr + iv;
+                PieceT<WT> *o = yr + iv * es;
                 o->k1 = k1;
                 o->k2 = k2;
                 o->k3 = k3;
@@ -2207,6 +2257,35 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
               n0 = m0;
               n1 = m1;
             }
+          } else if constexpr (kMixed) {
+            const int e = threadIdx.x % kCellLanes, grp = threadIdx.x / kCellLanes;
+            auto sums = [&](auto cached, auto per_lane) {
+              constexpr int Z = decltype(per_lane)::value;
+              const AreaF<decltype(cached)::value> ar{sm.fcarea, cellA};
+              for (int k0 = 0; k0 < N_P; k0 += kThreads / kCellLanes) {
+                const int k = k0 + grp, kc = min(k, N_P - 1);
+                double *dst = part + (size_t)kc * N_E + e0 + e;
+                bool bad;
+                float v[Z];
+                cell_phase_sums_f<Z>(cell_phase(cached, kc), ar, M.S1, rad,
+                                     reinterpret_cast<const float4 *>(co4), EC + 1, *sm.cells,
+                                     bad, v);
+                if (bad) {
+                  atomicExch(&a.member_status[m], (int)kPulseFail);
+                } else if (k < N_P) {
+#pragma unroll
+                  for (int z = 0; z < Z; z++)
+                    if (e + kCellLanes * z < ne) dst[kCellLanes * z] += (double)v[z] * fix;
+                }
+              }
+            };
+            auto by_cells = [&](auto per_lane) {
+              if (M.S1 <= kMaxCellsF) sums(std::true_type{}, per_lane);
+              else sums(std::false_type{}, per_lane);
+            };
+            if (EC == 32) by_cells(std::integral_constant<int, 4>{});
+            else if (EC == 16) by_cells(std::integral_constant<int, 2>{});
+            else by_cells(std::integral_constant<int, 1>{});
           } else {
             const int ntasks = N_P * (EC / kEPT);
             auto sums = [&](auto cached) {
@@ -2216,34 +2295,19 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
                 const int pb = grp * kEPT;
                 if (pb >= ne) continue;
                 const CellPhaseF<kCached> cp = cell_phase(cached, k);
-                if constexpr (kMixed) {
-                  WT acc[kEPT];
+                DF acc[kEPT];
 #pragma unroll
-                  for (int e = 0; e < kEPT; e++) acc[e] = WT(0);
-                  const AreaF<kCached> ar{sm.fcarea, cellA};
-                  if (!cell_phase_sums<WT>(cp, ar, M.S1, rad, co4, N_L, pb, ne, acc)) {
-                    atomicExch(&a.member_status[m], (int)kPulseFail);
-                    continue;
-                  }
-#pragma unroll
-                  for (int e = 0; e < kEPT; e++)
-                    if (pb + e < ne)
-                      part[(size_t)(e0 + pb + e) * N_P + k] += (double)acc[e] * fix;
-                } else {
-                  DF acc[kEPT];
-#pragma unroll
-                  for (int e = 0; e < kEPT; e++) acc[e] = DF{0.0f, 0.0f};
-                  const AreaDF<kCached> ar{sm.fcarea, sm.fcarea_lo, cellA};
-                  if (!cell_phase_sums_df(cp, ar, M.S1, rad, pr, pb, corr, acc)) {
-                    atomicExch(&a.member_status[m], (int)kPulseFail);
-                    continue;
-                  }
-#pragma unroll
-                  for (int e = 0; e < kEPT; e++)
-                    if (pb + e < ne)
-                      part[(size_t)k * N_E + e0 + pb + e] +=
-                          scale_pow2(df_value(acc[e]), sm.sc_exp[pb + e]);
+                for (int e = 0; e < kEPT; e++) acc[e] = DF{0.0f, 0.0f};
+                const AreaDF<kCached> ar{sm.fcarea, sm.fcarea_lo, cellA};
+                if (!cell_phase_sums_df(cp, ar, M.S1, rad, pr, pb, corr, acc)) {
+                  atomicExch(&a.member_status[m], (int)kPulseFail);
+                  continue;
                 }
+#pragma unroll
+                for (int e = 0; e < kEPT; e++)
+                  if (pb + e < ne)
+                    part[(size_t)k * N_E + e0 + pb + e] +=
+                        scale_pow2(df_value(acc[e]), sm.sc_exp[pb + e]);
               }
             };
             if (M.S1 <= kMaxCellsF) sums(std::true_type{});
@@ -2821,9 +2885,7 @@ __global__ void reduce_flux_kernel(IntegrateArgs a) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int c = c0; c < c1; c++) s += a.partial[(size_t)c * n + t];
-    // the FP64 form's partials are [N_P][N_E], the mixed form's [N_E][N_P]
-    const int p = a.mixed ? t / a.N_P : t % a.N_E;
-    const int k = a.mixed ? t - p * a.N_P : t / a.N_E;
+    const int p = t % a.N_E, k = t / a.N_E;  // partials are [N_P][N_E]
     a.flux[M.flux_off + (int64_t)p * a.N_P + k] = s / (a.energies[p] * kKeV);
   }
 }
@@ -2854,8 +2916,15 @@ bool integrate_runs_fit(int N_L, int N_P, int EC, int nmu, int nE, int table2d) 
 int64_t integrate_image_doubles(int N_L) { return image_doubles(N_L); }
 
 int integrate_energy_chunk(int N_L, int N_P, int N_E, int mixed) {
-  return energy_chunk(N_L, N_P, N_E,
-                      mixed ? (int)sizeof(PieceT<float>) : (int)sizeof(PieceDF));
+  if (!mixed) return energy_chunk(N_L, N_P, N_E, (int)sizeof(PieceDF));
+  // mixed form: lanes are energies, so the chunk that leaves the fewest lanes
+  // idle, the larger of two (a cell is placed once per chunk), in 96 KB
+  int best = 8;
+  for (int ec = 16; ec <= 32; ec *= 2)
+    if ((size_t)ec * N_L * sizeof(PieceT<float>) <= 96 * 1024 &&
+        (N_E + ec - 1) / ec * ec <= (N_E + best - 1) / best * best)
+      best = ec;
+  return best;
 }
 
 void launch_integrate(const IntegrateArgs &a, cudaStream_t st) {
