@@ -1287,6 +1287,8 @@ __device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_
     // independent, and the groups of the warp stay together
     while (__any_sync(0xffffffffu, todo != 0u)) {
       float h[2], x[2];
+      uint32_t at[2];
+      bool odd[2];
 #pragma unroll
       for (int z = 0; z < 2; z++) {
         const int r = todo ? __ffs(todo) - 1 : kStage;
@@ -1316,16 +1318,22 @@ __device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_
         lead_acc(q.x, B.x, v, x[z]);
         lead_acc(q.z, B.z, v, x[z]);
         h[z] = __fsub_rn(v, lead);
-        const bool odd = r < kStage && ((m.y >> e) & 1u);
-        if (odd) h[z] = x[z] = 0.0f;
-        if (__any_sync(0xffffffffu, odd)) {
-          if (odd && !((m.z >> e) & 1u))
-            walked = run_cells(cp, area, rad, iv, (int)((m.x >> 10) & 1023u),
-                               (int)((m.x >> 20) & 1023u),
-                               PieceDF{{p.x, p.y}, {p.z, p.w}, {q.x, q.y}, {q.z, q.w}}, add_all,
-                               walked);
-          __syncwarp();
+        // (the empty record's meta has no flag set)
+        odd[z] = (m.y >> e) & 1u;
+        at[z] = (m.z >> e) & 1u ? 0u : m.x;
+      }
+      // (after both, so that no branch parts their chains)
+      if (__any_sync(0xffffffffu, odd[0] || odd[1])) {
+#pragma unroll
+        for (int z = 0; z < 2; z++) {
+          if (!odd[z]) continue;
+          h[z] = x[z] = 0.0f;
+          if (at[z] == 0u) continue;  // adds nothing
+          const int iv = (int)(at[z] & 1023u);
+          walked = run_cells(cp, area, rad, iv, (int)((at[z] >> 10) & 1023u),
+                             (int)((at[z] >> 20) & 1023u), pc.at(iv, e), add_all, walked);
         }
+        __syncwarp();
       }
 #pragma unroll
       for (int z = 0; z < 2; z++) {
