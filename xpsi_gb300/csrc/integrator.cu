@@ -1435,8 +1435,9 @@ struct EGrid {
   const int *xe;
   int nE;
 };
-__device__ __forceinline__ DF eval_num4d_dfx(const EGrid &E, const DF *slab, int b2, const DF *w2,
-                                             int b3, DF u0, int &xr) {
+// the energy stencil's weights (scaled to the largest column exponent xr)
+__device__ __forceinline__ void energy_weights(const EGrid &E, int b3, DF u0, DF (&w3)[4],
+                                               int &xr) {
   const DF *o = E.o + 3 * b3;
   const DF u1 = df_sub(u0, o[0]), u2 = df_sub(u0, o[1]), u3 = df_sub(u0, o[2]);
   const DF u01 = df_mul(u0, u1), u23 = df_mul(u2, u3);
@@ -1444,10 +1445,15 @@ __device__ __forceinline__ DF eval_num4d_dfx(const EGrid &E, const DF *slab, int
   // the nodes' column scales relative to the largest of the four (<= 1)
   const int x0 = E.xe[b3], x1 = E.xe[b3 + 1], x2 = E.xe[b3 + 2], x3 = E.xe[b3 + 3];
   xr = max(max(x0, x1), max(x2, x3));
-  const DF w3[4] = {df_scale(df_mul(df_mul(u1, u23), S[0]), x0 - xr),
-                    df_scale(df_mul(df_mul(u0, u23), S[1]), x1 - xr),
-                    df_scale(df_mul(df_mul(u01, u3), S[2]), x2 - xr),
-                    df_scale(df_mul(df_mul(u01, u2), S[3]), x3 - xr)};
+  w3[0] = df_scale(df_mul(df_mul(u1, u23), S[0]), x0 - xr);
+  w3[1] = df_scale(df_mul(df_mul(u0, u23), S[1]), x1 - xr);
+  w3[2] = df_scale(df_mul(df_mul(u01, u3), S[2]), x2 - xr);
+  w3[3] = df_scale(df_mul(df_mul(u01, u2), S[3]), x3 - xr);
+}
+__device__ __forceinline__ DF eval_num4d_dfx(const EGrid &E, const DF *slab, int b2, const DF *w2,
+                                             int b3, DF u0, int &xr) {
+  DF w3[4];
+  energy_weights(E, b3, u0, w3, xr);
   float sh = 0.0f, sl = 0.0f;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
@@ -1459,6 +1465,52 @@ __device__ __forceinline__ DF eval_num4d_dfx(const EGrid &E, const DF *slab, int
   }
   return df_norm(sh, sl);
 }
+
+// The same along one profile column, whose mu stencil every energy shares: the
+// four energy nodes of the stencil with the mu contraction done, kept from one
+// energy to the next (the nodes move by one or none between neighbouring
+// energies of a fine grid), so that an energy costs four products and four
+// per new node instead of twenty.
+struct NodeWindow {
+  DF T[4];
+  int at = -1;  // the base node T holds
+  __device__ __forceinline__ static DF node(const EGrid &E, const DF *slab, const DF *w2, int n) {
+    float h = 0.0f, l = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) df_acc_mul(w2[k], slab[(size_t)k * E.nE + n], h, l);
+    return df_norm(h, l);
+  }
+  // slab: at the mu stencil's base row
+  __device__ __forceinline__ DF eval(const EGrid &E, const DF *slab, const DF *w2, int b3, DF u0,
+                                     int &xr) {
+    if (at < 0 || b3 > at + 4 || b3 < at - 4) {
+      at = b3;
+#pragma unroll 1
+      for (int i = 0; i < 4; i++) {
+        T[0] = T[1]; T[1] = T[2]; T[2] = T[3];
+        T[3] = node(E, slab, w2, b3 + i);
+      }
+    }
+#pragma unroll 1
+    while (at < b3) {
+      at++;
+      T[0] = T[1]; T[1] = T[2]; T[2] = T[3];
+      T[3] = node(E, slab, w2, at + 3);
+    }
+#pragma unroll 1
+    while (at > b3) {
+      at--;
+      T[3] = T[2]; T[2] = T[1]; T[1] = T[0];
+      T[0] = node(E, slab, w2, at);
+    }
+    DF w3[4];
+    energy_weights(E, b3, u0, w3, xr);
+    float h = 0.0f, l = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) df_acc_mul(w3[i], T[i], h, l);
+    return df_norm(h, l);
+  }
+};
 
 // ---------------------------------------------------------------------------
 // main integrator kernel
@@ -1980,14 +2032,16 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
           }
           __syncthreads();
           // specific intensities of every profile column (:445-478): a thread
-          // takes one column and every parts-th energy of the chunk, so the
+          // takes one column and its part of the chunk's energies, so the
           // energy stencil moves by a node or two from one to the next
+          const int per = (ne + parts - 1) / parts, pl0 = part0 * per, pl1 = min(ne, pl0 + per);
           for (int col = col0; col < N_L; col += kThreads) {
             const int f = sm.flag[col];
             int lo = -1;
             MuStencil ms{};
+            NodeWindow nodes;
             if (tab2 && (f & kColLit)) ms = mu_stencil(a.atmos, as, sm.abb[col], false);
-            for (int pl = part0; pl < ne; pl += parts) {
+            for (int pl = pl0; pl < pl1; pl++) {
               const int p = e0 + pl;
               if (!(f & kColLit)) {
                 if constexpr (kMixed) co4[col * (EC + 1) + pl].y = 0.0f;
@@ -2044,7 +2098,8 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
                     for (int q = 0; q < 4; q++) w2[q] = df_split(mc.w2[q]);
                     I = eval_num4d_dfx(eg4, slabd, mc.b2, w2, b3, u, xr);
                   } else {
-                    I = eval_num4d_dfx(eg4, slabd, sm.mb[col], sm.mw + 4 * col, b3, u, xr);
+                    I = nodes.eval(eg4, slabd + (size_t)sm.mb[col] * nEt, sm.mw + 4 * col, b3, u,
+                                   xr);
                   }
                   if (I.h < 0.0f) I = DF{0.0f, 0.0f};
                   if (dfy) {
@@ -2078,7 +2133,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
               // the beaming modification (hot_wrapper.pyx:153-199) of the
               // column's intensities
               int lb = -1;
-              for (int pl = part0; pl < ne; pl += parts) {
+              for (int pl = pl0; pl < pl1; pl++) {
                 const int p = e0 + pl;
                 const double I_raw = pr.yd(col, pl);
                 double I_E;
