@@ -66,7 +66,10 @@ struct InPair {
 // weights and error estimate per integrand)
 // (not inlined: one copy per integrand pair, so that the kernel's code stays in
 // the instruction cache)
-template <typename P>
+// kOne: the two nodes of a pair in turn by one copy of the integrand's code,
+// where the 31-point rule's code shares the instruction cache; alone, the two
+// nodes side by side are faster (64 vectors' rows: 7.7 ms)
+template <bool kOne, typename P>
 __device__ __noinline__ void gk61_pair_panel(const P &pf, double a, double b, double res[2],
                                                 double err[2], double rabs[2], double rasc[2]) {
   constexpr int NH = XG_K61_HALF - 1;
@@ -89,8 +92,17 @@ __device__ __noinline__ void gk61_pair_panel(const P &pf, double a, double b, do
   for (int j = 0; j < NH; j++) {
     const DF dx = df_mul(h, DF{XG_K61_X2[2 * j], XG_K61_X2[2 * j + 1]});
     DF f1[2], f2[2];
-    pf(df_sub(c, dx), f1[0], f1[1]);
-    pf(df_add(c, dx), f2[0], f2[1]);
+    if constexpr (kOne) {
+#pragma unroll 1
+      for (int z = 0; z < 2; z++) {
+        f1[0] = f2[0];
+        f1[1] = f2[1];
+        pf(z ? df_add(c, dx) : df_sub(c, dx), f2[0], f2[1]);
+      }
+    } else {
+      pf(df_sub(c, dx), f1[0], f1[1]);
+      pf(df_add(c, dx), f2[0], f2[1]);
+    }
     const DF wk{XG_K61_WK2[2 * j], XG_K61_WK2[2 * j + 1]};
     const DF wg{XG_K61_WG2[2 * j], XG_K61_WG2[2 * j + 1]};
 #pragma unroll
@@ -161,8 +173,12 @@ __device__ __noinline__ bool gk31_pair(const P &pf, double a, double b, double r
   for (int j = 0; j < NH; j++) {
     const DF dx = df_mul(h, DF{XG_K31_X2[2 * j], XG_K31_X2[2 * j + 1]});
     DF f1[2], f2[2];
-    pf(df_sub(c, dx), f1[0], f1[1]);
-    pf(df_add(c, dx), f2[0], f2[1]);
+#pragma unroll 1
+    for (int z = 0; z < 2; z++) {  // (one copy of the integrand's code)
+      f1[0] = f2[0];
+      f1[1] = f2[1];
+      pf(z ? df_add(c, dx) : df_sub(c, dx), f2[0], f2[1]);
+    }
     const DF wk{XG_K31_WK2[2 * j], XG_K31_WK2[2 * j + 1]};
     const DF wg{XG_K31_WG2[2 * j], XG_K31_WG2[2 * j + 1]};
 #pragma unroll
@@ -207,7 +223,7 @@ __device__ __noinline__ int q61_pair(const P &pf, double a, double b, double &r1
   const double epsrel = 1.0e-12;
   double al[LIMIT], bl[LIMIT], rl[2][LIMIT], el[2][LIMIT];
   double r0[2], e0[2], ra0[2], rc0[2];
-  gk61_pair_panel(pf, a, b, r0, e0, ra0, rc0);
+  gk61_pair_panel<k31>(pf, a, b, r0, e0, ra0, rc0);
   bool done[2];
   int st0[2];
 #pragma unroll
@@ -237,8 +253,8 @@ __device__ __noinline__ int q61_pair(const P &pf, double a, double b, double &r1
     const double ai = al[k], bi = bl[k];
     const double a1 = ai, b1 = 0.5 * (ai + bi), a2 = b1, b2 = bi;
     double R1[2], E1[2], RA1[2], RC1[2], R2[2], E2[2], RA2[2], RC2[2];
-    gk61_pair_panel(pf, a1, b1, R1, E1, RA1, RC1);
-    gk61_pair_panel(pf, a2, b2, R2, E2, RA2, RC2);
+    gk61_pair_panel<k31>(pf, a1, b1, R1, E1, RA1, RC1);
+    gk61_pair_panel<k31>(pf, a2, b2, R2, E2, RA2, RC2);
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const double ri = rl[q][k], ei = el[q][k];
@@ -464,10 +480,13 @@ __global__ void __launch_bounds__(128) rays_finish_kernel(RaysArgs a) {
 // A row's rays are shared by `parts` CTAs, a ray to a thread, and
 // rays_finish_kernel follows.  (A CTA with a whole row in turn ran 8 % slower:
 // its warps waited for the rays near the limb.)  Bound: FP32 issue through
-// long dependent double-float chains, 45-60 % of the issue slots, and the
-// instruction cache.  24 vectors (5628 rows of 1024 rays): 7.9 ms with 61
-// points everywhere and every panel inlined, 4.3 ms now (61 points alone: 64
-// vectors' 10810 rows 13.7 -> 7.7 ms); 64 rows: 252 us in turn on 64 SMs, 67 us.
+// long dependent double-float chains, 54 % of the issue slots, and the
+// instruction cache: one copy of an integrand for both sides of a node pair
+// took 256 prior vectors from 25.4 to 21.0 ms, and five or six CTAs per SM
+// instead of four only wait for instructions (21.3, 21.5 ms).  24 vectors
+// (5628 rows of 1024 rays): 7.9 ms with 61 points everywhere and every panel
+// inlined, 3.8 ms now (61 points alone: 64 vectors' 10810 rows 13.7 -> 7.7 ms);
+// 64 rows: 252 us in turn on 64 SMs, 60 us.
 template <bool k31>
 __global__ void __launch_bounds__(128) rays_kernel(RaysArgs a, int parts) {
   const int row = blockIdx.x / parts;
