@@ -50,15 +50,16 @@ __device__ __forceinline__ DF df_log_t(DF m, const DF *tab) {
   return df_add(df_fma(DF{(float)e, 0.0f}, ln2, tab[i]), df_mul(df_add(s, s), p));
 }
 
+__device__ __noinline__ double exp_large(double x) { return exp(x); }
 // exp(x) of a double-float x, returned as a double: x = k ln 2 + r with
 // |r| <= ln 2 / 2 (ln 2 in parts, gen_log_table.py: k times the first two
 // exact for |k| < 2^11), exp(r) by its Taylor series through r^13 / 13! in
-// double-float (truncation below 4e-18 relative), then 2^k in FP64; 0 below
+// double-float (truncation below 4e-18 relative), joined with 2^k by bits; 0 below
 // the double range, the FP64 exp beyond ln 2^1000.
 __device__ __forceinline__ double df_exp_d(DF x) {
   if (x.h != x.h) return (double)x.h;
   if (x.h < -760.0f) return 0.0;
-  if (x.h > 690.0f) return exp((double)x.h + (double)x.l);
+  if (x.h > 690.0f) return exp_large((double)x.h + (double)x.l);
   const float kf = rintf(x.h * 1.44269504088896341f);
   const int k = (int)kf;
   DF r = df_add(x, DF{-kf * XG_LN2_1, 0.0f});
@@ -67,11 +68,7 @@ __device__ __forceinline__ double df_exp_d(DF x) {
   DF p{XG_EXPT[XG_EXPT_N - 1][0], XG_EXPT[XG_EXPT_N - 1][1]};
 #pragma unroll
   for (int n = XG_EXPT_N - 2; n >= 0; n--) p = df_fma(p, r, DF{XG_EXPT[n][0], XG_EXPT[n][1]});
-  // 2^k from the bit pattern, split in two factors to stay normal
-  const int k1 = k / 2, k2 = k - k1;
-  const double f1 = __hiloint2double((k1 + 1023) << 20, 0);
-  const double f2 = __hiloint2double((k2 + 1023) << 20, 0);
-  return df_value(p) * f1 * f2;
+  return df_join_bits(p, k);
 }
 
 constexpr int kWarps = 4;
@@ -101,7 +98,7 @@ struct Marg {
 };
 
 // :84-138, as the reference writes it
-__device__ __forceinline__ double marginal_integrand_direct(const Marg &m, double B) {
+__device__ __noinline__ double marginal_integrand_direct(const Marg &m, double B) {
   double x = 0.0;
   for (int j = 0; j < m.n; j++) {
     double c = m.SCALE * (m.star[j] + B);
@@ -122,14 +119,19 @@ __device__ __forceinline__ double marginal_integrand_direct(const Marg &m, doubl
 // some ratio is not positive (c_j(B) <= 0) takes the direct form, which
 // holds the reference's tests for that case.
 __device__ __forceinline__ double marginal_integrand(const Marg &m, double B) {
-  if (!m.rel) return marginal_integrand_direct(m, B);
-  const double dBd = B - m.Bi;
-  const DF dB = df_split(dBd);
+  if (!m.rel) {
+    const Marg mc = m;
+    return marginal_integrand_direct(mc, B);
+  }
+  const DF dB = df_split_bits(B - m.Bi, 0);
   const DF one{1.0f, 0.0f};
   DF acc{0.0f, 0.0f};
   for (int j = 0; j < m.n; j++) {
     const DF r = df_fma(dB, m.q[j], one);
-    if (!(r.h > 0.0f)) return marginal_integrand_direct(m, B);
+    if (!(r.h > 0.0f)) {
+      const Marg mc = m;
+      return marginal_integrand_direct(mc, B);
+    }
     if (m.dataf[j] != 0.0f) acc = df_fma(DF{m.dataf[j], 0.0f}, df_log_t(r, m.logt), acc);
   }
   return df_exp_d(df_sub(acc, df_mul(m.nS, dB)));
@@ -141,6 +143,30 @@ __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+// warp_sum of two and of four values, each half (quarter) of the warp carrying
+// one of them once the others' share is handed over: five and six additions
+// in place of ten and twenty, the same bits (the FP64 pipe takes 64 cycles
+// for one, a shuffle two)
+__device__ __forceinline__ double hand_over(double low, double high, int lane, int o) {
+  const bool up = lane & o;
+  return (up ? high : low) + __shfl_xor_sync(0xffffffffu, up ? low : high, o);
+}
+__device__ __forceinline__ void warp_sum2(double &a, double &b, int lane) {
+  double v = hand_over(a, b, lane, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  a = __shfl_sync(0xffffffffu, v, 0);
+  b = __shfl_sync(0xffffffffu, v, 16);
+}
+__device__ __forceinline__ void warp_sum4(double (&a)[4], int lane) {
+  const double u = hand_over(a[0], a[1], lane, 16), w = hand_over(a[2], a[3], lane, 16);
+  double v = hand_over(u, w, lane, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    a[i] = __shfl_sync(0xffffffffu, v, (i & 1 ? 16 : 0) + (i & 2 ? 8 : 0));
 }
 
 // The Akima-periodic pieces of one component's pulse through (x[i], y[i]),
@@ -196,35 +222,35 @@ __device__ __forceinline__ int akima_pieces_warp_df(const double *x, const doubl
 }
 // akima_periodic_integral over [lo, hi] from the pieces of
 // akima_pieces_warp_df (yd in yd[]), in units of 2^e
-__device__ __forceinline__ DF akima_integral_df(const double *x, const DF *yd, int n,
-                                                const DF *k1, const DF *k2, const DF *k3,
+// (hd: the intervals' lengths; only the two ends' offsets are formed in FP64,
+// and the lower end's value in the first interval alone, which the lanes take
+// together)
+__device__ __forceinline__ DF akima_integral_df(const double *x, const DF *hd, const DF *yd,
+                                                int n, const DF *k1, const DF *k2, const DF *k3,
                                                 double lo, double hi) {
   const DF third{0.3333333432674408f, -9.934107758624577e-09f};
   const int ia = locate_bits(x, n, lo), ib = locate_bits(x, n, hi);
+  const DF u = df_split_bits(lo - x[ia], 0), w = df_split_bits(hi - x[ib], 0);
   DF acc{0.0f, 0.0f};
+#pragma unroll 1
   for (int i = ia; i <= ib; i++) {
-    const double u = (i == ia) ? lo - x[i] : 0.0;
-    const double w = (i == ib) ? hi - x[i] : x[i + 1] - x[i];
-    // F(t) = t (y + t (k1 / 2 + t (k2 / 3 + t k3 / 4))) at w and u
+    // F(t) = t (y + t (k1 / 2 + t (k2 / 3 + t k3 / 4)))
     const DF c1{0.5f * k1[i].h, 0.5f * k1[i].l}, c3{0.25f * k3[i].h, 0.25f * k3[i].l};
-    const DF c2 = df_mul(k2[i], third);
-    DF F[2];
-    const double ts[2] = {w, u};
-#pragma unroll
-    for (int z = 0; z < 2; z++) {
-      const DF t = df_split_bits(ts[z], 0);
-      F[z] = df_mul(t, df_fma(t, df_fma(t, df_fma(t, c3, c2), c1), yd[i]));
-    }
-    acc = df_add(acc, df_sub(F[0], F[1]));
+    const DF c2 = df_mul(k2[i], third), y = yd[i];
+    auto F = [&](DF t) { return df_mul(t, df_fma(t, df_fma(t, df_fma(t, c3, c2), c1), y)); };
+    DF v = F(i == ib ? w : hd[i]);
+    if (i == ia) v = df_sub(v, F(u));
+    acc = df_add(acc, v);
   }
   return acc;
 }
 
-// :140-173 (returns the step; writes the Gaussian width); lane-parallel over
-// the phase bins.  pow(s, 2.0) of the reference is s * s, as its C compiler
-// emits it.
-__device__ __forceinline__ double newton_delta(const Marg &m, double B, int lane, double &std) {
-  double x = 0.0, y = 0.0;
+// :140-173: y and x of the Newton step -y / x at B, whose Gaussian width is
+// sqrt(2 / x); lane-parallel over the phase bins.  pow(s, 2.0) of the
+// reference is s * s, as its C compiler emits it.
+__device__ __forceinline__ void newton_sums(const Marg &m, double B, int lane, double &y,
+                                            double &x) {
+  x = y = 0.0;
   for (int j = lane; j < m.n; j += 32) {
     // d / s and d / s^2 from one reciprocal (an ulp from the two divisions)
     const double is = 1.0 / (m.star[j] + B);
@@ -232,12 +258,15 @@ __device__ __forceinline__ double newton_delta(const Marg &m, double B, int lane
     y += t;
     x += t * is;
   }
-  y = warp_sum(y);
-  x = warp_sum(x);
+  warp_sum2(y, x, lane);
   y = 2.0 * m.T - 2.0 * y;
   x *= 2.0;
-  std = sqrt(2.0 / x);
-  return -1.0 * y / x;
+}
+// |step| > epsilon width (:336), as y^2 > 2 epsilon^2 x where that says the
+// same: no root and no division
+__device__ __forceinline__ bool newton_far(double y, double x, double epsilon) {
+  if (epsilon > 0.0 && x > 0.0 && x < 1.0e300) return y * y > 2.0 * epsilon * epsilon * x;
+  return fabs(y / x) > epsilon * sqrt(2.0 / x);
 }
 
 // The 21-point Gauss-Kronrod panels of the marginal quadrature, evaluated by
@@ -349,7 +378,7 @@ __device__ __forceinline__ int warp_worst(const double *el, int size, int lane) 
 }
 
 // adaptive GK21 (same scheme as the rays' QAG), warp-cooperative; a < b
-__device__ double warp_qag21_core(const Marg &m, WarpSmem &w, int lane, double a, double b,
+__device__ __noinline__ double warp_qag21_core(const Marg &m, WarpSmem &w, int lane, double a, double b,
                                   double epsabs, double er) {
   const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
   Panel P0, Pu;
@@ -428,75 +457,76 @@ __device__ double warp_dyadic(const Marg &m, WarpSmem &w, int lane, double lo, d
   return sum;
 }
 
-// A 61-point Gauss-Kronrod panel over [a, b] by the warp, two nodes to a lane
-// (61 of its 64 slots).  The integrand is an exponential, so its own sum is
-// the rule's |f| sum; the error estimate is QUADPACK's.
-__device__ __forceinline__ void warp_panel61(const Marg &m, int lane, double a, double b,
-                                             double &res, double &err) {
-  const int NH = XG_K61_HALF - 1;  // 30
-  const double c = 0.5 * (a + b), h = 0.5 * (b - a);
-  double f[2] = {0.0, 0.0}, wk[2] = {0.0, 0.0}, wg[2] = {0.0, 0.0};
-#pragma unroll 1
-  for (int z = 0; z < 2; z++) {
-    const int n = lane + 32 * z;
-    if (n > 2 * NH) break;
-    const int s = n <= NH ? n : n - NH - 1;
-    const double x = n < NH ? -XG_K61_X[s] : (n == NH ? 0.0 : XG_K61_X[s]);
-    f[z] = marginal_integrand(m, fma(h, x, c));
-    wk[z] = XG_K61_WK[s];
-    wg[z] = XG_K61_WG[s];
-  }
-  const double rk = warp_sum(fma(wk[1], f[1], wk[0] * f[0]));
-  const double rg = warp_sum(fma(wg[1], f[1], wg[0] * f[0]));
-  const double mean = 0.5 * rk;
-  const double rc = warp_sum(fma(wk[1], fabs(f[1] - mean), wk[0] * fabs(f[0] - mean))) * h;
-  res = rk * h;
-  double e = fabs((rk - rg) * h);
-  if (rc != 0.0 && e != 0.0) {
-    const double x = 200.0 * e / rc, sc = x * sqrt(x);
-    e = sc < 1.0 ? rc * sc : rc;
-  }
-  err = fmax(e, 50.0 * 2.220446049250313e-16 * res);
-}
-
-// The marginal integral over [a, b] from one such panel on each side of the
-// integrand's peak (one in all where the peak lies on an end): a window of
-// ten standard deviations either way is smooth enough that they meet the
-// adaptive rule's tolerance, at two node evaluations per lane and panel
-// against two for each of the eight or so bisections, whose sums and error
-// estimates (FP64, one per warp) were the kernel's larger half.  Returns false
-// where they do not.
+// The marginal integral over [a, b] from one 61-point Gauss-Kronrod panel on
+// each side of the integrand's peak (one in all where the peak lies on an
+// end), two nodes to a lane (61 of its 64 slots): a window of ten standard
+// deviations either way is smooth enough that they meet the adaptive rule's
+// tolerance, at two node evaluations per lane and panel against two for each
+// of the eight or so bisections, whose sums and error estimates (FP64, one per
+// warp) were the kernel's larger half.  The integrand is an exponential, so
+// its own sum is the rule's |f| sum; the error estimate is QUADPACK's, its
+// ratio in float.  Returns false where they do not meet it.  One copy of the
+// integrand's code serves the four nodes.
 __device__ __forceinline__ bool warp_peak61(const Marg &m, int lane, double a, double b,
                                             double er, double &out) {
+  const int NH = XG_K61_HALF - 1;  // 30
   const bool inside = a < m.Bi && m.Bi < b;
-  double r, e;
-  warp_panel61(m, lane, a, inside ? m.Bi : b, r, e);
-  if (inside) {
-    double r2, e2;
-    warp_panel61(m, lane, m.Bi, b, r2, e2);
-    r += r2;
-    e += e2;
+  const double mid = inside ? m.Bi : b;
+  double c[2], h[2];
+  c[0] = 0.5 * (a + mid), h[0] = 0.5 * (mid - a);
+  c[1] = 0.5 * (mid + b), h[1] = 0.5 * (b - mid);
+  // the four values, shifted through registers: panel 0 in f3, f2
+  double f3 = 0.0, f2 = 0.0, f1 = 0.0, f0 = 0.0;
+#pragma unroll 1
+  for (int z = 0; z < 4; z++) {
+    const int n = lane + 32 * (z & 1);
+    double v = 0.0;
+    if (n <= 2 * NH && (z < 2 || inside)) {
+      const int s = n <= NH ? n : n - NH - 1;
+      const double x = n < NH ? -XG_K61_X[s] : (n == NH ? 0.0 : XG_K61_X[s]);
+      v = marginal_integrand(m, fma(z < 2 ? h[0] : h[1], x, z < 2 ? c[0] : c[1]));
+    }
+    f3 = f2; f2 = f1; f1 = f0; f0 = v;
+  }
+  const int n1 = lane + 32;
+  const int s0 = lane <= NH ? lane : lane - NH - 1;
+  const bool two = n1 <= 2 * NH;
+  const double k0 = XG_K61_WK[s0], g0 = XG_K61_WG[s0];
+  const double k1 = two ? XG_K61_WK[n1 - NH - 1] : 0.0, g1 = two ? XG_K61_WG[n1 - NH - 1] : 0.0;
+  double sum[4] = {fma(k1, f2, k0 * f3), fma(g1, f2, g0 * f3), fma(k1, f0, k0 * f1),
+                   fma(g1, f0, g0 * f1)};
+  warp_sum4(sum, lane);
+  const double ma = 0.5 * sum[0], mb = 0.5 * sum[2];
+  double rc[2] = {fma(k1, fabs(f2 - ma), k0 * fabs(f3 - ma)),
+                  fma(k1, fabs(f0 - mb), k0 * fabs(f1 - mb))};
+  warp_sum2(rc[0], rc[1], lane);
+  double r = 0.0, e = 0.0;
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    if (p == 1 && !inside) break;
+    const double res = sum[2 * p] * h[p];
+    // err = rasc min(1, (200 |K - G| / rasc)^1.5): the half-width cancels from
+    // the ratio
+    const float dk = fabsf((float)(sum[2 * p] - sum[2 * p + 1])), rcf = (float)rc[p];
+    float q = dk;
+    if (rcf != 0.0f && dk != 0.0f) {
+      const float x = 200.0f * dk / rcf, sc = x * sqrtf(x);
+      q = sc < 1.0f ? rcf * sc : rcf;
+    }
+    r += res;
+    e += fmax((double)q * h[p], 50.0 * 2.220446049250313e-16 * res);
   }
   out = r;
   return r > 0.0 && e <= er * r;
 }
 
-// the marginal integral over [a, b]: adaptive GK21 at relative
-// min(epsrel, 1e-13); when every interior node sees zero but an endpoint
+// adaptive GK21 over [a, b]; when every interior node sees zero but an endpoint
 // does not (a channel without counts has a window ~1e91 wide whose integrand
 // decays on the scale 1 / exposure), the window is cut into dyadic pieces
 // toward that endpoint, as a Clenshaw-Curtis rule with endpoint nodes would
 // resolve it.
-__device__ double warp_marginal(const Marg &m, WarpSmem &w, int lane, double a, double b,
-                                double epsabs, double epsrel) {
-  const double eps = 2.220446049250313e-16;
-  double sign = 1.0;
-  if (b < a) { double t = a; a = b; b = t; sign = -1.0; }
-  if (a == b) return 0.0;
-  double er = epsrel < 1.0e-13 ? epsrel : 1.0e-13;
-  if (epsabs <= 0.0 && er < 50.0 * eps) er = 50.0 * eps;
-  double peak;
-  if (m.rel && warp_peak61(m, lane, a, b, er, peak)) return sign * peak;
+__device__ __noinline__ double warp_adaptive(const Marg &m, WarpSmem &w, int lane, double a,
+                                            double b, double epsabs, double er) {
   double r = warp_qag21_core(m, w, lane, a, b, epsabs, er);
   if (r == 0.0) {
     double fa = marginal_integrand(m, a);
@@ -510,26 +540,28 @@ __device__ double warp_marginal(const Marg &m, WarpSmem &w, int lane, double a, 
       r = rl + rr;
     }
   }
-  return sign * r;
+  return r;
+}
+// the marginal integral over [a, b] at relative min(epsrel, 1e-13)
+__device__ __forceinline__ double warp_marginal(const Marg &m, WarpSmem &w, int lane, double a, double b,
+                                double epsabs, double epsrel) {
+  const double eps = 2.220446049250313e-16;
+  double sign = 1.0;
+  if (b < a) { double t = a; a = b; b = t; sign = -1.0; }
+  if (a == b) return 0.0;
+  double er = epsrel < 1.0e-13 ? epsrel : 1.0e-13;
+  if (epsabs <= 0.0 && er < 50.0 * eps) er = 50.0 * eps;
+  double peak;
+  if (m.rel && warp_peak61(m, lane, a, b, er, peak)) return sign * peak;
+  const Marg mc = m;  // (what the calls below see stays out of the hot path's registers)
+  return sign * warp_adaptive(mc, w, lane, a, b, epsabs, er);
 }
 
-__global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
-  __shared__ WarpSmem ws[kWarps];
-  __shared__ DF s_logt[XG_LOGT_N];
-  // the phase grid's 1 / h and 1 / h^2 as pairs, shared by the warps' Akima builds
-  __shared__ DF s_ih[kQagLimit], s_ih2[kQagLimit];
-  for (int t = threadIdx.x; t < XG_LOGT_N; t += blockDim.x) s_logt[t] = DF{XG_LOGT[t][0], XG_LOGT[t][1]};
-  for (int t = threadIdx.x; t < a.N_P - 1 && t < kQagLimit; t += blockDim.x) {
-    const double h = a.comp_phases[t + 1] - a.comp_phases[t];
-    s_ih[t] = df_split(1.0 / h);
-    s_ih2[t] = df_split(1.0 / (h * h));
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long gw = (long)blockIdx.x * kWarps + wid;
-  if (gw >= (long)a.n_vec * a.K) return;
-  const int v = (int)(gw / a.K), ch = (int)(gw % a.K);
-  WarpSmem &w = ws[wid];
+// one channel of one evaluation, by a warp
+__device__ __forceinline__ void like_channel(const LikeArgs &a, WarpSmem &w, const DF *s_logt,
+                                             const DF *s_h, const DF *s_ih, const DF *s_ih2,
+                                             int lane, int v, int ch) {
+  __syncwarp();  // the last channel's readers of w are done
   const int B = a.B, N_P = a.N_P;
   const double n = (double)B;
   const double SCALE = a.exposure / n;
@@ -545,6 +577,7 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
     DF *yd = reinterpret_cast<DF *>(w.el), *k1 = reinterpret_cast<DF *>(w.al);
     DF *k2 = reinterpret_cast<DF *>(w.bl), *k3 = reinterpret_cast<DF *>(w.rl);
     const double *xs = a.comp_phases;
+    const long long x_lo = ordered(xs[0]), x_hi = ordered(xs[N_P - 1]);
     for (int h = 0; h < a.H; h++) {
       const double *pulse = a.signals + (((size_t)v * a.H + h) * a.K + ch) * N_P;
       const double sh = a.shifts[(size_t)v * a.H + h];
@@ -556,19 +589,17 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
         if (are_equal(pb - pa, 1.0)) { pa = 0.0; pb = 1.0; }
         else { pa -= floor(pa); pb -= floor(pb); }
         // the reference's argument checks (akima_periodic_integral)
+        // (comparisons by bits; a NaN gives a NaN as before)
         auto piece = [&](double lo, double hi) -> double {
-          if (lo > hi || lo < xs[0] || hi > xs[N_P - 1]) return nan("");
-          if (lo == hi) return 0.0;
-          return df_join_bits(akima_integral_df(xs, yd, N_P, k1, k2, k3, lo, hi), ex);
+          const long long lb = ordered(lo), hb = ordered(hi);
+          if (lb > hb || lb < x_lo || hb > x_hi) return nan("");
+          if (lb == hb) return 0.0;
+          return df_join_bits(akima_integral_df(xs, s_h, yd, N_P, k1, k2, k3, lo, hi), ex);
         };
-        double val;
-        if (pa < pb) {
-          val = piece(pa, pb);
-          if (val > 0.0 || neg) st += val;
-        } else {
-          val = piece(pa, 1.0);
-          if (val > 0.0 || neg) st += val;
-          val = piece(0.0, pb);
+        const bool whole = ordered(pa) < ordered(pb);  // else the bin wraps: two parts
+#pragma unroll 1
+        for (int part = 0; part < (whole ? 1 : 2); part++) {
+          const double val = piece(part ? 0.0 : pa, whole || part ? pb : 1.0);
           if (val > 0.0 || neg) st += val;
         }
         w.star[j] = st;
@@ -612,8 +643,8 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
     av_STAR += w.star[j];
     av_DATA += w.data[j];
   }
-  av_STAR = warp_sum(av_STAR);
-  av_DATA = warp_sum(av_DATA);
+  warp_sum2(av_STAR, av_DATA, lane);
+  const double dsum = av_DATA;
   const size_t o = (size_t)v * a.K + ch;
   int flag = 0;
   double term = 0.0, Bout = 0.0;
@@ -639,35 +670,41 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
       double B_min = 0.0;
       Bv = av_DATA - av_STAR;
       if (Bv <= B_min) {
-        double min_counts = -1.0;
-        for (int j = 0; j < B; j++)
-          if (are_equal(w.star[j], 0.0)) { min_counts = -2.0; break; }
-        if (are_equal(min_counts, -2.0)) {
-          for (int j = 0; j < B; j++)
-            if ((are_equal(min_counts, -2.0) && w.data[j] > 0.0) ||
-                (0.0 < w.data[j] && w.data[j] < min_counts))
-              min_counts = w.data[j];
+        // where some bin's star rate is zero (within 1e-12), the smallest
+        // positive count (by bits, a lane per bin)
+        bool dark = false;
+        long long least = LLONG_MAX;
+        for (int j = lane; j < B; j += 32) {
+          const long long sb = __double_as_longlong(w.star[j]) & LLONG_MAX;
+          const long long db = __double_as_longlong(w.data[j]);
+          dark |= sb < __double_as_longlong(1.0e-12);
+          if (db > 0 && db <= __double_as_longlong(INFINITY)) least = min(least, db);
         }
-        if (!are_equal(min_counts, -1.0)) {
-          if (are_equal(min_counts, -2.0)) { Bv = 0.0; B_min = 0.0; }
-          else { Bv = 0.01 * min_counts / SCALE; B_min = 0.1 * Bv; }
-        } else {
-          Bv = B_min;
+        Bv = B_min;
+        if (__any_sync(0xffffffffu, dark)) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+            least = min(least, __shfl_xor_sync(0xffffffffu, least, o));
+          if (least != LLONG_MAX) {
+            Bv = 0.01 * __longlong_as_double(least) / SCALE;
+            B_min = 0.1 * Bv;
+          }
         }
       }
-      double stdv;
-      double dB = newton_delta(m, Bv, lane, stdv);
-      int counter = 0, steps = 0;
+      int counter = 0;
       // the reference's Newton loop (:336-352) has no step limit; 10000 steps
       // bound it here (convergence takes a handful)
-      while (fabs(dB) > a.epsilon * stdv && counter < 2 && steps++ < 10000) {
-        Bv += dB;
+#pragma unroll 1
+      for (int steps = 0;; steps++) {
+        double y, x;
+        newton_sums(m, Bv, lane, y, x);
+        if (counter >= 2 || steps >= 10000 || !newton_far(y, x, a.epsilon)) break;
+        Bv += -1.0 * y / x;
         if (Bv < B_min) {
           if (B_min > 0.0) counter += 1;
           else counter = 2;
           Bv = B_min;
         }
-        dB = newton_delta(m, Bv, lane, stdv);
       }
       double std_est = 0.0;
       for (int j = lane; j < B; j += 32) {
@@ -691,16 +728,14 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
       }
       if (Bi < lower) Bi = lower;
       else if (Bi > upper) Bi = upper;
-      double A = 0.0, dsum = 0.0;
+      double A = 0.0;
       for (int j = lane; j < B; j += 32) {
         double c = SCALE * (w.star[j] + Bi);
         if (c > 0.0) A += w.data[j] * log(c) - c;
         else if (are_equal(c, 0.0) && are_equal(w.data[j], 0.0)) {}
         else A += a.llzero;
-        dsum += w.data[j];
       }
       A = warp_sum(A);
-      dsum = warp_sum(dsum);
       m.A = A;
       // relative form of the integrand when every c_j(Bi) > 0
       bool pos = true;
@@ -749,6 +784,35 @@ __global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
       a.star[o * B + j] = s;
     }
   }
+}
+
+// What bounds it: the FP64 pipe (Newton's reciprocals, the sums over the bins,
+// the normalisation's logarithm: some 300 instructions of 16 cycles per SM),
+// then FP32 issue (the integrand's logarithms) and instruction fetch, so the
+// integrand, the bins' integrals and Newton's sums are one copy of code each
+// and the adaptive rule a call.  Persistent CTAs form the phase grid's
+// reciprocals once.  With some 600 FP64 instructions per channel and inlined
+// copies (FP64 pipe 66 % busy, a third of the stalls for instructions): 1500
+// channels 134 us, 100 vectors of 300 channels 1188 us, 24 vectors of 1500
+// 1779 us; now 110, 910 and 1417 us.
+__global__ void __launch_bounds__(32 * kWarps) like_channel_kernel(LikeArgs a) {
+  __shared__ WarpSmem ws[kWarps];
+  __shared__ DF s_logt[XG_LOGT_N];
+  // the phase grid's h, 1 / h and 1 / h^2 as pairs, shared by the warps' Akima builds
+  __shared__ DF s_h[kQagLimit], s_ih[kQagLimit], s_ih2[kQagLimit];
+  for (int t = threadIdx.x; t < XG_LOGT_N; t += blockDim.x) s_logt[t] = DF{XG_LOGT[t][0], XG_LOGT[t][1]};
+  for (int t = threadIdx.x; t < a.N_P - 1 && t < kQagLimit; t += blockDim.x) {
+    const double h = a.comp_phases[t + 1] - a.comp_phases[t];
+    s_h[t] = df_split_bits(h, 0);
+    s_ih[t] = df_split(1.0 / h);
+    s_ih2[t] = df_split(1.0 / (h * h));
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  WarpSmem &w = ws[wid];
+  const long total = (long)a.n_vec * a.K;
+  for (long gw = (long)blockIdx.x * kWarps + wid; gw < total; gw += (long)gridDim.x * kWarps)
+    like_channel(a, w, s_logt, s_h, s_ih, s_ih2, lane, (int)(gw / a.K), (int)(gw % a.K));
 }
 
 // (s, c) += x with Neumaier's compensation: s + c carries the sum to about
@@ -827,7 +891,8 @@ void launch_likelihood(const LikeArgs &a, cudaStream_t st) {
   long warps = (long)a.n_vec * a.K;
   if (warps <= 0) return;
   unsigned blocks = (unsigned)((warps + kWarps - 1) / kWarps);
-  like_channel_kernel<<<blocks, 32 * kWarps, 0, st>>>(a);
+  // (persistent: four CTAs are resident per SM)
+  like_channel_kernel<<<blocks < 152u * 16u ? blocks : 152u * 16u, 32 * kWarps, 0, st>>>(a);
   like_finalize_kernel<<<a.n_vec, 32 * kFinalWarps, 0, st>>>(a);
 }
 
