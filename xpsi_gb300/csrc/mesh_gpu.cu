@@ -681,7 +681,9 @@ __device__ __forceinline__ void finish_cell(const MeshJob &J, xgpu_mesh_batch_ou
 // left to the boundary kernel.
 // Measured, CTA per cell against this: 100 blackbody spots 6.35, 5.33 ms; 256
 // prior vectors of two regions 80.8, 66.5 ms; 13 such vectors 3.9, 5.0 ms (too
-// few cells to fill the groups: the rule kPackedMin).  Two CTAs per SM keep the
+// few cells to fill the groups: the rule kPackedMin).  With the nodes queued
+// between the integrand's stages (PackQueue) and four sums to a reduction the
+// two large batches take 4.23 and 49.4 ms (5.32 and 60.3 without).  Two CTAs per SM keep the
 // pipe full (82-85 % busy) and leave each group several cells; four leave
 // lone cells in their warps at the end (6.33 ms for the 100 spots).
 // ---------------------------------------------------------------------------
@@ -690,6 +692,21 @@ constexpr int kPackCtasPerSm = 2;
 struct PackLists {
   double al[kPackList], bl[kPackList], rl[kPackList], el[kPackList];
   double v[2][21];
+  CutCell f;
+};
+// The nodes of a warp's step: cosine and sine of the colatitude, and the
+// queues of those that need a boundary's azimuth and of those whose value is
+// wanted (group 42 + panel 21 + node, and the node's place above 8 bits).  An
+// FP64 instruction costs the same for one lane as for 32, and only 43 % and 63
+// % of the nodes get there: queued, they take 3 and 4 turns in place of 6.
+constexpr int kPackNodes = 4 * 42;
+struct PackQueue {
+  double mu[kPackNodes], st[kPackNodes];
+  unsigned short edge[kPackNodes], value[kPackNodes];
+};
+struct PackSmem {
+  PackLists lists[kPackCells];
+  PackQueue queues[kPackThreads / 32];
 };
 constexpr unsigned kPackedMin = 10000;
 struct CellQueue {
@@ -697,25 +714,37 @@ struct CellQueue {
   unsigned *count;        // queued, next of the boundary kernel, left, next of the packed one
   unsigned packed_min;    // queued cells from which the packed kernel takes them
 };
-__device__ __forceinline__ double group_sum(double s) {
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
+// sums of four values over the lanes of a group, to every lane, with four
+// additions (the bits of four butterflies of three): a lane carries one of them
+// once the others' share is handed over
+__device__ __forceinline__ double hand_over(double low, double high, int lane, int o) {
+  const bool up = lane & o;
+  return (up ? high : low) + __shfl_xor_sync(0xffffffffu, up ? low : high, o);
+}
+__device__ __forceinline__ void group_sum4(double &a, double &b, double &c, double &d, int lane) {
+  double v = hand_over(hand_over(a, b, lane, 4), hand_over(c, d, lane, 4), lane, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  const int g0 = lane & 24;
+  a = __shfl_sync(0xffffffffu, v, g0);
+  b = __shfl_sync(0xffffffffu, v, g0 + 4);
+  c = __shfl_sync(0xffffffffu, v, g0 + 2);
+  d = __shfl_sync(0xffffffffu, v, g0 + 6);
 }
 __global__ void __launch_bounds__(kPackThreads, kPackCtasPerSm) mesh_packed_kernel(
     const MeshJob *jobs, int n_mesh, xgpu_mesh_batch_out o, const RowTmp *row_tmp,
     const MeshTrig *trig, const ColTrig *cols, int S_max, CellQueue Q) {
   extern __shared__ double pack_smem[];
-  PackLists *lists = reinterpret_cast<PackLists *>(pack_smem);
+  PackSmem &S = *reinterpret_cast<PackSmem *>(pack_smem);
   const unsigned n = Q.count[0];
   if (n < Q.packed_min) return;
   const double eps = 2.220446049250313e-16, dmin = 2.2250738585072014e-308;
   const int lane = threadIdx.x & 31, l = lane & 7, g0 = lane & 24;
-  PackLists &L = lists[threadIdx.x >> 3];
+  PackLists &L = S.lists[threadIdx.x >> 3];
+  PackLists *LW = S.lists + (threadIdx.x >> 5) * 4;  // the warp's four
+  PackQueue &N = S.queues[threadIdx.x >> 5];
   int64_t c = 0;
   int m = 0;
   size_t i = 0, j = 0;
-  CutCell f;
   bool have = false, more = true, first = false;
   double ai = 0.0, bi = 0.0, area = 0.0, errsum = 0.0;
   int size = 0, iter = 0, k = 0, rnd1 = 0, rnd2 = 0;
@@ -727,59 +756,108 @@ __global__ void __launch_bounds__(kPackThreads, kPackCtasPerSm) mesh_packed_kern
       more = q < n;
       if (more) {
         c = Q.cells[q];
+        CutCell f;
         cut_cell(jobs, n_mesh, row_tmp, trig, cols, S_max, c, m, i, j, ai, bi, f);
+        if (l == 0) L.f = f;
         have = first = true;
       }
     }
     __syncwarp();
     if (!__any_sync(0xffffffffu, have)) return;
-    // the step's nodes
+    // the step's nodes: their places
     const double mid = first ? bi : 0.5 * (ai + bi);
+    int n_edge = 0, n_value = 0;
+    const unsigned below_me = (1u << lane) - 1u;
+    auto push = [&](unsigned short *queue, int &count, bool on, int item) {
+      const unsigned mask = __ballot_sync(0xffffffffu, on);
+      if (on) queue[count + __popc(mask & below_me)] = (unsigned short)item;
+      count += __popc(mask);
+    };
 #pragma unroll 1
     for (int p = 0; p < 6; p++) {
       const int z = p >= 3, nd = l + 8 * (p - 3 * z);
       const double a = z ? mid : ai, b = z ? bi : mid;
       const double ctr = 0.5 * (a + b), h = 0.5 * (b - a);
+      const int id = (g0 >> 3) * 42 + z * 21 + nd;
+      int where = -1;
       if (have && nd < 21 && !(first && z)) {
         const double x = nd == 10 ? 0.0 : XG_K21_X[k21_slot(nd)];
-        L.v[z][nd] = f(fma(h, nd < 10 ? -x : x, ctr));
+        const double theta = fma(h, nd < 10 ? -x : x, ctr);
+        double mu, st, keep = 0.0;
+        where = L.f.place(theta, mu, st);
+        if (where >= 0) {
+          N.mu[id] = mu;
+          N.st[id] = st;
+          keep = where & CutCell::kEdge ? theta : L.f.f.pb - L.f.f.pa;
+        }
+        L.v[z][nd] = keep;  // the colatitude, the width, then the value
       }
+      push(N.edge, n_edge, where >= 0 && (where & CutCell::kEdge), id | where << 8);
+      push(N.value, n_value, where >= 0 && !(where & CutCell::kEdge), id);
+    }
+    // the widths of those at a boundary
+#pragma unroll 1
+    for (int t = lane; t - lane < n_edge; t += 32) {
+      __syncwarp();
+      int id = 0;
+      bool some = false;
+      if (t < n_edge) {
+        const int item = N.edge[t];
+        id = item & 255;
+        PackLists &G = LW[id / 42];
+        double &v = G.v[0][id % 42];
+        const double w = G.f.width(v, item >> 8, N.mu[id], N.st[id]);
+        some = ordered_bits(w) != 0;
+        v = some ? w : 0.0;
+      }
+      push(N.value, n_value, some, id);
+    }
+    // the values
+    __syncwarp();
+#pragma unroll 1
+    for (int t = lane; t < n_value; t += 32) {
+      const int id = N.value[t];
+      PackLists &G = LW[id / 42];
+      double &v = G.v[0][id % 42];
+      v = G.f.value(v, N.mu[id], N.st[id]);
     }
     __syncwarp();
     // the four sums of either panel; even lanes keep the first's
-    double ps[4];
+    double ps[4], v1[2][2], v2[2][2], k1[2][2], k2[2][2], sk[2], sg[2], sm[2], sa[2];
 #pragma unroll
     for (int z = 0; z < 2; z++) {
-      double v1[2], v2[2], k1[2], k2[2], sk, sg;
 #pragma unroll
       for (int t = 0; t < 2; t++) {
         const int lo = l + 8 * t;
         const int m1 = z ? (lo < 5 ? lo + 11 : lo - 5) : lo;
         const bool two = z ? (lo >= 5 && lo < 10) : lo < 5;
         const int m2 = z ? lo + 11 : lo + 16;
-        v1[t] = L.v[z][m1];
-        v2[t] = two ? L.v[z][m2] : v1[t];
-        k1[t] = XG_K21_WK[k21_slot(m1)];
-        k2[t] = two ? XG_K21_WK[k21_slot(m2)] : 0.0;
+        v1[z][t] = L.v[z][m1];
+        v2[z][t] = two ? L.v[z][m2] : v1[z][t];
+        k1[z][t] = XG_K21_WK[k21_slot(m1)];
+        k2[z][t] = two ? XG_K21_WK[k21_slot(m2)] : 0.0;
         const double g1 = XG_K21_WG[k21_slot(m1)], g2 = two ? XG_K21_WG[k21_slot(m2)] : 0.0;
-        const double a = fma(k2[t], v2[t], k1[t] * v1[t]), b = fma(g2, v2[t], g1 * v1[t]);
-        sk = t ? sk + a : a;
-        sg = t ? sg + b : b;
-      }
-      sk = group_sum(sk);
-      sg = group_sum(sg);
-      const double mean = 0.5 * sk;
-      double sm = fma(k2[0], fabs(v2[0] - mean), k1[0] * fabs(v1[0] - mean));
-      sm += fma(k2[1], fabs(v2[1] - mean), k1[1] * fabs(v1[1] - mean));
-      double sa = fma(k2[0], fabs(v2[0]), k1[0] * fabs(v1[0]));
-      sa += fma(k2[1], fabs(v2[1]), k1[1] * fabs(v1[1]));
-      sm = group_sum(sm);
-      sa = group_sum(sa);
-      if (z == 0 || (lane & 1)) {
-        ps[0] = sk; ps[1] = sg; ps[2] = sm; ps[3] = sa;
+        const double a = fma(k2[z][t], v2[z][t], k1[z][t] * v1[z][t]);
+        const double b = fma(g2, v2[z][t], g1 * v1[z][t]);
+        sk[z] = t ? sk[z] + a : a;
+        sg[z] = t ? sg[z] + b : b;
       }
     }
+    group_sum4(sk[0], sg[0], sk[1], sg[1], lane);
+#pragma unroll
+    for (int z = 0; z < 2; z++) {
+      const double mean = 0.5 * sk[z];
+      sm[z] = fma(k2[z][0], fabs(v2[z][0] - mean), k1[z][0] * fabs(v1[z][0] - mean));
+      sm[z] += fma(k2[z][1], fabs(v2[z][1] - mean), k1[z][1] * fabs(v1[z][1] - mean));
+      sa[z] = fma(k2[z][0], fabs(v2[z][0]), k1[z][0] * fabs(v1[z][0]));
+      sa[z] += fma(k2[z][1], fabs(v2[z][1]), k1[z][1] * fabs(v1[z][1]));
+    }
+    group_sum4(sm[0], sa[0], sm[1], sa[1], lane);
     const bool odd = lane & 1;
+    ps[0] = odd ? sk[1] : sk[0];
+    ps[1] = odd ? sg[1] : sg[0];
+    ps[2] = odd ? sm[1] : sm[0];
+    ps[3] = odd ? sa[1] : sa[0];
     const WPanel P = k21_finish(ps, odd ? mid : ai, odd ? bi : mid);
     const double r1 = __shfl_sync(0xffffffffu, P.res, g0);
     const double r2 = __shfl_sync(0xffffffffu, P.res, g0 + 1);
@@ -1058,7 +1136,7 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
   mesh_cells_kernel<<<(unsigned)((n_cells + 127) / 128), 128, 0, st>>>(
       d_jobs, n, n_cells, *out, row_tmp, mesh_tmp, trig, cols, S_m, queue, n_queue);
   if (pack) {
-    const size_t lists = sizeof(PackLists) * kPackCells;
+    const size_t lists = sizeof(PackSmem);
     cudaFuncSetAttribute(mesh_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)lists);
     mesh_packed_kernel<<<152 * kPackCtasPerSm, kPackThreads, lists, st>>>(

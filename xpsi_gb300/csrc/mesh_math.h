@@ -503,8 +503,22 @@ struct CutCell {
     return 0;
   }
   XG_HD double operator()(double theta) const {
-    if (!off_pole && are_equal(theta, 0.0)) return 0.0;
     double mu, st;
+    const int where = place(theta, mu, st);
+    if (where < 0) return 0.0;
+    double dphi = f.pb - f.pa;
+    if (where & kEdge) {
+      dphi = width(theta, where, mu, st);
+      if (ordered_bits(dphi) == 0) return 0.0;
+    }
+    return value(dphi, mu, st);
+  }
+  // The integrand in three stages, which the packed kernel takes apart: the
+  // node's place (negative: the cell has none of this ring), the azimuthal
+  // width where a boundary's azimuth is needed (kEdge), and the value.
+  enum { kCede1 = 1, kSup2 = 2, kFar = 4, kEdge = 8 };
+  XG_HD int place(double theta, double &mu, double &st) const {
+    if (!off_pole && are_equal(theta, 0.0)) return -1;
 #ifdef __CUDA_ARCH__
     sincos(theta, &st, &mu);
 #else
@@ -515,20 +529,26 @@ struct CutCell {
     const double na = g.cos_cede - g.cos_colat * mu, da = g.sin_colat * st;
     const double nc = g.cos_sr - g.cos_sc * mu, dc = g.sin_sc * st;
     const int cede = side(na, da, c_near, c_far);
-    if (cede == 2) return 0.0;
+    if (cede == 2) return -1;
     const bool far = no_super || negative(g.superRadius - fabs(theta - g.superColat));
     const int sup = far ? 2 : side(nc, dc, s_near, s_far);
-    if (sup == 1) return 0.0;
-    double dphi = f.pb - f.pa;
-    if (cede == 0 || sup == 0) {
-      // the boundary azimuths that matter: one inverse cosine for the lanes
-      // that need one of the two, a second only for those that need both
-      const double phi1 = edge_azimuth(cede == 0 ? na : nc, cede == 0 ? da : dc);
-      double phi2 = phi1;
-      if (cede == 0 && sup == 0) phi2 = edge_azimuth(nc, dc);
-      dphi = extent(theta, cede, sup, far, phi1, phi2);
-      if (ordered_bits(dphi) == 0) return 0.0;
-    }
+    if (sup == 1) return -1;
+    return (cede == 1 ? kCede1 : 0) | (sup == 2 ? kSup2 : 0) | (far ? kFar : 0) |
+           (cede == 0 || sup == 0 ? kEdge : 0);
+  }
+  XG_HD double width(double theta, int where, double mu, double st) const {
+    const Region &g = f.g;
+    const double na = g.cos_cede - g.cos_colat * mu, da = g.sin_colat * st;
+    const double nc = g.cos_sr - g.cos_sc * mu, dc = g.sin_sc * st;
+    const int cede = where & kCede1 ? 1 : 0, sup = where & kSup2 ? 2 : 0;
+    // the boundary azimuths that matter: one inverse cosine for the lanes
+    // that need one of the two, a second only for those that need both
+    const double phi1 = edge_azimuth(cede == 0 ? na : nc, cede == 0 ? da : dc);
+    double phi2 = phi1;
+    if (cede == 0 && sup == 0) phi2 = edge_azimuth(nc, dc);
+    return extent(theta, cede, sup, (where & kFar) != 0, phi1, phi2);
+  }
+  XG_HD double value(double dphi, double mu, double st) const {
     const Star &s = f.s;
     const double radius = radiusNormalised(mu, s.epsilon, s.zeta, s.shape);
     const double ft2 = f_theta_sq(mu, st, radius, s.epsilon, s.zeta, s.shape);
