@@ -7,6 +7,7 @@
 // vectors are built concurrently on the host's cores (one std::thread per
 // slice); mesh_gpu.cu builds the same meshes on the GPU.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -253,10 +254,13 @@ int xgpu_allocate_cells_many(int n, xgpu_alloc_request *req, int n_threads) {
   if (n <= 0) return 0;
   if (n_threads <= 0) n_threads = (int)std::max(1u, std::thread::hardware_concurrency());
   n_threads = std::min(n_threads, n);
+  // the calling thread takes requests too, each the next one (their quadratures
+  // differ several times over in length)
   std::vector<std::thread> pool;
-  auto work = [&](int t) {
+  std::atomic<int> next{0};
+  auto work = [&]() {
     std::unique_ptr<Work> w(new Work);
-    for (int i = t; i < n; i += n_threads) {
+    for (int i = next++; i < n; i = next++) {
       xgpu_alloc_request &q = req[i];
       Star s{q.R_eq, q.epsilon, q.zeta, q.Omega, q.star_shape_ind};
       allocate(q.num_cells, q.min_sqrt, q.max_sqrt, s, q.super_radius, q.cede_radius,
@@ -264,7 +268,8 @@ int xgpu_allocate_cells_many(int n, xgpu_alloc_request *req, int n_threads) {
                q.hole_radius, q.hole_azimuth, q.out, *w);
     }
   };
-  for (int t = 0; t < n_threads; t++) pool.emplace_back(work, t);
+  for (int t = 1; t < n_threads; t++) pool.emplace_back(work);
+  work();
   for (auto &th : pool) th.join();
   return 0;
 }
