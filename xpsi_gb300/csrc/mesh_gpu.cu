@@ -680,8 +680,8 @@ __device__ __forceinline__ void finish_cell(const MeshJob &J, xgpu_mesh_batch_ou
 // bits.  A cell whose integral vanishes (the reference looks at it again) is
 // left to the boundary kernel.
 // Measured, CTA per cell against this: 100 blackbody spots 6.35, 5.33 ms; 256
-// prior vectors of two regions 80.8, 66.5 ms; 13 such vectors 3.9, 5.0 ms (too
-// few cells to fill the groups: the rule kPackedMin).  With the nodes queued
+// prior vectors of two regions 80.8, 66.5 ms (fewer cells do not fill the
+// groups: the rule kPackedMin).  With the nodes queued
 // between the integrand's stages (PackQueue) and four sums to a reduction the
 // two large batches take 4.23 and 49.4 ms (5.32 and 60.3 without).  Two CTAs per SM keep the
 // pipe full (82-85 % busy) and leave each group several cells; four leave
@@ -708,7 +708,10 @@ struct PackSmem {
   PackLists lists[kPackCells];
   PackQueue queues[kPackThreads / 32];
 };
-constexpr unsigned kPackedMin = 10000;
+// about 130 cells a spot and 460 a vector of two regions; CTA per cell against
+// packed: 20 spots 1.55, 1.90 ms, 40 2.70, 2.12, 60 3.96, 2.96; 7 vectors 2.49,
+// 2.57, 11 3.33, 3.28, 13 4.05, 3.60; 9 prior vectors 2.78, 3.18
+constexpr unsigned kPackedMin = 5000;
 struct CellQueue {
   int64_t *cells, *left;  // queued; left to the boundary kernel
   unsigned *count;        // queued, next of the boundary kernel, left, next of the packed one
