@@ -753,9 +753,135 @@ __device__ int image_record(const RowCtx &c, int I, int N_L, const double *leave
   return out;
 }
 
-__global__ void __launch_bounds__(128) geometry_kernel(IntegrateArgs a) {
+constexpr int kPlanThreads = 128;  // the geometry pre-pass's CTA
+
+// chunks of mesh m for a target cost: count (write == false) or write them
+// from index c0; returns the count.  Costs are whole numbers, so that nothing
+// here waits for the FP64 pipe.
+__device__ int plan_mesh(const IntegrateArgs &a, int m, long long target, bool write, int c0) {
+  const MemberDesc M = a.members[m];
+  int n = 0;
+  long long acc = 0;
+  int64_t start = M.row_off;
+  for (int64_t s = 0; s < M.S0; s++) {
+    const int64_t row = M.row_off + s;
+    const long long c = (long long)a.row_cost[row];
+    if (acc > 0 && acc + c > target) {
+      if (write) {
+        a.chunk_r0[c0 + n] = start;
+        a.chunk_r1[c0 + n] = row;
+        a.chunk_cost[c0 + n] = (float)acc;
+      }
+      n++;
+      acc = 0;
+      start = row;
+    }
+    acc += c;
+  }
+  if (M.S0 > 0) {
+    if (write) {
+      a.chunk_r0[c0 + n] = start;
+      a.chunk_r1[c0 + n] = M.row_off + M.S0;
+      a.chunk_cost[c0 + n] = (float)acc;
+    }
+    n++;
+  }
+  return n;
+}
+
+// exclusive scan of per-thread values over the block; returns the total
+__device__ int block_exclusive_scan(int v, int *s_buf, int &excl) {
+  const int t = threadIdx.x;
+  s_buf[t] = v;
+  __syncthreads();
+  for (int o = 1; o < kPlanThreads; o <<= 1) {
+    const int x = t >= o ? s_buf[t - o] : 0;
+    __syncthreads();
+    s_buf[t] += x;
+    __syncthreads();
+  }
+  excl = s_buf[t] - v;
+  const int total = s_buf[kPlanThreads - 1];
+  __syncthreads();
+  return total;
+}
+
+// The chunks of the call, by the first CTA of the geometry pre-pass, which
+// neither needs them nor leaves the chip before it (also log10 of the
+// energies).  As a launch of its own between the costs and the pre-pass it took
+// 40 us of a 64-parallel call's 690, 29 of one spot's 1205.
+__device__ __noinline__ void plan_chunks(const IntegrateArgs &a) {
+  __shared__ long long s_sum[kPlanThreads];
+  __shared__ int s_scan[kPlanThreads];
+  __shared__ int s_hist[64], s_cur[64];
+  const int t = threadIdx.x;
+  for (int p = t; p < a.N_E; p += kPlanThreads) a.lgE[p] = log10(a.energies[p]);
+  // total cost
+  long long sum = 0;
+  for (int64_t r = t; r < a.n_rows; r += kPlanThreads) sum += (long long)a.row_cost[r];
+  s_sum[t] = sum;
+  __syncthreads();
+  for (int o = kPlanThreads / 2; o > 0; o >>= 1) {
+    if (t < o) s_sum[t] += s_sum[t + o];
+    __syncthreads();
+  }
+  // (whole costs exceed the quotient where they exceed its whole part)
+  long long target = max(1ll, s_sum[0] / max(1, a.target_chunks));
+  // meshes [m0, m1) of this thread
+  const int per = (a.n_members + kPlanThreads - 1) / kPlanThreads;
+  const int m0 = min(a.n_members, t * per), m1 = min(a.n_members, m0 + per);
+  int excl = 0, total = 0;
+  for (int pass = 0; pass < 2; pass++) {
+    int cnt = 0;
+    for (int m = m0; m < m1; m++) cnt += plan_mesh(a, m, target, false, 0);
+    total = block_exclusive_scan(cnt, s_scan, excl);
+    if (total <= a.max_chunks) break;
+    // the bound cannot be exceeded in exact arithmetic; should rounding ever
+    // do it, one chunk per mesh fits
+    target = LLONG_MAX / 2;
+  }
+  int c = excl;
+  for (int m = m0; m < m1; m++) {
+    a.chunk_first[m] = c;
+    c += plan_mesh(a, m, target, true, c);
+  }
+  if (t == 0) {
+    a.chunk_first[a.n_members] = total;
+    *a.chunk_count = total;
+  }
+  // heaviest first: counting sort on floor(log2 cost), descending
+  if (t < 64) s_hist[t] = 0;
+  __syncthreads();
+  for (int k = t; k < total; k += kPlanThreads) {
+    int e = 0;
+    frexpf(a.chunk_cost[k], &e);
+    atomicAdd(&s_hist[min(63, max(0, e))], 1);
+  }
+  __syncthreads();
+  if (t == 0) {
+    int run = 0;
+    for (int b = 63; b >= 0; b--) {
+      s_cur[b] = run;
+      run += s_hist[b];
+    }
+  }
+  __syncthreads();
+  for (int k = t; k < total; k += kPlanThreads) {
+    int e = 0;
+    frexpf(a.chunk_cost[k], &e);
+    a.chunk_order[atomicAdd(&s_cur[min(63, max(0, e))], 1)] = k;
+  }
+}
+
+// a CTA per parallel; kPlan: after one that plans the call's chunks
+template <bool kPlan>
+__global__ void __launch_bounds__(kPlanThreads) geometry_kernel(IntegrateArgs a) {
   extern __shared__ __align__(16) char smem[];
-  const int64_t row = blockIdx.x;
+  if (kPlan && blockIdx.x == 0) {
+    plan_chunks(a);
+    return;
+  }
+  const int64_t row = (int64_t)blockIdx.x - (kPlan ? 1 : 0);
   const int m = a.row_member[row];
   const MemberDesc M = a.members[m];
   const int i = (int)(row - M.row_off);
@@ -2796,11 +2922,14 @@ __global__ void split_reduce_kernel(SplitArgs a) {
 // ---------------------------------------------------------------------------
 constexpr float kCostImage = 28.0f;
 constexpr float kCostRow = 6.0f;
-constexpr int kPlanThreads = 1024;
 
 __global__ void row_cost_kernel(IntegrateArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // the call's counters
+    *a.item_next = 0;
+    *a.geo_count = 0;
+  }
   if (row >= a.n_rows) return;
   const MemberDesc M = a.members[a.row_member[row]];
   const int64_t i = row - M.row_off;
@@ -2818,124 +2947,6 @@ __global__ void row_cost_kernel(IntegrateArgs a) {
       c = (float)io * (kCostImage + (float)cr) + kCostRow;
     }
     a.row_cost[row] = c;
-  }
-}
-
-// chunks of mesh m for a target cost: count (write == false) or write them
-// from index c0; returns the count
-__device__ int plan_mesh(const IntegrateArgs &a, int m, double target, bool write, int c0) {
-  const MemberDesc M = a.members[m];
-  int n = 0;
-  double acc = 0.0;
-  int64_t start = M.row_off;
-  for (int64_t s = 0; s < M.S0; s++) {
-    const int64_t row = M.row_off + s;
-    const double c = a.row_cost[row];
-    if (acc > 0.0 && acc + c > target) {
-      if (write) {
-        a.chunk_r0[c0 + n] = start;
-        a.chunk_r1[c0 + n] = row;
-        a.chunk_cost[c0 + n] = (float)acc;
-      }
-      n++;
-      acc = 0.0;
-      start = row;
-    }
-    acc += c;
-  }
-  if (M.S0 > 0) {
-    if (write) {
-      a.chunk_r0[c0 + n] = start;
-      a.chunk_r1[c0 + n] = M.row_off + M.S0;
-      a.chunk_cost[c0 + n] = (float)acc;
-    }
-    n++;
-  }
-  return n;
-}
-
-// exclusive scan of per-thread values over the block; returns the total
-__device__ int block_exclusive_scan(int v, int *s_buf, int &excl) {
-  const int t = threadIdx.x;
-  s_buf[t] = v;
-  __syncthreads();
-  for (int o = 1; o < kPlanThreads; o <<= 1) {
-    const int x = t >= o ? s_buf[t - o] : 0;
-    __syncthreads();
-    s_buf[t] += x;
-    __syncthreads();
-  }
-  excl = s_buf[t] - v;
-  const int total = s_buf[kPlanThreads - 1];
-  __syncthreads();
-  return total;
-}
-
-// one CTA of kPlanThreads threads
-// (also the call's other constants: log10 of the energies, zeroed counters)
-__global__ void __launch_bounds__(kPlanThreads) plan_chunks_kernel(IntegrateArgs a) {
-  __shared__ double s_sum[kPlanThreads];
-  __shared__ int s_scan[kPlanThreads];
-  __shared__ int s_hist[64], s_cur[64];
-  const int t = threadIdx.x;
-  for (int p = t; p < a.N_E; p += kPlanThreads) a.lgE[p] = log10(a.energies[p]);
-  if (t == 0) {
-    *a.item_next = 0;
-    *a.geo_count = 0;
-  }
-  // total cost (fixed summation order)
-  double sum = 0.0;
-  for (int64_t r = t; r < a.n_rows; r += kPlanThreads) sum += a.row_cost[r];
-  s_sum[t] = sum;
-  __syncthreads();
-  for (int o = kPlanThreads / 2; o > 0; o >>= 1) {
-    if (t < o) s_sum[t] += s_sum[t + o];
-    __syncthreads();
-  }
-  double target = fmax(1.0, s_sum[0] / (double)max(1, a.target_chunks));
-  // meshes [m0, m1) of this thread
-  const int per = (a.n_members + kPlanThreads - 1) / kPlanThreads;
-  const int m0 = min(a.n_members, t * per), m1 = min(a.n_members, m0 + per);
-  int excl = 0, total = 0;
-  for (int pass = 0; pass < 2; pass++) {
-    int cnt = 0;
-    for (int m = m0; m < m1; m++) cnt += plan_mesh(a, m, target, false, 0);
-    total = block_exclusive_scan(cnt, s_scan, excl);
-    if (total <= a.max_chunks) break;
-    // the bound cannot be exceeded in exact arithmetic; should rounding ever
-    // do it, one chunk per mesh fits
-    target = 1.0e300;
-  }
-  int c = excl;
-  for (int m = m0; m < m1; m++) {
-    a.chunk_first[m] = c;
-    c += plan_mesh(a, m, target, true, c);
-  }
-  if (t == 0) {
-    a.chunk_first[a.n_members] = total;
-    *a.chunk_count = total;
-  }
-  // heaviest first: counting sort on floor(log2 cost), descending
-  if (t < 64) s_hist[t] = 0;
-  __syncthreads();
-  for (int k = t; k < total; k += kPlanThreads) {
-    int e = 0;
-    frexpf(a.chunk_cost[k], &e);
-    atomicAdd(&s_hist[min(63, max(0, e))], 1);
-  }
-  __syncthreads();
-  if (t == 0) {
-    int run = 0;
-    for (int b = 63; b >= 0; b--) {
-      s_cur[b] = run;
-      run += s_hist[b];
-    }
-  }
-  __syncthreads();
-  for (int k = t; k < total; k += kPlanThreads) {
-    int e = 0;
-    frexpf(a.chunk_cost[k], &e);
-    a.chunk_order[atomicAdd(&s_cur[min(63, max(0, e))], 1)] = k;
   }
 }
 
@@ -2957,11 +2968,14 @@ __global__ void reduce_flux_kernel(IntegrateArgs a) {
 
 // the geometry pre-pass and, for a table atmosphere, each parallel's entry
 // state of the mu walk: a scan of the parallels in call order
+template <bool kPlan>
 static void launch_geometry(const IntegrateArgs &a, cudaStream_t st) {
   const size_t smem = geometry_bytes(a.N_L, a.N_R);
   // (the attribute is per device: set on every launch, which is cheap)
-  cudaFuncSetAttribute(geometry_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  geometry_kernel<<<(unsigned)a.n_rows, 128, smem, st>>>(a);
+  cudaFuncSetAttribute(geometry_kernel<kPlan>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       200 * 1024);
+  const unsigned grid = (unsigned)(a.n_rows + (kPlan ? 1 : 0));
+  geometry_kernel<kPlan><<<grid, kPlanThreads, smem, st>>>(a);
   if (a.atmos.I != nullptr) num4d_scan_kernel<<<(a.n_members + 127) / 128, 128, 0, st>>>(a);
 }
 
@@ -2993,10 +3007,10 @@ int integrate_energy_chunk(int N_L, int N_P, int N_E, int mixed) {
 void launch_integrate(const IntegrateArgs &a, cudaStream_t st) {
   if (a.n_members <= 0) return;
   const int nmu = a.atmos.I ? a.atmos.nmu : 0, nE = a.atmos.I ? a.atmos.nE : 0;
-  // the work plan from the parallels' costs (needs the ray tables)
-  if (a.n_rows > 0) row_cost_kernel<<<(unsigned)((a.n_rows * 32 + 255) / 256), 256, 0, st>>>(a);
-  plan_chunks_kernel<<<1, kPlanThreads, 0, st>>>(a);
-  if (a.n_rows > 0) launch_geometry(a, st);
+  // the work plan from the parallels' costs (needs the ray tables), beside the
+  // geometry pre-pass
+  row_cost_kernel<<<(unsigned)((a.n_rows * 32 + 256) / 256), 256, 0, st>>>(a);
+  launch_geometry<true>(a, st);
   const long items = (long)a.max_chunks * a.n_eg;
   const unsigned ctas = (unsigned)(items < a.ctas ? items : a.ctas);
   if (a.mixed) {
@@ -3035,7 +3049,7 @@ int launch_stokes(const IntegrateArgs &a, cudaStream_t st) {
   const int nmu = a.atmos.I ? a.atmos.nmu : 0, nE = a.atmos.I ? a.atmos.nE : 0;
   const size_t smem = stokes_smem(a.N_L, a.N_P, a.N_E, a.N_R, nmu, nE);
   if (smem > 227 * 1024) return -2;
-  if (a.atmos.I != nullptr) launch_geometry(a, st);
+  if (a.atmos.I != nullptr) launch_geometry<false>(a, st);
   if (cudaFuncSetAttribute(stokes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return -5;

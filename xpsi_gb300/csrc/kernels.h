@@ -76,7 +76,7 @@ struct IntegrateArgs {
   const double *energies, *leaves, *phases;
   Atmos4D atmos;
   // work chunks, planned on the device from per-parallel costs before the
-  // integrator runs (integrator.cu, plan_chunks_kernel): chunk c covers rows
+  // integrator runs (integrator.cu, plan_chunks): chunk c covers rows
   // [chunk_r0[c], chunk_r1[c]) of one member.  An item is a chunk and one of
   // n_eg groups of its energy chunks (of at most EC energies); `ctas` CTAs take
   // items from the counter item_next, chunk_order[0] (heaviest) first
