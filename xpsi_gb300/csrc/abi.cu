@@ -317,7 +317,7 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
   // the photon sphere has up to about eight; the integrator forms those that
   // find no room again), then one per CTA
   const int64_t img = xg::integrate_image_doubles(N_L);
-  const int64_t geo_cap = 2 * n_rows + 1024;
+  int64_t geo_cap = 2 * n_rows + 1024;
   // one allocation for the call's scratch, parts at 256-byte boundaries
   size_t total = 0;
   auto part = [&](size_t bytes) {
@@ -336,10 +336,18 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
   const size_t o_wsum =
       part(use_w ? (size_t)ctas * xg::integrate_wsum_bytes(N_P, max_cells, &w_cap) : 0);
   const size_t o_lgE = part((size_t)N_E * 8);
-  const size_t o_geo = part((size_t)(geo_cap + ctas) * img * 8);
   const size_t o_info = part((size_t)std::max<int64_t>(1, n_rows) * sizeof(xg::RowInfo));
+  const size_t o_geo = total;
   Dev dscratch;
-  if ((rc = dalloc(dscratch, total, st))) return rc;
+  rc = dalloc(dscratch, o_geo + (size_t)(geo_cap + ctas) * img * 8, st);
+  if (rc) {
+    // a batch that fills the device does without the records, as a parallel
+    // does that finds no room
+    cudaGetLastError();
+    geo_cap = 0;
+    rc = dalloc(dscratch, o_geo + (size_t)ctas * img * 8, st);
+  }
+  if (rc) return rc;
   unsigned char *sp = dscratch.as<unsigned char>();
   CK(cudaMemsetAsync(d->mesh_status, 0, n_meshes * sizeof(int32_t), st));
 
