@@ -303,13 +303,13 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
   int rc;
   if ((rc = upload(dm, reinterpret_cast<const xg::MemberDesc *>(meshes), n_meshes, st))) return rc;
   // run records of the FP64 form's power sums (parallels of up to 256 cells,
-  // which the integrator holds in shared memory, 1024 leaves and 1024 phases,
+  // which the integrator holds in shared memory, 1023 leaves and 1024 phases,
   // and leaf counts that leave shared memory for them, about 470; beyond that
   // the per-cell form runs)
   int w_cap = 0;
   int max_cells = 0;
   for (int m = 0; m < n_meshes; m++) max_cells = std::max(max_cells, (int)meshes[m].S1);
-  const bool use_w = !mixed && max_cells <= 256 && N_L <= 1024 && wsum_enabled() &&
+  const bool use_w = !mixed && max_cells <= 256 && N_L <= 1023 && wsum_enabled() &&
                      xg::integrate_runs_fit(N_L, N_P, EC, d->atmos.intensity ? d->atmos.nmu : 0,
                                             d->atmos.intensity ? d->atmos.nE : 0, table2d);
   const bool tab4 = d->atmos.intensity != nullptr && !table2d;

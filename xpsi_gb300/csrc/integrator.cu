@@ -1216,7 +1216,10 @@ __host__ __device__ inline size_t integrate_wsum_bytes_dev(int N_P, int cap) {
   return (n * (2 * sizeof(float4) + sizeof(int)) + 255) & ~size_t(255);
 }
 constexpr int kStage = 8;
-struct RunStage {  // the last record is empty
+// The last record is empty: no area, in an interval of zeros that follows the
+// pieces (of an actual piece, whose coefficients need not be finite where knots
+// nearly coincide, it would add 0 times infinity).
+struct RunStage {
   float4 w[2 * kStage + 2];
   uint4 meta[kStage + 1];  // interval and cells, class masks of the interval
 };
@@ -1444,7 +1447,7 @@ __device__ __forceinline__ DF run_sum(const CP &cp, const AR &area, const int32_
         lead_acc(q.x, B.x, v, x[z]);
         lead_acc(q.z, B.z, v, x[z]);
         h[z] = __fsub_rn(v, lead);
-        // (the empty record's meta has no flag set)
+        // (the empty record has no flag set)
         odd[z] = (m.y >> e) & 1u;
         at[z] = (m.z >> e) & 1u ? 0u : m.x;
       }
@@ -1687,8 +1690,9 @@ __host__ __device__ inline IntSmem int_smem(char *base, int N_L, int N_P, int EC
     p = reinterpret_cast<T *>(base + at);
     at += n * sizeof(T);
   };
+  // (with runs, an interval of zeros after the last)
   const size_t pieces = kMixed ? (size_t)(EC + 1) * N_L * sizeof(PieceT<float>)
-                               : (size_t)2 * (EC + 1) * N_L * sizeof(float4);
+                               : (size_t)2 * (EC + 1) * (N_L + (runs ? 1 : 0)) * sizeof(float4);
   const size_t geo = (size_t)N_L * 8 * sizeof(double) + (size_t)(4 * N_L + 8) * sizeof(int) + 64;
   take(o.piece, pieces > geo ? pieces : geo);
   take(o.Z, N_L); take(o.abb, N_L); take(o.geom, N_L);
@@ -1757,7 +1761,9 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
   const IntSmem sm = int_smem<kMixed>(smem, N_L, N_P, EC, nmu, nEt, a.table2d != 0, use_w);
   PieceT<WT> *co4 = reinterpret_cast<PieceT<WT> *>(sm.piece);  // mixed form
   const PieceRows pr{reinterpret_cast<float4 *>(sm.piece),
-                     reinterpret_cast<float4 *>(sm.piece) + (size_t)N_L * (EC + 1), EC + 1};
+                     reinterpret_cast<float4 *>(sm.piece) +
+                         (size_t)(N_L + (use_w ? 1 : 0)) * (EC + 1),
+                     EC + 1};
   __shared__ RowAtm s_ra;
   __shared__ RowCtx s_row;
   __shared__ int s_item, s_jalt, s_state[3], s_win[2];
@@ -1816,12 +1822,17 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
       const DF v = df_split(a.phases[t]);
       sm.phase[t] = make_float2(v.h, v.l);
     }
-  if (use_w)
+  if (use_w) {
+    // (the geometry formed in the pieces' place ends before interval N_L of
+    // either array: 80 N_L + 48 bytes against 144 N_L or more)
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = threadIdx.x; t <= EC; t += blockDim.x)
+      pr.a[N_L * (EC + 1) + t] = pr.b[N_L * (EC + 1) + t] = zero;
     for (int t = threadIdx.x; t < kThreads / EC; t += blockDim.x) {
-      sm.stages[t].w[2 * kStage] = sm.stages[t].w[2 * kStage + 1] =
-          make_float4(0.f, 0.f, 0.f, 0.f);
-      sm.stages[t].meta[kStage] = make_uint4(0u, 0u, 0u, 0u);
+      sm.stages[t].w[2 * kStage] = sm.stages[t].w[2 * kStage + 1] = zero;
+      sm.stages[t].meta[kStage] = make_uint4((uint32_t)N_L, 0u, 0u, 0u);
     }
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_iv = N_L - 1, strips = (n_iv + kStrip - 1) / kStrip;
   // energy chunks of equal size, at most EC energies each
