@@ -338,7 +338,9 @@ __device__ bool load_row(const IntegrateArgs &a, const MemberDesc &M, int64_t ro
       r.inclination = M.inclination;
       r.cos_i = cos(M.inclination);
       r.sin_i = sin(M.inclination);
-      r.IO = M.image_order_limit > 0 ? M.image_order_limit : (int)ceil(r.maxDefl / kPi);
+      // (a failed row's deflection, NaN or below zero, has no images)
+      r.IO = M.image_order_limit > 0 ? M.image_order_limit
+                                     : (r.maxDefl > 0.0 ? (int)ceil(r.maxDefl / kPi) : 0);
       const double *vec = a.params + (M.cell_off + (int64_t)i * M.S1 + best) * a.n_params;
       r.vec0 = vec[0];
       r.vec1 = vec[1];
@@ -901,9 +903,14 @@ __global__ void __launch_bounds__(kPlanThreads) geometry_kernel(IntegrateArgs a)
   const bool lit = load_row(a, M, row, i, c, &s_row);
   int n = 0;
   if (lit) {
-    if (threadIdx.x == 0 && a.geo) {
-      const long long b = (long long)atomicAdd(a.geo_count, (unsigned long long)c.IO);
-      s_base = b + c.IO <= a.geo_cap ? b : -1;
+    // records for the images the parallel's deflection reaches (image I lies
+    // beyond I pi); none for one beyond what a ray table keeps (100 pi), NaN or
+    // infinite, so that no row can take or move the others' room
+    const int need =
+        c.maxDefl >= 0.0 && c.maxDefl <= 101.0 * kPi ? min(c.IO, (int)(c.maxDefl / kPi) + 1) : 0;
+    if (threadIdx.x == 0 && a.geo && need > 0) {
+      const long long b = (long long)atomicAdd(a.geo_count, (unsigned long long)need);
+      s_base = b + need <= a.geo_cap ? b : -1;
     }
     stage_deflection(c, g, &s_jalt);
     const bool table = a.atmos.I != nullptr;
@@ -911,13 +918,14 @@ __global__ void __launch_bounds__(kPlanThreads) geometry_kernel(IntegrateArgs a)
     const double mu_top3 = table ? a.atmos.mu[a.atmos.nmu - 3] : 0.0;
     for (int I = 0; I < c.IO; I++) {
       // (without room for the parallel's images the integrator forms them again)
-      double *rec = s_base >= 0 ? a.geo + (s_base + I) * image_doubles(N_L) : nullptr;
+      double *rec = s_base >= 0 && I < need ? a.geo + (s_base + I) * image_doubles(N_L) : nullptr;
       const int got = image_record(c, I, N_L, a.leaves, g, table, mu_top3, mu_max, s_state, s_z,
                                    rec);
       if (got == 0) { n++; continue; }
       if (got == 2) n |= kImgTerm;
       break;
     }
+    if ((n & ~kImgTerm) > need && threadIdx.x == 0) s_base = -1;
   }
   if (threadIdx.x == 0) {
     if (a.row_has_eval) {
