@@ -68,13 +68,22 @@ __device__ __forceinline__ long long ordered(double v) {
   const long long b = __double_as_longlong(v);
   return b < 0 ? -(b & 0x7fffffffffffffffLL) : b;
 }
-// locate() on a table of non-negative values
+// a <= b, false where either is NaN
+__device__ __forceinline__ bool at_most(double a, double b) {
+  constexpr unsigned long long inf2 = 0xffe0000000000000ull;  // of +-infinity, doubled
+  return ordered(a) <= ordered(b) && 2ull * __double_as_longlong(a) <= inf2 &&
+         2ull * __double_as_longlong(b) <= inf2;
+}
+// locate() on a table of non-negative values (a NaN in the table is above
+// nothing, as there)
 __device__ __forceinline__ int locate_bits(const double *x, int n, double v) {
-  const long long vb = __double_as_longlong(v);
+  using U = unsigned long long;
+  // x[mid] > v: its bits above those of v and at most those of infinity
+  const U vb = (U)__double_as_longlong(v), span = 0x7ff0000000000000ull - vb;
   int lo = 0, hi = n - 1;
   while (hi > lo + 1) {
     const int mid = (lo + hi) >> 1;
-    if (__double_as_longlong(x[mid]) > vb) hi = mid; else lo = mid;
+    if ((U)__double_as_longlong(x[mid]) - vb - 1 < span) hi = mid; else lo = mid;
   }
   return lo;
 }

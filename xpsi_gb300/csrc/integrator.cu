@@ -296,7 +296,7 @@ __device__ void state_machine(int N_L, int leaf_lim, const double *leaves, GeoSm
       invis = 1;
     } else {
       for (int m = 1; m < N_L; m++)
-        if (!(ordered(g.phase[m]) > ordered(g.phase[m - 1]))) { term = 1; break; }
+        if (at_most(g.phase[m], g.phase[m - 1])) { term = 1; break; }
     }
   }
   g.flags[0] = term;
@@ -356,14 +356,15 @@ __device__ bool load_row(const IntegrateArgs &a, const MemberDesc &M, int64_t ro
 // Copy the parallel's deflection table to shared memory (the leaf searches
 // probe it ~10 times per lookup) and find the first ray deflected beyond
 // pi/2 (:301-303; the reference's scan is unbounded, here it stops at the
-// last ray).  All threads of the CTA call it.
+// last ray; a NaN ends it, as there, and its cosine rules the second table
+// out).  All threads of the CTA call it.
 __device__ void stage_deflection(RowCtx &c, GeoSmem &g, int *s_jalt) {
   const int N_R = c.N_R;
   for (int t = threadIdx.x; t < N_R; t += blockDim.x) g.rD[t] = c.D[t];
   if (threadIdx.x == 0) *s_jalt = N_R - 1;
   __syncthreads();
   for (int t = threadIdx.x; t < N_R - 1; t += blockDim.x)
-    if (ordered(g.rD[t]) > ordered(kHalfPi)) atomicMin(s_jalt, t);
+    if (!at_most(g.rD[t], kHalfPi)) atomicMin(s_jalt, t);
   __syncthreads();
   c.jalt = *s_jalt;
   c.D = g.rD;
@@ -2063,7 +2064,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
           if (threadIdx.x == 0) s_jalt = c.N_R - 1;
           __syncthreads();
           for (int t = threadIdx.x; t < c.N_R - 1; t += blockDim.x)
-            if (ordered(c.D[t]) > ordered(kHalfPi)) atomicMin(&s_jalt, t);
+            if (!at_most(c.D[t], kHalfPi)) atomicMin(&s_jalt, t);
           __syncthreads();
           c.jalt = s_jalt;
           c.alt_xmin = cos(c.D[c.jalt]);
