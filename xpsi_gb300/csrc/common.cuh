@@ -461,16 +461,14 @@ __device__ __forceinline__ double df_join_bits(DF a, int e) {
     if (a.h == 0.0f) return 0.0;
     return scale_pow2(df_value(a), e);
   }
-  // in units of 2^(eh - 52): the high part's 24 bits and the low part rounded
-  const int li = __float2int_rn(a.l * __int_as_float((52 - eh + 127) << 23));
+  // in units of 2^(eh - 52), the high part's 24 bits and the low part rounded;
+  // half of that where the low part takes a power of two into the binade below
   const bool neg = hb < 0;
-  long long m = ((long long)((hb & 0x7fffff) | 0x800000) << 29) + (neg ? -li : li);
-  int x = ex;
-  if (m < (1ll << 52)) {
-    m <<= 1;
-    x -= 1;
-  }
-  const long long bits = ((long long)(x + 1023) << 52) + (m - (1ll << 52));
+  const int dip = (hb & 0x7fffff) == 0 && (hb ^ __float_as_int(a.l)) < 0 ? 1 : 0;
+  const int li = __float2int_rn(a.l * __int_as_float((52 + dip - eh + 127) << 23));
+  const long long m =
+      ((long long)((hb & 0x7fffff) | 0x800000) << (29 + dip)) + (neg ? -li : li);
+  const long long bits = ((long long)(ex - dip + 1023) << 52) + (m - (1ll << 52));
   return __longlong_as_double(neg ? bits | (long long)0x8000000000000000ull : bits);
 }
 
