@@ -1094,6 +1094,15 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
     S_max = std::max(S_max, q.S);
   }
   if (rows != n_rows || cells != n_cells) return -2;
+  // (the parallels' shared memory: up to 14,000 of them a mesh)
+  const size_t smem = sizeof(double) * (kAreaTab + 2 * S_max + 1);
+  if (smem > 48 * 1024 &&
+      (smem > 227 * 1024 ||
+       cudaFuncSetAttribute(mesh_parallels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)smem) != cudaSuccess)) {
+    cudaGetLastError();
+    return -5;
+  }
   // one allocation for the call's scratch, parts at 256-byte boundaries
   const int S_m = (int)S_max;
   size_t total = 0;
@@ -1145,7 +1154,6 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
   else
     mesh_table_kernel<false><<<dim3((kAreaTab + 127) / 128, (unsigned)n), 128, 0, st>>>(d_jobs,
                                                                                        tab);
-  const size_t smem = sizeof(double) * (kAreaTab + 2 * S_max + 1);
   mesh_parallels_kernel<<<(unsigned)n, 128, smem, st>>>(d_jobs, tab, par, mesh_tmp, trig, cols,
                                                         S_m);
   mesh_rows_kernel<<<(unsigned)((n_rows + 3) / 4), 128, 0, st>>>(d_jobs, n, n_rows, par, S_m,
