@@ -381,6 +381,36 @@ int xgpu_integrate_batch_mixed(int n_meshes, const xgpu_mesh *meshes,
                                int N_P, const xgpu_integrate_batch_data *d,
                                int target_ctas, void *stream);
 
+/* xgpu_integrate_batch (mixed == 0) or xgpu_integrate_batch_mixed with a bound
+ * on the call's device scratch, and what became of it.  Where the scratch does
+ * not fit limit_bytes, or the device, the call does without the parallels'
+ * geometry records (their images are formed again: slower, the same values)
+ * and then without the run records of the FP64 form's power sums (the per-cell
+ * form: slower, another order of summation); what is left is allocated whatever
+ * the limit. */
+typedef struct {
+  int64_t limit_bytes;           /* in: 0 for no limit */
+  int64_t *rows_without_records; /* in: device counter or NULL: the parallels
+                                  * whose images found no room in the records */
+  int64_t used_bytes;            /* out: the scratch taken */
+  int64_t record_room;           /* out: images the records hold */
+  int32_t run_sums;              /* out: 1 where the power sums ran */
+} xgpu_integrate_scratch;
+
+int xgpu_integrate_batch_scratch(int n_meshes, const xgpu_mesh *meshes,
+                                 int64_t n_rows, int N_R, int N_E, int N_L,
+                                 int N_P, const xgpu_integrate_batch_data *d,
+                                 int target_ctas, int mixed,
+                                 xgpu_integrate_scratch *scratch, void *stream);
+
+/* The scratch that xgpu_integrate_batch (or, mixed != 0, the mixed form) takes
+ * without a limit on a device of `sms` multiprocessors: max_cells is the largest
+ * S1 of the meshes, nmu and nE the table's grid sizes (0 without one).  No
+ * device is needed. */
+int64_t xgpu_integrate_scratch_bytes(int n_meshes, int64_t n_rows, int max_cells,
+                                     int N_E, int N_L, int N_P, int nmu, int nE,
+                                     int mixed, int target_ctas, int sms);
+
 /* Energy integration of n_signals [N_E][N_P] signals at in_off[s] (device
  * int64 offsets) into [n_edges-1][N_P] at out_off[s]; d_sq[s] divides the
  * signal first (Likelihood.py:361-364); accumulate adds into out. */
@@ -546,6 +576,10 @@ typedef struct {
 
 int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n_rows,
                     int64_t n_cells, const xgpu_mesh_batch_out *out, void *stream);
+
+/* The device scratch xgpu_mesh_batch takes for n meshes of at most S_max
+ * parallels (no device is needed). */
+int64_t xgpu_mesh_scratch_bytes(int n, int64_t n_rows, int64_t n_cells, size_t S_max);
 
 /* ---------------------------------------------------------------------- */
 /* The photosphere elsewhere: closed mesh and time-invariant integrator.    */

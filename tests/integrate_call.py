@@ -35,3 +35,18 @@ def integrate(ev, B):
               C.byref(d), int(ev.target_ctas), torch.cuda.current_stream().cuda_stream))
     torch.cuda.synchronize()
     return B["flux"].cpu().numpy(), B["mesh_status"].cpu().numpy()
+
+
+def integrate_scratch(ev, B, limit_bytes=0):
+    """integrate() with a bound on the call's scratch: fluxes, statuses, what
+    the call reports, and the parallels that found no geometry records."""
+    torch = ev.torch
+    P, d = B["P"], batch_data(ev, B)
+    count = torch.full((1,), -1, dtype=torch.int64, device=ev.dev)
+    s = N.IntegrateScratch(limit_bytes, count.data_ptr())
+    N.check(N.lib().xgpu_integrate_batch_scratch(
+        P.V * P.H, P.meshes, P.n_rows, ev.N_R, len(ev.model.energies), ev.N_L, ev.N_L, C.byref(d),
+        int(ev.target_ctas), int(ev.precision == "mixed"), C.byref(s),
+        torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    return B["flux"].cpu().numpy(), B["mesh_status"].cpu().numpy(), s, int(count.item())

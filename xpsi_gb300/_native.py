@@ -156,6 +156,11 @@ class ElsewhereBatchData(C.Structure):
                 ("signal_stride", I64), ("signal_N_P", I32)]
 
 
+class IntegrateScratch(C.Structure):
+    _fields_ = [("limit_bytes", I64), ("rows_without_records", P), ("used_bytes", I64),
+                ("record_room", I64), ("run_sums", I32)]
+
+
 class Component(C.Structure):
     _fields_ = [("signal", P), ("phases", P), ("ld", I64), ("n", I32), ("shift", D)]
 
@@ -197,6 +202,11 @@ def _bind(L):
         "xgpu_integrate_batch_mixed": (C.c_int, [C.c_int, C.POINTER(Mesh), I64, C.c_int,
                                                  C.c_int, C.c_int, C.c_int,
                                                  C.POINTER(IntegrateBatchData), C.c_int, P]),
+        "xgpu_integrate_batch_scratch": (C.c_int, [C.c_int, C.POINTER(Mesh), I64, C.c_int,
+                                                   C.c_int, C.c_int, C.c_int,
+                                                   C.POINTER(IntegrateBatchData), C.c_int,
+                                                   C.c_int, C.POINTER(IntegrateScratch), P]),
+        "xgpu_integrate_scratch_bytes": (I64, [C.c_int, I64] + [C.c_int] * 9),
         "xgpu_energy_batch": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, P, P, P, P,
                                         P, P, P, C.c_int, P]),
         "xgpu_fold_batch": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, P, C.c_int, P,
@@ -214,6 +224,7 @@ def _bind(L):
         "xgpu_allocate_cells_many": (C.c_int, [C.c_int, C.POINTER(AllocRequest), C.c_int]),
         "xgpu_mesh_batch": (C.c_int, [C.c_int, C.POINTER(MeshMember), I64, I64,
                                       C.POINTER(MeshBatchOut), P]),
+        "xgpu_mesh_scratch_bytes": (I64, [C.c_int, I64, I64, SZ]),
         "xgpu_peak_probe": (C.c_double, [C.c_int, C.c_int, C.c_int, C.c_int, P, P]),
         "xgpu_gaussian_loglike": (C.c_int, [SZ, SZ, P, SZ, P, P, P]),
         "xgpu_gaussian_loglike_batch": (C.c_int, [C.c_int, C.c_int, C.c_int, P, I64, I64, P, P,
@@ -271,7 +282,9 @@ EXPORTED = ["xgpu_abi_version", "xgpu_last_error", "xgpu_compute_rays", "xgpu_in
             "xgpu_energy_batch", "xgpu_fold_batch", "xgpu_likelihood_batch",
             "xgpu_allocate_cells", "xgpu_cell_mesh", "xgpu_cell_mesh_many", "xgpu_peak_probe",
             "xgpu_likelihood_batch_static", "xgpu_integrate_batch_mixed",
-            "xgpu_fold_batch_tc", "xgpu_mesh_batch", "xgpu_allocate_cells_many",
+            "xgpu_integrate_batch_scratch", "xgpu_integrate_scratch_bytes",
+            "xgpu_fold_batch_tc", "xgpu_mesh_batch", "xgpu_mesh_scratch_bytes",
+            "xgpu_allocate_cells_many",
             "xgpu_closed_cell_mesh", "xgpu_closed_cell_mesh_many",
             "xgpu_integrate_time_invariant", "xgpu_elsewhere_batch",
             "xgpu_integrate_general", "xgpu_compute_expected_counts",

@@ -476,6 +476,7 @@ class BatchEvaluator:
         self.torch = torch
         self.model = model
         self.dev = torch.device("cuda", device)
+        self.sms = torch.cuda.get_device_properties(self.dev).multi_processor_count
         t = lambda a, dt=torch.float64: torch.as_tensor(np.ascontiguousarray(a), dtype=dt,
                                                           device=self.dev)
         self.energies = t(model.energies)

@@ -212,7 +212,8 @@ int xgpu_rays_batch_rule(int64_t n_rows, int N_R, const double *u, const double 
 namespace {
 int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, int N_R,
                          int N_E, int N_L, int N_P, const xgpu_integrate_batch_data *d,
-                         int target_ctas, void *stream, int mixed, int table2d = 0);
+                         int target_ctas, void *stream, int mixed, int table2d = 0,
+                         xgpu_integrate_scratch *scratch = nullptr);
 }
 
 int xgpu_integrate_batch(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, int N_R,
@@ -229,6 +230,15 @@ int xgpu_integrate_batch_mixed(int n_meshes, const xgpu_mesh *meshes, int64_t n_
                               stream, 1);
 }
 
+int xgpu_integrate_batch_scratch(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, int N_R,
+                                 int N_E, int N_L, int N_P, const xgpu_integrate_batch_data *d,
+                                 int target_ctas, int mixed, xgpu_integrate_scratch *scratch,
+                                 void *stream) {
+  if (scratch == nullptr) return fail_msg("no xgpu_integrate_scratch");
+  return integrate_batch_impl(n_meshes, meshes, n_rows, N_R, N_E, N_L, N_P, d, target_ctas,
+                              stream, mixed != 0, 0, scratch);
+}
+
 }  // extern "C"
 
 namespace {
@@ -243,9 +253,81 @@ bool wsum_enabled() {
   return on;
 }
 
+// A call's work split and device scratch: one allocation, parts at 256-byte
+// boundaries.
+struct IntegrateShape {
+  int n_meshes;
+  int64_t n_rows;
+  int max_cells, N_E, N_L, N_P, nmu, nE;  // cells of a parallel at most; grid sizes, 0: no table
+  int table2d, mixed, target_ctas, sms;
+};
+struct IntegratePlan {
+  int64_t target_chunks, max_chunks, geo_cap;
+  int ctas, EC, n_eg, w_cap;
+  bool use_w;
+  size_t r0, r1, first, order, count, rowcost, chunkcost, part, state, slab, wsum, lgE, info, geo;
+  size_t total;
+};
+// what a call does without where its scratch finds no room: nothing, the
+// geometry records (the integrator forms the images again, the same values), or
+// the run records too (the per-cell form, another order of summation)
+enum ScratchLevel { kAllScratch, kNoRecords, kNoRuns };
+
+IntegratePlan integrate_plan(const IntegrateShape &s, ScratchLevel level) {
+  IntegratePlan p{};
+  // the chunks are planned on the device from the parallels' costs (image
+  // counts are known only after the ray tables): about 4 per CTA slot of
+  // the target, at most 2 target + members and at most one per parallel
+  // (integrator.cu)
+  p.target_chunks = 4 * (int64_t)(s.target_ctas > 0 ? s.target_ctas : 8 * 152);
+  p.max_chunks = std::min<int64_t>(2 * p.target_chunks + s.n_meshes, s.n_rows) + 16;
+  p.ctas = 2 * std::max(1, s.sms);  // two integrator CTAs are resident per SM
+  // With fewer parallels than CTAs a parallel's energy chunks are shared by
+  // four items, by two up to twice as many; above that the items' own setup
+  // (records, runs, table window: 15-20 % of one parallel) costs more than it
+  // gives.  Measured, one item per parallel against this: 64 parallels 1036 ->
+  // 711 us, 166 3170 -> 2973, 500 5222 -> 5115; four for 500: 5190.
+  p.EC = xg::integrate_energy_chunk(s.N_L, s.N_P, s.N_E, s.mixed);
+  const int want_eg = s.n_rows <= p.ctas ? 4 : s.n_rows <= 2 * p.ctas ? 2 : 1;
+  while (p.EC > 16 && (s.N_E + p.EC - 1) / p.EC < want_eg) p.EC /= 2;
+  p.n_eg = std::min(want_eg, (s.N_E + p.EC - 1) / p.EC);
+  // run records of the FP64 form's power sums (parallels of up to 256 cells,
+  // which the integrator holds in shared memory, 1023 leaves and 1024 phases,
+  // and leaf counts that leave shared memory for them, about 490 with the full
+  // table; beyond that the per-cell form runs)
+  p.use_w = level != kNoRuns && !s.mixed && s.max_cells <= 256 && s.N_L <= 1023 &&
+            wsum_enabled() &&
+            xg::integrate_runs_fit(s.N_L, s.N_P, p.EC, s.nmu, s.nE, s.table2d);
+  // geometry records: two images per parallel and some room (a parallel near
+  // the photon sphere has up to about eight; the integrator forms those that
+  // find no room again), then one per CTA
+  p.geo_cap = level == kAllScratch ? 2 * s.n_rows + 1024 : 0;
+  auto part = [&](size_t bytes) {
+    const size_t at = p.total;
+    p.total += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  const size_t chunks = (size_t)p.max_chunks, rows = (size_t)std::max<int64_t>(1, s.n_rows);
+  p.r0 = part(chunks * 8), p.r1 = part(chunks * 8);
+  p.first = part((size_t)(s.n_meshes + 1) * 4), p.order = part(chunks * 4);
+  p.count = part(64), p.rowcost = part(rows * 4);
+  p.chunkcost = part(chunks * 4);
+  // each item's CTA zeroes its own part of a partial before accumulating
+  p.part = part(chunks * s.N_E * s.N_P * 8);
+  p.state = part((size_t)3 * s.n_rows + 16);
+  p.slab = part(s.table2d ? 0 : (size_t)p.ctas * s.nmu * s.nE * 8);
+  p.wsum = part(p.use_w ? (size_t)p.ctas * xg::integrate_wsum_bytes(s.N_P, s.max_cells, &p.w_cap)
+                        : 0);
+  p.lgE = part((size_t)s.N_E * 8);
+  p.info = part(rows * sizeof(xg::RowInfo));
+  p.geo = part((size_t)(p.geo_cap + p.ctas) * xg::integrate_image_doubles(s.N_L) * 8);
+  return p;
+}
+
 int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, int N_R,
                          int N_E, int N_L, int N_P, const xgpu_integrate_batch_data *d,
-                         int target_ctas, void *stream, int mixed, int table2d) {
+                         int target_ctas, void *stream, int mixed, int table2d,
+                         xgpu_integrate_scratch *scratch) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (n_meshes <= 0) return 0;
   if (N_L < 5) return fail_msg("num_leaves must be at least 5 (Akima spline)");
@@ -277,77 +359,40 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
     return fail_msg("the elsewhere correction is computed by the FP64 integrator only");
   if (d->correction != nullptr && d->n_correction < 1)
     return fail_msg("correction vectors need at least 1 parameter per cell");
-  if (target_ctas <= 0) target_ctas = 8 * 152;
-  // the chunks are planned on the device from the parallels' costs (image
-  // counts are known only after the ray tables): about 4 per CTA slot of
-  // the target, at most 2 target + members and at most one per parallel
-  // (integrator.cu)
-  const int64_t target_chunks = 4 * (int64_t)target_ctas;
-  const int64_t max_chunks = std::min<int64_t>(2 * target_chunks + n_meshes, n_rows) + 16;
-  if (max_chunks > (int64_t)INT32_MAX / 2) return fail_msg("too many meshes in one call");
-  const int n_chunks = (int)max_chunks;
-  int dev = 0, sms = 0;
+  int dev = 0;
+  IntegrateShape shape{n_meshes, n_rows, 0, N_E, N_L, N_P, 0, 0, table2d, mixed, target_ctas, 0};
   CK(cudaGetDevice(&dev));
-  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int ctas = 2 * std::max(1, sms);  // two integrator CTAs are resident per SM
-  // With fewer parallels than CTAs a parallel's energy chunks are shared by
-  // four items, by two up to twice as many; above that the items' own setup
-  // (records, runs, table window: 15-20 % of one parallel) costs more than it
-  // gives.  Measured, one item per parallel against this: 64 parallels 1036 ->
-  // 711 us, 166 3170 -> 2973, 500 5222 -> 5115; four for 500: 5190.
-  int EC = xg::integrate_energy_chunk(N_L, N_P, N_E, mixed);
-  const int want_eg = n_rows <= ctas ? 4 : n_rows <= 2 * ctas ? 2 : 1;
-  while (EC > 16 && (N_E + EC - 1) / EC < want_eg) EC /= 2;
-  const int n_eg = std::min(want_eg, (N_E + EC - 1) / EC);
-  Dev dm;
+  CK(cudaDeviceGetAttribute(&shape.sms, cudaDevAttrMultiProcessorCount, dev));
+  for (int m = 0; m < n_meshes; m++)
+    shape.max_cells = std::max(shape.max_cells, (int)meshes[m].S1);
+  if (d->atmos.intensity != nullptr) {
+    shape.nmu = (int)d->atmos.nmu;
+    shape.nE = (int)d->atmos.nE;
+  }
+  const bool tab4 = d->atmos.intensity != nullptr && !table2d;
+  IntegratePlan p = integrate_plan(shape, kAllScratch);
+  if (p.max_chunks > (int64_t)INT32_MAX / 2) return fail_msg("too many meshes in one call");
+  Dev dm, dscratch;
   int rc;
   if ((rc = upload(dm, reinterpret_cast<const xg::MemberDesc *>(meshes), n_meshes, st))) return rc;
-  // run records of the FP64 form's power sums (parallels of up to 256 cells,
-  // which the integrator holds in shared memory, 1023 leaves and 1024 phases,
-  // and leaf counts that leave shared memory for them, about 470; beyond that
-  // the per-cell form runs)
-  int w_cap = 0;
-  int max_cells = 0;
-  for (int m = 0; m < n_meshes; m++) max_cells = std::max(max_cells, (int)meshes[m].S1);
-  const bool use_w = !mixed && max_cells <= 256 && N_L <= 1023 && wsum_enabled() &&
-                     xg::integrate_runs_fit(N_L, N_P, EC, d->atmos.intensity ? d->atmos.nmu : 0,
-                                            d->atmos.intensity ? d->atmos.nE : 0, table2d);
-  const bool tab4 = d->atmos.intensity != nullptr && !table2d;
-  // geometry records: two images per parallel and some room (a parallel near
-  // the photon sphere has up to about eight; the integrator forms those that
-  // find no room again), then one per CTA
-  const int64_t img = xg::integrate_image_doubles(N_L);
-  int64_t geo_cap = 2 * n_rows + 1024;
-  // one allocation for the call's scratch, parts at 256-byte boundaries
-  size_t total = 0;
-  auto part = [&](size_t bytes) {
-    const size_t at = total;
-    total += (bytes + 255) & ~size_t(255);
-    return at;
-  };
-  const size_t o_r0 = part((size_t)n_chunks * 8), o_r1 = part((size_t)n_chunks * 8);
-  const size_t o_first = part((size_t)(n_meshes + 1) * 4), o_order = part((size_t)n_chunks * 4);
-  const size_t o_count = part(64), o_rowcost = part((size_t)std::max<int64_t>(1, n_rows) * 4);
-  const size_t o_chunkcost = part((size_t)n_chunks * 4);
-  // each item's CTA zeroes its own part of a partial before accumulating
-  const size_t o_part = part((size_t)n_chunks * N_E * N_P * 8);
-  const size_t o_state = part((size_t)3 * n_rows + 16);
-  const size_t o_slab = part(tab4 ? (size_t)ctas * d->atmos.nmu * d->atmos.nE * 8 : 0);
-  const size_t o_wsum =
-      part(use_w ? (size_t)ctas * xg::integrate_wsum_bytes(N_P, max_cells, &w_cap) : 0);
-  const size_t o_lgE = part((size_t)N_E * 8);
-  const size_t o_info = part((size_t)std::max<int64_t>(1, n_rows) * sizeof(xg::RowInfo));
-  const size_t o_geo = total;
-  Dev dscratch;
-  rc = dalloc(dscratch, o_geo + (size_t)(geo_cap + ctas) * img * 8, st);
-  if (rc) {
-    // a batch that fills the device does without the records, as a parallel
-    // does that finds no room
+  // a batch that fills the device, or the caller's limit, does without the
+  // records and then without the runs
+  const size_t limit = scratch && scratch->limit_bytes > 0 ? (size_t)scratch->limit_bytes : SIZE_MAX;
+  for (int level = kAllScratch;; level++) {
+    p = integrate_plan(shape, (ScratchLevel)level);
+    if (p.total > limit && level < kNoRuns) continue;
+    rc = dalloc(dscratch, p.total, st);
+    if (!rc) break;
+    if (level == kNoRuns) return rc;
     cudaGetLastError();
-    geo_cap = 0;
-    rc = dalloc(dscratch, o_geo + (size_t)ctas * img * 8, st);
   }
-  if (rc) return rc;
+  if (scratch) {
+    scratch->used_bytes = (int64_t)p.total;
+    scratch->record_room = p.geo_cap;
+    scratch->run_sums = p.use_w;
+    if (scratch->rows_without_records)
+      CK(cudaMemsetAsync(scratch->rows_without_records, 0, sizeof(int64_t), st));
+  }
   unsigned char *sp = dscratch.as<unsigned char>();
   CK(cudaMemsetAsync(d->mesh_status, 0, n_meshes * sizeof(int32_t), st));
 
@@ -369,35 +414,36 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
   a.atmos = xg::Atmos4D{d->atmos.logT, d->atmos.logg, d->atmos.mu, d->atmos.logE,
                         d->atmos.intensity, (int)d->atmos.nT, (int)d->atmos.ng,
                         (int)d->atmos.nmu, (int)d->atmos.nE, d->atmos.intensity_f32};
-  a.max_chunks = n_chunks;
-  a.target_chunks = (int)target_chunks;
-  a.chunk_r0 = reinterpret_cast<int64_t *>(sp + o_r0);
-  a.chunk_r1 = reinterpret_cast<int64_t *>(sp + o_r1);
-  a.partial = reinterpret_cast<double *>(sp + o_part);
-  a.chunk_first = reinterpret_cast<int32_t *>(sp + o_first);
-  a.chunk_order = reinterpret_cast<int32_t *>(sp + o_order);
-  a.chunk_count = reinterpret_cast<int32_t *>(sp + o_count);
+  a.max_chunks = (int)p.max_chunks;
+  a.target_chunks = (int)p.target_chunks;
+  a.chunk_r0 = reinterpret_cast<int64_t *>(sp + p.r0);
+  a.chunk_r1 = reinterpret_cast<int64_t *>(sp + p.r1);
+  a.partial = reinterpret_cast<double *>(sp + p.part);
+  a.chunk_first = reinterpret_cast<int32_t *>(sp + p.first);
+  a.chunk_order = reinterpret_cast<int32_t *>(sp + p.order);
+  a.chunk_count = reinterpret_cast<int32_t *>(sp + p.count);
   a.item_next = a.chunk_count + 1;
-  a.geo_count = reinterpret_cast<unsigned long long *>(sp + o_count + 16);
-  a.row_cost = reinterpret_cast<float *>(sp + o_rowcost);
-  a.chunk_cost = reinterpret_cast<float *>(sp + o_chunkcost);
-  uint8_t *sb = sp + o_state;
+  a.geo_count = reinterpret_cast<unsigned long long *>(sp + p.count + 16);
+  a.row_cost = reinterpret_cast<float *>(sp + p.rowcost);
+  a.chunk_cost = reinterpret_cast<float *>(sp + p.chunkcost);
+  uint8_t *sb = sp + p.state;
   a.row_has_eval = sb; a.row_last_top = sb + n_rows; a.row_entry_top = sb + 2 * n_rows;
-  a.n_eg = n_eg;
-  a.EC = EC;
-  a.ctas = ctas;
-  a.lgE = reinterpret_cast<double *>(sp + o_lgE);
-  a.geo = reinterpret_cast<double *>(sp + o_geo);
-  a.geo_cap = geo_cap;
-  a.row_info = reinterpret_cast<xg::RowInfo *>(sp + o_info);
+  a.n_eg = p.n_eg;
+  a.EC = p.EC;
+  a.ctas = p.ctas;
+  a.lgE = reinterpret_cast<double *>(sp + p.lgE);
+  a.geo = reinterpret_cast<double *>(sp + p.geo);
+  a.geo_cap = p.geo_cap;
+  a.row_info = reinterpret_cast<xg::RowInfo *>(sp + p.info);
   a.table2d = table2d;
   a.member_status = d->mesh_status;
   a.flux = d->flux;
   a.flop_counter = d->flop_counter;
-  a.slab = tab4 ? reinterpret_cast<double *>(sp + o_slab) : nullptr;
-  a.wsum = use_w ? sp + o_wsum : nullptr;
-  a.w_cap = w_cap;
+  a.slab = tab4 ? reinterpret_cast<double *>(sp + p.slab) : nullptr;
+  a.wsum = p.use_w ? sp + p.wsum : nullptr;
+  a.w_cap = p.w_cap;
   a.mixed = mixed;
+  a.rows_again = scratch ? scratch->rows_without_records : nullptr;
   xg::launch_integrate(a, st);
   CK(cudaGetLastError());
   return 0;
@@ -405,6 +451,16 @@ int integrate_batch_impl(int n_meshes, const xgpu_mesh *meshes, int64_t n_rows, 
 }  // namespace
 
 extern "C" {
+
+int64_t xgpu_integrate_scratch_bytes(int n_meshes, int64_t n_rows, int max_cells, int N_E, int N_L,
+                                     int N_P, int nmu, int nE, int mixed, int target_ctas,
+                                     int sms) {
+  if (n_meshes <= 0) return 0;
+  return (int64_t)integrate_plan(IntegrateShape{n_meshes, n_rows, max_cells, N_E, N_L, N_P, nmu,
+                                                nE, 0, mixed, target_ctas, sms},
+                                 kAllScratch)
+      .total;
+}
 
 int xgpu_energy_batch(int n_signals, int N_E, int N_P, int n_edges, const double *signal,
                       const int64_t *in_off, const double *log10_energies,

@@ -936,6 +936,8 @@ __global__ void __launch_bounds__(kPlanThreads) geometry_kernel(IntegrateArgs a)
     if (a.row_info) {
       RowInfo r;
       r.geo = s_base;
+      if (a.rows_again && s_base < 0 && (n & ~kImgTerm) > 0)
+        atomicAdd(reinterpret_cast<unsigned long long *>(a.rows_again), 1ull);
       r.images = n;
       r.cell = c.J;
       r.z_lo = __int_as_float(s_z[0]);

@@ -96,6 +96,7 @@ struct IntegrateArgs {
   long long geo_cap;
   unsigned long long *geo_count;
   RowInfo *row_info;        // [rows]
+  int64_t *rows_again = nullptr;  // parallels that found no records are counted here, or null
   int table2d;              // the atmosphere is a 2-D table (atm 4, 6)
   float *row_cost;          // [n_rows] scratch: estimated cost of each parallel
   float *chunk_cost;        // [max_chunks] scratch

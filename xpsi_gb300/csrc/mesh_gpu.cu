@@ -1061,8 +1061,45 @@ __global__ void __launch_bounds__(kCutThreads) mesh_split_kernel(
   }
 }
 
+// a call's device scratch: one allocation, parts at 256-byte boundaries
+struct MeshScratch {
+  size_t jobs, tab, row, mesh, par, trig, cols, queue, left, count, split, piece, total;
+  unsigned cap;  // of the split list
+  bool pack;     // the packed kernel is launched
+};
+MeshScratch mesh_scratch(size_t n, size_t n_rows, size_t n_cells, size_t S_max) {
+  MeshScratch o{};
+  auto part = [&](size_t bytes) {
+    const size_t at = o.total;
+    o.total += (bytes + 255) & ~size_t(255);
+    return at;
+  };
+  o.jobs = part(sizeof(MeshJob) * n);
+  o.tab = part(sizeof(double) * n * kAreaTab);
+  o.row = part(sizeof(RowTmp) * n_rows);
+  o.mesh = part(sizeof(double) * 2 * n);
+  o.par = part(sizeof(double) * n * S_max);
+  o.trig = part(sizeof(MeshTrig) * n);
+  o.cols = part(sizeof(ColTrig) * n * (S_max + 1));
+  o.queue = part(sizeof(int64_t) * n_cells);
+  // the packed kernel is launched where the batch may queue enough cells (a
+  // region's edge cuts some two cells of each parallel, up to about six)
+  o.pack = n_rows >= kPackedMin / 6;
+  o.left = part(o.pack ? sizeof(int64_t) * n_cells : 0);
+  o.count = part(6 * sizeof(unsigned));
+  o.cap = (unsigned)(4 * n + 64);
+  o.split = part(sizeof(SplitCell) * o.cap);
+  o.piece = part(sizeof(double) * 2 * kPieces * o.cap);
+  return o;
+}
+
 }  // namespace
 }  // namespace xg
+
+extern "C" int64_t xgpu_mesh_scratch_bytes(int n, int64_t n_rows, int64_t n_cells, size_t S_max) {
+  if (n <= 0) return 0;
+  return (int64_t)xg::mesh_scratch((size_t)n, (size_t)n_rows, (size_t)n_cells, S_max).total;
+}
 
 extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n_rows,
                                int64_t n_cells, const xgpu_mesh_batch_out *out, void *stream) {
@@ -1103,47 +1140,26 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
     cudaGetLastError();
     return -5;
   }
-  // one allocation for the call's scratch, parts at 256-byte boundaries
+  const MeshScratch o = mesh_scratch((size_t)n, (size_t)n_rows, (size_t)n_cells, S_max);
   const int S_m = (int)S_max;
-  size_t total = 0;
-  auto part = [&](size_t bytes) {
-    const size_t at = total;
-    total += (bytes + 255) & ~size_t(255);
-    return at;
-  };
-  const size_t o_jobs = part(sizeof(MeshJob) * (size_t)n);
-  const size_t o_tab = part(sizeof(double) * (size_t)n * kAreaTab);
-  const size_t o_row = part(sizeof(RowTmp) * (size_t)n_rows);
-  const size_t o_mesh = part(sizeof(double) * 2 * (size_t)n);
-  const size_t o_par = part(sizeof(double) * (size_t)n * S_max);
-  const size_t o_trig = part(sizeof(MeshTrig) * (size_t)n);
-  const size_t o_cols = part(sizeof(ColTrig) * (size_t)n * (S_max + 1));
-  const size_t o_queue = part(sizeof(int64_t) * (size_t)n_cells);
-  // the packed kernel is launched where the batch may queue enough cells (a
-  // region's edge cuts some two cells of each parallel, up to about six)
-  const bool pack = n_rows >= (int64_t)(kPackedMin / 6);
-  const size_t o_left = part(pack ? sizeof(int64_t) * (size_t)n_cells : 0);
-  const size_t o_count = part(6 * sizeof(unsigned));
-  SplitList sl{};
-  sl.cap = (unsigned)(4 * (size_t)n + 64);
-  const size_t o_split = part(sizeof(SplitCell) * sl.cap);
-  const size_t o_piece = part(sizeof(double) * 2 * kPieces * sl.cap);
   unsigned char *base = nullptr;
-  if (cudaMallocAsync(reinterpret_cast<void **>(&base), total, st) != cudaSuccess) return -5;
-  MeshJob *d_jobs = reinterpret_cast<MeshJob *>(base + o_jobs);
-  double *tab = reinterpret_cast<double *>(base + o_tab);
-  RowTmp *row_tmp = reinterpret_cast<RowTmp *>(base + o_row);
-  double *mesh_tmp = reinterpret_cast<double *>(base + o_mesh);
-  double *par = reinterpret_cast<double *>(base + o_par);
-  MeshTrig *trig = reinterpret_cast<MeshTrig *>(base + o_trig);
-  ColTrig *cols = reinterpret_cast<ColTrig *>(base + o_cols);
-  int64_t *queue = reinterpret_cast<int64_t *>(base + o_queue);
-  unsigned *n_queue = reinterpret_cast<unsigned *>(base + o_count);
-  sl.cells = reinterpret_cast<SplitCell *>(base + o_split);
-  sl.piece = reinterpret_cast<double *>(base + o_piece);
+  if (cudaMallocAsync(reinterpret_cast<void **>(&base), o.total, st) != cudaSuccess) return -5;
+  MeshJob *d_jobs = reinterpret_cast<MeshJob *>(base + o.jobs);
+  double *tab = reinterpret_cast<double *>(base + o.tab);
+  RowTmp *row_tmp = reinterpret_cast<RowTmp *>(base + o.row);
+  double *mesh_tmp = reinterpret_cast<double *>(base + o.mesh);
+  double *par = reinterpret_cast<double *>(base + o.par);
+  MeshTrig *trig = reinterpret_cast<MeshTrig *>(base + o.trig);
+  ColTrig *cols = reinterpret_cast<ColTrig *>(base + o.cols);
+  int64_t *queue = reinterpret_cast<int64_t *>(base + o.queue);
+  unsigned *n_queue = reinterpret_cast<unsigned *>(base + o.count);
+  SplitList sl{};
+  sl.cap = o.cap;
+  sl.cells = reinterpret_cast<SplitCell *>(base + o.split);
+  sl.piece = reinterpret_cast<double *>(base + o.piece);
   sl.count = n_queue + 4;
-  const CellQueue Q{queue, reinterpret_cast<int64_t *>(base + o_left), n_queue,
-                    pack ? kPackedMin : UINT_MAX};
+  const CellQueue Q{queue, reinterpret_cast<int64_t *>(base + o.left), n_queue,
+                    o.pack ? kPackedMin : UINT_MAX};
   // (a copy from pageable memory has been staged when cudaMemcpyAsync
   // returns, so the host jobs may go out of scope)
   cudaMemcpyAsync(d_jobs, jobs.data(), sizeof(MeshJob) * (size_t)n, cudaMemcpyHostToDevice, st);
@@ -1160,7 +1176,7 @@ extern "C" int xgpu_mesh_batch(int n, const xgpu_mesh_member *members, int64_t n
                                                                  mesh_tmp, *out, row_tmp);
   mesh_cells_kernel<<<(unsigned)((n_cells + 127) / 128), 128, 0, st>>>(
       d_jobs, n, n_cells, *out, row_tmp, mesh_tmp, trig, cols, S_m, queue, n_queue);
-  if (pack) {
+  if (o.pack) {
     const size_t lists = sizeof(PackSmem);
     cudaFuncSetAttribute(mesh_packed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)lists);

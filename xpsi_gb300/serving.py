@@ -32,6 +32,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import batch as BT
+from ._native import lib
 
 
 @dataclass(eq=False)
@@ -66,25 +67,26 @@ class ServerStats:
 
 
 def estimate_bytes(ev: BT.BatchEvaluator, P) -> int:
-    """Device footprint of one prepared launch (inputs, ray tables, fluxes,
-    integrated signals, folded signals, likelihood scratch, integrator
-    partials and table slabs)."""
+    """Device footprint of one prepared launch: inputs, ray tables, fluxes,
+    integrated signals, folded signals, likelihood scratch, and the largest of
+    the mesh builder's, the integrator's and the fold's scratch (each is given
+    back to the launch's stream before the next stage takes its own)."""
     n_m = P.V * P.H
     N_E = len(ev.model.energies)
     N_P = ev.N_L
     # packed rows (8 FP64 + mesh index) and cells (area, azimuth, 2 params,
-    # flag), whether uploaded or built on the device, plus the GPU mesh
-    # builder's scratch (area tables, per-row temporaries)
+    # flag), whether uploaded or built on the device
     b = P.n_rows * (8 * 8 + 4) + P.n_cells * (4 * 8 + 4) + P.d_sq.nbytes + P.shifts.nbytes
-    b += len(P.meshes) * 1000 * 8 + P.n_rows * 4 * 8
     b += 3 * P.n_rows * ev.N_R * 8 + P.n_rows * 12
-    b += n_m * (N_E * N_P + ev.q * N_P + ev.K * N_P) * 8
+    b += n_m * (N_E * N_P + ev.q * N_P + ev.K * N_P) * 8 + n_m * 20 + 4
     b += P.V * ev.K * 12 + P.V * 12
-    b += 8 * 152 * (N_E * N_P * 8)           # chunk partials (bounded)
-    # the integrator's geometry records: two images per parallel
-    b += (2 * P.n_rows + 1024) * (4 * 8 + 1) * ev.N_L
-    if ev.atmos is not None:
-        b += 8 * 152 * ev.atmos.nmu * ev.atmos.nE * 8
+    S_max = max((m.S1 for m in P.meshes), default=2)
+    nmu, nE = (ev.atmos.nmu, ev.atmos.nE) if ev.atmos is not None else (0, 0)
+    b += max(lib().xgpu_mesh_scratch_bytes(n_m, P.n_rows, P.n_cells, S_max),
+             lib().xgpu_integrate_scratch_bytes(n_m, P.n_rows, S_max, N_E, ev.N_L, N_P, nmu, nE,
+                                                int(ev.precision == "mixed"),
+                                                int(ev.target_ctas), ev.sms),
+             (n_m * N_P + ev.K) * (ev.q * 8 + 4) + 1024)
     if getattr(P, "else_V", 0):
         # elsewhere: packed parallels and cells, ray tables, per-parallel
         # spectra, the spectra, and the hot regions' correction vectors
