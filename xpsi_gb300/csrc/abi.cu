@@ -293,8 +293,8 @@ IntegratePlan integrate_plan(const IntegrateShape &s, ScratchLevel level) {
   p.n_eg = std::min(want_eg, (s.N_E + p.EC - 1) / p.EC);
   // run records of the FP64 form's power sums (parallels of up to 256 cells,
   // which the integrator holds in shared memory, 1023 leaves and 1024 phases,
-  // and leaf counts that leave shared memory for them, about 490 with the full
-  // table; beyond that the per-cell form runs)
+  // and leaf counts that leave shared memory for them, about 470 with the full
+  // table and as many phases; beyond that the per-cell form runs)
   p.use_w = level != kNoRuns && !s.mixed && s.max_cells <= 256 && s.N_L <= 1023 &&
             wsum_enabled() &&
             xg::integrate_runs_fit(s.N_L, s.N_P, p.EC, s.nmu, s.nE, s.table2d);
