@@ -334,8 +334,11 @@ int xgpu_rays_batch(int64_t n_rows, int N_R, const double *u,
                     const double *lag_scale, void *stream);
 /* The same with a choice of each integral's first panel: 31 points, which most
  * rays need no more than (xgpu_rays_batch), or 61, the reference's rule from
- * the start.  The two agree to 1e-14; what rounds to FP32 downstream (the
- * mixed form) keeps its values to the last bit with 61. */
+ * the start.  Either holds each integral to 1e-12 of itself by its own error
+ * estimate; the largest difference measured between their tables, u from 0.02
+ * to 0.6666, is 3e-14.  What rounds to FP32 downstream (the mixed form) keeps
+ * its values to the last bit with 61, which a caller who feeds
+ * xgpu_integrate_batch_mixed asks for here. */
 int xgpu_rays_batch_rule(int64_t n_rows, int N_R, const double *u,
                          const double *r_s, double *maxAlpha, double *deflection,
                          double *cos_alpha, double *lag, double *maxDeflection,
