@@ -42,7 +42,6 @@ constexpr int kThreads = 256;
 constexpr int kEPT = 8;  // energies per accumulation task
 constexpr int kMaxCellsF = 256;  // cells per parallel held as FP32 pairs in shared memory
 constexpr int kMaxPhases = 1024;  // signal phases held as FP32 pairs in shared memory
-constexpr int kMaxEnergiesF = 256;  // energies held in FP32 (mixed form)
 constexpr int kStrip = 8;  // Akima pieces per thread, built from a sliding window of chords
 
 // Akima piece of one energy row: value at the left knot and the three
@@ -69,12 +68,13 @@ struct GeoSmem {
   double *rD;  // the parallel's deflection table, staged for the binary searches
   int *src, *calc, *term, *clamp0;
   int *flags;  // [0] terminate, [1] invisible image, [2] any evaluation, [3] last_top
-  double *lgE;  // [EC] log10 of the chunk's energies (FP64 path, Num4D)
-  double *lzs;  // [N_L] log10(Z) + log10(E_eff) per leaf (FP64 path, Num4D)
+  // the rest is the Stokes kernel's:
+  double *lgE;  // [EC] log10 of the chunk's energies, or the energies (2-D tables)
+  double *lzs;  // [N_L] log10(Z), or Z, per leaf (2-D tables)
   int *sc_exp;  // [EC] binary exponent of the largest |profile value| per energy row
-  DF *ih, *ih2;  // [N_L] 1/h and 1/h^2 of the phase intervals (FP64 path)
+  DF *ih, *ih2;  // [N_L] 1/h and 1/h^2 of the phase intervals
   double *c2chi = nullptr, *s2chi = nullptr;  // [N_L] cos, sin of twice the polarisation
-                                              // angle (Stokes kernel only)
+                                              // angle
 };
 
 
@@ -377,19 +377,11 @@ __device__ void stage_deflection(RowCtx &c, GeoSmem &g, int *s_jalt) {
 struct AtmSmem {
   double *gmu, *gE;      // grids of mu and log10(E/kT)
   double *smu, *sE;      // inverse Lagrange denominators per stencil base, 4 each
-  float *fgmu, *fgE, *fsmu, *fsE;  // FP32 copies for the mixed-precision form
-  float *fgEo;           // [3 nE] offsets gE[b + i] - gE[b], i = 1..3 (mixed form)
-  // FP64 form with a contracted 4-D table: the offsets gE[b + i] - gE[b]
-  // (i = 1..3) and the inverse Lagrange denominators of the energy grid as
-  // double-float pairs (in the space of the mixed form's FP32 arrays and of sE)
-  DF *dgEo, *dsE;
-  int *xe;               // [nE] binary exponent of each energy column of the slab
+  float *fgmu, *fgE;     // FP32 copies of the grids, for the guided searches
   float *fphase;         // FP32 copy of the phase knots
   float *fphase_lo;      // phase knot minus its FP32 copy
   float *fcphi, *fcphi_lo;  // cell azimuths of the parallel as float pairs (<= kMaxCellsF)
   float *fcarea, *fcarea_lo;  // cell areas of the parallel as float pairs (<= kMaxCellsF)
-  float *finvZ, *fabb, *fgeom;  // per profile column: 1/Z, mu eta, geometric factor
-  float *fE;                // energies
 };
 
 // inverse denominators of the 4-point Lagrange basis on grid[b..b+3]
@@ -611,10 +603,8 @@ __host__ __device__ inline Layout make_layout(int N_L, int N_P, int N_E, int nmu
   L.bytes = (size_t)5 * N_L * sizeof(double)      // phase, leafphase, Z, ABB, GEOM
             + (size_t)ec * N_L * piece_bytes       // coefficients
             + (size_t)(nmu + nE) * 5 * sizeof(double)  // Num4D grids + inverse denominators
-            + (size_t)(nmu + nE) * 5 * sizeof(float)   // their FP32 copies (mixed form)
-            + (size_t)3 * nE * sizeof(float)           // energy-grid node offsets (mixed)
-            + (size_t)nE * sizeof(int)                 // slab column exponents (FP64 form)
-            + (size_t)(5 * N_L + 4 * kMaxCellsF + kMaxEnergiesF) * sizeof(float)
+            + (size_t)(nmu + nE) * sizeof(float)       // the grids' FP32 copies
+            + (size_t)(2 * N_L + 4 * kMaxCellsF) * sizeof(float)  // knots, cells as pairs
             + (size_t)N_R * sizeof(double)  // staged deflection table
             + (size_t)(ec + N_L) * sizeof(double)  // lgE, lzs
             + (size_t)2 * N_L * sizeof(DF)         // ih, ih2
@@ -653,25 +643,12 @@ __device__ GeoSmem carve(char *base, int N_L, int EC, double **coef, int nmu = 0
     float *f = reinterpret_cast<float *>(d);
     atm->fgmu = f; f += nmu;
     atm->fgE = f; f += nE;
-    atm->fsmu = f; f += (size_t)4 * nmu;
-    atm->fsE = f; f += (size_t)4 * nE;
-    atm->fgEo = f; f += (size_t)3 * nE;
-    // the FP64 form's double-float energy-grid data reuse the mixed form's
-    // FP32 arrays (fsmu .. fgEo: 4 nmu + 7 nE floats >= 6 nE + 1) and sE
-    atm->dgEo = reinterpret_cast<DF *>((reinterpret_cast<uintptr_t>(atm->fsmu) + 7) &
-                                       ~uintptr_t(7));
-    atm->dsE = reinterpret_cast<DF *>(atm->sE);
     atm->fphase = f; f += N_L;
     atm->fphase_lo = f; f += N_L;
     atm->fcphi = f; f += kMaxCellsF;
     atm->fcphi_lo = f; f += kMaxCellsF;
     atm->fcarea = f; f += kMaxCellsF;
     atm->fcarea_lo = f; f += kMaxCellsF;
-    atm->finvZ = f; f += N_L;
-    atm->fabb = f; f += N_L;
-    atm->fgeom = f; f += N_L;
-    atm->fE = f; f += kMaxEnergiesF;
-    atm->xe = reinterpret_cast<int *>(f); f += nE;
     d = reinterpret_cast<double *>((reinterpret_cast<uintptr_t>(f) + 15) & ~uintptr_t(15));
   }
   int *ip = reinterpret_cast<int *>(d);
