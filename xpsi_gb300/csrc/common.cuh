@@ -74,16 +74,19 @@ __device__ __forceinline__ bool at_most(double a, double b) {
   return ordered(a) <= ordered(b) && 2ull * __double_as_longlong(a) <= inf2 &&
          2ull * __double_as_longlong(b) <= inf2;
 }
-// locate() on a table of non-negative values (a NaN in the table is above
+// locate() on a table of non-negative values; kNaN: which may hold NaN (above
 // nothing, as there)
+template <bool kNaN = false>
 __device__ __forceinline__ int locate_bits(const double *x, int n, double v) {
   using U = unsigned long long;
+  const long long vb = __double_as_longlong(v);
   // x[mid] > v: its bits above those of v and at most those of infinity
-  const U vb = (U)__double_as_longlong(v), span = 0x7ff0000000000000ull - vb;
+  const U first = (U)vb + 1, span = 0x7ff0000000000000ull - (U)vb;
   int lo = 0, hi = n - 1;
   while (hi > lo + 1) {
     const int mid = (lo + hi) >> 1;
-    if ((U)__double_as_longlong(x[mid]) - vb - 1 < span) hi = mid; else lo = mid;
+    const long long b = __double_as_longlong(x[mid]);
+    if (kNaN ? (U)b - first < span : b > vb) hi = mid; else lo = mid;
   }
   return lo;
 }
