@@ -4,7 +4,8 @@
 // blackbody (hot_BB.pyx:54-98) and numerical 4-D (hot_Num4D.pyx:248-461)
 // atmospheres.
 //
-// Work decomposition (one CTA per chunk of consecutive parallels of one mesh):
+// Work decomposition (CTAs that take items in turn: a chunk of consecutive
+// parallels of one mesh, and all or a share of its energies):
 //   1. leaf geometry, in a pre-pass with a CTA per parallel, one thread per leaf
 //      pair (k, N_L-1-k): image deflection,
 //      cos alpha / lag / d cos alpha from the Steffen ray tables, Doppler and
@@ -1740,7 +1741,7 @@ struct RowAtm {
 // stencils and 1 / h of the knots; energy coordinates are integers, and values
 // change between double and float pair on the integer pipe.  24 vectors at
 // sqrt_num_cells 96 (two Num4D regions, 128 leaves, 128 energies): 30 ms with
-// those in FP64 and the geometry formed here, 16.7 ms now; 100 blackbody spots
+// those in FP64 and the geometry formed here, 16.0 ms now; 100 blackbody spots
 // (64 leaves, 64 energies): 4.7 ms, 1.9 ms now.
 // WT = double: the plain FP64 drop-in.  WT = float: the mixed-precision form
 // (geometry, visibility and knots in FP64; atmosphere, Akima pieces and the
@@ -1870,7 +1871,7 @@ __global__ void __launch_bounds__(kThreads, 2) integrate_kernel(IntegrateArgs a)
     // scaling (uniform over the CTA: a chunk is one mesh's rows)
     const bool dfy = !kMixed && t4 && M.beam_opt == 0 && !corr;
     double *part = a.partial + (size_t)chunk * N_E * N_P;
-    // partials: FP64 form [N_P][N_E] (the sums' lanes are energies), mixed [N_E][N_P]
+    // partials [N_P][N_E] in either form: the sums' lanes are energies
     for (int t = threadIdx.x; t < N_P * (e_hi - e_lo); t += blockDim.x) {
       const int k = t / (e_hi - e_lo), e = e_lo + t - k * (e_hi - e_lo);
       part[(size_t)k * N_E + e] = 0.0;

@@ -83,7 +83,7 @@ struct IntegrateArgs {
   int max_chunks;           // bound on the planned chunks (2 target + members)
   int target_chunks;        // chunks the plan aims at
   int64_t *chunk_r0, *chunk_r1;  // [max_chunks]
-  double *partial;          // [max_chunks][N_P][N_E] (mixed: [N_E][N_P]), by each chunk's CTA
+  double *partial;          // [max_chunks][N_P][N_E] (Stokes: see below), by each item's CTA
   int32_t *chunk_first;     // [n_members + 1] first chunk of each member
   int32_t *chunk_order;     // [max_chunks]
   int32_t *chunk_count;     // [1]

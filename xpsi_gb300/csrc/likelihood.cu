@@ -8,9 +8,11 @@
 // and hold one phase bin each for the channel sums (Newton steps, Gaussian
 // width, the normalisation A), which are reduced with xor-butterfly shuffles
 // so every lane holds the same bits and control flow stays warp-uniform;
-// the marginal integral is a QUADPACK-style adaptive Gauss-Kronrod-21 quadrature run to
-// relative 1e-13 whose 21 node evaluations per panel are spread over the
-// lanes.  The reference's CQUAD call (:416-419) asks for relative 1e-8 on
+// the marginal integral is one 61-point Gauss-Kronrod panel on each side of
+// the peak, two nodes to a lane, where those meet relative 1e-13 by their own
+// error estimate, else a QUADPACK-style adaptive Gauss-Kronrod-21 quadrature run
+// to it, whose 21 node evaluations per panel are spread over the lanes.  The
+// reference's CQUAD call (:416-419) asks for relative 1e-8 on
 // this smooth integrand, so both converge to the same integral.  The channel
 // terms are summed per evaluation in channel order by a second kernel, which
 // also applies the reference's early exits (slim cut :677-684, vanished
@@ -935,7 +937,8 @@ void launch_likelihood(const LikeArgs &a, cudaStream_t st) {
   long warps = (long)a.n_vec * a.K;
   if (warps <= 0) return;
   unsigned blocks = (unsigned)((warps + kWarps - 1) / kWarps);
-  // (persistent: four CTAs are resident per SM)
+  // (at most 16 CTAs per SM, four of them resident: each takes several channels,
+  // and the phase grid's reciprocals are formed 16 times per SM at most)
   like_channel_kernel<<<blocks < 152u * 16u ? blocks : 152u * 16u, 32 * kWarps, 0, st>>>(a);
   like_finalize_kernel<<<a.n_vec, 32 * kFinalWarps, 0, st>>>(a);
 }

@@ -5,7 +5,8 @@
 // (the packing of xpsi/HotRegion.py:774-1017 / Likelihood.py:297-432 that
 // the host path does in numpy).
 //
-// Seven launches over all meshes of the batch:
+// Seven launches over all meshes of the batch, eight where it may queue many
+// cells:
 //   1. the 1000-point table of area(colat..lims[1]) per mesh, one thread (few
 //      meshes: one warp) per entry (1000 independent adaptive quadratures);
 //   2. per mesh: the cell area, the S - 1 parallels and the columns' edges (the
@@ -15,11 +16,14 @@
 //   4. one thread per cell: the corner / centre membership tests; cells
 //      wholly inside or outside get their area at once, cells cut by a
 //      region boundary (~1 %) are queued;
-//   5. one CTA of two warps per queued cell, taken from a shared counter: its
-//      area quadrature, a panel to each warp (21 Gauss-Kronrod nodes over the
-//      lanes, the interval list in shared memory) -- the same adaptive scheme
-//      the host builder runs serially; two more launches for the pieces of
-//      cells touched at a corner.
+//   5. from 5000 queued cells on, their area quadratures four cells to a warp,
+//      eight lanes a cell (those whose integral vanishes are left to 6);
+//   6. one CTA of two warps per queued cell, or per cell left, taken from a
+//      shared counter: its area quadrature, a panel to each warp (21
+//      Gauss-Kronrod nodes over the lanes, the interval list in shared memory)
+//      -- the same adaptive scheme the host builder runs serially;
+//   7. a CTA for each dyadic piece of the cells touched at a corner, and one
+//      for each of those cells' sums (two launches).
 // The serial quadratures of steps 1 and 3 keep their interval list (128
 // intervals) in local memory; the host builder's limit of 4000 gives bitwise
 // the same meshes (these integrals converge in far fewer intervals).

@@ -330,7 +330,7 @@ __device__ __forceinline__ double turning_radius(double b) {
   return 2.0 * b * cos((atan(sqrt(4.0 * b * b * i27 - 1.0)) - kPi) * i3) * isq3;
 }
 
-// what a row's rays share: u sqrt(1 - u), 1 / u, 1 / (1/u - 1) as a pair, 1 / c
+// what a row's rays share: u sqrt(1 - u), 1 / u, 1 / (1/u - 1) as a pair
 struct RowRay {
   double r_s, u, u_sq1u, iu;
   DF q;
